@@ -110,6 +110,9 @@ struct rg_ctx {
     DevBuf samples, workCounter;               // per-sample payload sums, persistent-kernel work counter
     // wavefront path state
     DevBuf wfPayload, wfMeta, wfFrames, wfQO0, wfQO1, wfQD0, wfQD1, wfQP0, wfQP1, wfHitTUV, wfHitInst, wfCounts, wfOverflow;
+    // ray trees of the frames: node pool (its nodes per sample grow when a frame filled it)
+    DevBuf trO, trD, trState, trHit, trInst, trSurf, trLink, trOver, trCand, trCtl;
+    uint32_t treeNodes = kTreeNodesMin;
     uint32_t* hostCount = nullptr;             // pinned words for polling the queue length and work counter
     int lastIterations = 0;
     // batch rendering: job table, per-slot job / sample index, ray-sort scratch, per-job images
@@ -455,8 +458,8 @@ uint64_t scene_bytes(const SceneState& st) {
 
 // path state of the wavefront loop for `paths` path slots
 // path state for `paths` paths; queues and hit records for max(paths, hitSlots) entries
-rg_status ensure_wavefront(rg_ctx* c, size_t paths, WavefrontBuffers& w, size_t hitSlots = 0) {
-    const size_t P = paths ? paths : 1, Q = std::max(P, hitSlots);
+rg_status ensure_wavefront(rg_ctx* c, size_t paths, WavefrontBuffers& w) {
+    const size_t P = paths ? paths : 1, Q = P;
     TRY(ensure(c, c->wfPayload, 64 * P));
     TRY(ensure(c, c->wfMeta, 8 * P));
     TRY(ensure(c, c->wfFrames, 144ull * kMaxFrames * P));
@@ -486,6 +489,37 @@ rg_status ensure_wavefront(rg_ctx* c, size_t paths, WavefrontBuffers& w, size_t 
     w.hitInst = c->wfHitInst.as<uint32_t>();
     w.counts = c->wfCounts.as<uint32_t>();
     w.overflow = c->wfOverflow.as<uint32_t>();
+    return RG_OK;
+}
+
+// ray-tree buffers for a frame of `work` samples; frames of more than 2^25 samples go in chunks
+rg_status ensure_tree(rg_ctx* c, size_t work, RayTree& t) {
+    const size_t roots = std::min<size_t>(work, 1u << 25);
+    size_t cap = std::max<size_t>(roots * c->treeNodes, 1u << 16);
+    // (RG_TREE_POOL overrides the pool's nodes; tests use a small pool to make chunks fill it)
+    if (const char* env = getenv("RG_TREE_POOL")) cap = std::max<size_t>(strtoull(env, nullptr, 10), 4608);
+    TRY(ensure(c, c->trO, 16 * cap));
+    TRY(ensure(c, c->trD, 16 * cap));
+    TRY(ensure(c, c->trState, 16 * cap));
+    TRY(ensure(c, c->trHit, 16 * cap));
+    TRY(ensure(c, c->trInst, 4 * cap));
+    TRY(ensure(c, c->trSurf, 16 * cap));
+    TRY(ensure(c, c->trLink, 16 * cap));
+    TRY(ensure(c, c->trOver, 4 * cap));
+    TRY(ensure(c, c->trCand, 8 * cap));
+    TRY(ensure(c, c->trCtl, kTreeCtlWords * sizeof(uint32_t)));
+    t.rayO = c->trO.as<float4>();
+    t.rayD = c->trD.as<float4>();
+    t.state = c->trState.as<uint4>();
+    t.hitTUV = c->trHit.as<float4>();
+    t.hitInst = c->trInst.as<uint32_t>();
+    t.surf = c->trSurf.as<float4>();
+    t.link = c->trLink.as<uint4>();
+    t.overflow = c->trOver.as<uint32_t>();
+    t.cand[0] = c->trCand.as<uint32_t>();
+    t.cand[1] = c->trCand.as<uint32_t>() + cap;
+    t.ctl = c->trCtl.as<uint32_t>();
+    t.capacity = (uint32_t)cap;
     return RG_OK;
 }
 
@@ -551,7 +585,8 @@ rg_status rg_destroy(rg_ctx* c) {
                       &c->tmpD, &c->samples, &c->workCounter, &c->wfPayload, &c->wfMeta, &c->wfFrames, &c->wfQO0, &c->wfQO1,
                       &c->wfQD0, &c->wfQD1, &c->wfQP0, &c->wfQP1, &c->wfHitTUV, &c->wfHitInst, &c->wfCounts, &c->wfOverflow, &c->jobTable,
                       &c->slotJob, &c->slotSample, &c->sortKeys, &c->sortPerm, &c->sortHist, &c->bBase, &c->bNormal, &c->bRough,
-                      &c->bFinal, &c->bFxaa, &c->batchFb};
+                      &c->bFinal, &c->bFxaa, &c->batchFb, &c->trO, &c->trD, &c->trState, &c->trHit, &c->trInst, &c->trSurf, &c->trLink,
+                      &c->trOver, &c->trCand, &c->trCtl};
     for (DevBuf* b : bufs) release(c, *b);
     for (SceneState* st : c->scenes)
         if (st) {
@@ -839,9 +874,7 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     tp.glossySeed = c->glossySeed;
     c->lastSamples = (uint32_t)ubo->numSamples;
     const bool mega = (c->flags & RG_FLAG_MEGAKERNEL) != 0;
-    if (!mega)
-        TRY(ensure_wavefront(c, (size_t)c->W * c->H * (uint32_t)ubo->numSamples, tp.wf,
-                             frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples)));
+    if (!mega) TRY(ensure_tree(c, frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), tp.tree));
     CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
     FrameEvents* fe;
     TRY(cur_events(c, &fe));
@@ -849,11 +882,12 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     if (mega) {
         c->lastIterations = 0;
         CK(launch_trace(tp, c->stream));
+    } else {
+        bool full = false;
+        const bool timed = (c->flags & RG_FLAG_KERNEL_TIMING) != 0;
+        CK(launch_trace_tree(tp, c->stream, c->hostCount, &c->lastIterations, &full, timed ? next_kernel_events : nullptr, timed ? fe : nullptr));
+        if (full && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
     }
-    else if (c->flags & RG_FLAG_KERNEL_TIMING)
-        CK(launch_trace_wavefront(tp, c->stream, c->hostCount, &c->lastIterations, next_kernel_events, fe));
-    else
-        CK(launch_trace_wavefront(tp, c->stream, c->hostCount, &c->lastIterations));
     return run_post(c, ubo, fxaa);
 }
 

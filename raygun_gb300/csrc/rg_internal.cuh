@@ -201,6 +201,35 @@ struct WavefrontBuffers {
     uint32_t* overflow; // per queue slot: slots of rays whose short traversal stack overflowed
 };
 
+// Ray trees (trace.cu): one node per traced ray.  The roots, one per sample of the chunk, are nodes
+// 0 .. treeRoots - 1 (their rays and states are recomputed, not stored).
+struct RayTree {
+    float4* rayO;       // origin, tmin; once composed: colour, payload depth
+    float4* rayD;       // direction, tmax
+    uint4* state;       // curIOR bits, recDepth | rayType << 4 | job << 6, parent and flags, refDepth bits
+    float4* hitTUV;     // t, u, v, primitive bits
+    uint32_t* hitInst;  // instance or 0xFFFFFFFF (miss)
+    float4* surf;       // of a hit: world normal, material index bits
+    uint4* link;        // of a hit: its shadow, reflection and refraction node
+    uint32_t* overflow; // nodes of rays whose short traversal stack overflowed
+    uint32_t* cand[2];  // nodes whose assumptions k_tree_check verifies (the list in use: treeCand)
+    uint32_t* ctl;      // kTreeCtlWords words
+    uint32_t capacity;  // nodes, below kTreeMaxNodes
+};
+// words of RayTree::ctl: nodes appended after the roots; rays that the last check changed, 16 minus the
+// least recursion depth of the rays replaced since the last round, nodes traced when the last check ran;
+// the traversal kernel's work counter, overflow list length and finished blocks; lengths of the candidate
+// lists; then the first node of every round
+enum : int { kTreeAlloc = 0, kTreeChanges = 1, kTreeLevels = 2, kTreeTraced = 3, kTreeFetch = 4, kTreeCand = 7, kTreeBounds = 9 };
+constexpr uint32_t kTreeMaxNodes = 1u << 29;
+// a sample's GENERIC hits (at most 2^9 - 1 at 8 recursions) bound the checks that can change a ray
+constexpr int kTreeMaxRounds = 512 * 9;
+constexpr int kTreeCtlWords = kTreeBounds + kTreeMaxRounds + 1;
+// Pool size: nodes per sample.  The benchmark scenes trace 2.5 to 4 rays a sample; a chunk of samples
+// that fills the pool goes again in smaller chunks, and the next frame's pool is twice as large, up to
+// kTreeNodesMax a sample (less than the 1.6 KB that a path of the batch loop takes).
+constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 14;
+
 // one render job of a batch: a scene, its UBO and its image size.  Work items of the batch are
 // numbered job after job; job j owns [workBase, workBase + workCount) and writes its per-sample
 // payload sums to samples[sampleBase + (y * W + x) * S + s].
@@ -238,9 +267,12 @@ struct TraceParams {
     uint32_t* slotSample;
     const uint32_t* perm;  // nullable: order in which the trace kernel takes the queue's rays
     uint32_t glossySeed;   // 0: the reference's mirror shading; else glossy reference shading (seed)
-    // frame loop: the first (trace, shade) round computes the camera rays and initial payloads of
-    // work items 0 .. W*H*S-1 (8x4-tile order) itself instead of reading a raygen queue
+    // ray trees: the first round computes the camera rays of the roots itself
     int firstRound;
+    // ray trees: node pool; the current chunk of samples (work items treeBase + k, k < treeRoots), the
+    // candidate list in use
+    RayTree tree;
+    uint32_t treeBase, treeRoots, treeCand;
     // ray query (rg_trace_rays_device): queryCount rays read from the caller's buffer (origin, tmin,
     // direction, tmax: two float4 per ray) and hits written in rg_trace_rays' layout, so the query
     // needs neither a queue copy before the traversal nor a read-out pass after it
@@ -257,12 +289,13 @@ constexpr int kTileW = 8, kTileH = 4;
 inline size_t frame_work_items(uint32_t W, uint32_t H, uint32_t S) {
     return (size_t)((W + kTileW - 1) / kTileW) * ((H + kTileH - 1) / kTileH) * (kTileW * kTileH) * S;
 }
-// hostCount: pinned host word used to poll the queue length; iterations: trace/shade rounds run
 // kernelEvents (nullable): callback that returns a (start, end) event pair to record around each
 // traversal launch
 typedef bool (*EventPairFn)(void* user, cudaEvent_t* start, cudaEvent_t* end);
-cudaError_t launch_trace_wavefront(const TraceParams& p, cudaStream_t s, uint32_t* hostCount, int* iterations,
-                                   EventPairFn kernelEvents = nullptr, void* user = nullptr);
+// a frame through ray trees, and its resolve.  hostWords: three pinned words polled after each check;
+// iterations: rounds run; *poolFull: a chunk of samples filled the node pool
+cudaError_t launch_trace_tree(const TraceParams& p, cudaStream_t s, uint32_t* hostWords, int* iterations, bool* poolFull,
+                              EventPairFn kernelEvents = nullptr, void* user = nullptr);
 // traversal launch shape of the batch loop: block size {64,128,256}, stack entries {16,24,32,48},
 // ray-sort key applied to each queue before it is traced
 struct TraceTune {

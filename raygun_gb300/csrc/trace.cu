@@ -20,10 +20,13 @@
 // GLSL-undefined cases follow fixed policies: r/(tr+r) with tr+r == 0 -> 0; pow(x, n) with
 // integer n -> repeated multiply; a zero direction (refract at total internal reflection) -> no
 // traversal, miss shader; clamp/min/max treat a NaN operand as absent (fminf/fmaxf).
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "rg_internal.cuh"
 
@@ -202,6 +205,7 @@ struct SmemStackT {
     __device__ __forceinline__ uint32_t& operator[](int i) const { return base[i * THREADS]; }
     __device__ __forceinline__ float& w(int i) const { return saved[i * THREADS]; }
     __device__ __forceinline__ uint32_t& over() const { return base[(DEPTH - 1) * THREADS]; }
+    static constexpr int kStride = THREADS;  // words from one entry to the next
 };
 // the same stack in (L1-cached) local memory
 #ifndef RG_STACK_SMEM
@@ -254,6 +258,10 @@ struct Trav {
     uint32_t ref, inst;
     int sp;
     bool inBlas, active;
+    // shared rays only (see drain): first stack word not given away; whether the stack holds the marker
+    // of the instance the lane is in (a lane that was given a BLAS node has none)
+    int sb;
+    bool marker;
 };
 
 template <class STACK>
@@ -278,7 +286,7 @@ __device__ __forceinline__ void trav_begin(Trav& T, const DevScene& sc, float ox
     T.active = true;
 }
 
-template <bool COUNT, class STACK>
+template <bool COUNT, bool SHARED = false, class STACK>
 __device__ __forceinline__ void trav_step(Trav& T, const DevScene& sc, const STACK& stack, VisitCounts& vc) {
     const uint32_t ref = T.ref;
     const float tmin = T.tmin;
@@ -350,6 +358,7 @@ __device__ __forceinline__ void trav_step(Trav& T, const DevScene& sc, const STA
                         T.tris = reinterpret_cast<const float4*>(pp.y);
                         T.inst = __float_as_uint(hi.w);
                         T.inBlas = true;
+                        if (SHARED) T.marker = true;
                         T.ref = bn == 1 ? kLeaf : 0u;
                         return;
                     }
@@ -360,7 +369,7 @@ __device__ __forceinline__ void trav_step(Trav& T, const DevScene& sc, const STA
     }
     // pop (a marker leaves the BLAS: back to the world-space ray and the TLAS)
     for (;;) {
-        if (T.sp == 0) {
+        if (T.sp == (SHARED ? T.sb : 0)) {
             T.active = false;
             return;
         }
@@ -451,6 +460,7 @@ __device__ __forceinline__ V3 refract(V3 I, V3 N, float eta) {
 }
 __device__ __forceinline__ float glsl_mod(float x, float y) { return x - y * floorf(x / y); }
 __device__ __forceinline__ float len(V3 v) { return sqrtf(dot(v, v)); }
+__device__ __forceinline__ bool is_zero(V3 v) { return v.x == 0.0f && v.y == 0.0f && v.z == 0.0f; }
 
 enum : int { RT_GENERIC = 0, RT_SHADOW_TRACE = 1, RT_SHADOW_INTERNAL = 2 };
 
@@ -579,6 +589,109 @@ __device__ __forceinline__ V3 ggx_normal(V3 n, float roughness, uint32_t seed, u
     return normalize(t * (sinT * cosf(phi)) + b * (sinT * sinf(phi)) + n * cosT);
 }
 
+__device__ __forceinline__ void load_material(const rg_material* M, Frame& cur) {
+    cur.diffuse = v3(__ldg(&M->diffuse[0]), __ldg(&M->diffuse[1]), __ldg(&M->diffuse[2]));
+    cur.specular = v3(__ldg(&M->specular[0]), __ldg(&M->specular[1]), __ldg(&M->specular[2]));
+    cur.transparency = __ldg(&M->transparency);
+    cur.reflectivity = __ldg(&M->reflectivity);
+    cur.roughness = __ldg(&M->roughness);
+    cur.ior = __ldg(&M->ior);
+    cur.emission = __ldg(&M->emission);
+    cur.rayConsumption = (int)__ldg(&M->rayConsumption);
+}
+
+// gridEffect, closesthit.rchit:74-91
+__device__ __forceinline__ void grid_effect(V3 pos, float refDepth, float hitT, Frame& cur) {
+    float aa = ((refDepth + hitT) + 8.0f) / 30.0f;
+    float aa2 = aa / 2.0f;
+    float minmod = fminf(fabsf(glsl_mod((pos.x + 1000.0f) * 10.0f + aa2, 20.0f) - aa2),
+                         fabsf(glsl_mod((pos.z + 1000.0f) * 10.0f + aa2, 20.0f) - aa2));
+    if (minmod < aa2) {
+        float aa_sq = aa * aa;
+        minmod = minmod - (aa2 - aa_sq / 3.0f);
+        minmod = minmod * (3.0f / aa_sq);
+        float f = mixs(aa / 10.0f, 1.0f, minmod);
+        cur.diffuse = cur.diffuse * f;
+        cur.specular = cur.specular * f;
+        cur.reflectivity = cur.reflectivity * f;
+    }
+    if (glsl_mod((pos.x + 1000.0f) * 5.0f, 20.0f) < 10.0f && glsl_mod((pos.z + 1000.0f) * 5.0f, 20.0f) < 10.0f)
+        cur.reflectivity = cur.reflectivity * 1.5f;
+}
+
+// Whether the sign of the grid effect's factor f can depend on refDepth at pos.  With D the distance to
+// the nearest line (in tenths of a unit) and a = (refDepth + t + 8) / 30, f <= 0 needs D <=
+// a (1.5 - 1.15 a) / (3 - 0.3 a), which is at most 0.175 and negative from a = 1.305 on; refDepth only
+// grows while siblings run.  The margins cover the rounding of pos * 10.
+__device__ __forceinline__ bool grid_sign_varies(V3 pos, float refDepth, float hitT) {
+    if (((refDepth + hitT) + 8.0f) / 30.0f > 1.32f) return false;
+    const float wx = glsl_mod((pos.x + 1000.0f) * 10.0f, 20.0f), wz = glsl_mod((pos.z + 1000.0f) * 10.0f, 20.0f);
+    const float d = fminf(fminf(wx, 20.0f - wx), fminf(wz, 20.0f - wz));
+    return !(d > 0.25f);
+}
+
+// closesthit.rchit:95-122 of hit h of `ray`: attribute fetch, world position, world normal and grid
+// effect (returned: whether the material has it); matId: the material's index
+__device__ __forceinline__ bool closest_hit_surface(const DevScene& sc, const Hit& h, const RayReq& ray, float refDepth, Frame& cur,
+                                                    uint32_t& matId) {
+    const DevInstance* in = sc.inst + h.inst;
+    const uint32_t vOff = __ldg(&in->vOff), iOff = __ldg(&in->iOff), mOff = __ldg(&in->mOff);
+    const float4 m0 = __ldg(&in->m[0]), m1 = __ldg(&in->m[1]), m2 = __ldg(&in->m[2]);
+    const float bx = (1.0f - h.u) - h.v, by = h.u, bz = h.v;
+    const uint32_t ib = iOff + 3 * h.prim;
+    const rg_vertex* v0 = sc.vertices + vOff + __ldg(sc.indices + ib);
+    const rg_vertex* v1 = sc.vertices + vOff + __ldg(sc.indices + ib + 1);
+    const rg_vertex* v2 = sc.vertices + vOff + __ldg(sc.indices + ib + 2);
+    V3 n0 = v3(__ldg(&v0->normal[0]), __ldg(&v0->normal[1]), __ldg(&v0->normal[2]));
+    V3 n1 = v3(__ldg(&v1->normal[0]), __ldg(&v1->normal[1]), __ldg(&v1->normal[2]));
+    V3 n2 = v3(__ldg(&v2->normal[0]), __ldg(&v2->normal[1]), __ldg(&v2->normal[2]));
+    matId = mOff + __ldg(&v0->matIndex);
+    const rg_material* M = sc.materials + matId;
+    load_material(M, cur);
+    cur.origin = ray.o + ray.d * h.t;
+    cur.D = ray.d;
+    cur.t = h.t;
+    V3 vn = (n0 * bx + n1 * by) + n2 * bz;
+    V3 wn = v3((m0.x * vn.x + m0.y * vn.y) + m0.z * vn.z, (m1.x * vn.x + m1.y * vn.y) + m1.z * vn.z,
+               (m2.x * vn.x + m2.y * vn.y) + m2.z * vn.z);
+    cur.n = normalize(wn);
+    const bool effect = __ldg(&M->effectId) == 1;
+    if (effect) grid_effect(cur.origin, refDepth, h.t, cur);
+    return effect;
+}
+
+// what a SHADOW_TRACE invocation reads of its hit: position and material
+__device__ __forceinline__ void shadow_hit_surface(const DevScene& sc, const Hit& h, const RayReq& ray, Frame& cur, uint32_t& matId) {
+    const DevInstance* in = sc.inst + h.inst;
+    const rg_vertex* v0 = sc.vertices + __ldg(&in->vOff) + __ldg(sc.indices + __ldg(&in->iOff) + 3 * h.prim);
+    matId = __ldg(&in->mOff) + __ldg(&v0->matIndex);
+    cur.transparency = __ldg(&sc.materials[matId].transparency);
+    cur.origin = ray.o + ray.d * h.t;
+    cur.D = ray.d;
+    cur.n = v3s(0.0f);
+}
+
+// the reflection and refraction directions of a GENERIC hit (closesthit.rchit:206-251), eta given; with
+// glossy reference shading (a seed, at the sample's primary hit) through a sampled microfacet
+template <bool GLOSSY>
+__device__ __forceinline__ V3 reflect_dir(const Frame& cur, uint32_t seed, int recDepth) {
+    V3 dir = reflect(cur.D, cur.n);
+    if (GLOSSY && seed && recDepth == 0 && cur.roughness > 0.0f) {
+        const V3 g = reflect(cur.D, ggx_normal(cur.n, cur.roughness, seed, 1u));
+        if (dot(g, cur.n) > 0.0f) dir = g;
+    }
+    return dir;
+}
+template <bool GLOSSY>
+__device__ __forceinline__ V3 refract_dir(const Frame& cur, float eta, uint32_t seed, int recDepth) {
+    V3 dir = refract(cur.D, cur.n, eta);
+    if (GLOSSY && seed && recDepth == 0 && cur.roughness > 0.0f) {
+        const V3 g = refract(cur.D, ggx_normal(cur.n, cur.roughness, seed, 2u), eta);
+        if (!is_zero(g)) dir = g;
+    }
+    return dir;
+}
+
 // One step of the closest-hit / miss state machine: consume the result `h` of the pending trace and
 // run the paused invocations on the frame stack until the next trace is needed (returns true, `ray`
 // set) or the sample's primary trace has returned (returns false).
@@ -597,55 +710,9 @@ __device__ __forceinline__ bool shade_step(const DevScene& sc, const V3 L, const
     V3 refractColor = v3s(1.0f);
     while (!newRay) {
         if (ph == PH_HIT) {
-            // closesthit.rchit:95-122 -- fetch, world position, world normal, grid effect
-            const DevInstance* in = sc.inst + h.inst;
-            const uint32_t vOff = __ldg(&in->vOff), iOff = __ldg(&in->iOff), mOff = __ldg(&in->mOff);
-            const float4 m0 = __ldg(&in->m[0]), m1 = __ldg(&in->m[1]), m2 = __ldg(&in->m[2]);
+            uint32_t matId;
+            closest_hit_surface(sc, h, ray, p.refDepth, cur, matId);
             const float hitT = h.t;
-            const float bx = (1.0f - h.u) - h.v, by = h.u, bz = h.v;
-            const uint32_t ib = iOff + 3 * h.prim;
-            const rg_vertex* v0 = sc.vertices + vOff + __ldg(sc.indices + ib);
-            const rg_vertex* v1 = sc.vertices + vOff + __ldg(sc.indices + ib + 1);
-            const rg_vertex* v2 = sc.vertices + vOff + __ldg(sc.indices + ib + 2);
-            const uint32_t matIndex = __ldg(&v0->matIndex);
-            V3 n0 = v3(__ldg(&v0->normal[0]), __ldg(&v0->normal[1]), __ldg(&v0->normal[2]));
-            V3 n1 = v3(__ldg(&v1->normal[0]), __ldg(&v1->normal[1]), __ldg(&v1->normal[2]));
-            V3 n2 = v3(__ldg(&v2->normal[0]), __ldg(&v2->normal[1]), __ldg(&v2->normal[2]));
-            const rg_material* M = sc.materials + mOff + matIndex;
-            cur.diffuse = v3(__ldg(&M->diffuse[0]), __ldg(&M->diffuse[1]), __ldg(&M->diffuse[2]));
-            cur.specular = v3(__ldg(&M->specular[0]), __ldg(&M->specular[1]), __ldg(&M->specular[2]));
-            cur.transparency = __ldg(&M->transparency);
-            cur.reflectivity = __ldg(&M->reflectivity);
-            cur.roughness = __ldg(&M->roughness);
-            cur.ior = __ldg(&M->ior);
-            cur.emission = __ldg(&M->emission);
-            cur.rayConsumption = (int)__ldg(&M->rayConsumption);
-            const uint32_t effectId = __ldg(&M->effectId);
-            cur.origin = ray.o + ray.d * hitT;
-            cur.D = ray.d;
-            cur.t = hitT;
-            V3 vn = (n0 * bx + n1 * by) + n2 * bz;
-            V3 wn = v3((m0.x * vn.x + m0.y * vn.y) + m0.z * vn.z, (m1.x * vn.x + m1.y * vn.y) + m1.z * vn.z,
-                       (m2.x * vn.x + m2.y * vn.y) + m2.z * vn.z);
-            cur.n = normalize(wn);
-            if (effectId == 1) {  // gridEffect, closesthit.rchit:74-91
-                V3 pos = cur.origin;
-                float aa = ((p.refDepth + hitT) + 8.0f) / 30.0f;
-                float aa2 = aa / 2.0f;
-                float minmod = fminf(fabsf(glsl_mod((pos.x + 1000.0f) * 10.0f + aa2, 20.0f) - aa2),
-                                     fabsf(glsl_mod((pos.z + 1000.0f) * 10.0f + aa2, 20.0f) - aa2));
-                if (minmod < aa2) {
-                    float aa_sq = aa * aa;
-                    minmod = minmod - (aa2 - aa_sq / 3.0f);
-                    minmod = minmod * (3.0f / aa_sq);
-                    float f = mixs(aa / 10.0f, 1.0f, minmod);
-                    cur.diffuse = cur.diffuse * f;
-                    cur.specular = cur.specular * f;
-                    cur.reflectivity = cur.reflectivity * f;
-                }
-                if (glsl_mod((pos.x + 1000.0f) * 5.0f, 20.0f) < 10.0f && glsl_mod((pos.z + 1000.0f) * 5.0f, 20.0f) < 10.0f)
-                    cur.reflectivity = cur.reflectivity * 1.5f;
-            }
             if (p.rayType == RT_SHADOW_INTERNAL) {  // :125-152
                 float thick = clampf(hitT * (1.0f - cur.transparency) * 10.0f, 0.0f, 1.0f);
                 V3 shadowCol = p.hitValue - mix(v3s(0.0f), normalize(v3s(1.1f) - cur.diffuse) + v3s(0.1f), thick);
@@ -711,11 +778,7 @@ __device__ __forceinline__ bool shade_step(const DevScene& sc, const V3 L, const
             }
         } else if (ph == PH_G_REFLECT) {  // :206-221
             if (p.recDepth < maxRec && cur.reflectivity > 0.0f) {
-                V3 dir = reflect(cur.D, cur.n);
-                if (GLOSSY && p.seed && p.recDepth == 0 && cur.roughness > 0.0f) {  // glossy reference shading
-                    const V3 g = reflect(cur.D, ggx_normal(cur.n, cur.roughness, p.seed, 1u));
-                    if (dot(g, cur.n) > 0.0f) dir = g;
-                }
+                const V3 dir = reflect_dir<GLOSSY>(cur, p.seed, p.recDepth);
                 p.recDepth += cur.rayConsumption;
                 p.refDepth = p.refDepth + cur.t;
                 cnt.secondary++;
@@ -728,30 +791,11 @@ __device__ __forceinline__ bool shade_step(const DevScene& sc, const V3 L, const
             }
         } else if (ph == PH_G_REFRACT) {  // :223-251
             if (p.recDepth < maxRec && cur.transparency > 0.0f) {
-                V3 dir;
-                const bool glossy = GLOSSY && p.seed && p.recDepth == 0 && cur.roughness > 0.0f;
-                const V3 mn = glossy ? ggx_normal(cur.n, cur.roughness, p.seed, 2u) : cur.n;
-                if (cur.front) {
-                    float eta = p.curIOR / cur.ior;
-                    dir = refract(cur.D, cur.n, eta);
-                    if (glossy) {  // glossy reference shading: refraction through the sampled microfacet
-                        const V3 g = refract(cur.D, mn, eta);
-                        if (!(g.x == 0.0f && g.y == 0.0f && g.z == 0.0f)) dir = g;
-                    }
-                    p.curIOR = cur.ior;
-                    cur.kind = R_G_REFR_F;
-                } else {
-                    float eta = cur.ior / 1.0f;
-                    dir = refract(cur.D, cur.n, eta);
-                    if (glossy) {
-                        const V3 g = refract(cur.D, mn, eta);
-                        if (!(g.x == 0.0f && g.y == 0.0f && g.z == 0.0f)) dir = g;
-                    }
-                    p.curIOR = 1.0f;
-                    cur.kind = R_G_REFR_B;
-                }
+                const V3 dir = refract_dir<GLOSSY>(cur, cur.front ? p.curIOR / cur.ior : cur.ior / 1.0f, p.seed, p.recDepth);
+                p.curIOR = cur.front ? cur.ior : 1.0f;
+                cur.kind = cur.front ? R_G_REFR_F : R_G_REFR_B;
                 p.recDepth++;
-                if (!(dir.x == 0.0f && dir.y == 0.0f && dir.z == 0.0f)) cnt.secondary++;  // only rays that traverse
+                if (!is_zero(dir)) cnt.secondary++;  // only rays that traverse
                 frames[fsp++] = cur;
                 ray.o = cur.origin; ray.d = dir; ray.tmin = 0.01f; ray.tmax = 1000.0f; ray.missIndex = 0; ray.masked = false;
                 newRay = true;
@@ -1035,16 +1079,12 @@ __global__ void k_resolve_job(const float4* __restrict__ samples, uint32_t W, ui
 }
 
 // ---------------------------------------------------------------------------------------------
-// Wavefront form of the same path: every (pixel, sample) is a path with exactly one outstanding
-// ray at a time (the reference's recursion is depth-first on one payload), so a frame is a loop of
-// (trace all pending rays, shade all their results).  The trace kernel only traverses: few
-// registers, high occupancy, dynamic ray fetch.  The shade kernel runs the same state machine as
-// the megakernel on the path's payload and frame stack, which live in device memory between the
-// two kernels, and appends each path's next ray to the other queue.
-
-struct PathMeta {
-    int fsp, missIndex;
-};
+// Batch loop: every path slot has exactly one outstanding ray at a time (the reference's recursion is
+// depth-first on one payload), so a batch is a loop of (trace all pending rays, shade all their
+// results).  The trace kernel only traverses: few registers, high occupancy, dynamic ray fetch.  The
+// shade kernel runs the same state machine as the megakernel on the path's payload and frame stack,
+// which live in device memory between the two kernels, and appends each path's next ray to the other
+// queue.
 
 __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
     const unsigned mask = __ballot_sync(0xFFFFFFFFu, want);
@@ -1144,12 +1184,7 @@ __device__ __forceinline__ void store_sample(float4* so, const Payload& p) {
     so[2] = make_float4(p.roughRGB.x, p.roughRGB.y, p.roughRGB.z, p.roughA);
 }
 
-// work items of the frame loop: one path per (pixel, sample) in 8x4-tile order, all of them in the
-// first round; path = (py * W + px) * S + sample
-__device__ __forceinline__ uint32_t frame_work_total(const TraceParams& P) {
-    const uint32_t S = (uint32_t)P.ubo.numSamples;
-    return ((P.W + kTileW - 1) / kTileW) * ((P.H + kTileH - 1) / kTileH) * (kTileW * kTileH) * S;
-}
+// work items of a frame: one per (pixel, sample) in 8x4-tile order; path = (py * W + px) * S + sample
 // camera ray and initial payload of work item id (raygen.h:84-102); false outside the image
 __device__ __forceinline__ bool frame_work_item(const TraceParams& P, uint32_t id, uint32_t& path, Payload& p, RayReq& ray) {
     const rg_ubo& U = P.ubo;
@@ -1190,18 +1225,157 @@ __global__ void __launch_bounds__(256) k_wfb_raygen(const TraceParams P) {
     flush_counts(P, c, 1);
 }
 
-// closest hit of every ray of queue q.  Lanes whose ray finished take new rays from the queue (one
-// atomic per warp) as soon as RG_FETCH_THRESHOLD lanes of the warp are idle, so a warp does not wait
-// for its longest ray; between fetches every lane advances its ray by RG_WF_STEPS steps.  BATCH: the
-// ray's scene is its path's job's scene.  P.perm (nullable) gives the order the rays are taken in.
+#ifndef RG_DRAIN_LANES
+#define RG_DRAIN_LANES 8
+#endif
+#ifndef RG_DRAIN_ROUNDS
+#define RG_DRAIN_ROUNDS 2
+#endif
+// The end of a launch of few rays: it lasts as long as its longest ray, whose record steps (up to 90 on
+// the sphere scene, 200 on the game frame) wait for memory one after another while the other lanes of
+// its warp idle.  The closest hit does not depend on the order in which subtrees are visited, so the
+// warp's idle lanes take them over: each live lane gives the bottom entry of its stack (the largest
+// subtree left) to an idle lane, with the ray at that entry's level.  Lanes of one ray share the best t as
+// hits are found; a lane that finishes hands its hit to another lane of the same ray, and the last one
+// writes it.  Ties go to the smaller (instance, primitive) as everywhere, so the hit is the one the ray's
+// own lane would have found.  One game-frame ray of 153 records: 43 us against 57; the 1280x720 game frame
+// with the filter: 2.20 ms against 2.25 ms without.  From RG_DRAIN_LANES live lanes on only: with 16 and
+// 32 the sphere frame is 1 % and 7 % slower.
+template <bool COUNT, class STACK, class SceneOf, class HitOut>
+__device__ __forceinline__ void drain(Trav& T, uint32_t& slot, const DevScene*& scp, const STACK& stk, VisitCounts& vc, SceneOf&& sceneOf,
+                                      HitOut&& hitOut) {
+    const unsigned lane = threadIdx.x & 31, full = 0xFFFFFFFFu, below = (1u << lane) - 1u;
+    T.sb = 0;
+    T.marker = T.inBlas;
+    for (;;) {
+        const unsigned live = __ballot_sync(full, T.active);
+        if (!live) break;
+        // what the lane can give: TLAS entry (bottom of a stack at TLAS level or below the marker), or
+        // a BLAS entry (just above the marker, or the bottom of a stack without one)
+        const int held = T.active ? T.sp - T.sb : 0;
+        const bool atMarker = held > 0 && T.inBlas && T.marker && stk[T.sb] == kMarker;
+        const unsigned givers = __ballot_sync(full, held > (atMarker ? 1 : 0));
+        if (givers && live != full) {
+            const unsigned idle = ~live;
+            const int pairs = min(__popc(givers), __popc(idle));
+            const bool gives = (givers >> lane & 1u) && __popc(givers & below) < pairs;
+            const bool takes = (idle >> lane & 1u) && __popc(idle & below) < pairs;
+            const bool blasLevel = T.inBlas && (atMarker || !T.marker);
+            uint32_t entry = 0;
+            if (gives) {
+                entry = stk[T.sb + (atMarker ? 1 : 0)];
+                if (atMarker) stk[T.sb + 1] = kMarker;
+                ++T.sb;
+                if (!T.inBlas) {  // the taker reads the world ray where a ray inside a BLAS has parked it
+                    stk.w(0) = T.r.ox; stk.w(1) = T.r.oy; stk.w(2) = T.r.oz;
+                    stk.w(3) = T.r.jx; stk.w(4) = T.r.jy; stk.w(5) = T.r.jz;
+                }
+            }
+            __syncwarp();
+            unsigned from = lane;
+            if (takes) {  // the giver of the same rank
+                unsigned m = givers;
+                for (int r = __popc(idle & below); r > 0; --r) m &= m - 1u;
+                from = (unsigned)__ffs(m) - 1u;
+            }
+            Trav N;
+            N.tmin = __shfl_sync(full, T.tmin, from);
+            N.h.t = __shfl_sync(full, T.h.t, from);
+            N.ref = __shfl_sync(full, entry, from);
+            N.inst = __shfl_sync(full, T.inst, from);
+            N.inBlas = __shfl_sync(full, (int)blasLevel, from) != 0;
+            N.nodes = reinterpret_cast<const WideNode*>(__shfl_sync(full, reinterpret_cast<unsigned long long>(T.nodes), from));
+            N.tris = reinterpret_cast<const float4*>(__shfl_sync(full, reinterpret_cast<unsigned long long>(T.tris), from));
+            N.r.ox = __shfl_sync(full, T.r.ox, from); N.r.oy = __shfl_sync(full, T.r.oy, from); N.r.oz = __shfl_sync(full, T.r.oz, from);
+            N.r.dx = __shfl_sync(full, T.r.dx, from); N.r.dy = __shfl_sync(full, T.r.dy, from); N.r.dz = __shfl_sync(full, T.r.dz, from);
+            N.r.jx = __shfl_sync(full, T.r.jx, from); N.r.jy = __shfl_sync(full, T.r.jy, from); N.r.jz = __shfl_sync(full, T.r.jz, from);
+            N.r.clx = __shfl_sync(full, T.r.clx, from); N.r.cly = __shfl_sync(full, T.r.cly, from); N.r.clz = __shfl_sync(full, T.r.clz, from);
+            N.r.chx = __shfl_sync(full, T.r.chx, from); N.r.chy = __shfl_sync(full, T.r.chy, from); N.r.chz = __shfl_sync(full, T.r.chz, from);
+            N.r.Sx = __shfl_sync(full, T.r.Sx, from); N.r.Sy = __shfl_sync(full, T.r.Sy, from); N.r.Sz = __shfl_sync(full, T.r.Sz, from);
+            N.r.bits = __shfl_sync(full, T.r.bits, from);
+            const uint32_t slotN = __shfl_sync(full, slot, from);
+            const DevScene* scN = reinterpret_cast<const DevScene*>(__shfl_sync(full, reinterpret_cast<unsigned long long>(scp), from));
+            if (takes) {
+                slot = slotN;
+                scp = scN;
+                N.h.hit = false;
+                N.h.u = N.h.v = 0.0f;
+                N.h.inst = N.h.prim = 0xFFFFFFFFu;
+                N.sp = N.sb = 0;
+                N.marker = false;
+                N.active = true;
+                if (!N.inBlas) {
+                    const float* w = stk.saved + ((int)from - (int)lane);
+                    N.r.ox = w[0]; N.r.oy = w[STACK::kStride]; N.r.oz = w[2 * STACK::kStride];
+                    box_terms(N.r.ox, w[3 * STACK::kStride], N.h.t, N.r.jx, N.r.clx, N.r.chx);
+                    box_terms(N.r.oy, w[4 * STACK::kStride], N.h.t, N.r.jy, N.r.cly, N.r.chy);
+                    box_terms(N.r.oz, w[5 * STACK::kStride], N.h.t, N.r.jz, N.r.clz, N.r.chz);
+                    N.r.bits = octant(N.r.jx, N.r.jy, N.r.jz) << 6;
+                    N.nodes = sceneOf(scN).tlasWide;
+                    N.tris = nullptr;
+                }
+                T = N;
+                stk.over() = 0u;
+            }
+            __syncwarp();
+        }
+        const bool was = T.active;
+        const float before = T.h.t;
+#pragma unroll 1
+        for (int j = 0; j < RG_DRAIN_ROUNDS; ++j) {
+            const bool inner = T.active && !(T.ref & kLeaf);
+            if (!__any_sync(full, inner)) break;
+            if (inner) trav_step<COUNT, true>(T, sceneOf(scp), stk, vc);
+        }
+        if (T.active && (T.ref & kLeaf)) trav_step<COUNT, true>(T, sceneOf(scp), stk, vc);
+        // a closer hit shortens the ray for its other lanes
+        for (unsigned m = __ballot_sync(full, T.h.t < before && T.h.hit); m; m &= m - 1u) {
+            const int f = __ffs(m) - 1;
+            const float t = __shfl_sync(full, T.h.t, f);
+            if (__shfl_sync(full, slot, f) == slot && T.h.t > t) {
+                T.h.t = t;
+                T.h.hit = false;
+            }
+        }
+        for (unsigned m = __ballot_sync(full, was && !T.active); m;) {
+            const int f = __ffs(m) - 1;
+            m &= m - 1u;
+            const uint32_t sf = __shfl_sync(full, slot, f);
+            const unsigned peers = __ballot_sync(full, (T.active || (m >> lane & 1u)) && slot == sf);
+            if (!peers) {
+                if ((int)lane == f) hitOut();
+                continue;
+            }
+            Hit h;
+            h.t = __shfl_sync(full, T.h.t, f);
+            h.u = __shfl_sync(full, T.h.u, f);
+            h.v = __shfl_sync(full, T.h.v, f);
+            h.inst = __shfl_sync(full, T.h.inst, f);
+            h.prim = __shfl_sync(full, T.h.prim, f);
+            h.hit = __shfl_sync(full, (int)T.h.hit, f) != 0;
+            const uint32_t over = __shfl_sync(full, stk.over(), f);
+            if ((int)lane == __ffs(peers) - 1) {
+                if (h.hit && accept(h.t, h.t, h.inst, h.prim, T.h)) T.h = h;
+                if (over) stk.over() = 1u;
+            }
+        }
+    }
+}
+
+// closest hit of every ray of a set.  Lanes whose ray finished take new rays (one atomic per warp) as
+// soon as RG_FETCH_THRESHOLD lanes of the warp are idle, so a warp does not wait for its longest ray;
+// between fetches every lane advances its ray by RG_WF_STEPS steps.  Its forms:
+//   kFormTree   the nodes of one round of a frame's ray trees (q: the round); the first round computes
+//               the camera rays of the roots itself;
+//   kFormBatch  queue q of the batch loop; the ray's scene is its path's job's scene, and P.perm
+//               (nullable) gives the order the rays are taken in;
+//   kFormQuery  rg_trace_rays_device: rays and hits in the caller's buffers.
+enum TraceForm : int { kFormTree, kFormBatch, kFormQuery };
 #ifndef RG_FETCH_THRESHOLD
 #define RG_FETCH_THRESHOLD 8
 #endif
 #ifndef RG_WF_STEPS
 #define RG_WF_STEPS 6
-#endif
-#ifndef RG_WHILE_WHILE
-#define RG_WHILE_WHILE 1
 #endif
 #ifndef RG_INNER_ROUNDS
 #define RG_INNER_ROUNDS 3
@@ -1213,9 +1387,9 @@ __global__ void __launch_bounds__(256) k_wfb_raygen(const TraceParams P) {
 // a finished ray's hit: the frame loop's hit record (t, u, v, primitive; instance or 0xFFFFFFFF), or
 // for a ray query rg_trace_rays' layout in the caller's buffers (t, u, v and (instance, primitive);
 // zeros and 0xFFFFFFFF for a miss)
-template <bool QUERY>
+template <TraceForm FORM>
 __device__ __forceinline__ void put_hit(const TraceParams& P, uint32_t slot, const Hit& h, bool hit) {
-    if (QUERY) {
+    if (FORM == kFormQuery) {
         float* t = P.queryTuv + 3 * (size_t)slot;
         uint32_t* id = P.queryIds + 2 * (size_t)slot;
         t[0] = hit ? h.t : 0.0f;
@@ -1224,19 +1398,42 @@ __device__ __forceinline__ void put_hit(const TraceParams& P, uint32_t slot, con
         id[0] = hit ? h.inst : 0xFFFFFFFFu;
         id[1] = hit ? h.prim : 0xFFFFFFFFu;
     } else {
-        P.wf.hitTUV[slot] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
-        P.wf.hitInst[slot] = hit ? h.inst : 0xFFFFFFFFu;
+        float4* t = FORM == kFormTree ? P.tree.hitTUV : P.wf.hitTUV;
+        uint32_t* i = FORM == kFormTree ? P.tree.hitInst : P.wf.hitInst;
+        t[slot] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
+        i[slot] = hit ? h.inst : 0xFFFFFFFFu;
     }
 }
 
-// QUERY: the ray-query form (rg_trace_rays_device), rays and hits in the caller's buffers
-template <bool COUNT, bool BATCH, int THREADS, int DEPTH, bool QUERY = false>
+// lanes of a warp that take rays in a launch of `count`, and blocks that have rays
+__device__ __forceinline__ uint32_t trace_width(uint32_t count, uint32_t threads) {
+    const uint32_t warps = gridDim.x * (threads / 32);
+    return min(32u, max(1u, (count + warps - 1u) / warps));
+}
+__device__ __forceinline__ uint32_t trace_workers(uint32_t count, uint32_t threads) {
+    const uint32_t perBlock = trace_width(count, threads) * (threads / 32);
+    return min(gridDim.x, (count + perBlock - 1u) / perBlock);
+}
+
+template <bool COUNT, TraceForm FORM, int THREADS, int DEPTH>
 __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k_wf_trace(const __grid_constant__ TraceParams P, int q) {
     RG_DECLARE_SMEM_STACK(stk, THREADS, DEPTH);
     const WavefrontBuffers& wf = P.wf;
-    const bool first = !BATCH && !QUERY && P.firstRound;
-    const uint32_t count = QUERY ? P.queryCount : first ? frame_work_total(P) : *(volatile uint32_t*)(wf.counts + q);
-    if (blockIdx.x == 0 && threadIdx.x == 0) wf.counts[q ^ 1] = 0;  // the shade kernel appends there next
+    constexpr bool TREE = FORM == kFormTree, BATCH = FORM == kFormBatch, QUERY = FORM == kFormQuery;
+    const bool first = TREE && P.firstRound;
+    uint32_t node0 = 0, count;  // TREE: the round's first node
+    if (TREE) {
+        node0 = first ? 0u : P.tree.ctl[kTreeBounds + q];
+        const uint32_t end = first ? P.treeRoots : min(P.treeRoots + *(volatile uint32_t*)(P.tree.ctl + kTreeAlloc), P.tree.capacity);
+        count = end - node0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            P.tree.ctl[kTreeBounds + q + 1] = end;  // the next round's first node
+            P.tree.ctl[kTreeChanges] = P.tree.ctl[kTreeLevels] = P.tree.ctl[kTreeCand + (P.treeCand ^ 1u)] = 0;  // k_tree_check's
+        }
+    } else {
+        count = QUERY ? P.queryCount : *(volatile uint32_t*)(wf.counts + q);
+        if (BATCH && blockIdx.x == 0 && threadIdx.x == 0) wf.counts[q ^ 1] = 0;  // the shade kernel appends there next
+    }
     const unsigned lane = threadIdx.x & 31;
     const unsigned ltmask = (1u << lane) - 1u;
     VisitCounts vc = {0, 0, 0};
@@ -1253,50 +1450,36 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
             vc.overflow++;                                                                   \
             wf.overflow[atomicAdd(wf.counts + 3, 1u)] = slot;                                \
         }                                                                                    \
-        put_hit<QUERY>(P, slot, T.h, T.h.hit);                                               \
+        put_hit<FORM>(P, slot, T.h, T.h.hit);                                                \
     } while (0)
-    bool exhausted = false;
-    for (;;) {
-        const unsigned idle = __ballot_sync(0xFFFFFFFFu, !T.active);
-        if (__popc(idle) >= RG_FETCH_THRESHOLD || idle == 0xFFFFFFFFu) {
-            const bool need = !T.active && !exhausted;
-            const unsigned needMask = __ballot_sync(0xFFFFFFFFu, need);
-            if (needMask) {
-                const int leader = __ffs(needMask) - 1;
-                uint32_t base = 0;
-                if ((int)lane == leader) base = atomicAdd(wf.counts + 2, (uint32_t)__popc(needMask));
-                base = __shfl_sync(0xFFFFFFFFu, base, leader);
-                if (need) {
-                    const uint32_t k = base + (uint32_t)__popc(needMask & ltmask);
-                    if (k >= count) {
-                        exhausted = true;
-                    } else if (first) {  // camera ray of work item k, computed here
-                        slot = k;
-                        uint32_t path;
-                        Payload p0;
-                        RayReq r0;
-                        if (frame_work_item(P, k, path, p0, r0)) {
-                            trav_begin(T, P.scene, r0.o.x, r0.o.y, r0.o.z, r0.d.x, r0.d.y, r0.d.z, r0.tmin, r0.tmax, stk);
-                            if (!T.active) {
-                                wf.hitTUV[slot] = make_float4(T.h.t, T.h.u, T.h.v, __uint_as_float(T.h.prim));
-                                wf.hitInst[slot] = 0xFFFFFFFFu;
-                            }
-                        }
-                    } else {
-                        slot = P.perm ? P.perm[k] : k;
-                        if (BATCH) scp = &P.jobs[P.slotJob[wf.qPath[q][slot]]].scene;
-                        const float4 o = QUERY ? P.queryRays[2 * (size_t)slot] : wf.qO[q][slot];
-                        const float4 d = QUERY ? P.queryRays[2 * (size_t)slot + 1] : wf.qD[q][slot];
-                        trav_begin(T, RG_SC, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, stk);
-                        if (!T.active) put_hit<QUERY>(P, slot, T.h, false);  // zero direction or the scene box missed
-                    }
-                }
+    // starts ray k of the launch
+    auto begin = [&](uint32_t k) {
+        if (first) {  // camera ray of root k, computed here
+            slot = k;
+            uint32_t sample;
+            Payload p0;
+            RayReq r0;
+            if (frame_work_item(P, P.treeBase + k, sample, p0, r0)) {
+                trav_begin(T, P.scene, r0.o.x, r0.o.y, r0.o.z, r0.d.x, r0.d.y, r0.d.z, r0.tmin, r0.tmax, stk);
+                if (!T.active) put_hit<FORM>(P, slot, T.h, false);
             }
-            if (!__any_sync(0xFFFFFFFFu, T.active || !exhausted)) break;
+        } else if (TREE) {
+            slot = node0 + k;
+            const float4 o = P.tree.rayO[slot], d = P.tree.rayD[slot];
+            trav_begin(T, P.scene, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, stk);
+            if (!T.active) put_hit<FORM>(P, slot, T.h, false);
+        } else {
+            slot = P.perm ? P.perm[k] : k;
+            if (BATCH) scp = &P.jobs[P.slotJob[wf.qPath[q][slot]]].scene;
+            const float4 o = QUERY ? P.queryRays[2 * (size_t)slot] : wf.qO[q][slot];
+            const float4 d = QUERY ? P.queryRays[2 * (size_t)slot + 1] : wf.qD[q][slot];
+            trav_begin(T, RG_SC, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, stk);
+            if (!T.active) put_hit<FORM>(P, slot, T.h, false);  // zero direction or the scene box missed
         }
-#if RG_WHILE_WHILE
-        // while-while: lanes on inner nodes descend together (the others wait), then every lane at a
-        // leaf processes it, so each pass runs one kind of step across most of the warp
+    };
+    // while-while: lanes on inner nodes descend together (the others wait), then every lane at a
+    // leaf processes it, so each pass runs one kind of step across most of the warp
+    auto passes = [&]() {
 #pragma unroll 1
         for (int k = 0; k < RG_WF_STEPS; ++k) {
 #pragma unroll 1
@@ -1313,18 +1496,38 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
                 if (!T.active) RG_WF_HIT_OUT();
             }
         }
-#else
-        if (T.active) {
-#pragma unroll 1
-            for (int k = 0; k < RG_WF_STEPS; ++k) {
-                trav_step<COUNT>(T, RG_SC, stk, vc);
-                if (!T.active) {
-                    RG_WF_HIT_OUT();
-                    break;
+    };
+    const uint32_t workers = trace_workers(count, THREADS);
+    if (blockIdx.x >= workers) return;
+    if (workers < gridDim.x || trace_width(count, THREADS) < 32u) {
+        // Fewer rays than lanes: spread over all warps, whose other lanes join in.  Warp w takes rays
+        // w * width .. + width - 1 without the fetch counter, and blocks without a ray are done.
+        const uint32_t width = trace_width(count, THREADS), k = (blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5)) * width + lane;
+        if (lane < width && k < count) begin(k);
+        while (__popc(__ballot_sync(0xFFFFFFFFu, T.active)) > RG_DRAIN_LANES) passes();
+        drain<COUNT>(T, slot, scp, stk, vc, [&](const DevScene* sc) -> const DevScene& { return BATCH ? *sc : P.scene; }, [&] { RG_WF_HIT_OUT(); });
+    } else {
+        bool exhausted = false;
+        for (;;) {
+            const unsigned idle = __ballot_sync(0xFFFFFFFFu, !T.active);
+            if (__popc(idle) >= RG_FETCH_THRESHOLD || idle == 0xFFFFFFFFu) {
+                const bool need = !T.active && !exhausted;
+                const unsigned needMask = __ballot_sync(0xFFFFFFFFu, need);
+                if (needMask) {
+                    const int leader = __ffs(needMask) - 1;
+                    uint32_t base = 0;
+                    if ((int)lane == leader) base = atomicAdd(wf.counts + 2, (uint32_t)__popc(needMask));
+                    base = __shfl_sync(0xFFFFFFFFu, base, leader);
+                    if (need) {
+                        const uint32_t k = base + (uint32_t)__popc(needMask & ltmask);
+                        if (k >= count) exhausted = true;
+                        else begin(k);
+                    }
                 }
+                if (!__any_sync(0xFFFFFFFFu, T.active || !exhausted)) break;
             }
+            passes();
         }
-#endif
     }
 #undef RG_WF_HIT_OUT
 #undef RG_SC
@@ -1345,7 +1548,7 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        stk.over() = atomicAdd(wf.counts + 4, 1u) == gridDim.x - 1 ? 1u : 0u;
+        stk.over() = atomicAdd(wf.counts + 4, 1u) == trace_workers(count, THREADS) - 1 ? 1u : 0u;
     }
     __syncthreads();
     const uint32_t lastBlock = *reinterpret_cast<volatile uint32_t*>(&stk_mem[DEPTH - 1][0]);
@@ -1356,13 +1559,16 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
         const uint32_t s = __ldcg(wf.overflow + i);
         float4 o, d;
         const DevScene* sc = &P.scene;
-        if (first) {  // work item s's camera ray, as the first round computed it
-            uint32_t path;
+        if (first) {  // root s's camera ray, as the first round computed it
+            uint32_t sample;
             Payload p0;
             RayReq r0;
-            frame_work_item(P, s, path, p0, r0);
+            frame_work_item(P, P.treeBase + s, sample, p0, r0);
             o = make_float4(r0.o.x, r0.o.y, r0.o.z, r0.tmin);
             d = make_float4(r0.d.x, r0.d.y, r0.d.z, r0.tmax);
+        } else if (TREE) {
+            o = P.tree.rayO[s];
+            d = P.tree.rayD[s];
         } else if (QUERY) {
             o = P.queryRays[2 * (size_t)s];
             d = P.queryRays[2 * (size_t)s + 1];
@@ -1373,7 +1579,7 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
         }
         Hit h;
         retrace_deep(sc, o, d, &h, P.counters);
-        put_hit<QUERY>(P, s, h, h.hit);
+        put_hit<FORM>(P, s, h, h.hit);
     }
     if (threadIdx.x == 0) {
         wf.counts[3] = 0;
@@ -1381,13 +1587,610 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
     }
 }
 
+// ---- ray trees -------------------------------------------------------------------------------------
+// The reference's recursion is depth-first on one payload, so a path traced as the shaders run it has
+// one ray in flight at a time: up to 70 rays in sequence, and a frame as many rounds.  But which rays a
+// hit issues follows from the hit, its recursion depth and its ray type; of the payload's state that
+// earlier siblings leave behind, only curIOR (the direction of a front-face refraction) and refDepth (a
+// grid material's colour and reflectivity) matter.  So every sample's rays are a tree of nodes:
+//   rounds    k_wf_trace and k_tree_expand grow all trees breadth first, one recursion level a round:
+//             the shadow, reflection and refraction rays of a level's hits are traced by one launch,
+//             curIOR and refDepth taken as if no sibling had changed them.  Every nested trace is at
+//             least one recursion level deeper, so maxRecursions + 1 rounds finish the trees.
+//             A refraction in a reflection's subtree that changes the curIOR of the refraction after
+//             it (0.07 - 0.6 % of the samples on the benchmark scenes) replaces that ray at once, and
+//             one or two more rounds grow the replacements.
+//   check     k_tree_check compares what the finished subtrees leave in curIOR and refDepth with what
+//             was assumed.  A refraction ray that still comes out different, or a reflection ray that
+//             must or must not be there, is replaced, its new subtree grown by further rounds, and the
+//             check repeated until nothing changes.
+//   compose   k_tree_compose evaluates the hits bottom-up, a round at a time from the last: a hit's
+//             colour is a function of its surface, its shadow chain and its children's colours.
+// All of it evaluates the shaders' expressions on the shaders' operands, in their order, so the images
+// are the depth-first ones bit for bit.
+//
+// A node: ray (origin, tmin; direction, tmax), state (curIOR and refDepth on entry, recursion depth,
+// ray type, job, parent), hit, surface of the hit (world normal -- flipped toward the ray for GENERIC
+// hits --, material), links to its shadow / reflection / refraction node.  Roots (nodes 0 ..
+// treeRoots - 1, one per sample of the chunk) have no stored ray and state: both are recomputed.
+constexpr uint32_t kNodeMask = kTreeMaxNodes - 1u;  // links: node ids below kTreeMaxNodes, or
+constexpr uint32_t kNoNode = kNodeMask;             //   no ray issued
+constexpr uint32_t kZeroFront = kNodeMask - 1u;     //   a front-face refraction of zero direction: misses,
+constexpr uint32_t kZeroBack = kNodeMask - 2u;      //   leaves curIOR = ior; a back-face one: leaves 1
+constexpr uint32_t kFrontBit = 0x80000000u;         // links.x: the ray hit the front face
+constexpr uint32_t kOffBit = 0x40000000u;           // state.z: a sibling may have changed refDepth
+constexpr uint32_t kDeadBit = 0x80000000u;          // state.z: below a ray that was replaced
+__device__ __forceinline__ bool is_node(uint32_t link) { return link < kZeroBack; }
+
+struct NodeState {
+    float curIOR, refDepth;
+    uint32_t rec, type, job, parent;  // parent: with kOffBit / kDeadBit
+};
+__device__ __forceinline__ NodeState node_state(const TraceParams& P, uint32_t i) {
+    if (i < P.treeRoots) return {1.0f, 0.0f, 0u, (uint32_t)RT_GENERIC, 0u, kNodeMask};
+    const uint4 s = P.tree.state[i];
+    return {__uint_as_float(s.x), __uint_as_float(s.w), s.y & 15u, (s.y >> 4) & 3u, s.y >> 6, s.z};
+}
+__device__ __forceinline__ uint4 pack_state(float curIOR, uint32_t rec, uint32_t type, uint32_t job, uint32_t parent, float refDepth) {
+    return make_uint4(__float_as_uint(curIOR), rec | type << 4 | job << 6, parent, __float_as_uint(refDepth));
+}
+
+// the camera ray of root k of the chunk, its fresh payload and its sample index; false outside the image
+template <bool BATCH>
+__device__ __forceinline__ bool tree_root(const TraceParams& P, uint32_t k, uint32_t& job, uint32_t& sample, Payload& p, RayReq& ray) {
+    job = 0;
+    if (BATCH) return batch_primary(P, P.treeBase + k, job, sample, p, ray);
+    return frame_work_item(P, P.treeBase + k, sample, p, ray);
+}
+template <bool BATCH>
+__device__ __forceinline__ const DevScene& tree_scene(const TraceParams& P, uint32_t job) { return BATCH ? P.jobs[job].scene : P.scene; }
+template <bool BATCH>
+__device__ __forceinline__ const rg_ubo& tree_ubo(const TraceParams& P, uint32_t job) { return BATCH ? P.jobs[job].ubo : P.ubo; }
+__device__ __forceinline__ V3 light_of(const rg_ubo& u) { return v3(u.lightDir[0], u.lightDir[1], u.lightDir[2]); }
+
+__device__ __forceinline__ bool node_hit(const RayTree& t, uint32_t i) { return t.hitInst[i] != 0xFFFFFFFFu; }
+
+// marks the GENERIC nodes from y down as replaced (what nodes from `fresh` on issued or will issue
+// learns it from its parent)
+__device__ void bury(const RayTree& t, uint32_t y, uint32_t fresh) {
+    uint32_t st[2 * kMaxFrames];
+    int n = 0;
+    st[n++] = y;
+    while (n) {
+        y = st[--n];
+        atomicOr(&t.state[y].z, kDeadBit);
+        if (y >= fresh || !node_hit(t, y)) continue;
+        const uint4 c = t.link[y];
+        if (is_node(c.y)) st[n++] = c.y;
+        if (is_node(c.z)) st[n++] = c.z;
+    }
+}
+
+// GENERIC node x's ray and hit, for rays it issues anew
+template <bool BATCH>
+__device__ __forceinline__ void reissue_frame(const TraceParams& P, uint32_t x, NodeState& st, uint32_t& seed, Frame& cur) {
+    const RayTree& t = P.tree;
+    RayReq ray;
+    seed = 0;
+    if (x < P.treeRoots) {
+        Payload p;
+        uint32_t sample;
+        tree_root<BATCH>(P, x, st.job, sample, p, ray);
+        seed = p.seed;
+    } else {
+        const float4 o = t.rayO[x], d = t.rayD[x];
+        ray.o = v3(o.x, o.y, o.z);
+        ray.d = v3(d.x, d.y, d.z);
+    }
+    const float4 sf = t.surf[x];
+    cur.t = t.hitTUV[x].x;
+    cur.D = ray.d;
+    cur.n = v3(sf.x, sf.y, sf.z);
+    cur.origin = ray.o + ray.d * cur.t;
+    load_material(tree_scene<BATCH>(P, st.job).materials + __float_as_uint(sf.w), cur);
+}
+
+// a new GENERIC node for a ray of direction dir from cur; kNoNode when the pool is full
+__device__ __forceinline__ uint32_t append_ray(const TraceParams& P, const Frame& cur, V3 dir, float ior, uint32_t rec, uint32_t job,
+                                               uint32_t parent, float refDepth) {
+    const RayTree& t = P.tree;
+    const uint32_t at = P.treeRoots + atomicAdd(t.ctl + kTreeAlloc, 1u);
+    if (at >= t.capacity) return kNoNode;
+    t.rayO[at] = make_float4(cur.origin.x, cur.origin.y, cur.origin.z, 0.01f);
+    t.rayD[at] = make_float4(dir.x, dir.y, dir.z, 1000.0f);
+    t.state[at] = pack_state(ior, rec, RT_GENERIC, job, parent, refDepth);
+    atomicMax(t.ctl + kTreeLevels, 16u - rec);
+    __threadfence();  // before the link to it: whoever replaces it finds its state
+    return at;
+}
+
+// front-face hit x (cur) refracts with curIOR = ior; refDepth: v before its reflection ray
+template <bool GLOSSY>
+__device__ __forceinline__ void replace_refraction(const TraceParams& P, uint32_t x, const NodeState& st, uint32_t seed, const Frame& cur,
+                                                   float ior, float v, uint32_t fresh) {
+    const RayTree& t = P.tree;
+    const V3 dir = refract_dir<GLOSSY>(cur, ior / cur.ior, seed, (int)st.rec);
+    const uint32_t to = is_zero(dir) ? kZeroFront
+                                     : append_ray(P, cur, dir, cur.ior, st.rec + 1u, st.job, x | kOffBit, is_node(t.link[x].y) ? v + cur.t : v);
+    // the refraction link and the curIOR it was issued with, in one exchange
+    const unsigned long long pair = (unsigned long long)__float_as_uint(ior) << 32 | to;
+    const uint32_t old = (uint32_t)atomicExch(reinterpret_cast<unsigned long long*>(&t.link[x].z), pair);
+    if (is_node(old)) bury(t, old, fresh);
+}
+
+// GENERIC node y refracts and leaves curIOR = ior (as far as is known yet): the refraction that runs next
+// in depth-first order outside y's subtree is that of the nearest ancestor whose reflection subtree y is
+// the last refraction of.  `fresh`: first node of the current round.
+template <bool BATCH, bool GLOSSY>
+__device__ __forceinline__ void refraction_left(const TraceParams& P, uint32_t y, float ior, uint32_t fresh) {
+    const RayTree& t = P.tree;
+    while (y >= P.treeRoots) {
+        const uint32_t x = t.state[y].z & kNodeMask;
+        const uint4 c = t.link[x];
+        if (c.y == y && c.z != kNoNode) {
+            if (!(c.x & kFrontBit) || c.w == __float_as_uint(ior)) return;
+            NodeState st = node_state(P, x);
+            if (x >= P.treeRoots && (st.parent & kDeadBit)) return;
+            uint32_t seed;
+            Frame cur;
+            reissue_frame<BATCH>(P, x, st, seed, cur);
+            replace_refraction<GLOSSY>(P, x, st, seed, cur, ior, st.refDepth, fresh);
+            return;
+        }
+        if (c.y != y && c.z != y) return;  // y was replaced
+        y = x;
+    }
+}
+
+// Surfaces and child rays of one round's hits.  A warp appends its shadow rays, then its reflection,
+// then its refraction rays, with one atomic: 32 hits of a few surfaces give runs of similar rays.
+template <bool BATCH, bool GLOSSY>
+__global__ void __launch_bounds__(128) k_tree_expand(const __grid_constant__ TraceParams P, int round) {
+    const RayTree& t = P.tree;
+    const bool first = P.firstRound != 0;
+    const uint32_t begin = first ? 0u : t.ctl[kTreeBounds + round], end = t.ctl[kTreeBounds + round + 1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) t.ctl[kTreeFetch] = 0;  // the next trace launch's work counter
+    const unsigned lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+    for (uint32_t base = begin + blockIdx.x * blockDim.x; base < end; base += gridDim.x * blockDim.x) {
+        const uint32_t i = base + threadIdx.x;
+        bool want[3] = {false, false, false}, candidate = false;
+        V3 dir[3];
+        float depthC = 0.0f, iorT = 0.0f, tminS = 0.01f;
+        uint32_t recR = 0, typeS = RT_SHADOW_TRACE, link[3] = {kNoNode, kNoNode, kNoNode}, off = 0, offT = 0, matId = 0;
+        Frame cur;
+        NodeState st = {1.0f, 0.0f, 0u, (uint32_t)RT_GENERIC, 0u, 0u};
+        const uint32_t inst = i < end ? t.hitInst[i] : 0xFFFFFFFFu;
+        bool live = inst != 0xFFFFFFFFu;
+        if (live) {
+            RayReq ray;
+            uint32_t seed = 0;
+            if (first) {
+                uint32_t sample;
+                Payload p;
+                live = tree_root<BATCH>(P, i, st.job, sample, p, ray);
+                seed = p.seed;
+            } else {
+                st = node_state(P, i);
+                if (round > 1 && (st.parent & kNodeMask) >= P.treeRoots && (t.state[st.parent & kNodeMask].z & kDeadBit)) {  // its parent was replaced
+                    st.parent |= kDeadBit;
+                    t.state[i].z = st.parent;
+                }
+                live = !(st.parent & kDeadBit);
+                const float4 o = t.rayO[i], d = t.rayD[i];
+                ray.o = v3(o.x, o.y, o.z);
+                ray.d = v3(d.x, d.y, d.z);
+            }
+            if (live) {
+                const float4 ht = t.hitTUV[i];
+                const Hit h = {ht.x, ht.y, ht.z, inst, __float_as_uint(ht.w), true};
+                const DevScene& sc = tree_scene<BATCH>(P, st.job);
+                bool effect = false;
+                if (st.type == RT_SHADOW_TRACE) shadow_hit_surface(sc, h, ray, cur, matId);
+                else effect = closest_hit_surface(sc, h, ray, st.refDepth, cur, matId);
+                const rg_ubo& u = tree_ubo<BATCH>(P, st.job);
+                const bool deeper = (int)st.rec < u.maxRecursions;
+                off = st.parent & kOffBit;
+                if (st.type == RT_SHADOW_INTERNAL) {
+                    want[0] = deeper;
+                    dir[0] = cur.D;
+                } else if (st.type == RT_SHADOW_TRACE) {
+                    want[0] = deeper && cur.transparency > 0.0f;
+                    dir[0] = cur.D;
+                    typeS = RT_SHADOW_INTERNAL;
+                } else {
+                    cur.front = dot(-cur.D, cur.n) > 0.0f;
+                    if (!cur.front) cur.n = normalize(-cur.n);
+                    const V3 L = light_of(u);
+                    if (deeper && dot(-L, cur.n) > 0.07f) {
+                        want[0] = true;
+                        dir[0] = -L;
+                        tminS = 0.01f * 10.0f;
+                    }
+                    depthC = st.refDepth;
+                    offT = off;
+                    if (deeper && cur.reflectivity > 0.0f) {
+                        want[1] = true;
+                        dir[1] = reflect_dir<GLOSSY>(cur, seed, (int)st.rec);
+                        recR = st.rec + (uint32_t)cur.rayConsumption;
+                        depthC = st.refDepth + cur.t;
+                        offT = kOffBit;
+                    }
+                    if (deeper && cur.transparency > 0.0f) {
+                        dir[2] = refract_dir<GLOSSY>(cur, cur.front ? st.curIOR / cur.ior : cur.ior / 1.0f, seed, (int)st.rec);
+                        iorT = cur.front ? cur.ior : 1.0f;
+                        want[2] = !is_zero(dir[2]);
+                        if (!want[2]) link[2] = cur.front ? kZeroFront : kZeroBack;
+                    }
+                    candidate = deeper && ((cur.front && want[1] && cur.transparency > 0.0f) ||
+                                            (effect && off && grid_sign_varies(cur.origin, st.refDepth, cur.t)));
+                }
+            }
+        }
+        const unsigned m0 = __ballot_sync(0xFFFFFFFFu, want[0]), m1 = __ballot_sync(0xFFFFFFFFu, want[1]),
+                       m2 = __ballot_sync(0xFFFFFFFFu, want[2]);
+        const uint32_t n0 = (uint32_t)__popc(m0), n1 = (uint32_t)__popc(m1), n2 = (uint32_t)__popc(m2);
+        uint32_t at = 0;
+        if (n0 + n1 + n2) {
+            if (lane == 0) at = atomicAdd(t.ctl + kTreeAlloc, n0 + n1 + n2);
+            at = P.treeRoots + __shfl_sync(0xFFFFFFFFu, at, 0);
+        }
+        const uint32_t cp = warp_append(t.ctl + kTreeCand + P.treeCand, candidate);
+        if (candidate && cp < t.capacity) t.cand[P.treeCand][cp] = i;
+        if (!live && inst != 0xFFFFFFFFu && !first) t.link[i] = make_uint4(kNoNode, kNoNode, kNoNode, 0u);
+        if (live) {
+            const uint32_t c[3] = {at + (uint32_t)__popc(m0 & below), at + n0 + (uint32_t)__popc(m1 & below),
+                                   at + n0 + n1 + (uint32_t)__popc(m2 & below)};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                if (!want[k] || c[k] >= t.capacity) continue;  // a full pool discards the whole chunk (launch_trace_tree)
+                link[k] = c[k];
+                t.rayO[c[k]] = make_float4(cur.origin.x, cur.origin.y, cur.origin.z, k == 0 ? tminS : 0.01f);
+                t.rayD[c[k]] = make_float4(dir[k].x, dir[k].y, dir[k].z, 1000.0f);
+                t.state[c[k]] = k == 0 ? pack_state(st.curIOR, st.rec + 1u, typeS, st.job, i, st.refDepth)
+                              : k == 1 ? pack_state(st.curIOR, recR, RT_GENERIC, st.job, i | off, depthC)
+                                       : pack_state(iorT, st.rec + 1u, RT_GENERIC, st.job, i | offT, depthC);
+            }
+            const bool front = cur.front && st.type == RT_GENERIC;
+            t.link[i] = make_uint4(link[0] | (front ? kFrontBit : 0u), link[1], link[2], __float_as_uint(st.curIOR));
+            t.surf[i] = make_float4(cur.n.x, cur.n.y, cur.n.z, __uint_as_float(matId));
+            // a refraction behind some ancestor's reflection sets the curIOR of that ancestor's refraction.
+            // A front-face one is expected to leave the object again (curIOR 1) unless the recursion
+            // limit stops it inside.
+            if (link[2] != kNoNode && !first) {
+                const bool stays = front && (link[2] == kZeroFront || (int)st.rec + 1 >= tree_ubo<BATCH>(P, st.job).maxRecursions);
+                refraction_left<BATCH, GLOSSY>(P, i, stays ? cur.ior : 1.0f, begin);
+            }
+        }
+    }
+}
+
+// refDepth after the shaders ran the invocation at node y and everything below it, from value v before
+// it: every reflection ray adds the t of the hit that issued it, in depth-first order.  Nodes from
+// `fresh` on are not traced yet and count as misses.
+__device__ float fold_ref_depth(const RayTree& t, uint32_t y, float v, uint32_t fresh) {
+    uint32_t st[2 * kMaxFrames];
+    int n = 0;
+    st[n++] = y;
+    while (n) {
+        y = st[--n];
+        if (y >= fresh || !node_hit(t, y)) continue;
+        const uint4 c = t.link[y];
+        if (is_node(c.z)) st[n++] = c.z;
+        if (is_node(c.y)) {
+            v = v + t.hitTUV[y].x;
+            st[n++] = c.y;
+        }
+    }
+    return v;
+}
+
+// refDepth on entry of GENERIC node x as the depth-first order leaves it
+__device__ float exact_ref_depth(const TraceParams& P, uint32_t x, uint32_t fresh) {
+    const RayTree& t = P.tree;
+    uint32_t way[kMaxFrames];
+    int n = 0;
+    NodeState s = node_state(P, x);
+    while (x >= P.treeRoots && (s.parent & kOffBit) && n < kMaxFrames) {
+        way[n++] = x;
+        x = s.parent & kNodeMask;
+        s = node_state(P, x);
+    }
+    float v = s.refDepth;  // no sibling changed it here
+    while (n) {
+        const uint4 c = t.link[x];
+        const uint32_t next = way[--n];
+        if (is_node(c.y)) v = v + t.hitTUV[x].x;
+        if (c.y != next && is_node(c.y)) v = fold_ref_depth(t, c.y, v, fresh);
+        x = next;
+    }
+    return v;
+}
+
+// The candidates -- front-face hits with a reflection and a refraction ray, and grid-effect hits whose
+// refDepth a sibling may have changed -- against the finished subtrees (nodes below `fresh`).  What a
+// subtree leaves in curIOR is set by its last refraction: the end of the walk along refraction links,
+// or along the reflection link where an invocation refracts nothing.  Replaced rays are appended for the
+// next rounds; candidates whose subtree could still change stay in the other list.
+template <bool BATCH, bool GLOSSY>
+__global__ void __launch_bounds__(128) k_tree_check(const __grid_constant__ TraceParams P, int round) {
+    const RayTree& t = P.tree;
+    const uint32_t n = min(t.ctl[kTreeCand + P.treeCand], t.capacity), fresh = t.ctl[kTreeBounds + round];
+    if (blockIdx.x == 0 && threadIdx.x == 0) t.ctl[kTreeTraced] = fresh;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const uint32_t k = base + threadIdx.x;
+        bool keep = false;
+        uint32_t x = 0;
+        if (k < n) {
+            x = t.cand[P.treeCand][k];
+            NodeState st = node_state(P, x);
+            if (x < P.treeRoots) st.parent = 0u;
+            uint4 c = t.link[x];
+            const bool sibling = is_node(c.y) && c.y < fresh && node_hit(t, c.y);  // a reflection ray with a subtree
+            if (!(st.parent & kDeadBit) && is_node(c.y) && c.y >= fresh) keep = true;
+            else if (!(st.parent & kDeadBit) && (sibling || (st.parent & kOffBit))) {
+                uint32_t seed;
+                Frame cur;
+                reissue_frame<BATCH>(P, x, st, seed, cur);
+                const rg_material* materials = tree_scene<BATCH>(P, st.job).materials;
+                const bool grid = __ldg(&materials[__float_as_uint(t.surf[x].w)].effectId) == 1 && (st.parent & kOffBit) &&
+                                  grid_sign_varies(cur.origin, st.refDepth, cur.t);
+                uint32_t changes = 0;
+                float v = st.refDepth;
+                if (grid) {
+                    v = exact_ref_depth(P, x, fresh);
+                    grid_effect(cur.origin, v, cur.t, cur);
+                    const bool reflects = cur.reflectivity > 0.0f;
+                    if (reflects && !is_node(c.y)) {
+                        c.y = append_ray(P, cur, reflect_dir<GLOSSY>(cur, seed, (int)st.rec), st.curIOR,
+                                         st.rec + (uint32_t)cur.rayConsumption, st.job, x | kOffBit, v + cur.t);
+                        t.link[x].y = c.y;
+                        ++changes;
+                    } else if (!reflects && is_node(c.y)) {
+                        bury(t, c.y, fresh);
+                        t.link[x].y = c.y = kNoNode;
+                        ++changes;
+                    }
+                }
+                if ((c.x & kFrontBit) && cur.transparency > 0.0f) {
+                    float ior = st.curIOR;
+                    for (uint32_t y = c.y; is_node(y) && y < fresh && node_hit(t, y);) {
+                        const uint4 cy = t.link[y];
+                        if (is_node(cy.z)) {
+                            ior = __uint_as_float(t.state[cy.z].x);
+                            y = cy.z;
+                        } else if (cy.z == kNoNode) {
+                            y = cy.y;
+                        } else {
+                            ior = cy.z == kZeroBack ? 1.0f : __ldg(&materials[__float_as_uint(t.surf[y].w)].ior);
+                            break;
+                        }
+                    }
+                    if (c.w != __float_as_uint(ior)) {
+                        replace_refraction<GLOSSY>(P, x, st, seed, cur, ior, v, fresh);
+                        ++changes;
+                    }
+                }
+                if (changes) atomicAdd(t.ctl + kTreeChanges, changes);
+                if (sibling) {
+                    const uint4 cy = t.link[c.y < fresh ? c.y : x];
+                    keep = cy.y != kNoNode || cy.z != kNoNode || (st.parent & kOffBit);  // (off: c.y may yet reflect)
+                }
+                keep = keep || grid || changes;
+            }
+        }
+        const uint32_t pos = warp_append(t.ctl + kTreeCand + (P.treeCand ^ 1u), keep);
+        if (keep && pos < t.capacity) t.cand[P.treeCand ^ 1u][pos] = x;
+    }
+}
+
+// Whether the shadow chain of GENERIC node x ends in the sky: its last ray goes on behind a
+// SHADOW_INTERNAL hit (closesthit.rchit:133) and misses.
+__device__ bool chain_meets_sky(const TraceParams& P, uint32_t x) {
+    const RayTree& t = P.tree;
+    uint32_t s = t.link[x].x & kNodeMask;
+    for (bool behind = false;; behind = true) {
+        if (!is_node(s)) return false;
+        if (!node_hit(t, s)) return behind;
+        const uint32_t j = t.link[s].x & kNodeMask;  // SHADOW_INTERNAL (none at an opaque hit)
+        if (!is_node(j) || !node_hit(t, j)) return false;
+        s = t.link[j].x & kNodeMask;
+    }
+}
+
+// payload.depth < 1000 on entry of GENERIC node x: the last GENERIC hit or sky miss that the
+// depth-first order finished before it (0 before any)
+__device__ bool depth_is_near(const TraceParams& P, uint32_t x) {
+    const RayTree& t = P.tree;
+    while (x >= P.treeRoots) {
+        const uint32_t p = t.state[x].z & kNodeMask;
+        const uint4 c = t.link[p];
+        if (c.z == x && is_node(c.y)) return node_hit(t, c.y) && t.hitTUV[c.y].x < 1000.0f;
+        if (chain_meets_sky(P, p)) return false;
+        x = p;
+    }
+    return true;
+}
+
+// shadowCol of SHADOW_INTERNAL hit j (closesthit.rchit:126-128); every such hit finds hitValue at 1
+__device__ __forceinline__ V3 internal_shadow(const RayTree& t, uint32_t j, const Frame& m) {
+    const float thick = clampf(t.hitTUV[j].x * (1.0f - m.transparency) * 10.0f, 0.0f, 1.0f);
+    return v3s(1.0f) - mix(v3s(0.0f), normalize(v3s(1.1f) - m.diffuse) + v3s(0.1f), thick);
+}
+
+// hitValue that the shadow ray s of GENERIC node x returns with (closesthit.rchit:125-166, 193): the
+// chain SHADOW_TRACE, SHADOW_INTERNAL, SHADOW_TRACE, ... walked to its end and unwound
+__device__ V3 shadow_chain(const TraceParams& P, const DevScene& sc, const V3 L, uint32_t x, uint32_t s, RayCounts& cnt) {
+    const RayTree& t = P.tree;
+    uint32_t inner[kMaxFrames];  // SHADOW_INTERNAL hits passed
+    int n = 0;
+    V3 value = v3s(1.0f);
+    bool far = false;
+    Frame m;
+    auto surface = [&](uint32_t k) {
+        const uint32_t id = __float_as_uint(t.surf[k].w);
+        load_material(sc.materials + id, m);
+        if (__ldg(&sc.materials[id].effectId) == 1) {  // the chain's rays carry x's refDepth
+            const NodeState sk = node_state(P, x);
+            const float4 o = t.rayO[k], d = t.rayD[k];
+            const float ht = t.hitTUV[k].x;
+            grid_effect(v3(o.x, o.y, o.z) + v3(d.x, d.y, d.z) * ht, (sk.parent & kOffBit) && x >= P.treeRoots ? exact_ref_depth(P, x, kNodeMask) : sk.refDepth, ht, m);
+        }
+    };
+    for (;;) {
+        cnt.shadow++;
+        if (!node_hit(t, s)) {
+            if (n) {  // behind a SHADOW_INTERNAL hit: miss shader 0
+                const float4 d = t.rayD[s];
+                Payload p;
+                sky(p, v3(d.x, d.y, d.z), L);
+                value = p.hitValue;
+                far = true;
+            }
+            break;
+        }
+        const float transparency = __ldg(&sc.materials[__float_as_uint(t.surf[s].w)].transparency);
+        if (!(transparency > 0.0f)) {
+            value = value * mixs(0.4f, 0.8f, clampf(logf(t.hitTUV[s].x) / 8.0f, 0.0f, 1.0f));
+            break;
+        }
+        const uint32_t j = t.link[s].x & kNodeMask;
+        if (!is_node(j)) break;  // recursion limit
+        cnt.shadow++;
+        if (!node_hit(t, j)) break;  // shadow miss: 1
+        const uint32_t a = t.link[j].x & kNodeMask;
+        if (!is_node(a)) {  // recursion limit
+            surface(j);
+            value = internal_shadow(t, j, m) * 0.4f;
+            break;
+        }
+        inner[n++] = j;
+        s = a;
+    }
+    if (n && !far) far = !depth_is_near(P, x);
+    while (n) {
+        const uint32_t j = inner[--n];
+        surface(j);
+        V3 col = internal_shadow(t, j, m);
+        if (!far) {
+            value = value * col;
+            continue;
+        }
+        const float4 d = t.rayD[j], sf = t.surf[j];
+        const V3 dir = refract(v3(d.x, d.y, d.z), v3(sf.x, sf.y, sf.z), m.ior / 1.0f);
+        const float q = dot(L, dir);
+        col = col * (q * q * q * q * q + 0.75f);
+        cnt.masked++;
+        Payload p;
+        sky(p, -dir, L);
+        value = col + p.hitValue * 0.1f;
+    }
+    return value;
+}
+
+// Colours of one round's GENERIC nodes from their children's (rayO of a child: colour; its ray is no
+// longer needed once its own colour is known); roots write their sample's payload sums.
+template <bool BATCH>
+__global__ void __launch_bounds__(128) k_tree_compose(const __grid_constant__ TraceParams P, int round) {
+    const RayTree& t = P.tree;
+    const bool roots = round == 0;
+    const uint32_t begin = roots ? 0u : t.ctl[kTreeBounds + round], end = t.ctl[kTreeBounds + round + 1];
+    RayCounts cnt = {0, 0, 0, 0};
+    for (uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x) {
+        uint32_t sample = 0;
+        Payload p;
+        RayReq ray;
+        NodeState st = {1.0f, 0.0f, 0u, (uint32_t)RT_GENERIC, 0u, 0u};
+        if (roots) {
+            if (!tree_root<BATCH>(P, i, st.job, sample, p, ray)) continue;
+            cnt.primary++;
+        } else {
+            st = node_state(P, i);
+            if (st.type != RT_GENERIC || (st.parent & kDeadBit)) continue;
+            const float4 d = t.rayD[i];
+            ray.d = v3(d.x, d.y, d.z);
+        }
+        const rg_ubo& u = tree_ubo<BATCH>(P, st.job);
+        const V3 L = light_of(u);
+        if (!node_hit(t, i)) {
+            sky(p, ray.d, L);
+        } else {
+            const DevScene& sc = tree_scene<BATCH>(P, st.job);
+            const float4 sf = t.surf[i];
+            const uint4 c = t.link[i];
+            Frame cur;
+            cur.t = t.hitTUV[i].x;
+            cur.n = v3(sf.x, sf.y, sf.z);
+            const rg_material* M = sc.materials + __float_as_uint(sf.w);
+            load_material(M, cur);
+            if (__ldg(&M->effectId) == 1) {
+                if (!roots) {
+                    const float4 o = t.rayO[i];
+                    ray.o = v3(o.x, o.y, o.z);
+                }
+                grid_effect(ray.o + ray.d * cur.t, (st.parent & kOffBit) ? exact_ref_depth(P, i, kNodeMask) : st.refDepth, cur.t, cur);
+            }
+            // closesthit.rchit:168-204
+            const bool deeper = (int)st.rec < u.maxRecursions;
+            const float ndl = dot(-L, cur.n);
+            V3 base = cur.diffuse * fmaxf(ndl, 0.2f), shadow = v3s(1.0f);
+            if (ndl > 0.07f) {
+                if (deeper) shadow = shadow_chain(P, sc, L, i, c.x & kNodeMask, cnt);
+            } else {
+                const float tr = cur.transparency, sm = tr * tr;
+                shadow = tr < 1.0f ? mix(v3s(1.0f), cur.diffuse * sm, tr) : v3s(0.4f);
+            }
+            // :206-221
+            V3 reflectColor = v3s(1.0f), refractColor = v3s(1.0f);
+            float reflectDepth = 0.0f;
+            if (is_node(c.y)) {
+                cnt.secondary++;
+                const float4 r = t.rayO[c.y];
+                reflectColor = v3(r.x, r.y, r.z) * cur.specular;
+                reflectDepth = r.w;
+            }
+            // :223-251
+            if (c.z != kNoNode) {
+                V3 value;
+                if (is_node(c.z)) {
+                    cnt.secondary++;
+                    const float4 r = t.rayO[c.z];
+                    value = v3(r.x, r.y, r.z);
+                } else {
+                    Payload q;
+                    sky(q, v3s(0.0f), L);
+                    value = q.hitValue;
+                }
+                refractColor = (c.x & kFrontBit) ? value : mix(v3s(1.0f), cur.diffuse, logf(1.0f + cur.t)) * value;
+            }
+            // :253-267
+            base = base * shadow;
+            base = base + cur.diffuse * cur.emission;
+            const float total = fmaxf(cur.transparency, cur.reflectivity), den = cur.transparency + cur.reflectivity;
+            const V3 roughCol = mix(refractColor, reflectColor, den == 0.0f ? 0.0f : cur.reflectivity / den);
+            p.hitValue = mix(base, roughCol, total);
+            p.depth = cur.t;
+            if (roots) {
+                p.hitValue = base;
+                p.normal = cur.n;
+                p.roughRGB = roughCol;
+                p.roughA = fminf((reflectDepth / 50.0f) * cur.roughness, cur.roughness / 2.1f);
+                p.reflectContribution = total;
+            }
+        }
+        if (roots) store_sample(P.samples + 3 * (size_t)sample, p);
+        else t.rayO[i] = make_float4(p.hitValue.x, p.hitValue.y, p.hitValue.z, p.depth);
+    }
+    __syncwarp();
+    unsigned long long c[4] = {cnt.primary, cnt.shadow, cnt.secondary, cnt.masked};
+    flush_counts(P, c, 4);
+}
+
 // shading of one path from a trace result up to its next traversed ray (false) or to the end of
 // its sample (true); mask-0 traces and zero directions run their miss shader right away
-template <bool GLOSSY>
 __device__ __forceinline__ bool shade_until_trace(const DevScene& sc, const V3 L, const int maxRec, Hit h, Payload& p, RayReq& ray,
                                                   Frame* frames, int& fsp, Frame& cur, RayCounts& cnt) {
     for (;;) {
-        if (!shade_step<GLOSSY>(sc, L, maxRec, h, p, ray, frames, fsp, cur, cnt)) return true;
+        if (!shade_step<false>(sc, L, maxRec, h, p, ray, frames, fsp, cur, cnt)) return true;
         if (ray.masked || (ray.d.x == 0.0f && ray.d.y == 0.0f && ray.d.z == 0.0f)) {
             h.hit = false;
             continue;
@@ -1396,18 +2199,11 @@ __device__ __forceinline__ bool shade_until_trace(const DevScene& sc, const V3 L
     }
 }
 
-// shading of every result of queue q; next rays go to queue q^1, finished samples to P.samples.
-// BATCH: a slot whose path finished starts the batch's next work item in place.
-#ifndef RG_SHADE_MIN_BLOCKS
-#define RG_SHADE_MIN_BLOCKS 6  // 85 registers, a few spilled: 6 blocks of 128 per SM beat 4 unspilled
-#endif
-template <bool BATCH, bool GLOSSY = false>
-__global__ void __launch_bounds__(128, BATCH ? 1 : RG_SHADE_MIN_BLOCKS) k_wf_shade(const TraceParams P, int q) {
+// shading of every result of queue q of the batch loop; next rays go to queue q^1, finished samples to
+// P.samples, and a slot whose path finished starts the batch's next work item in place
+__global__ void __launch_bounds__(128) k_wf_shade(const TraceParams P, int q) {
     const WavefrontBuffers& wf = P.wf;
-    const V3 L = v3(P.ubo.lightDir[0], P.ubo.lightDir[1], P.ubo.lightDir[2]);
-    const int maxRec = P.ubo.maxRecursions;
-    const bool first = !BATCH && P.firstRound;
-    const uint32_t count = first ? frame_work_total(P) : *(volatile uint32_t*)(wf.counts + q);
+    const uint32_t count = *(volatile uint32_t*)(wf.counts + q);
     if (blockIdx.x == 0 && threadIdx.x == 0) wf.counts[2] = 0;  // the next trace kernel's work counter
     const unsigned lane = threadIdx.x & 31;
     RayCounts cnt = {0, 0, 0, 0};
@@ -1421,12 +2217,8 @@ __global__ void __launch_bounds__(128, BATCH ? 1 : RG_SHADE_MIN_BLOCKS) k_wf_sha
         Frame cur;
         RayReq ray;
         int fsp = 0;
-        bool live = i < count;
-        if (live && first) {  // the work item's camera ray and initial payload, as the trace kernel made them
-            live = frame_work_item(P, i, path, p, ray);
-            fsp = 0;
-            if (live) cnt.primary++;
-        } else if (live) {
+        const bool live = i < count;
+        if (live) {
             path = wf.qPath[q][i];
             const float4 o = wf.qO[q][i], d = wf.qD[q][i];
             const int2 meta = wf.meta[path];
@@ -1449,44 +2241,36 @@ __global__ void __launch_bounds__(128, BATCH ? 1 : RG_SHADE_MIN_BLOCKS) k_wf_sha
             h.v = ht.z;
             h.prim = __float_as_uint(ht.w);
             Frame* frames = framesBase + (size_t)path * kMaxFrames;
-            bool done;
-            if constexpr (BATCH) {
-                const JobDesc& J = P.jobs[P.slotJob[path]];
-                done = shade_until_trace<GLOSSY>(J.scene, v3(J.ubo.lightDir[0], J.ubo.lightDir[1], J.ubo.lightDir[2]), J.ubo.maxRecursions, h,
-                                                 p, ray, frames, fsp, cur, cnt);
-            } else {
-                done = shade_until_trace<GLOSSY>(P.scene, L, maxRec, h, p, ray, frames, fsp, cur, cnt);
-            }
-            if (done) {
-                store_sample(P.samples + 3 * (size_t)(BATCH ? P.slotSample[path] : path), p);
-                regen = BATCH;
+            const JobDesc& J = P.jobs[P.slotJob[path]];
+            if (shade_until_trace(J.scene, v3(J.ubo.lightDir[0], J.ubo.lightDir[1], J.ubo.lightDir[2]), J.ubo.maxRecursions, h, p, ray, frames,
+                                  fsp, cur, cnt)) {
+                store_sample(P.samples + 3 * (size_t)P.slotSample[path], p);
+                regen = true;
             } else {
                 emit = true;
             }
         }
-        if constexpr (BATCH) {
-            // path regeneration: finished slots take the next work items (one atomic per warp and try)
-            for (;;) {
-                const bool need = regen && !exhausted;
-                const unsigned needMask = __ballot_sync(0xFFFFFFFFu, need);
-                if (!needMask) break;
-                const int leader = __ffs(needMask) - 1;
-                uint32_t b0 = 0;
-                if ((int)lane == leader) b0 = atomicAdd(P.workCounter, (uint32_t)__popc(needMask));
-                b0 = __shfl_sync(0xFFFFFFFFu, b0, leader);
-                if (need) {
-                    const uint32_t id = b0 + (uint32_t)__popc(needMask & ((1u << lane) - 1u));
-                    uint32_t job = 0, si = 0;
-                    if (id >= P.totalWork) {
-                        exhausted = true;
-                    } else if (batch_primary(P, id, job, si, p, ray)) {
-                        P.slotJob[path] = job;
-                        P.slotSample[path] = si;
-                        fsp = 0;
-                        regen = false;
-                        emit = true;
-                        cnt.primary++;
-                    }
+        // path regeneration: finished slots take the next work items (one atomic per warp and try)
+        for (;;) {
+            const bool need = regen && !exhausted;
+            const unsigned needMask = __ballot_sync(0xFFFFFFFFu, need);
+            if (!needMask) break;
+            const int leader = __ffs(needMask) - 1;
+            uint32_t b0 = 0;
+            if ((int)lane == leader) b0 = atomicAdd(P.workCounter, (uint32_t)__popc(needMask));
+            b0 = __shfl_sync(0xFFFFFFFFu, b0, leader);
+            if (need) {
+                const uint32_t id = b0 + (uint32_t)__popc(needMask & ((1u << lane) - 1u));
+                uint32_t job = 0, si = 0;
+                if (id >= P.totalWork) {
+                    exhausted = true;
+                } else if (batch_primary(P, id, job, si, p, ray)) {
+                    P.slotJob[path] = job;
+                    P.slotSample[path] = si;
+                    fsp = 0;
+                    regen = false;
+                    emit = true;
+                    cnt.primary++;
                 }
             }
         }
@@ -1502,7 +2286,7 @@ __global__ void __launch_bounds__(128, BATCH ? 1 : RG_SHADE_MIN_BLOCKS) k_wf_sha
 }
 
 // the rest of one path, traced and shaded back to back
-template <bool GLOSSY, class STACK>
+template <class STACK>
 __device__ __forceinline__ void finish_path(const DevScene& sc, const V3 L, const int maxRec, RayReq& ray, Payload& p, Frame* frames,
                                             int& fsp, const STACK& stk, VisitCounts& vc, RayCounts& cnt, unsigned long long* counters) {
     Frame cur;
@@ -1511,19 +2295,16 @@ __device__ __forceinline__ void finish_path(const DevScene& sc, const V3 L, cons
         h.hit = false;
         if (!ray.masked)
             h = closest_hit<false>(sc, ray.o.x, ray.o.y, ray.o.z, ray.d.x, ray.d.y, ray.d.z, ray.tmin, ray.tmax, stk, vc, counters);
-        if (!shade_step<GLOSSY>(sc, L, maxRec, h, p, ray, frames, fsp, cur, cnt)) break;
+        if (!shade_step<false>(sc, L, maxRec, h, p, ray, frames, fsp, cur, cnt)) break;
     }
 }
 
-// Tail of the wavefront loop: once few paths remain, one launch finishes every remaining path --
-// each thread traces and shades its path's remaining sequence back to back -- instead of one
-// (trace, shade) launch pair per remaining round.  BATCH: only after the last work item was taken.
-template <bool BATCH, bool GLOSSY = false>
+// Tail of the batch loop: once few paths and no work items remain, one launch finishes every remaining
+// path -- each thread traces and shades its path's remaining sequence back to back -- instead of one
+// (trace, shade) launch pair per remaining round.
 __global__ void __launch_bounds__(kTraceThreads) k_wf_tail(const __grid_constant__ TraceParams P, int q) {
     RG_DECLARE_STACK(stk);
     const WavefrontBuffers& wf = P.wf;
-    const V3 L0 = v3(P.ubo.lightDir[0], P.ubo.lightDir[1], P.ubo.lightDir[2]);
-    const int maxRec0 = P.ubo.maxRecursions;
     const uint32_t count = *(volatile uint32_t*)(wf.counts + q);
     RayCounts cnt = {0, 0, 0, 0};
     VisitCounts vc = {0, 0, 0};
@@ -1543,14 +2324,10 @@ __global__ void __launch_bounds__(kTraceThreads) k_wf_tail(const __grid_constant
         Payload p;
         load_payload(wf.payload + 4 * (size_t)path, p);
         Frame* frames = framesBase + (size_t)path * kMaxFrames;
-        if constexpr (BATCH) {
-            const JobDesc& J = P.jobs[P.slotJob[path]];
-            finish_path<GLOSSY>(J.scene, v3(J.ubo.lightDir[0], J.ubo.lightDir[1], J.ubo.lightDir[2]), J.ubo.maxRecursions, ray, p, frames, fsp,
-                        stk, vc, cnt, P.counters);
-        } else {
-            finish_path<GLOSSY>(P.scene, L0, maxRec0, ray, p, frames, fsp, stk, vc, cnt, P.counters);
-        }
-        store_sample(P.samples + 3 * (size_t)(BATCH ? P.slotSample[path] : path), p);
+        const JobDesc& J = P.jobs[P.slotJob[path]];
+        finish_path(J.scene, v3(J.ubo.lightDir[0], J.ubo.lightDir[1], J.ubo.lightDir[2]), J.ubo.maxRecursions, ray, p, frames, fsp, stk, vc, cnt,
+                    P.counters);
+        store_sample(P.samples + 3 * (size_t)P.slotSample[path], p);
     }
     unsigned long long c[6] = {cnt.shadow, cnt.secondary, cnt.masked, vc.nodes, vc.tris, vc.overflow};
     const int slot[6] = {1, 2, 3, 4, 5, 6};
@@ -1744,10 +2521,10 @@ typedef void (*TraceKernel)(const TraceParams, int);
 
 // the traversal kernel of one launch shape
 static TraceKernel trace_kernel(bool batch, bool count, int threads, int depth) {
-    if (count) return batch ? k_wf_trace<true, true, kTraceThreads, kTraversalStack> : k_wf_trace<true, false, kTraceThreads, kTraversalStack>;
-    if (!batch) return k_wf_trace<false, false, kTraceThreads, kTraversalStack>;
+    if (count) return batch ? k_wf_trace<true, kFormBatch, kTraceThreads, kTraversalStack> : k_wf_trace<true, kFormTree, kTraceThreads, kTraversalStack>;
+    if (!batch) return k_wf_trace<false, kFormTree, kTraceThreads, kTraversalStack>;
 #define RG_TK(T, D) \
-    if (threads == T && depth == D) return k_wf_trace<false, true, T, D>;
+    if (threads == T && depth == D) return k_wf_trace<false, kFormBatch, T, D>;
     RG_TK(64, 16) RG_TK(64, 24) RG_TK(64, 32) RG_TK(64, 48)
     RG_TK(128, 16) RG_TK(128, 24) RG_TK(128, 32) RG_TK(128, 48)
     RG_TK(256, 16) RG_TK(256, 24) RG_TK(256, 32)  // 256 x 48 exceeds the 48 KB of static shared memory
@@ -1761,12 +2538,12 @@ bool tune_supported(const TraceTune& t) {
 
 // the query form of the traversal kernel for a stack depth (visit counting: the default depth only)
 static TraceKernel query_kernel(bool count, int depth) {
-    if (count) return k_wf_trace<true, false, kTraceThreads, kTraversalStack, true>;
+    if (count) return k_wf_trace<true, kFormQuery, kTraceThreads, kTraversalStack>;
     switch (depth) {
-        case 16: return k_wf_trace<false, false, kTraceThreads, 16, true>;
-        case 24: return k_wf_trace<false, false, kTraceThreads, 24, true>;
-        case 32: return k_wf_trace<false, false, kTraceThreads, 32, true>;
-        case 48: return k_wf_trace<false, false, kTraceThreads, 48, true>;
+        case 16: return k_wf_trace<false, kFormQuery, kTraceThreads, 16>;
+        case 24: return k_wf_trace<false, kFormQuery, kTraceThreads, 24>;
+        case 32: return k_wf_trace<false, kFormQuery, kTraceThreads, 32>;
+        case 48: return k_wf_trace<false, kFormQuery, kTraceThreads, 48>;
         default: return nullptr;
     }
 }
@@ -1795,53 +2572,73 @@ cudaError_t launch_trace_queue(const TraceParams& p, const float* rays, uint32_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_trace_wavefront(const TraceParams& p, cudaStream_t s, uint32_t* hostCount, int* iterations,
-                                   EventPairFn kernelEvents, void* user) {
-    const int c = p.countVisits ? 1 : 0;
-    const TraceKernel trace = trace_kernel(false, c, kTraceThreads, kTraversalStack);
-    const int gTrace = grid_of((const void*)trace, kTraceThreads);
+cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, uint32_t* hostWords, int* iterations, bool* poolFull,
+                              EventPairFn kernelEvents, void* user) {
+    TraceParams p = p0;
+    p.wf.counts = p.tree.ctl + kTreeFetch - 2;  // the traversal kernel's work counter, overflow list length and finished blocks
+    p.wf.overflow = p.tree.overflow;
+    const TraceKernel trace = trace_kernel(false, p.countVisits != 0, kTraceThreads, kTraversalStack);
     // glossy reference shading has kernels of its own; the reference's shading keeps the lean ones
-    typedef void (*WfKernel)(const TraceParams, int);
-    const WfKernel shade = p.glossySeed ? k_wf_shade<false, true> : k_wf_shade<false, false>;
-    const WfKernel tail = p.glossySeed ? k_wf_tail<false, true> : k_wf_tail<false, false>;
-    const int gShade = grid_of((const void*)shade, 128);
-    const int gTail = grid_of((const void*)tail, kTraceThreads);
-    if (!gTrace || !gShade || !gTail) return cudaErrorUnknown;
-    cudaError_t e = cudaMemsetAsync(p.wf.counts, 0, 4 * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    // the first round generates the camera rays itself (no raygen queue)
-    TraceParams p1 = p;
-    p1.firstRound = 1;
-    // the pending-ray count below which the remaining paths finish in one k_wf_tail launch; the
-    // visit-counting build stays in the round loop (the tail kernel does not count visits)
-    const uint32_t tailBelow = c ? 0u : (uint32_t)RG_TAIL_RAYS;
-    int q = 0, it = 0;
-    const int kChunk = RG_POLL_ROUNDS, kMaxIterations = 100000;
-    for (;;) {
-        for (int k = 0; k < kChunk; ++k, ++it) {
-            cudaEvent_t e0 = nullptr, e1 = nullptr;
-            if (kernelEvents && !kernelEvents(user, &e0, &e1)) e0 = e1 = nullptr;
-            if (e0) cudaEventRecord(e0, s);
-            trace<<<gTrace, kTraceThreads, 0, s>>>(it == 0 ? p1 : p, q);
-            if (e1) cudaEventRecord(e1, s);
-            shade<<<gShade, 128, 0, s>>>(it == 0 ? p1 : p, q);
-            count_launch(2);
-            q ^= 1;
-        }
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(hostCount, p.wf.counts + q, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
-        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-        if (*hostCount == 0) break;
-        if (*hostCount < tailBelow) {
-            cudaEvent_t e0 = nullptr, e1 = nullptr;
-            if (kernelEvents && !kernelEvents(user, &e0, &e1)) e0 = e1 = nullptr;
-            if (e0) cudaEventRecord(e0, s);
-            tail<<<gTail, kTraceThreads, 0, s>>>(p, q);
-            if (e1) cudaEventRecord(e1, s);
+    const auto expand = p.glossySeed ? k_tree_expand<false, true> : k_tree_expand<false, false>;
+    const auto check = p.glossySeed ? k_tree_check<false, true> : k_tree_check<false, false>;
+    const int gTrace = grid_of((const void*)trace, kTraceThreads), gExpand = grid_of((const void*)expand, 128),
+              gCheck = grid_of((const void*)check, 128), gCompose = grid_of((const void*)k_tree_compose<false>, 128);
+    if (!gTrace || !gExpand || !gCheck || !gCompose) return cudaErrorUnknown;
+    const int maxRec = p.ubo.maxRecursions;
+    const uint32_t work = (uint32_t)frame_work_items(p.W, p.H, (uint32_t)p.ubo.numSamples), cap = p.tree.capacity;
+    cudaError_t e;
+    int it = 0;
+    *poolFull = false;
+    // chunks of samples (first work item, samples) whose trees share the node pool; a chunk that fills it
+    // goes again in eight parts (one sample's tree, replaced rays included, is far smaller than any pool)
+    std::vector<std::pair<uint32_t, uint32_t>> todo;
+    auto split = [&](uint32_t base, uint32_t n, uint32_t m) {
+        for (uint32_t b = (n - 1) / m * m + m; b; b -= m) todo.emplace_back(base + b - m, std::min(m, n - (b - m)));  // popped in order
+    };
+    split(0, work, std::max(1u, std::min(work, cap / kTreeNodesMin)));
+    while (!todo.empty()) {
+        p.treeBase = todo.back().first;
+        p.treeRoots = todo.back().second;
+        todo.pop_back();
+        p.treeCand = 0;
+        if ((e = cudaMemsetAsync(p.tree.ctl, 0, kTreeBounds * sizeof(uint32_t), s)) != cudaSuccess) return e;
+        int k = 0, levels = maxRec + 1;
+        bool full = false;
+        for (;;) {
+            for (int l = 0; l < levels; ++l, ++k, ++it) {
+                p.firstRound = k == 0;
+                cudaEvent_t e0 = nullptr, e1 = nullptr;
+                if (kernelEvents && !kernelEvents(user, &e0, &e1)) e0 = e1 = nullptr;
+                if (e0) cudaEventRecord(e0, s);
+                trace<<<gTrace, kTraceThreads, 0, s>>>(p, k);
+                if (e1) cudaEventRecord(e1, s);
+                expand<<<gExpand, 128, 0, s>>>(p, k);
+                count_launch(2);
+            }
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            if (maxRec == 0) break;  // no hit issues a ray
+            check<<<gCheck, 128, 0, s>>>(p, k);
             count_launch();
-            break;
+            if ((e = cudaMemcpyAsync(hostWords, p.tree.ctl, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+            if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+            full = p.treeRoots + hostWords[kTreeAlloc] > cap;
+            const bool pending = p.treeRoots + hostWords[kTreeAlloc] > hostWords[kTreeTraced];
+            if (full || (!pending && !hostWords[kTreeChanges])) break;
+            // from the shallowest new ray down
+            levels = pending && hostWords[kTreeLevels] ? std::max(1, maxRec + 1 - (16 - (int)hostWords[kTreeLevels])) : 1;
+            if (k + levels >= kTreeMaxRounds) return cudaErrorUnknown;
+            p.treeCand ^= 1u;
         }
-        if (it >= kMaxIterations) return cudaErrorLaunchTimeout;
+        if (full) {
+            *poolFull = true;
+            if (p.treeRoots == 1) return cudaErrorUnknown;
+            split(p.treeBase, p.treeRoots, (p.treeRoots + 7) / 8);
+            continue;
+        }
+        while (k--) {
+            k_tree_compose<false><<<gCompose, 128, 0, s>>>(p, k);
+            count_launch();
+        }
     }
     if (iterations) *iterations = it;
     dim3 grid((p.W + 31) / 32, (p.H + 7) / 8);
@@ -1873,9 +2670,9 @@ cudaError_t launch_trace_batch(const TraceParams& p0, const TraceTune& tune, con
     const TraceKernel trace = trace_kernel(true, c, threads, c ? kTraversalStack : tune.depth);
     if (!trace || !tune_supported(tune)) return cudaErrorInvalidValue;
     const int gTrace = grid_of((const void*)trace, threads);
-    const int gShade = grid_of((const void*)k_wf_shade<true>, 128);
+    const int gShade = grid_of((const void*)k_wf_shade, 128);
     const int gRaygen = grid_of((const void*)k_wfb_raygen, 256);
-    const int gTail = grid_of((const void*)k_wf_tail<true>, kTraceThreads);
+    const int gTail = grid_of((const void*)k_wf_tail, kTraceThreads);
     const int gSort = grid_of((const void*)k_sort_scatter<RG_SORT_MORTON>, 256);
     if (!gTrace || !gShade || !gRaygen || !gTail || !gSort) return cudaErrorUnknown;
     const bool sorted = tune.sortKey != RG_SORT_NONE;
@@ -1896,7 +2693,7 @@ cudaError_t launch_trace_batch(const TraceParams& p0, const TraceTune& tune, con
             if (e0) cudaEventRecord(e0, s);
             trace<<<gTrace, threads, 0, s>>>(p, q);
             if (e1) cudaEventRecord(e1, s);
-            k_wf_shade<true><<<gShade, 128, 0, s>>>(p, q);
+            k_wf_shade<<<gShade, 128, 0, s>>>(p, q);
             count_launch(2);
             q ^= 1;
         }
@@ -1909,7 +2706,7 @@ cudaError_t launch_trace_batch(const TraceParams& p0, const TraceTune& tune, con
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             if (kernelEvents && !kernelEvents(user, &e0, &e1)) e0 = e1 = nullptr;
             if (e0) cudaEventRecord(e0, s);
-            k_wf_tail<true><<<gTail, kTraceThreads, 0, s>>>(p, q);
+            k_wf_tail<<<gTail, kTraceThreads, 0, s>>>(p, q);
             if (e1) cudaEventRecord(e1, s);
             count_launch();
             break;
@@ -1948,9 +2745,9 @@ cudaError_t capture_trace_batch(const TraceParams& p0, const TraceTune& tune, co
     const TraceKernel trace = trace_kernel(true, false, tune.threads, tune.depth);
     if (!trace || !tune_supported(tune)) return cudaErrorInvalidValue;
     const int gTrace = grid_of((const void*)trace, tune.threads);
-    const int gShade = grid_of((const void*)k_wf_shade<true>, 128);
+    const int gShade = grid_of((const void*)k_wf_shade, 128);
     const int gRaygen = grid_of((const void*)k_wfb_raygen, 256);
-    const int gTail = grid_of((const void*)k_wf_tail<true>, kTraceThreads);
+    const int gTail = grid_of((const void*)k_wf_tail, kTraceThreads);
     const int gSort = grid_of((const void*)k_sort_scatter<RG_SORT_MORTON>, 256);
     if (!gTrace || !gShade || !gRaygen || !gTail || !gSort) return cudaErrorUnknown;
     const bool sorted = tune.sortKey != RG_SORT_NONE;
@@ -1980,7 +2777,7 @@ cudaError_t capture_trace_batch(const TraceParams& p0, const TraceTune& tune, co
     for (int q = 0; q < 2; ++q) {
         if (sorted) enqueue_sort(p, tune.sortKey, sort, gSort, q, s2);
         trace<<<gTrace, tune.threads, 0, s2>>>(p, q);
-        k_wf_shade<true><<<gShade, 128, 0, s2>>>(p, q);
+        k_wf_shade<<<gShade, 128, 0, s2>>>(p, q);
     }
     // body runs before the loop stops with its limit flag set (RG_BATCH_LOOP_LIMIT overrides, read
     // when the graph is captured; tests use a small limit to check the reported error)
@@ -1992,7 +2789,7 @@ cudaError_t capture_trace_batch(const TraceParams& p0, const TraceTune& tune, co
     if (e != cudaSuccess) return e;
     if ((e = cudaStreamUpdateCaptureDependencies(s, &node, nullptr, 1, cudaStreamSetCaptureDependencies)) != cudaSuccess) return e;
     // after an even number of rounds the pending rays are in queue 0
-    k_wf_tail<true><<<gTail, kTraceThreads, 0, s>>>(p, 0);
+    k_wf_tail<<<gTail, kTraceThreads, 0, s>>>(p, 0);
     return cudaGetLastError();
 }
 
