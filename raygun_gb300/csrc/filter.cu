@@ -76,51 +76,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// 16 consecutive FP32 columns of this thread's TMEM lane, without waiting (tmem_wait_ld before use)
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* r) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ uint4 add_bf16x8(uint4 a, uint4 b) {
-    const bf16* x = reinterpret_cast<const bf16*>(&a);
-    const bf16* y = reinterpret_cast<const bf16*>(&b);
-    uint4 o;
-    bf16* z = reinterpret_cast<bf16*>(&o);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) z[j] = __float2bfloat16(__bfloat162float(x[j]) + __bfloat162float(y[j]));
-    return o;
-}
-
-constexpr int kTileRows = 2, kTilePx = 128, kPatchRows = kTileRows + 2, kPatchW = kTilePx + 2;
-constexpr int kPatchPlane = kPatchRows * kPatchW * 16;  // bytes of one channel-chunk plane of the patch
-
-// stages the (kTileRows + 2) x 130 input patch of tile (b, y0, x0) as [chunk][pixel][8]; x2 (nullable)
-// is added element-wise; outside the image reads zero
-template <int CIN>
-__device__ __forceinline__ void load_patch(uint8_t* patch, const bf16* __restrict__ x, const bf16* __restrict__ x2, int b, int y0,
-                                           int x0, int H, int W) {
-    constexpr int CC = CIN / 8, NP = kPatchRows * kPatchW;
-    for (int i = threadIdx.x; i < CC * NP; i += blockDim.x) {
-        const int pix = i % NP, cc = i / NP;
-        const int gy = y0 - 1 + pix / kPatchW, gx = x0 - 1 + pix % kPatchW;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (gy >= 0 && gy < H && gx >= 0 && gx < W) {
-            const size_t off = (((size_t)b * H + gy) * W + gx) * CIN + cc * 8;
-            v = *reinterpret_cast<const uint4*>(x + off);
-            if (x2) v = add_bf16x8(v, *reinterpret_cast<const uint4*>(x2 + off));
-        }
-        *reinterpret_cast<uint4*>(patch + (size_t)cc * kPatchPlane + (size_t)pix * 16) = v;
-    }
-}
-
-}  // namespace
-
-namespace {
 
 // Row-streaming convolution.  A work item is a strip of 128 output pixels x a segment of rows of
 // one image; a CTA walks its items down the rows, three output rows (a group) at a time.  Input rows
@@ -466,97 +422,190 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
     if (warp == 1) tmem_dealloc(tmem, S::kCols);
 }
 
-// ---- weight gradient: dW[co][tap][ci] = sum_p g[p][co] * x[p + tap][ci] ----------------------------
-// D (M = 128 rows: output channels, padded with zero planes) x (N = CIN per tap) over K = pixels.  Both
-// operands MN-major: A = g tile [co chunk][pixel][8], B = the shifted input patch [ci chunk][pixel][8].
-// Each CTA accumulates its tiles for a group of taps in TMEM, then writes its partial sums.
+// ---- weight and bias gradients: dW[co][tap][ci] = sum_p g[p][co] * x[p + tap][ci], db[co] = sum_p g[p][co]
+// D (M = 128 rows: output channels) x (N = CIN per tap) over K = pixels, both operands MN-major: A = a
+// row of g as channel-chunk planes [chunk][pixel][8], B = a row of x in the same layout at the tap's
+// pixel offset.  The bias sum is one more product, with a tile of ones as B.
+// A CTA takes an equal run of the (image, strip of 128 pixels, row) list, so all CTAs end together, and
+// streams it: each row of g once, each row of x once (plus two rows where a run starts or enters the next
+// strip), through rings of shared-memory slots filled by TMA, while one thread issues a row's 72 MMAs
+// (M = 128, N = CIN, K = 16) with constant descriptor offsets; everything accumulates in tensor memory.
+// Rows of A beyond COUT read whatever lies behind the slot; their results are not read.  64 input
+// channels take two tap groups (9 x 64 columns exceed the 512 of an SM).
+// Bound: the copies' 16-byte rows (CIN / 8 x 130 + COUT / 8 x 128 of them per image row) and the MMA
+// issue, about one of either per clock at CIN = COUT = 64.  32 crops of 128 x 128, 64 -> 64: 410 us with
+// one tile staged, multiplied and waited for at a time by one warp quartet; 141 us now, bias sum (113 us
+// in a kernel of its own) included.
 template <int CIN, int COUT>
 struct DwShape {
-    static constexpr int kTaps = CIN == 64 ? 5 : 9;          // taps per CTA (two tap groups for 64 channels)
+    static constexpr int kTaps = CIN == 64 ? 5 : 9;  // taps per CTA
     static constexpr int kGroups = CIN == 64 ? 2 : 1;
-    static constexpr int kGPlane = kTileRows * kTilePx * 16;  // bytes of one chunk plane of the g tile
-    static constexpr int kGBytes = 16 * kGPlane;              // 16 planes = 128 rows of A
-    static constexpr int kPatchBytes = (CIN / 8) * kPatchPlane;
-    // at least 120 KB so that one CTA holds an SM (and all 512 TMEM columns) at a time
-    static constexpr int kSmem = kGBytes + kPatchBytes + 1024 > 120 * 1024 ? kGBytes + kPatchBytes + 1024 : 120 * 1024;
-    static constexpr uint32_t kCols = 512;
-    static_assert(kTaps * CIN <= 512, "TMEM columns");
+    static constexpr int kGPlane = kStripPx * 16, kGBytes = (COUT / 8) * kGPlane, kXBytes = (CIN / 8) * kRowPlane;
+    static constexpr int kGRing = 4, kXRing = 6;
+    static constexpr uint32_t kGTx = kGBytes, kXTx = (CIN / 8) * kRowW * 16;
+    static constexpr int kOnes = 2 * 256;  // B tile of ones: [2 chunks][16 pixels][8]
+    static constexpr int kUsed = kGRing * kGBytes + kXRing * kXBytes + kOnes;
+    static constexpr int kReach = (kGRing - 1) * kGBytes + 16 * kGPlane;  // A's 128 rows from the last slot
+    // at least 120 KB: one CTA holds an SM (and its tensor memory) at a time
+    static constexpr int kSmem = (kUsed > kReach ? kUsed : kReach) + 1024 > 120 * 1024 ? (kUsed > kReach ? kUsed : kReach) + 1024 : 120 * 1024;
+    static constexpr uint32_t kCols = kTaps * CIN + 16 <= 256 ? 256 : 512;
+    static_assert(kTaps * CIN + 16 <= 512 && kGBytes % 128 == 0 && kXBytes % 128 == 0, "shape");
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(128, 1) k_filter_dw(const bf16* __restrict__ x, const bf16* __restrict__ x2, const bf16* __restrict__ g,
-                                                      int B, int H, int W, float* __restrict__ partial, int* status) {
+__global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapG, int B,
+                                                      int H, int W, float* __restrict__ partial, float* __restrict__ biasPartial, int* status) {
     using S = DwShape<CIN, COUT>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* gsm = smem;
-    uint8_t* patch = smem + S::kGBytes;
+    uint8_t *gring = smem, *xring = smem + S::kGRing * S::kGBytes, *ones = xring + S::kXRing * S::kXBytes;
     __shared__ uint32_t tmem_base;
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t xFull[S::kXRing], xEmpty[S::kXRing], gFull[S::kGRing], gEmpty[S::kGRing], drain;
+    __shared__ int abortFlag, issuedX, issuedG, consumedX, consumedG;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tap0 = blockIdx.y * S::kTaps, ntaps = min(S::kTaps, 9 - tap0);
-    for (int i = tid; i < S::kGBytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(gsm)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid == 0) mbar_init(&mbar, 1);
+    const int tap0 = S::kGroups == 1 ? 0 : blockIdx.y * S::kTaps;
+    for (int i = tid; i < S::kOnes / 2; i += blockDim.x) reinterpret_cast<bf16*>(ones)[i] = __float2bfloat16(1.0f);
+    if (tid == 0) {
+        for (int k = 0; k < S::kXRing; ++k) {
+            mbar_init(&xFull[k], 1);
+            mbar_init(&xEmpty[k], 1);
+        }
+        for (int k = 0; k < S::kGRing; ++k) {
+            mbar_init(&gFull[k], 1);
+            mbar_init(&gEmpty[k], 1);
+        }
+        mbar_init(&drain, 1);
+        abortFlag = 0;
+        issuedX = issuedG = consumedX = consumedG = 0;
+        mbar_init_fence();
+    }
+    async_proxy_fence();  // the ones are read by the tensor core
     if (warp == 0) tmem_alloc(&tmem_base, S::kCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
-    const int tilesX = (W + kTilePx - 1) / kTilePx, tilesY = (H + kTileRows - 1) / kTileRows;
-    const int tiles = B * tilesY * tilesX;
-    constexpr uint32_t idesc = umma_idesc(128, CIN, true, true);
-    uint32_t phase = 0;
-    bool ok = true, first = true;
-    for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const int b = t / (tilesY * tilesX), rem = t % (tilesY * tilesX);
-        const int y0 = (rem / tilesX) * kTileRows, x0 = (rem % tilesX) * kTilePx;
-        load_patch<CIN>(patch, x, x2, b, y0, x0, H, W);
-        for (int i = tid; i < (COUT / 8) * kTileRows * kTilePx; i += blockDim.x) {  // g tile, zero outside the image
-            const int pix = i % (kTileRows * kTilePx), cc = i / (kTileRows * kTilePx);
-            const int gy = y0 + pix / kTilePx, gx = x0 + pix % kTilePx;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (gy < H && gx < W) v = *reinterpret_cast<const uint4*>(g + (((size_t)b * H + gy) * W + gx) * COUT + cc * 8);
-            *reinterpret_cast<uint4*>(gsm + (size_t)cc * S::kGPlane + (size_t)pix * 16) = v;
-        }
-        async_proxy_fence();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t pbase = smem_u32(patch), gbase = smem_u32(gsm);
+    volatile int* abort = &abortFlag;
+    const int strips = (W + kStripPx - 1) / kStripPx;
+    const long long rows = (long long)B * strips * H, r0 = rows * blockIdx.x / gridDim.x, r1 = rows * (blockIdx.x + 1) / gridDim.x;
+    // the run of rows from r on that lie in one strip of one image: its image, first pixel, first row, length
+    auto run_at = [&](long long r, int& b, int& x0, int& y0) {
+        const long long bs = r / H;
+        b = (int)(bs / strips);
+        x0 = (int)(bs % strips) * kStripPx;
+        y0 = (int)(r % H);
+        return (int)min((long long)(H - y0), r1 - r);
+    };
+    if (warp == 0) {
+        if (lane == 0) {  // copies: x rows y0 - 1 .. y0 + n, g rows y0 .. y0 + n - 1 of each run
+            int sx = 0, sg = 0;
+            bool ok = true;
+            for (long long r = r0; r < r1 && ok;) {
+                int b, x0, y0;
+                const int n = run_at(r, b, x0, y0);
+                for (int k = 0; k < n + 2 && ok; ++k) {
+                    const int xs = sx % S::kXRing;
+                    ok = sx < S::kXRing || mbar_wait_or_abort(&xEmpty[xs], (uint32_t)((sx / S::kXRing - 1) & 1), abort, status);
+                    if (!ok) break;
+                    mbar_expect_tx(&xFull[xs], S::kXTx);
 #pragma unroll 1
-            for (int j = 0; j < ntaps; ++j) {
-                const int tap = tap0 + j, dy = tap / 3, dx = tap % 3;
+                    for (int cc = 0; cc < CIN / 8; ++cc)
+                        tma_load_4d(xring + xs * S::kXBytes + cc * kRowPlane, &mapX, cc * 8, x0 - 1, y0 - 1 + k, b, &xFull[xs]);
+                    issuedX = ++sx;
+                    if (k >= n) continue;
+                    const int gs = sg % S::kGRing;
+                    ok = sg < S::kGRing || mbar_wait_or_abort(&gEmpty[gs], (uint32_t)((sg / S::kGRing - 1) & 1), abort, status);
+                    if (!ok) break;
+                    mbar_expect_tx(&gFull[gs], S::kGTx);
 #pragma unroll 1
-                for (int r = 0; r < kTileRows; ++r)
-#pragma unroll 1
-                    for (int kk = 0; kk < kTilePx / 16; ++kk) {
-                        const uint64_t ad = umma_desc(gbase + (uint32_t)((r * kTilePx + 16 * kk) * 16), 128, S::kGPlane);
-                        const uint64_t bd = umma_desc(pbase + (uint32_t)(((r + dy) * kPatchW + 16 * kk + dx) * 16), 128, kPatchPlane);
-                        umma(tmem + (uint32_t)(j * CIN), ad, bd, idesc, (first && r == 0 && kk == 0) ? 0u : 1u);
-                    }
+                    for (int cc = 0; cc < COUT / 8; ++cc)
+                        tma_load_4d(gring + gs * S::kGBytes + cc * S::kGPlane, &mapG, cc * 8, x0, y0 + k, b, &gFull[gs]);
+                    issuedG = ++sg;
+                }
+                r += n;
             }
-            umma_commit(&mbar);
         }
-        first = false;
-        ok = __syncthreads_and(mbar_wait(&mbar, phase, status, 1u << 24, 3)) != 0;  // also: the next tile overwrites the operands
-        phase ^= 1u;
-        tc_fence_after();
+    } else if (warp == 1) {
+        if (lane == 0) {  // MMA issuer: output row j of a run takes x rows j, j + 1, j + 2 of the run
+            const uint64_t a0 = umma_desc(smem_u32(gring), 128, S::kGPlane), b0 = umma_desc(smem_u32(xring), 128, kRowPlane),
+                           one = umma_desc(smem_u32(ones), 128, 256);
+            constexpr uint32_t id = umma_idesc(128, CIN, true, true), idOne = umma_idesc(128, 16, true, true);
+            int sx = 0, sg = 0, seen = 0;  // first x row of the run, g row, x rows waited for
+            uint32_t acc = 0;
+            bool ok = true;
+            for (long long r = r0; r < r1 && ok;) {
+                int b, x0, y0;
+                const int n = run_at(r, b, x0, y0);
+                for (int j = 0; j < n && ok; ++j, ++sg) {
+                    for (; seen < sx + j + 3 && ok; ++seen)
+                        ok = mbar_wait_or_abort(&xFull[seen % S::kXRing], (uint32_t)((seen / S::kXRing) & 1), abort, status);
+                    consumedX = seen;
+                    ok = ok && mbar_wait_or_abort(&gFull[sg % S::kGRing], (uint32_t)((sg / S::kGRing) & 1), abort, status);
+                    if (!ok) break;
+                    consumedG = sg + 1;
+                    tc_fence_after();
+                    const uint64_t ad = a0 + (uint64_t)(((sg % S::kGRing) * S::kGBytes) >> 4);
+                    uint64_t bd[3];
+#pragma unroll
+                    for (int dy = 0; dy < 3; ++dy) bd[dy] = b0 + (uint64_t)((((sx + j + dy) % S::kXRing) * S::kXBytes) >> 4);
+#pragma unroll
+                    for (int t = 0; t < S::kTaps; ++t) {
+                        const int tap = tap0 + t;
+                        if (S::kGroups > 1 && tap >= 9) break;
+                        const int dy = tap / 3, dx = tap - 3 * dy;
+                        const uint64_t bt = (dy == 0 ? bd[0] : dy == 1 ? bd[1] : bd[2]) + (uint64_t)dx;
+#pragma unroll
+                        for (int kk = 0; kk < kStripPx / 16; ++kk)
+                            umma(tmem + (uint32_t)(t * CIN), ad + (uint64_t)(16 * kk), bt + (uint64_t)(16 * kk), id, kk == 0 ? acc : 1u);
+                    }
+                    if (tap0 == 0)
+#pragma unroll
+                        for (int kk = 0; kk < kStripPx / 16; ++kk)
+                            umma(tmem + (uint32_t)(S::kTaps * CIN), ad + (uint64_t)(16 * kk), one, idOne, kk == 0 ? acc : 1u);
+                    acc = 1u;
+                    umma_commit(&gEmpty[sg % S::kGRing]);
+                    umma_commit(&xEmpty[(sx + j) % S::kXRing]);
+                    if (j == n - 1) {
+                        umma_commit(&xEmpty[(sx + n) % S::kXRing]);
+                        umma_commit(&xEmpty[(sx + n + 1) % S::kXRing]);
+                    }
+                }
+                sx += n + 2;
+                r += n;
+            }
+            umma_commit(&drain);  // completes when every MMA issued above has
+            mbar_wait(&drain, 0u, nullptr);
+        }
     }
-    // partial[blockIdx.x][co][tap][ci] for this CTA's taps (zero when it had no tile)
+    __syncthreads();
+    // an abandoned pipeline may still have copies in flight: wait for them (bounded) before the shared
+    // memory goes away
+    if (tid == 0 && abortFlag) {
+        for (int k = consumedX; k < issuedX; ++k) mbar_wait(&xFull[k % S::kXRing], (uint32_t)((k / S::kXRing) & 1), nullptr);
+        for (int k = consumedG; k < issuedG; ++k) mbar_wait(&gFull[k % S::kGRing], (uint32_t)((k / S::kGRing) & 1), nullptr);
+    }
+    __syncthreads();
+    tc_fence_after();
+    // partial[blockIdx.x][co][tap][ci] for this CTA's taps (zero when it had no row)
     const int co = warp * 32 + lane;
+    const bool some = r1 > r0 && !abortFlag;
     float* out = partial + (size_t)blockIdx.x * COUT * 9 * CIN;
     if (warp * 32 < COUT) {
+        const uint32_t row = tmem + ((uint32_t)(warp * 32) << 16);
+        float v[16];
 #pragma unroll 1
-        for (int j = 0; j < ntaps; ++j)
+        for (int t = 0; t < S::kTaps && tap0 + t < 9; ++t)
 #pragma unroll 1
             for (int c0 = 0; c0 < CIN; c0 += 16) {
-                float v[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * CIN + c0), v);
+                tmem_ld16(row + (uint32_t)(t * CIN + c0), v);
                 if (co < COUT)
 #pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        out[((size_t)co * 9 + tap0 + j) * CIN + c0 + q] = (ok && !first) ? v[q] : 0.0f;
+                    for (int q = 0; q < 16; ++q) out[((size_t)co * 9 + tap0 + t) * CIN + c0 + q] = some ? v[q] : 0.0f;
             }
+        if (tap0 == 0) {
+            tmem_ld16(row + (uint32_t)(S::kTaps * CIN), v);
+            if (co < COUT) biasPartial[(size_t)blockIdx.x * COUT + co] = some ? v[0] : 0.0f;
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -584,39 +633,47 @@ __global__ void k_filter_pack(const float* __restrict__ W, int coutReal, int cin
     }
 }
 
-// dW (param layout [co][ci][3][3], real sizes) = sum over CTAs of the partials [cta][co][tap][ci]
-__global__ void k_filter_dw_reduce(const float* __restrict__ partial, int ctas, int cout, int cin, int coutReal, int cinReal,
-                                   float* __restrict__ dW) {
-    const int n = coutReal * cinReal * 9;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int tap = i % 9, ci = (i / 9) % cinReal, co = i / (9 * cinReal);
-        float s = 0.0f;
-        for (int c = 0; c < ctas; ++c) s += partial[(((size_t)c * cout + co) * 9 + tap) * cin + ci];
-        dW[i] = s;
-    }
-}
-
-// per-block channel sums of g [P][C] -> partial[block][C] (C divides 256)
-__global__ void __launch_bounds__(256) k_filter_bias_partial(const bf16* __restrict__ g, size_t P, int C, float* __restrict__ partial) {
-    __shared__ float acc[256];
-    const int c = threadIdx.x % C, rowsPer = 256 / C, r0 = threadIdx.x / C;
+// The end of a training step, all layers in one launch: gradients = sums of the CTAs' partials, Adam
+// (Kingma & Ba 2015) on the FP32 master parameters, and the packed BF16 weights of the new parameters.
+// A block takes 64 parameters, in the partials' order so that its loads are whole sectors; four threads
+// sum a quarter of the CTAs each (in a fixed order: a step is deterministic).  lr = 0: gradients only.
+// The five reductions of 152 partials took 244 us one thread a parameter; all of this takes 17 us.
+__global__ void __launch_bounds__(256) k_filter_finish(const FilterFinish f) {
+    __shared__ float part[4][64];
+    const int j = threadIdx.x & 63, q = threadIdx.x >> 6;
+    int l = 0;
+    while (l + 1 < 5 && (int)blockIdx.x >= f.layer[l + 1].block0) ++l;
+    const FilterFinish::Layer& L = f.layer[l];
+    const int nW = L.coutReal * 9 * L.cinReal, i = ((int)blockIdx.x - L.block0) * 64 + j;
+    const bool weight = i < nW, valid = i < nW + L.coutReal;
+    const int ci = weight ? i % L.cinReal : 0, tap = weight ? i / L.cinReal % 9 : 0, co = weight ? i / (9 * L.cinReal) : i - nW;
     float s = 0.0f;
-    for (size_t p = (size_t)blockIdx.x * rowsPer + r0; p < P; p += (size_t)gridDim.x * rowsPer) s += __bfloat162float(g[p * C + c]);
-    acc[threadIdx.x] = s;
+    if (valid) {
+        const size_t stride = weight ? (size_t)L.cout * 9 * L.cin : (size_t)L.cout;
+        const float* p = weight ? L.partial + ((size_t)co * 9 + tap) * L.cin + ci : L.biasPartial + co;
+#pragma unroll 8
+        for (int c = q; c < L.ctas; c += 4) s += p[stride * c];
+    }
+    part[q][j] = s;
     __syncthreads();
-    if (threadIdx.x < C) {
-        float t = 0.0f;
-        for (int k = 0; k < rowsPer; ++k) t += acc[k * C + threadIdx.x];
-        partial[(size_t)blockIdx.x * C + threadIdx.x] = t;
+    if (q || !valid) return;
+    const float gi = (part[0][j] + part[1][j]) + (part[2][j] + part[3][j]);
+    const int k = weight ? L.offW + (co * L.cinReal + ci) * 9 + tap : L.offB + co;
+    f.grad[k] = gi;
+    if (!(f.lr > 0.0f)) return;
+    const float mi = f.b1 * f.m[k] + (1.0f - f.b1) * gi, vi = f.b2 * f.v[k] + (1.0f - f.b2) * gi * gi;
+    f.m[k] = mi;
+    f.v[k] = vi;
+    const float w = f.w[k] - f.lr * (mi / f.c1) / (sqrtf(vi / f.c2) + f.eps);
+    f.w[k] = w;
+    if (!weight) {
+        L.bias[co] = w;
+        return;
     }
-}
-
-__global__ void k_filter_bias_reduce(const float* __restrict__ partial, int blocks, int C, int cReal, float* __restrict__ db) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cReal) return;
-    float s = 0.0f;
-    for (int b = 0; b < blocks; ++b) s += partial[(size_t)b * C + c];
-    db[c] = s;
+    // as k_filter_pack lays them out
+    const bf16 b = __float2bfloat16(w);
+    L.packed[((size_t)(tap * (L.cin / 8) + ci / 8) * L.cout + co) * 8 + ci % 8] = b;
+    if (L.packedT) L.packedT[((size_t)((8 - tap) * (L.cout / 8) + co / 8) * L.cin + ci) * 8 + co % 8] = b;
 }
 
 // mean-squared error over the 3 predicted channels; g = d(loss)/d(out) into channels 0..2 of [P][16]
@@ -644,18 +701,6 @@ __global__ void __launch_bounds__(256) k_filter_loss(const float4* __restrict__ 
         __syncthreads();
     }
     if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
-}
-
-// Adam (Kingma & Ba 2015) on the FP32 master parameters
-__global__ void k_filter_adam(float* __restrict__ w, const float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v, int n,
-                              float lr, float b1, float b2, float eps, float c1, float c2) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float gi = grad[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    }
 }
 
 __device__ __forceinline__ float4 unpack_half4(uint2 u) {
@@ -716,14 +761,14 @@ __global__ void k_filter_target(const uint2* __restrict__ rough, size_t P, float
 }
 
 
-// tensor map of an NHWC BF16 activation [B][H][W][C]: boxes of 8 channels x 130 pixels x 1 row
-cudaError_t patch_map(CUtensorMap* map, const void* x, int B, int H, int W, int C) {
+// tensor map of an NHWC BF16 activation [B][H][W][C]: boxes of 8 channels x `pixels` pixels x 1 row
+cudaError_t patch_map(CUtensorMap* map, const void* x, int B, int H, int W, int C, int pixels = kRowW) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return cudaErrorNotSupported;
     if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0) return cudaErrorMisalignedAddress;
     const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
     const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    const cuuint32_t box[4] = {8, (cuuint32_t)kRowW, 1, 1};
+    const cuuint32_t box[4] = {8, (cuuint32_t)pixels, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -776,7 +821,7 @@ cudaError_t conv_launch(const FilterConvArgs& a, cudaStream_t s) {
 }
 
 template <int CIN, int COUT>
-cudaError_t dw_launch(const bf16* x, const bf16* x2, const bf16* g, int B, int H, int W, float* partial, int ctas, int* status,
+cudaError_t dw_launch(const bf16* x, const bf16* g, int B, int H, int W, float* partial, float* biasPartial, int* ctas, int* status,
                       cudaStream_t s) {
     using S = DwShape<CIN, COUT>;
     static std::atomic<bool> attr{false};
@@ -785,7 +830,12 @@ cudaError_t dw_launch(const bf16* x, const bf16* x2, const bf16* g, int B, int H
         if (e != cudaSuccess) return e;
         attr.store(true, std::memory_order_release);
     }
-    k_filter_dw<CIN, COUT><<<dim3(ctas, S::kGroups), 128, S::kSmem, s>>>(x, x2, g, B, H, W, partial, status);
+    CUtensorMap mx, mg;
+    cudaError_t e = patch_map(&mx, x, B, H, W, CIN);
+    if (e == cudaSuccess) e = patch_map(&mg, g, B, H, W, COUT, kStripPx);
+    if (e != cudaSuccess) return e;
+    *ctas = std::max(1, filter_dw_ctas() / S::kGroups);
+    k_filter_dw<CIN, COUT><<<dim3(*ctas, S::kGroups), 128, S::kSmem, s>>>(mx, mg, B, H, W, partial, biasPartial, status);
     count_launch();
     return cudaGetLastError();
 }
@@ -809,14 +859,14 @@ int filter_dw_ctas() {
     return sms > 0 ? sms : 1;
 }
 
-cudaError_t filter_dw(int cin, int cout, const void* x, const void* x2, const void* g, int B, int H, int W, float* partial, int ctas,
+cudaError_t filter_dw(int cin, int cout, const void* x, const void* g, int B, int H, int W, float* partial, float* biasPartial, int* ctas,
                       int* status, cudaStream_t s) {
-    const bf16 *X = static_cast<const bf16*>(x), *X2 = static_cast<const bf16*>(x2), *G = static_cast<const bf16*>(g);
-    if (cin == 16 && cout == 32) return dw_launch<16, 32>(X, X2, G, B, H, W, partial, ctas, status, s);
-    if (cin == 32 && cout == 64) return dw_launch<32, 64>(X, X2, G, B, H, W, partial, ctas, status, s);
-    if (cin == 64 && cout == 64) return dw_launch<64, 64>(X, X2, G, B, H, W, partial, ctas, status, s);
-    if (cin == 64 && cout == 32) return dw_launch<64, 32>(X, X2, G, B, H, W, partial, ctas, status, s);
-    if (cin == 32 && cout == 16) return dw_launch<32, 16>(X, X2, G, B, H, W, partial, ctas, status, s);
+    const bf16 *X = static_cast<const bf16*>(x), *G = static_cast<const bf16*>(g);
+    if (cin == 16 && cout == 32) return dw_launch<16, 32>(X, G, B, H, W, partial, biasPartial, ctas, status, s);
+    if (cin == 32 && cout == 64) return dw_launch<32, 64>(X, G, B, H, W, partial, biasPartial, ctas, status, s);
+    if (cin == 64 && cout == 64) return dw_launch<64, 64>(X, G, B, H, W, partial, biasPartial, ctas, status, s);
+    if (cin == 64 && cout == 32) return dw_launch<64, 32>(X, G, B, H, W, partial, biasPartial, ctas, status, s);
+    if (cin == 32 && cout == 16) return dw_launch<32, 16>(X, G, B, H, W, partial, biasPartial, ctas, status, s);
     return cudaErrorInvalidValue;
 }
 
@@ -826,28 +876,19 @@ cudaError_t filter_pack(const float* W, int coutReal, int cinReal, int cin, int 
     return cudaGetLastError();
 }
 
-cudaError_t filter_dw_reduce(const float* partial, int ctas, int cout, int cin, int coutReal, int cinReal, float* dW, cudaStream_t s) {
-    k_filter_dw_reduce<<<64, 256, 0, s>>>(partial, ctas, cout, cin, coutReal, cinReal, dW);
+cudaError_t filter_finish(FilterFinish& f, cudaStream_t s) {
+    int blocks = 0;
+    for (FilterFinish::Layer& l : f.layer) {
+        l.block0 = blocks;
+        blocks += (l.coutReal * (9 * l.cinReal + 1) + 63) / 64;
+    }
+    k_filter_finish<<<blocks, 256, 0, s>>>(f);
     count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t filter_bias_grad(const void* g, size_t P, int C, int cReal, float* partial, int blocks, float* db, cudaStream_t s) {
-    k_filter_bias_partial<<<blocks, 256, 0, s>>>(static_cast<const bf16*>(g), P, C, partial);
-    k_filter_bias_reduce<<<1, 64, 0, s>>>(partial, blocks, C, cReal, db);
-    count_launch(2);
     return cudaGetLastError();
 }
 
 cudaError_t filter_loss(const float4* out, const float4* target, size_t P, float scale, void* g, float* partial, int blocks, cudaStream_t s) {
     k_filter_loss<<<blocks, 256, 0, s>>>(out, target, P, scale, static_cast<bf16*>(g), partial);
-    count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t filter_adam(float* w, const float* grad, float* m, float* v, int n, float lr, float b1, float b2, float eps, float c1,
-                        float c2, cudaStream_t s) {
-    k_filter_adam<<<128, 256, 0, s>>>(w, grad, m, v, n, lr, b1, b2, eps, c1, c2);
     count_launch();
     return cudaGetLastError();
 }

@@ -59,7 +59,7 @@ struct rg_filter {
     std::string err;
     int offW[kL], offB[kL];
     Dev params, grads, m, v, wf[kL], wt[kL], bias[kL], status;
-    Dev x0, y1, y2, y3, y4, x5, out, g5, gx5, gp4, gp3, gp2, gp1, target, dwPartial, bPartial, lossPartial;
+    Dev x0, y1, y2, y3, y4, x5, out, g5, gx5, gp4, gp3, gp2, gp1, target, dwPartial, lossPartial;
     size_t actPixels = 0;
     uint64_t steps = 0;
     bool packed = false;
@@ -235,7 +235,7 @@ rg_status rg_filter_destroy(rg_filter* f) {
     cudaSetDevice(f->device);
     if (f->stream) cudaStreamSynchronize(f->stream);
     Dev* all[] = {&f->params, &f->grads, &f->m, &f->v, &f->status, &f->x0, &f->y1, &f->y2, &f->y3, &f->y4, &f->x5, &f->out, &f->g5, &f->gx5,
-                  &f->gp4, &f->gp3, &f->gp2, &f->gp1, &f->target, &f->dwPartial, &f->bPartial, &f->lossPartial};
+                  &f->gp4, &f->gp3, &f->gp2, &f->gp1, &f->target, &f->dwPartial, &f->lossPartial};
     for (Dev* d : all) d->release();
     for (int l = 0; l < kL; ++l) {
         f->wf[l].release();
@@ -296,20 +296,25 @@ rg_status rg_filter_train_step(rg_filter* f, const void* d_input, const float* d
     using bf = __nv_bfloat16;
     const size_t P = (size_t)B * H * W;
     TRY_F(ensure_activations(f, P, true));
-    const int ctas = filter_dw_ctas(), lossBlocks = 512, biasBlocks = 256;
-    FCK(f->dwPartial.ensure(sizeof(float) * (size_t)ctas * 64 * 9 * 64));
-    FCK(f->bPartial.ensure(sizeof(float) * biasBlocks * 64));
+    const int lossBlocks = 512;
+    size_t partials = 0;  // floats of the CTAs' partial gradients, all layers
+    for (int l = 0; l < kL; ++l) partials += (size_t)filter_dw_ctas() * kCout[l] * (9 * kCin[l] + 1);
+    FCK(f->dwPartial.ensure(sizeof(float) * partials));
     FCK(f->lossPartial.ensure(sizeof(float) * lossBlocks));
     const bf* x0 = static_cast<const bf*>(d_input);
     TRY_F(forward(f, x0, (int)B, (int)H, (int)W, true));
     FCK(filter_loss(f->out.as<float4>(), reinterpret_cast<const float4*>(d_target), P, 1.0f / (3.0f * (float)P), f->g5.p,
                     f->lossPartial.as<float>(), lossBlocks, f->stream));
-    float* G = f->grads.as<float>();
     int* st = f->status.as<int>();
-    auto dW = [&](int l, const void* x, const void* x2, const void* g) -> rg_status {
-        FCK(filter_dw(kCin[l], kCout[l], x, x2, g, (int)B, (int)H, (int)W, f->dwPartial.as<float>(), ctas, st, f->stream));
-        FCK(filter_dw_reduce(f->dwPartial.as<float>(), ctas, kCout[l], kCin[l], kCoutR[l], kCinR[l], G + f->offW[l], f->stream));
-        FCK(filter_bias_grad(g, P, kCout[l], kCoutR[l], f->bPartial.as<float>(), biasBlocks, G + f->offB[l], f->stream));
+    FilterFinish fin;
+    float* room = f->dwPartial.as<float>();
+    auto dW = [&](int l, const void* x, const void* g) -> rg_status {
+        FilterFinish::Layer& L = fin.layer[l];
+        float* bias = room + (size_t)filter_dw_ctas() * kCout[l] * 9 * kCin[l];
+        FCK(filter_dw(kCin[l], kCout[l], x, g, (int)B, (int)H, (int)W, room, bias, &L.ctas, st, f->stream));
+        L = {room, bias, f->wf[l].as<bf>(), l > 0 ? f->wt[l].as<bf>() : nullptr, f->bias[l].as<float>(), L.ctas, kCout[l], kCin[l], kCoutR[l], kCinR[l],
+             f->offW[l], f->offB[l], 0};
+        room = bias + (size_t)filter_dw_ctas() * kCout[l];
         return RG_OK;
     };
     FilterConvArgs a;
@@ -319,7 +324,7 @@ rg_status rg_filter_train_step(rg_filter* f, const void* d_input, const float* d
     a.W = (int)W;
     a.status = st;
     // layer 5 (input x5 = y4 + y1)
-    TRY_F(dW(4, f->x5.p, nullptr, f->g5.p));
+    TRY_F(dW(4, f->x5.p, f->g5.p));
     {
         FilterConvArgs c = a;  // gx5 (kept for the skip), gp4 = gx5 where y4 > 0
         c.x = f->g5.as<bf>();
@@ -329,7 +334,7 @@ rg_status rg_filter_train_step(rg_filter* f, const void* d_input, const float* d
         c.mask = f->y4.as<bf>();
         FCK(filter_conv(kCout[4], kCin[4], c, f->stream));
     }
-    TRY_F(dW(3, f->y3.p, nullptr, f->gp4.p));
+    TRY_F(dW(3, f->y3.p, f->gp4.p));
     {
         FilterConvArgs c = a;
         c.x = f->gp4.as<bf>();
@@ -338,7 +343,7 @@ rg_status rg_filter_train_step(rg_filter* f, const void* d_input, const float* d
         c.mask = f->y3.as<bf>();
         FCK(filter_conv(kCout[3], kCin[3], c, f->stream));
     }
-    TRY_F(dW(2, f->y2.p, nullptr, f->gp3.p));
+    TRY_F(dW(2, f->y2.p, f->gp3.p));
     {
         FilterConvArgs c = a;
         c.x = f->gp3.as<bf>();
@@ -347,7 +352,7 @@ rg_status rg_filter_train_step(rg_filter* f, const void* d_input, const float* d
         c.mask = f->y2.as<bf>();
         FCK(filter_conv(kCout[2], kCin[2], c, f->stream));
     }
-    TRY_F(dW(1, f->y1.p, nullptr, f->gp2.p));
+    TRY_F(dW(1, f->y1.p, f->gp2.p));
     {
         FilterConvArgs c = a;  // through layer 2, plus the skip's gradient, masked by y1
         c.x = f->gp2.as<bf>();
@@ -357,16 +362,19 @@ rg_status rg_filter_train_step(rg_filter* f, const void* d_input, const float* d
         c.mask = f->y1.as<bf>();
         FCK(filter_conv(kCout[1], kCin[1], c, f->stream));
     }
-    TRY_F(dW(0, x0, nullptr, f->gp1.p));
-    // Adam
+    TRY_F(dW(0, x0, f->gp1.p));
     f->steps++;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.0f - std::pow(b1, (float)f->steps), c2 = 1.0f - std::pow(b2, (float)f->steps);
-    if (lr > 0.0f) {
-        FCK(filter_adam(f->params.as<float>(), G, f->m.as<float>(), f->v.as<float>(), RG_FILTER_PARAMS, lr, b1, b2, 1e-8f, c1, c2,
-                        f->stream));
-        TRY_F(refresh_weights(f));
-    }
+    fin.w = f->params.as<float>();
+    fin.grad = f->grads.as<float>();
+    fin.m = f->m.as<float>();
+    fin.v = f->v.as<float>();
+    fin.lr = lr;
+    fin.b1 = 0.9f;
+    fin.b2 = 0.999f;
+    fin.eps = 1e-8f;
+    fin.c1 = 1.0f - std::pow(fin.b1, (float)f->steps);
+    fin.c2 = 1.0f - std::pow(fin.b2, (float)f->steps);
+    FCK(filter_finish(fin, f->stream));
     std::vector<float> lp(lossBlocks);
     FCK(cudaMemcpyAsync(lp.data(), f->lossPartial.p, sizeof(float) * lossBlocks, cudaMemcpyDeviceToHost, f->stream));
     int status = 0;

@@ -348,15 +348,25 @@ struct FilterConvArgs {
     int* status;                // set when a tensor-core or copy completion wait gave up
 };
 cudaError_t filter_conv(int cin, int cout, const FilterConvArgs& a, cudaStream_t s);
-int filter_dw_ctas();
-cudaError_t filter_dw(int cin, int cout, const void* x, const void* x2, const void* g, int B, int H, int W, float* partial, int ctas,
+int filter_dw_ctas();  // most CTAs whose partials a weight gradient leaves
+// partial[cta][cout][9][cin] and biasPartial[cta][cout] of *ctas CTAs (x, g 16-byte aligned)
+cudaError_t filter_dw(int cin, int cout, const void* x, const void* g, int B, int H, int W, float* partial, float* biasPartial, int* ctas,
                       int* status, cudaStream_t s);
 cudaError_t filter_pack(const float* W, int coutReal, int cinReal, int cin, int cout, int transposed, void* out, cudaStream_t s);
-cudaError_t filter_dw_reduce(const float* partial, int ctas, int cout, int cin, int coutReal, int cinReal, float* dW, cudaStream_t s);
-cudaError_t filter_bias_grad(const void* g, size_t P, int C, int cReal, float* partial, int blocks, float* db, cudaStream_t s);
+// the end of a training step: gradients from the partials of all layers, Adam, packed weights
+struct FilterFinish {
+    struct Layer {
+        const float *partial, *biasPartial;
+        __nv_bfloat16 *packed, *packedT;  // packedT nullable (the first layer has no data gradient)
+        float* bias;                      // padded bias
+        int ctas, cout, cin, coutReal, cinReal, offW, offB;
+        int block0;                       // set by filter_finish
+    } layer[5];
+    float *w, *grad, *m, *v;
+    float lr, b1, b2, eps, c1, c2;
+};
+cudaError_t filter_finish(FilterFinish& f, cudaStream_t s);
 cudaError_t filter_loss(const float4* out, const float4* target, size_t P, float scale, void* g, float* partial, int blocks, cudaStream_t s);
-cudaError_t filter_adam(float* w, const float* grad, float* m, float* v, int n, float lr, float b1, float b2, float eps, float c1,
-                        float c2, cudaStream_t s);
 cudaError_t filter_gbuffer(const uint2* base, const uint2* normal, const uint2* rough, size_t P, float samples, void* out, cudaStream_t s);
 cudaError_t filter_composite(const uint2* base, const float4* pred, size_t P, const float fade[4], int showAlpha, uint2* finalImg,
                              cudaStream_t s);
