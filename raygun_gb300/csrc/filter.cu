@@ -92,8 +92,9 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 //   warp 0     TMA producer: refills a slot once the MMAs of the last group reading its row completed;
 //   warp 1     MMA issuer: group by group into alternating accumulator windows;
 //   warps 2-9  epilogue, two warps per TMEM lane quarter (half the channels each): drain a completed
-//              window (bias, ReLU, skip add, mask) and hand it back; BF16 rows leave through a small
-//              swizzled shared-memory stage so that each store instruction writes whole sectors.
+//              window, hand it back, then bias, ReLU, skip add, mask; a lane writes 16 channels of its
+//              pixel with one 32-byte store, a whole sector (through a swizzled shared-memory stage and
+//              16-byte stores the epilogue took 70 - 90 % of the time of the layers into 32 and 64 channels).
 constexpr int kStripPx = 128, kRowW = kStripPx + 2;
 constexpr int kRowPlane = 2176;  // 130 pixels x 16 B rounded up to 128 B (TMA destination alignment)
 constexpr int kEpiWarps = 8;
@@ -109,8 +110,7 @@ struct ConvShape {
     static constexpr int kRowBytes = CC * kRowPlane;              // one slot
     static constexpr uint32_t kRowTx = CC * kRowW * 16;           // bytes the TMA writes per row
     static constexpr int kWeightBytes = 9 * CIN * COUT * 2;       // [dx][ci/8][kernel row 2, 1, 0][co][8]
-    static constexpr int kStageBytes = 32 * COUT;                 // per epilogue warp: 32 pixels x COUT/2 channels (BF16)
-    static constexpr int kSmem = kWeightBytes + kRing * kRowBytes + kEpiWarps * kStageBytes + 1024;
+    static constexpr int kSmem = kWeightBytes + kRing * kRowBytes + 1024;
     static constexpr uint32_t kCols = kWindows * kWin <= 32 ? 32 : (kWindows * kWin <= 64 ? 64 : (kWindows * kWin <= 128 ? 128 : (kWindows * kWin <= 256 ? 256 : 512)));
     static_assert(CIN % 16 == 0 && COUT % 16 == 0 && kWin <= 256 && kWindows * kWin <= 512, "shape");
     static_assert(kWeightBytes % 128 == 0, "ring slots 128-byte aligned");
@@ -132,6 +132,20 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* mbar, uint32_t phas
     if (status) atomicExch(status, 3);  // 3: a wait of the learned filter gave up
     return false;
 }
+// The producer and MMA warps run their loops as whole warps, on values that are the same in all lanes --
+// the warp number through a shuffle, wait results through a vote -- and elect one lane only around the
+// copies and MMAs.  Descriptors and coordinates then live in uniform registers, where those
+// instructions take them; under a branch on the lane number each MMA took about 120 clocks to issue,
+// most of it moving its operands there.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ bool warp_wait_or_abort(uint64_t* mbar, uint32_t phase, volatile int* abort, int* status) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait_or_abort(mbar, phase, abort, status));
+}
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
 }
@@ -143,22 +157,35 @@ __device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t* r) {
                  : "r"(taddr));
 }
 
-// A warp's 32 pixels x NC 16-byte chunks in shared memory, chunk c of pixel p at slot c ^ f(p) so that
-// both the per-pixel writes and the row-order reads below touch 8 distinct bank groups per phase.
-template <int NC>
-__device__ __forceinline__ uint32_t stage_off(int p, int c) {
-    const int f = NC == 1 ? 0 : (p / (8 / NC)) % NC;
-    return (uint32_t)(p * NC * 16 + ((c ^ f) * 16));
+// N consecutive BF16 channels of one pixel (N = 8 or 16: one 16- or 32-byte access, a whole sector)
+template <int N>
+struct Chan {
+    uint32_t r[N / 2];
+};
+template <int N>
+__device__ __forceinline__ Chan<N> load_chan(const bf16* p) {
+    Chan<N> c;
+    if constexpr (N == 16)
+        asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(c.r[0]), "=r"(c.r[1]), "=r"(c.r[2]), "=r"(c.r[3]), "=r"(c.r[4]), "=r"(c.r[5]), "=r"(c.r[6]), "=r"(c.r[7])
+                     : "l"(p));
+    else
+        asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(c.r[0]), "=r"(c.r[1]), "=r"(c.r[2]), "=r"(c.r[3]) : "l"(p));
+    return c;
 }
-// copies the staged 32 x NC chunks to dst (pixel p at dst + p * pixStride bytes), pixels < valid only
-template <int NC>
-__device__ __forceinline__ void stage_out(const uint8_t* stage, uint8_t* dst, size_t pixStride, int valid, int lane) {
-#pragma unroll
-    for (int it = 0; it < NC; ++it) {
-        const int k = it * 32 + lane, p = k / NC, c = k % NC;
-        const uint4 v = *reinterpret_cast<const uint4*>(stage + stage_off<NC>(p, c));
-        if (p < valid) *reinterpret_cast<uint4*>(dst + (size_t)p * pixStride + c * 16) = v;
-    }
+template <int N>
+__device__ __forceinline__ void store_chan(bf16* p, const Chan<N>& c) {
+    if constexpr (N == 16)
+        asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(c.r[0]), "r"(c.r[1]), "r"(c.r[2]), "r"(c.r[3]), "r"(c.r[4]),
+                     "r"(c.r[5]), "r"(c.r[6]), "r"(c.r[7])
+                     : "memory");
+    else
+        asm volatile("st.global.v4.b32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(c.r[0]), "r"(c.r[1]), "r"(c.r[2]), "r"(c.r[3]) : "memory");
+}
+__device__ __forceinline__ float2 chan_pair(uint32_t r) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r)); }
+__device__ __forceinline__ uint32_t pack_pair(float x, float y) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+    return *reinterpret_cast<const uint32_t*>(&v);
 }
 
 template <int CIN, int COUT>
@@ -174,8 +201,8 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
     __shared__ uint32_t tmem_base;
     __shared__ __align__(8) uint64_t full[S::kRing], empty[S::kRing], accFull[NW], accEmpty[NW], drain;
     __shared__ int abortFlag, issuedRows, consumedRows;
-    __shared__ float biasSm[COUT];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ __align__(16) float biasSm[COUT];
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     // weights: packed [tap = dy * 3 + dx][ci/8][co][8] -> [dx][ci/8][kernel row 2, 1, 0][co][8]
     for (int i = tid; i < S::kWeightBytes / 16; i += blockDim.x) {
         const int co = i % COUT, dyr = (i / COUT) % 3, cc = (i / (3 * COUT)) % CC, dx = i / (3 * COUT * CC);
@@ -215,54 +242,47 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
         ys = (rem % segs) * segRows;
         ng = (min(ys + segRows, a.H) - ys + kGroupRows - 1) / kGroupRows;
     };
-    if (warp == 0) {
-        if (lane == 0) {  // producer: input rows ys - 1 .. ys + 3 ng of each item
-            int seq = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-                int b, x0, ys, ng;
-                item_of(item, b, x0, ys, ng);
-                for (int k = 0; k < kGroupRows * ng + 2 && ok; ++k, ++seq) {
-                    const int slot = seq % S::kRing, fill = seq / S::kRing;
-                    if (fill > 0 && !mbar_wait_or_abort(&empty[slot], (uint32_t)((fill - 1) & 1), abort, a.status)) {
-                        ok = false;
-                        break;
-                    }
+    if (warp == 0) {  // producer: input rows ys - 1 .. ys + 3 ng of each item
+        int seq = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            int b, x0, ys, ng;
+            item_of(item, b, x0, ys, ng);
+            for (int k = 0; k < kGroupRows * ng + 2; ++k, ++seq) {
+                const int slot = seq % S::kRing, fill = seq / S::kRing;
+                ok = fill == 0 || warp_wait_or_abort(&empty[slot], (uint32_t)((fill - 1) & 1), abort, a.status);
+                if (!ok) break;
+                if (elect_one()) {
                     mbar_expect_tx(&full[slot], S::kRowTx);
-#pragma unroll 1
+#pragma unroll
                     for (int cc = 0; cc < CC; ++cc)
                         tma_load_4d(ring + slot * S::kRowBytes + cc * kRowPlane, &tmapX, cc * 8, x0 - 1, ys - 1 + k, b, &full[slot]);
                     issuedRows = seq + 1;
                 }
+                __syncwarp();
             }
         }
-    } else if (warp == 1) {
-        if (lane == 0) {  // MMA issuer
-            // descriptors: the start address sits in the low 14 bits (address / 16) and every operand
-            // lies below 256 KB, so offsets add to it without a carry
-            const uint64_t adesc0 = umma_desc(smem_u32(ring), kRowPlane, 128), bdesc0 = umma_desc(smem_u32(wsm), 3 * COUT * 16, 128);
-            constexpr uint32_t id1 = umma_idesc(128, COUT, false, false), id2 = umma_idesc(128, 2 * COUT, false, false),
-                               id3 = umma_idesc(128, 3 * COUT, false, false);
-            int base = 0, waited = 0, g = 0;  // first input row of the item, input rows waited for, groups issued
-            bool ok = true;
-            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-                int b, x0, ys, ng;
-                item_of(item, b, x0, ys, ng);
-                for (int j = 0; j < ng && ok; ++j, ++g) {
-                    const int w = g % NW;
-                    if (g >= NW && !mbar_wait_or_abort(&accEmpty[w], (uint32_t)((g / NW - 1) & 1), abort, a.status)) {
-                        ok = false;
-                        break;
-                    }
-                    const int first = base + kGroupRows * j;  // input row r - 1 of this group
-                    for (; waited < first + 5; ++waited)
-                        if (!mbar_wait_or_abort(&full[waited % S::kRing], (uint32_t)((waited / S::kRing) & 1), abort, a.status)) {
-                            ok = false;
-                            break;
-                        }
-                    if (!ok) break;
+    } else if (warp == 1) {  // MMA issuer
+        // descriptors: the start address sits in the low 14 bits (address / 16) and every operand lies
+        // below 256 KB, so offsets add to it without a carry
+        const uint64_t adesc0 = umma_desc(smem_u32(ring), kRowPlane, 128), bdesc0 = umma_desc(smem_u32(wsm), 3 * COUT * 16, 128);
+        constexpr uint32_t id1 = umma_idesc(128, COUT, false, false), id2 = umma_idesc(128, 2 * COUT, false, false),
+                           id3 = umma_idesc(128, 3 * COUT, false, false);
+        int base = 0, waited = 0, g = 0;  // first input row of the item, input rows waited for, groups issued
+        bool ok = true;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+            int b, x0, ys, ng;
+            item_of(item, b, x0, ys, ng);
+            for (int j = 0; j < ng; ++j, ++g) {
+                const int w = g % NW;
+                ok = g < NW || warp_wait_or_abort(&accEmpty[w], (uint32_t)((g / NW - 1) & 1), abort, a.status);
+                const int first = base + kGroupRows * j;  // input row r - 1 of this group
+                for (; waited < first + 5 && ok; ++waited)
+                    ok = warp_wait_or_abort(&full[waited % S::kRing], (uint32_t)((waited / S::kRing) & 1), abort, a.status);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
                     consumedRows = waited;
-                    tc_fence_after();
                     uint64_t arow[5];
 #pragma unroll
                     for (int p = 0; p < 5; ++p) arow[p] = adesc0 + (uint64_t)((((first + p) % S::kRing) * S::kRowBytes) >> 4);
@@ -304,15 +324,16 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
                         umma_commit(&empty[(first + 4) % S::kRing]);
                     }
                 }
-                base += kGroupRows * ng + 2;
+                __syncwarp();
             }
-            umma_commit(&drain);  // completes when every MMA issued above has
-            mbar_wait(&drain, 0u, nullptr);
+            base += kGroupRows * ng + 2;
         }
+        if (elect_one()) umma_commit(&drain);  // completes when every MMA issued above has
+        __syncwarp();
+        mbar_wait(&drain, 0u, nullptr);
     } else {  // epilogue: TMEM lane quarter warp % 4 = pixels 32 (warp % 4) .. + 31; channel half h
-        constexpr int CH = COUT / 2, NC = CH / 8;
+        constexpr int CH = COUT / 2, N = CH >= 16 ? 16 : 8, NC = CH / N;
         const int q = warp & 3, h = (warp - 2) >> 2, cbase = h * CH;
-        uint8_t* stage = ring + S::kRing * S::kRowBytes + (warp - 2) * S::kStageBytes;
         int g = 0;
         bool ok = true;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
@@ -320,23 +341,22 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
             item_of(item, b, x0, ys, ng);
             const int ye = min(ys + segRows, a.H);
             const int xx = x0 + q * 32 + lane;
-            for (int j = 0; j < ng; ++j, ++g) {
-                const int w = g % NW;
+            const size_t rowStep = (size_t)a.W * COUT;
+            size_t at = (((size_t)b * a.H + ys) * a.W + xx) * COUT + cbase;  // this lane's channels in the group's first row
+            for (int j = 0; j < ng; ++j, ++g, at += kGroupRows * rowStep) {
+                const int w = g % NW, y0 = ys + kGroupRows * j;
+                auto live = [&](int r) { return y0 + r < ye && xx < a.W; };
                 // narrow layers fetch the skip input of the group's rows before waiting for the
                 // accumulators (registers allow it); 64-channel layers and masks load in place
-                constexpr bool kPre = NC <= 2;
-                constexpr int PR = kPre ? kGroupRows : 1;
-                uint4 addPre[PR][NC];
-                auto aux_load = [&](const bf16* src, int y, int c) {
-                    return src && y < ye && xx < a.W ? reinterpret_cast<const uint4*>(src + (((size_t)b * a.H + y) * a.W + xx) * COUT + cbase)[c]
-                                                     : make_uint4(0u, 0u, 0u, 0u);
-                };
-                if (kPre) {
+                constexpr bool kPre = CH <= 16;
+                Chan<N> addPre[kPre ? kGroupRows : 1][kPre ? NC : 1];
+                if constexpr (kPre)
+                    if (a.add)
 #pragma unroll
-                    for (int r = 0; r < PR; ++r)
+                        for (int r = 0; r < kGroupRows; ++r)
 #pragma unroll
-                        for (int c = 0; c < NC; ++c) addPre[r][c] = aux_load(a.add, ys + kGroupRows * j + r, c);
-                }
+                            for (int c = 0; c < NC; ++c)
+                                if (live(r)) addPre[r][c] = load_chan<N>(a.add + at + r * rowStep + c * N);
                 if (!mbar_wait_or_abort(&accFull[w], (uint32_t)((g / NW) & 1), abort, a.status)) {
                     ok = false;
                     break;
@@ -353,60 +373,53 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&accEmpty[w]);  // the window goes back before the math and stores
 #pragma unroll
-                for (int r = 0; r < kGroupRows; ++r) {
-                    const int y = ys + kGroupRows * j + r;
-                    if (y >= ye) continue;  // uniform across the warp
-                    const size_t px0 = ((size_t)b * a.H + y) * a.W + x0 + q * 32;  // pixel of lane 0
-                    const size_t px = px0 + lane;
-                    const bool in = xx < a.W;
-                    const int valid = min(32, a.W - (x0 + q * 32));
-                    float v[CH];
+                for (int c = 0; c < NC; ++c) {
+                    float bias[N];
 #pragma unroll
-                    for (int e = 0; e < CH; ++e) {
-                        v[e] = __uint_as_float(raw[r][e]) + biasSm[cbase + e];
-                        if (a.relu) v[e] = fmaxf(v[e], 0.0f);
-                    }
-                    auto put = [&](bf16* out, const float* vals, const uint4* mask) {  // BF16 row out through the stage
+                    for (int e = 0; e < N; e += 4) *reinterpret_cast<float4*>(bias + e) = *reinterpret_cast<const float4*>(biasSm + cbase + c * N + e);
 #pragma unroll
-                        for (int c = 0; c < NC; ++c) {
-                            __align__(16) bf16 o[8];
-                            if (mask) {
-                                const bf16* mv = reinterpret_cast<const bf16*>(&mask[c]);
+                    for (int r = 0; r < kGroupRows; ++r) {
+                        if (!live(r)) continue;
+                        const size_t o = at + r * rowStep + c * N;
+                        float v[N];
 #pragma unroll
-                                for (int e = 0; e < 8; ++e) o[e] = __float2bfloat16(__bfloat162float(mv[e]) > 0.0f ? vals[8 * c + e] : 0.0f);
-                            } else {
-#pragma unroll
-                                for (int e = 0; e < 8; ++e) o[e] = __float2bfloat16(vals[8 * c + e]);
-                            }
-                            *reinterpret_cast<uint4*>(stage + stage_off<NC>(lane, c)) = *reinterpret_cast<uint4*>(o);
+                        for (int e = 0; e < N; ++e) {
+                            v[e] = __uint_as_float(raw[r][c * N + e]) + bias[e];
+                            if (a.relu) v[e] = fmaxf(v[e], 0.0f);
                         }
-                        __syncwarp();
-                        stage_out<NC>(stage, reinterpret_cast<uint8_t*>(out + px0 * COUT + cbase), (size_t)COUT * 2, valid, lane);
-                        __syncwarp();
-                    };
-                    if (a.y) put(a.y, v, nullptr);
-                    if (a.add) {
-                        // forward skip (a.ya): the sum of the stored BF16 activations, x5 = bf16(bf16(y4) + y1);
-                        // backward (the skip gradient into layer 1's): FP32 sum, rounded once on the way out
-                        const bool storedSum = a.ya != nullptr;
+                        auto packed = [&] {
+                            Chan<N> p;
 #pragma unroll
-                        for (int c = 0; c < NC; ++c) {
-                            const uint4 av = kPre ? addPre[kPre ? r : 0][c] : aux_load(a.add, y, c);
-                            const bf16* hv = reinterpret_cast<const bf16*>(&av);
+                            for (int e = 0; e < N / 2; ++e) p.r[e] = pack_pair(v[2 * e], v[2 * e + 1]);
+                            return p;
+                        };
+                        if (a.y) store_chan<N>(a.y + o, packed());
+                        if (a.add) {
+                            // forward skip (a.ya): the sum of the stored BF16 activations, x5 = bf16(bf16(y4) + y1);
+                            // backward (the skip gradient into layer 1's): FP32 sum, rounded once on the way out
+                            const bool storedSum = a.ya != nullptr;
+                            const Chan<N> av = kPre ? addPre[kPre ? r : 0][kPre ? c : 0] : load_chan<N>(a.add + o);
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) {
-                                const float own = storedSum ? __bfloat162float(__float2bfloat16(v[8 * c + e])) : v[8 * c + e];
-                                v[8 * c + e] = own + __bfloat162float(hv[e]);
+                            for (int e = 0; e < N / 2; ++e) {
+                                const float2 ad = chan_pair(av.r[e]), own = storedSum ? chan_pair(pack_pair(v[2 * e], v[2 * e + 1]))
+                                                                                      : make_float2(v[2 * e], v[2 * e + 1]);
+                                v[2 * e] = own.x + ad.x;
+                                v[2 * e + 1] = own.y + ad.y;
                             }
                         }
-                    }
-                    if (a.ya) put(a.ya, v, nullptr);
-                    if (a.yf && cbase == 0 && in) reinterpret_cast<float4*>(a.yf)[px] = make_float4(v[0], v[1], v[2], v[3]);
-                    if (a.ym) {
-                        uint4 mk[NC];
+                        if (a.ya) store_chan<N>(a.ya + o, packed());
+                        if (a.yf && c == 0 && cbase == 0)
+                            reinterpret_cast<float4*>(a.yf)[((size_t)b * a.H + y0 + r) * a.W + xx] = make_float4(v[0], v[1], v[2], v[3]);
+                        if (a.ym) {
+                            const Chan<N> mk = load_chan<N>(a.mask + o);
 #pragma unroll
-                        for (int c = 0; c < NC; ++c) mk[c] = aux_load(a.mask, y, c);
-                        put(a.ym, v, mk);
+                            for (int e = 0; e < N / 2; ++e) {
+                                const float2 m = chan_pair(mk.r[e]);
+                                v[2 * e] = m.x > 0.0f ? v[2 * e] : 0.0f;
+                                v[2 * e + 1] = m.y > 0.0f ? v[2 * e + 1] : 0.0f;
+                            }
+                            store_chan<N>(a.ym + o, packed());
+                        }
                     }
                 }
             }
@@ -428,33 +441,37 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
 // pixel offset.  The bias sum is one more product, with a tile of ones as B.
 // A CTA takes an equal run of the (image, strip of 128 pixels, row) list, so all CTAs end together, and
 // streams it: each row of g once, each row of x once (plus two rows where a run starts or enters the next
-// strip), through rings of shared-memory slots filled by TMA, while one thread issues a row's 72 MMAs
-// (M = 128, N = CIN, K = 16) with constant descriptor offsets; everything accumulates in tensor memory.
-// Rows of A beyond COUT read whatever lies behind the slot; their results are not read.  64 input
-// channels take two tap groups (9 x 64 columns exceed the 512 of an SM).
-// Bound: the copies' 16-byte rows (CIN / 8 x 130 + COUT / 8 x 128 of them per image row) and the MMA
-// issue, about one of either per clock at CIN = COUT = 64.  32 crops of 128 x 128, 64 -> 64: 410 us with
-// one tile staged, multiplied and waited for at a time by one warp quartet; 141 us now, bias sum (113 us
-// in a kernel of its own) included.
+// strip), through rings of shared-memory slots filled by TMA, while one thread issues the MMAs with
+// constant descriptor offsets; everything accumulates in tensor memory.  The planes of the three x rows
+// that an output row needs lie one after another in the ring, so one MMA (M = 128, N = 3 CIN, K = 16)
+// takes the three taps of a column: reading A (4 KB) costs about 80 clocks an MMA whatever N is, and nine
+// MMAs of N = CIN for the nine taps took 92 - 142 us a layer on 32 crops of 128 x 128.  Where the ring
+// wraps inside the three rows, two MMAs share them.  Rows of A beyond COUT read whatever lies behind the
+// slot; their results are not read.  With 64 input channels the nine taps (576 columns) exceed tensor
+// memory: half of the CTAs take columns 0 and 1 of the kernel, the others column 2.
+// Those crops, 64 -> 64: 410 us with one tile staged, multiplied and waited for at a time by one warp
+// quartet, 98 us now, bias sum (113 us in a kernel of its own) included.
 template <int CIN, int COUT>
 struct DwShape {
-    static constexpr int kTaps = CIN == 64 ? 5 : 9;  // taps per CTA
     static constexpr int kGroups = CIN == 64 ? 2 : 1;
+    static constexpr int kCols0 = CIN == 64 ? 2 : 3;  // kernel columns of the first group
     static constexpr int kGPlane = kStripPx * 16, kGBytes = (COUT / 8) * kGPlane, kXBytes = (CIN / 8) * kRowPlane;
-    static constexpr int kGRing = 4, kXRing = 6;
+    static constexpr int kGRing = 4, kXRing = 8;
     static constexpr uint32_t kGTx = kGBytes, kXTx = (CIN / 8) * kRowW * 16;
     static constexpr int kOnes = 2 * 256;  // B tile of ones: [2 chunks][16 pixels][8]
     static constexpr int kUsed = kGRing * kGBytes + kXRing * kXBytes + kOnes;
     static constexpr int kReach = (kGRing - 1) * kGBytes + 16 * kGPlane;  // A's 128 rows from the last slot
     // at least 120 KB: one CTA holds an SM (and its tensor memory) at a time
     static constexpr int kSmem = (kUsed > kReach ? kUsed : kReach) + 1024 > 120 * 1024 ? (kUsed > kReach ? kUsed : kReach) + 1024 : 120 * 1024;
-    static constexpr uint32_t kCols = kTaps * CIN + 16 <= 256 ? 256 : 512;
-    static_assert(kTaps * CIN + 16 <= 512 && kGBytes % 128 == 0 && kXBytes % 128 == 0, "shape");
+    static constexpr int kBiasCol = kCols0 * 3 * CIN;  // tensor-memory column of the bias sums
+    static constexpr uint32_t kCols = kBiasCol + 16 <= 256 ? 256 : 512;
+    static_assert(kBiasCol + 16 <= 512 && 3 * CIN <= 256 && kGBytes % 128 == 0 && kXBytes % 128 == 0 && kSmem <= 227 * 1024, "shape");
 };
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapG, int B,
-                                                      int H, int W, float* __restrict__ partial, float* __restrict__ biasPartial, int* status) {
+                                                      int H, int W, int ctas0, float* __restrict__ partial, float* __restrict__ biasPartial,
+                                                      int* status) {
     using S = DwShape<CIN, COUT>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -462,8 +479,10 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
     __shared__ uint32_t tmem_base;
     __shared__ __align__(8) uint64_t xFull[S::kXRing], xEmpty[S::kXRing], gFull[S::kGRing], gEmpty[S::kGRing], drain;
     __shared__ int abortFlag, issuedX, issuedG, consumedX, consumedG;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tap0 = S::kGroups == 1 ? 0 : blockIdx.y * S::kTaps;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
+    // group 0 (CTAs 0 .. ctas0 - 1): kernel columns 0 .. kCols0 - 1 and the bias; group 1: the last column
+    const bool second = S::kGroups > 1 && (int)blockIdx.x >= ctas0;
+    const int cta = second ? (int)blockIdx.x - ctas0 : (int)blockIdx.x, ctas = second ? (int)gridDim.x - ctas0 : ctas0;
     for (int i = tid; i < S::kOnes / 2; i += blockDim.x) reinterpret_cast<bf16*>(ones)[i] = __float2bfloat16(1.0f);
     if (tid == 0) {
         for (int k = 0; k < S::kXRing; ++k) {
@@ -487,7 +506,7 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
     const uint32_t tmem = tmem_base;
     volatile int* abort = &abortFlag;
     const int strips = (W + kStripPx - 1) / kStripPx;
-    const long long rows = (long long)B * strips * H, r0 = rows * blockIdx.x / gridDim.x, r1 = rows * (blockIdx.x + 1) / gridDim.x;
+    const long long rows = (long long)B * strips * H, r0 = rows * cta / ctas, r1 = rows * (cta + 1) / ctas;
     // the run of rows from r on that lie in one strip of one image: its image, first pixel, first row, length
     auto run_at = [&](long long r, int& b, int& x0, int& y0) {
         const long long bs = r / H;
@@ -496,73 +515,90 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
         y0 = (int)(r % H);
         return (int)min((long long)(H - y0), r1 - r);
     };
-    if (warp == 0) {
-        if (lane == 0) {  // copies: x rows y0 - 1 .. y0 + n, g rows y0 .. y0 + n - 1 of each run
-            int sx = 0, sg = 0;
-            bool ok = true;
-            for (long long r = r0; r < r1 && ok;) {
-                int b, x0, y0;
-                const int n = run_at(r, b, x0, y0);
-                for (int k = 0; k < n + 2 && ok; ++k) {
-                    const int xs = sx % S::kXRing;
-                    ok = sx < S::kXRing || mbar_wait_or_abort(&xEmpty[xs], (uint32_t)((sx / S::kXRing - 1) & 1), abort, status);
-                    if (!ok) break;
+    if (warp == 0) {  // copies: x rows y0 - 1 .. y0 + n, g rows y0 .. y0 + n - 1 of each run
+        int sx = 0, sg = 0;
+        bool ok = true;
+        for (long long r = r0; r < r1 && ok;) {
+            int b, x0, y0;
+            const int n = run_at(r, b, x0, y0);
+            for (int k = 0; k < n + 2; ++k) {
+                const int xs = sx % S::kXRing;
+                ok = sx < S::kXRing || warp_wait_or_abort(&xEmpty[xs], (uint32_t)((sx / S::kXRing - 1) & 1), abort, status);
+                if (!ok) break;
+                ++sx;
+                if (elect_one()) {
                     mbar_expect_tx(&xFull[xs], S::kXTx);
-#pragma unroll 1
+#pragma unroll
                     for (int cc = 0; cc < CIN / 8; ++cc)
                         tma_load_4d(xring + xs * S::kXBytes + cc * kRowPlane, &mapX, cc * 8, x0 - 1, y0 - 1 + k, b, &xFull[xs]);
-                    issuedX = ++sx;
-                    if (k >= n) continue;
-                    const int gs = sg % S::kGRing;
-                    ok = sg < S::kGRing || mbar_wait_or_abort(&gEmpty[gs], (uint32_t)((sg / S::kGRing - 1) & 1), abort, status);
-                    if (!ok) break;
+                    issuedX = sx;
+                }
+                __syncwarp();
+                if (k >= n) continue;
+                const int gs = sg % S::kGRing;
+                ok = sg < S::kGRing || warp_wait_or_abort(&gEmpty[gs], (uint32_t)((sg / S::kGRing - 1) & 1), abort, status);
+                if (!ok) break;
+                ++sg;
+                if (elect_one()) {
                     mbar_expect_tx(&gFull[gs], S::kGTx);
-#pragma unroll 1
+#pragma unroll
                     for (int cc = 0; cc < COUT / 8; ++cc)
                         tma_load_4d(gring + gs * S::kGBytes + cc * S::kGPlane, &mapG, cc * 8, x0, y0 + k, b, &gFull[gs]);
-                    issuedG = ++sg;
+                    issuedG = sg;
                 }
-                r += n;
+                __syncwarp();
             }
+            r += n;
         }
-    } else if (warp == 1) {
-        if (lane == 0) {  // MMA issuer: output row j of a run takes x rows j, j + 1, j + 2 of the run
-            const uint64_t a0 = umma_desc(smem_u32(gring), 128, S::kGPlane), b0 = umma_desc(smem_u32(xring), 128, kRowPlane),
-                           one = umma_desc(smem_u32(ones), 128, 256);
-            constexpr uint32_t id = umma_idesc(128, CIN, true, true), idOne = umma_idesc(128, 16, true, true);
-            int sx = 0, sg = 0, seen = 0;  // first x row of the run, g row, x rows waited for
-            uint32_t acc = 0;
-            bool ok = true;
-            for (long long r = r0; r < r1 && ok;) {
-                int b, x0, y0;
-                const int n = run_at(r, b, x0, y0);
-                for (int j = 0; j < n && ok; ++j, ++sg) {
-                    for (; seen < sx + j + 3 && ok; ++seen)
-                        ok = mbar_wait_or_abort(&xFull[seen % S::kXRing], (uint32_t)((seen / S::kXRing) & 1), abort, status);
+    } else if (warp == 1) {  // MMA issuer: output row j of a run takes x rows j, j + 1, j + 2 of the run
+        const uint64_t a0 = umma_desc(smem_u32(gring), 128, S::kGPlane), b0 = umma_desc(smem_u32(xring), 128, kRowPlane),
+                       one = umma_desc(smem_u32(ones), 128, 256);
+        constexpr uint32_t id1 = umma_idesc(128, CIN, true, true), id2 = umma_idesc(128, 2 * CIN, true, true),
+                           id3 = umma_idesc(128, 3 * CIN, true, true), idOne = umma_idesc(128, 16, true, true);
+        int sx = 0, sg = 0, seen = 0;  // first x row of the run, g row, x rows waited for
+        uint32_t acc = 0;
+        bool ok = true;
+        for (long long r = r0; r < r1 && ok;) {
+            int b, x0, y0;
+            const int n = run_at(r, b, x0, y0);
+            for (int j = 0; j < n; ++j, ++sg) {
+                for (; seen < sx + j + 3 && ok; ++seen)
+                    ok = warp_wait_or_abort(&xFull[seen % S::kXRing], (uint32_t)((seen / S::kXRing) & 1), abort, status);
+                ok = ok && warp_wait_or_abort(&gFull[sg % S::kGRing], (uint32_t)((sg / S::kGRing) & 1), abort, status);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
                     consumedX = seen;
-                    ok = ok && mbar_wait_or_abort(&gFull[sg % S::kGRing], (uint32_t)((sg / S::kGRing) & 1), abort, status);
-                    if (!ok) break;
                     consumedG = sg + 1;
-                    tc_fence_after();
                     const uint64_t ad = a0 + (uint64_t)(((sg % S::kGRing) * S::kGBytes) >> 4);
-                    uint64_t bd[3];
+                    const int slot = (sx + j) % S::kXRing, ahead = S::kXRing - slot;  // slots before the ring wraps
+                    const uint64_t bd = b0 + (uint64_t)((slot * S::kXBytes) >> 4);
+                    // columns c .. of the kernel from the first one of this group on
+                    auto column = [&](int c, int dx) {
 #pragma unroll
-                    for (int dy = 0; dy < 3; ++dy) bd[dy] = b0 + (uint64_t)((((sx + j + dy) % S::kXRing) * S::kXBytes) >> 4);
+                        for (int kk = 0; kk < kStripPx / 16; ++kk) {
+                            const uint64_t ak = ad + (uint64_t)(16 * kk), off = (uint64_t)(16 * kk + dx);
+                            const uint32_t d = tmem + (uint32_t)(c * 3 * CIN), go = kk == 0 ? acc : 1u;
+                            if (ahead >= 3) {
+                                umma(d, ak, bd + off, id3, go);
+                            } else if (ahead == 2) {
+                                umma(d, ak, bd + off, id2, go);
+                                umma(d + 2 * CIN, ak, b0 + off, id1, go);
+                            } else {
+                                umma(d, ak, bd + off, id1, go);
+                                umma(d + CIN, ak, b0 + off, id2, go);
+                            }
+                        }
+                    };
+                    if (second) {
+                        column(0, S::kCols0);
+                    } else {
 #pragma unroll
-                    for (int t = 0; t < S::kTaps; ++t) {
-                        const int tap = tap0 + t;
-                        if (S::kGroups > 1 && tap >= 9) break;
-                        const int dy = tap / 3, dx = tap - 3 * dy;
-                        const uint64_t bt = (dy == 0 ? bd[0] : dy == 1 ? bd[1] : bd[2]) + (uint64_t)dx;
+                        for (int c = 0; c < S::kCols0; ++c) column(c, c);
 #pragma unroll
                         for (int kk = 0; kk < kStripPx / 16; ++kk)
-                            umma(tmem + (uint32_t)(t * CIN), ad + (uint64_t)(16 * kk), bt + (uint64_t)(16 * kk), id, kk == 0 ? acc : 1u);
+                            umma(tmem + (uint32_t)S::kBiasCol, ad + (uint64_t)(16 * kk), one, idOne, kk == 0 ? acc : 1u);
                     }
-                    if (tap0 == 0)
-#pragma unroll
-                        for (int kk = 0; kk < kStripPx / 16; ++kk)
-                            umma(tmem + (uint32_t)(S::kTaps * CIN), ad + (uint64_t)(16 * kk), one, idOne, kk == 0 ? acc : 1u);
-                    acc = 1u;
                     umma_commit(&gEmpty[sg % S::kGRing]);
                     umma_commit(&xEmpty[(sx + j) % S::kXRing]);
                     if (j == n - 1) {
@@ -570,12 +606,15 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
                         umma_commit(&xEmpty[(sx + n + 1) % S::kXRing]);
                     }
                 }
-                sx += n + 2;
-                r += n;
+                __syncwarp();
+                acc = 1u;
             }
-            umma_commit(&drain);  // completes when every MMA issued above has
-            mbar_wait(&drain, 0u, nullptr);
+            sx += n + 2;
+            r += n;
         }
+        if (elect_one()) umma_commit(&drain);  // completes when every MMA issued above has
+        __syncwarp();
+        mbar_wait(&drain, 0u, nullptr);
     }
     __syncthreads();
     // an abandoned pipeline may still have copies in flight: wait for them (bounded) before the shared
@@ -586,25 +625,26 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
     }
     __syncthreads();
     tc_fence_after();
-    // partial[blockIdx.x][co][tap][ci] for this CTA's taps (zero when it had no row)
+    // partial[cta][co][tap][ci] for this CTA's taps (zero when it had no row)
     const int co = warp * 32 + lane;
     const bool some = r1 > r0 && !abortFlag;
-    float* out = partial + (size_t)blockIdx.x * COUT * 9 * CIN;
+    float* out = partial + (size_t)cta * COUT * 9 * CIN;
     if (warp * 32 < COUT) {
         const uint32_t row = tmem + ((uint32_t)(warp * 32) << 16);
         float v[16];
+        const int cols = second ? 3 - S::kCols0 : S::kCols0, dx0 = second ? S::kCols0 : 0;
 #pragma unroll 1
-        for (int t = 0; t < S::kTaps && tap0 + t < 9; ++t)
+        for (int t = 0; t < 3 * cols; ++t)
 #pragma unroll 1
             for (int c0 = 0; c0 < CIN; c0 += 16) {
                 tmem_ld16(row + (uint32_t)(t * CIN + c0), v);
                 if (co < COUT)
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) out[((size_t)co * 9 + tap0 + t) * CIN + c0 + q] = some ? v[q] : 0.0f;
+                    for (int q = 0; q < 16; ++q) out[((size_t)co * 9 + (t % 3) * 3 + dx0 + t / 3) * CIN + c0 + q] = some ? v[q] : 0.0f;
             }
-        if (tap0 == 0) {
-            tmem_ld16(row + (uint32_t)(S::kTaps * CIN), v);
-            if (co < COUT) biasPartial[(size_t)blockIdx.x * COUT + co] = some ? v[0] : 0.0f;
+        if (!second) {
+            tmem_ld16(row + (uint32_t)S::kBiasCol, v);
+            if (co < COUT) biasPartial[(size_t)cta * COUT + co] = some ? v[0] : 0.0f;
         }
     }
     tc_fence_before();
@@ -652,7 +692,7 @@ __global__ void __launch_bounds__(256) k_filter_finish(const FilterFinish f) {
         const size_t stride = weight ? (size_t)L.cout * 9 * L.cin : (size_t)L.cout;
         const float* p = weight ? L.partial + ((size_t)co * 9 + tap) * L.cin + ci : L.biasPartial + co;
 #pragma unroll 8
-        for (int c = q; c < L.ctas; c += 4) s += p[stride * c];
+        for (int c = q, n = weight && tap % 3 == 2 ? L.ctas[1] : L.ctas[0]; c < n; c += 4) s += p[stride * c];
     }
     part[q][j] = s;
     __syncthreads();
@@ -834,8 +874,13 @@ cudaError_t dw_launch(const bf16* x, const bf16* g, int B, int H, int W, float* 
     cudaError_t e = patch_map(&mx, x, B, H, W, CIN);
     if (e == cudaSuccess) e = patch_map(&mg, g, B, H, W, COUT, kStripPx);
     if (e != cudaSuccess) return e;
-    *ctas = std::max(1, filter_dw_ctas() / S::kGroups);
-    k_filter_dw<CIN, COUT><<<dim3(*ctas, S::kGroups), 128, S::kSmem, s>>>(mx, mg, B, H, W, partial, biasPartial, status);
+    // one CTA per SM; two groups take half each: both copy every row, which bounds them (two thirds for the
+    // two columns: 106 us for 64 -> 64 on 32 crops against 98)
+    const int all = filter_dw_ctas();
+    ctas[0] = S::kGroups == 1 ? all : std::max(1, all / 2);
+    ctas[1] = S::kGroups == 1 ? all : std::max(1, all - ctas[0]);
+    const int grid = S::kGroups == 1 ? all : ctas[0] + ctas[1];
+    k_filter_dw<CIN, COUT><<<grid, 128, S::kSmem, s>>>(mx, mg, B, H, W, ctas[0], partial, biasPartial, status);
     count_launch();
     return cudaGetLastError();
 }

@@ -311,9 +311,9 @@ rg_status rg_filter_train_step(rg_filter* f, const void* d_input, const float* d
     auto dW = [&](int l, const void* x, const void* g) -> rg_status {
         FilterFinish::Layer& L = fin.layer[l];
         float* bias = room + (size_t)filter_dw_ctas() * kCout[l] * 9 * kCin[l];
-        FCK(filter_dw(kCin[l], kCout[l], x, g, (int)B, (int)H, (int)W, room, bias, &L.ctas, st, f->stream));
-        L = {room, bias, f->wf[l].as<bf>(), l > 0 ? f->wt[l].as<bf>() : nullptr, f->bias[l].as<float>(), L.ctas, kCout[l], kCin[l], kCoutR[l], kCinR[l],
-             f->offW[l], f->offB[l], 0};
+        L = {room, bias, f->wf[l].as<bf>(), l > 0 ? f->wt[l].as<bf>() : nullptr, f->bias[l].as<float>(), kCout[l], kCin[l], kCoutR[l], kCinR[l],
+             f->offW[l], f->offB[l], {0, 0}, 0};
+        FCK(filter_dw(kCin[l], kCout[l], x, g, (int)B, (int)H, (int)W, room, bias, L.ctas, st, f->stream));
         room = bias + (size_t)filter_dw_ctas() * kCout[l];
         return RG_OK;
     };

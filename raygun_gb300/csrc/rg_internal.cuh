@@ -349,7 +349,8 @@ struct FilterConvArgs {
 };
 cudaError_t filter_conv(int cin, int cout, const FilterConvArgs& a, cudaStream_t s);
 int filter_dw_ctas();  // most CTAs whose partials a weight gradient leaves
-// partial[cta][cout][9][cin] and biasPartial[cta][cout] of *ctas CTAs (x, g 16-byte aligned)
+// partial[cta][cout][9][cin] and biasPartial[cta][cout] of ctas[0] CTAs, ctas[1] for kernel column 2 (x, g
+// 16-byte aligned)
 cudaError_t filter_dw(int cin, int cout, const void* x, const void* g, int B, int H, int W, float* partial, float* biasPartial, int* ctas,
                       int* status, cudaStream_t s);
 cudaError_t filter_pack(const float* W, int coutReal, int cinReal, int cin, int cout, int transposed, void* out, cudaStream_t s);
@@ -359,7 +360,8 @@ struct FilterFinish {
         const float *partial, *biasPartial;
         __nv_bfloat16 *packed, *packedT;  // packedT nullable (the first layer has no data gradient)
         float* bias;                      // padded bias
-        int ctas, cout, cin, coutReal, cinReal, offW, offB;
+        int cout, cin, coutReal, cinReal, offW, offB;
+        int ctas[2];                      // CTAs with partials: kernel columns 0 and 1, column 2
         int block0;                       // set by filter_finish
     } layer[5];
     float *w, *grad, *m, *v;
