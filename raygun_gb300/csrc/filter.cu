@@ -6,10 +6,11 @@
 //   layers: 16(12 used) -> 32 -> 64 -> 64 -> 32 -> 16(3 used), ReLU after layers 1-4, the output of
 //   layer 1 added to the input of layer 5 (skip), every layer at full resolution.
 // Activations are BF16 NHWC, accumulation FP32 in tensor memory.  Each convolution is an implicit
-// GEMM: a CTA takes a tile of 2 image rows x 128 pixels (M = 128 output pixels per row), stages the
-// 4 x 130 input patch in shared memory as channel-chunk planes [chunk][pixel][8 channels] (16 B per
-// pixel and chunk) and issues, per row, 9 taps x Cin/16 tcgen05.mma (kind::f16, BF16 x BF16 -> F32)
-// whose A descriptors point straight into the patch at the tap's offset: no im2col copy.  The data
+// GEMM over strips of 128 pixels (M): input rows of 130 pixels lie in shared memory as the TMA writes
+// them, pixel after pixel, swizzled over a pixel's channels, and a tap's A descriptor starts at the tap's
+// pixel: no im2col copy.  Rows in boxes of 16 bytes (8 channels, one plane a box) took 1.3 - 1.5 times as
+// long to copy: 0.57 us against 0.40 us a row of 64 channels and SM, and 470 us against 433 us for the
+// network at 1080p.  The data
 // gradient is the same kernel on transposed, flipped weights; the weight gradient is a GEMM over
 // pixels with both operands MN-major (channels contiguous), accumulated in tensor memory per CTA and
 // reduced across CTAs in a fixed order (deterministic).
@@ -35,6 +36,17 @@ using bf16 = __nv_bfloat16;
 __device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+}
+
+// the same with a swizzle whose span is a row of C BF16 channels (32, 64 or 128 bytes), as the TMA writes
+// rows of pixels: the 16-byte chunks of a row are permuted by the row's address, so an operand may start
+// at any pixel of a row (its start address carries the pixel) and at any 32-byte step inside it.
+// K-major (channels are K): sbo = 8 pixels, lbo unused.  MN-major (pixels are K): sbo = 8 pixels, lbo = the
+// next C channels.
+template <int C>
+__device__ __forceinline__ uint64_t umma_desc_rows(uint32_t addr, uint32_t lbo) {
+    static_assert(C == 16 || C == 32 || C == 64, "swizzle spans");
+    return umma_desc(addr, lbo, 8 * C * 2) | ((uint64_t)(C == 64 ? 2 : C == 32 ? 4 : 6) << 61);
 }
 
 // instruction descriptor of tcgen05.mma kind::f16: D F32, A and B BF16, M x N, operand majors
@@ -81,8 +93,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // Row-streaming convolution.  A work item is a strip of 128 output pixels x a segment of rows of
 // one image; a CTA walks its items down the rows, three output rows (a group) at a time.  Input rows
 // (130 pixels: the strip and a 1-pixel halo, zero outside the image) stream through a ring of
-// shared-memory slots, each row loaded once per item as channel-chunk planes [chunk][pixel][8].  Input
-// row i feeds output rows i+1, i, i-1 through the kernel rows dy = 0, 1, 2, so a group's accumulator is
+// shared-memory slots, each row loaded once per item.  Input row i feeds output rows i+1, i, i-1 through the kernel rows dy = 0, 1, 2, so a group's accumulator is
 // a window of three adjacent TMEM blocks and each of its five input rows r-1 .. r+3 feeds it with ONE
 // tcgen05.mma per column tap dx and 16-channel step (M = 128 pixels, N = COUT, 2 COUT, 3 COUT, 2 COUT,
 // COUT), the B operand stacking the kernel rows' weights.  62 MMAs instead of 108 per 3 rows of a
@@ -96,7 +107,8 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 //              pixel with one 32-byte store, a whole sector (through a swizzled shared-memory stage and
 //              16-byte stores the epilogue took 70 - 90 % of the time of the layers into 32 and 64 channels).
 constexpr int kStripPx = 128, kRowW = kStripPx + 2;
-constexpr int kRowPlane = 2176;  // 130 pixels x 16 B rounded up to 128 B (TMA destination alignment)
+// bytes of a ring slot: `pixels` pixels of C channels, rounded up to the period of the widest swizzle
+constexpr int slot_bytes(int pixels, int C) { return (pixels * C * 2 + 1023) / 1024 * 1024; }
 constexpr int kEpiWarps = 8;
 constexpr int kConvThreads = 32 * (2 + kEpiWarps);
 constexpr int kGroupRows = 3;
@@ -107,13 +119,13 @@ struct ConvShape {
     static constexpr int kRing = 8;                               // input row slots
     static constexpr int kWin = 3 * COUT;                         // TMEM columns of one group's window
     static constexpr int kWindows = 3 * COUT * 4 <= 512 ? 4 : 2;  // accumulator windows (groups in flight)
-    static constexpr int kRowBytes = CC * kRowPlane;              // one slot
-    static constexpr uint32_t kRowTx = CC * kRowW * 16;           // bytes the TMA writes per row
+    static constexpr int kRowBytes = slot_bytes(kRowW, CIN);      // one slot
+    static constexpr uint32_t kRowTx = kRowW * CIN * 2;           // bytes the TMA writes per row
     static constexpr int kWeightBytes = 9 * CIN * COUT * 2;       // [dx][ci/8][kernel row 2, 1, 0][co][8]
     static constexpr int kSmem = kWeightBytes + kRing * kRowBytes + 1024;
     static constexpr uint32_t kCols = kWindows * kWin <= 32 ? 32 : (kWindows * kWin <= 64 ? 64 : (kWindows * kWin <= 128 ? 128 : (kWindows * kWin <= 256 ? 256 : 512)));
     static_assert(CIN % 16 == 0 && COUT % 16 == 0 && kWin <= 256 && kWindows * kWin <= 512, "shape");
-    static_assert(kWeightBytes % 128 == 0, "ring slots 128-byte aligned");
+    static_assert(kWeightBytes % 1024 == 0, "ring slots aligned to the swizzle period");
 };
 
 // bounded wait that also gives up when another role has given up (abort flag in shared memory)
@@ -254,9 +266,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
                 if (!ok) break;
                 if (elect_one()) {
                     mbar_expect_tx(&full[slot], S::kRowTx);
-#pragma unroll
-                    for (int cc = 0; cc < CC; ++cc)
-                        tma_load_4d(ring + slot * S::kRowBytes + cc * kRowPlane, &tmapX, cc * 8, x0 - 1, ys - 1 + k, b, &full[slot]);
+                    tma_load_4d(ring + slot * S::kRowBytes, &tmapX, 0, x0 - 1, ys - 1 + k, b, &full[slot]);
                     issuedRows = seq + 1;
                 }
                 __syncwarp();
@@ -265,7 +275,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
     } else if (warp == 1) {  // MMA issuer
         // descriptors: the start address sits in the low 14 bits (address / 16) and every operand lies
         // below 256 KB, so offsets add to it without a carry
-        const uint64_t adesc0 = umma_desc(smem_u32(ring), kRowPlane, 128), bdesc0 = umma_desc(smem_u32(wsm), 3 * COUT * 16, 128);
+        const uint64_t adesc0 = umma_desc_rows<CIN>(smem_u32(ring), 16), bdesc0 = umma_desc(smem_u32(wsm), 3 * COUT * 16, 128);
         constexpr uint32_t id1 = umma_idesc(128, COUT, false, false), id2 = umma_idesc(128, 2 * COUT, false, false),
                            id3 = umma_idesc(128, 3 * COUT, false, false);
         int base = 0, waited = 0, g = 0;  // first input row of the item, input rows waited for, groups issued
@@ -291,7 +301,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
                     for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
                         for (int kk = 0; kk < KK; ++kk) {
-                            const uint64_t aoff = (uint64_t)((2 * kk * kRowPlane + dx * 16) >> 4);
+                            const uint64_t aoff = (uint64_t)((kk * 32 + dx * CIN * 2) >> 4);
                             const uint64_t bk = bdesc0 + (uint64_t)((dx * CC + 2 * kk) * 3 * COUT);
                             const bool f = dx == 0 && kk == 0;  // the step where rows r+1 and r+2 start
                             // input r - 1: row r (kernel row 0)
@@ -437,35 +447,31 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_co
 
 // ---- weight and bias gradients: dW[co][tap][ci] = sum_p g[p][co] * x[p + tap][ci], db[co] = sum_p g[p][co]
 // D (M = 128 rows: output channels) x (N = CIN per tap) over K = pixels, both operands MN-major: A = a
-// row of g as channel-chunk planes [chunk][pixel][8], B = a row of x in the same layout at the tap's
-// pixel offset.  The bias sum is one more product, with a tile of ones as B.
+// row of g, B = a row of x from the tap's pixel on, both as the TMA writes them.  The bias sum is one more product, with a tile of ones as B.
 // A CTA takes an equal run of the (image, strip of 128 pixels, row) list, so all CTAs end together, and
 // streams it: each row of g once, each row of x once (plus two rows where a run starts or enters the next
 // strip), through rings of shared-memory slots filled by TMA, while one thread issues the MMAs with
-// constant descriptor offsets; everything accumulates in tensor memory.  The planes of the three x rows
-// that an output row needs lie one after another in the ring, so one MMA (M = 128, N = 3 CIN, K = 16)
-// takes the three taps of a column: reading A (4 KB) costs about 80 clocks an MMA whatever N is, and nine
-// MMAs of N = CIN for the nine taps took 92 - 142 us a layer on 32 crops of 128 x 128.  Where the ring
-// wraps inside the three rows, two MMAs share them.  Rows of A beyond COUT read whatever lies behind the
-// slot; their results are not read.  With 64 input channels the nine taps (576 columns) exceed tensor
+// constant descriptor offsets; everything accumulates in tensor memory.  The three x rows that an output
+// row needs lie one after another in the ring, so one MMA (M = 128, N = 3 CIN, K = 16) takes the three
+// taps of a kernel column: 24 MMAs a row instead of 72.  Where the ring wraps inside the three rows, two
+// MMAs share them.  Rows of A beyond COUT repeat its channels; their results are not read.  With 64 input channels the nine taps (576 columns) exceed tensor
 // memory: half of the CTAs take columns 0 and 1 of the kernel, the others column 2.
-// Those crops, 64 -> 64: 410 us with one tile staged, multiplied and waited for at a time by one warp
-// quartet, 98 us now, bias sum (113 us in a kernel of its own) included.
+// 32 crops of 128 x 128, 64 -> 64: 410 us with one tile staged, multiplied and waited for at a time by one warp
+// quartet, 96 us now, bias sum (113 us in a kernel of its own) included.
 template <int CIN, int COUT>
 struct DwShape {
     static constexpr int kGroups = CIN == 64 ? 2 : 1;
     static constexpr int kCols0 = CIN == 64 ? 2 : 3;  // kernel columns of the first group
-    static constexpr int kGPlane = kStripPx * 16, kGBytes = (COUT / 8) * kGPlane, kXBytes = (CIN / 8) * kRowPlane;
+    static constexpr int kGBytes = slot_bytes(kStripPx, COUT), kXBytes = slot_bytes(kRowW, CIN);
     static constexpr int kGRing = 4, kXRing = 8;
-    static constexpr uint32_t kGTx = kGBytes, kXTx = (CIN / 8) * kRowW * 16;
+    static constexpr uint32_t kGTx = kStripPx * COUT * 2, kXTx = kRowW * CIN * 2;
     static constexpr int kOnes = 2 * 256;  // B tile of ones: [2 chunks][16 pixels][8]
     static constexpr int kUsed = kGRing * kGBytes + kXRing * kXBytes + kOnes;
-    static constexpr int kReach = (kGRing - 1) * kGBytes + 16 * kGPlane;  // A's 128 rows from the last slot
     // at least 120 KB: one CTA holds an SM (and its tensor memory) at a time
-    static constexpr int kSmem = (kUsed > kReach ? kUsed : kReach) + 1024 > 120 * 1024 ? (kUsed > kReach ? kUsed : kReach) + 1024 : 120 * 1024;
+    static constexpr int kSmem = kUsed + 1024 > 120 * 1024 ? kUsed + 1024 : 120 * 1024;
     static constexpr int kBiasCol = kCols0 * 3 * CIN;  // tensor-memory column of the bias sums
     static constexpr uint32_t kCols = kBiasCol + 16 <= 256 ? 256 : 512;
-    static_assert(kBiasCol + 16 <= 512 && 3 * CIN <= 256 && kGBytes % 128 == 0 && kXBytes % 128 == 0 && kSmem <= 227 * 1024, "shape");
+    static_assert(kBiasCol + 16 <= 512 && 3 * CIN <= 256 && kSmem <= 227 * 1024, "shape");
 };
 
 template <int CIN, int COUT>
@@ -528,9 +534,7 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
                 ++sx;
                 if (elect_one()) {
                     mbar_expect_tx(&xFull[xs], S::kXTx);
-#pragma unroll
-                    for (int cc = 0; cc < CIN / 8; ++cc)
-                        tma_load_4d(xring + xs * S::kXBytes + cc * kRowPlane, &mapX, cc * 8, x0 - 1, y0 - 1 + k, b, &xFull[xs]);
+                    tma_load_4d(xring + xs * S::kXBytes, &mapX, 0, x0 - 1, y0 - 1 + k, b, &xFull[xs]);
                     issuedX = sx;
                 }
                 __syncwarp();
@@ -541,9 +545,7 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
                 ++sg;
                 if (elect_one()) {
                     mbar_expect_tx(&gFull[gs], S::kGTx);
-#pragma unroll
-                    for (int cc = 0; cc < COUT / 8; ++cc)
-                        tma_load_4d(gring + gs * S::kGBytes + cc * S::kGPlane, &mapG, cc * 8, x0, y0 + k, b, &gFull[gs]);
+                    tma_load_4d(gring + gs * S::kGBytes, &mapG, 0, x0, y0 + k, b, &gFull[gs]);
                     issuedG = sg;
                 }
                 __syncwarp();
@@ -551,7 +553,8 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
             r += n;
         }
     } else if (warp == 1) {  // MMA issuer: output row j of a run takes x rows j, j + 1, j + 2 of the run
-        const uint64_t a0 = umma_desc(smem_u32(gring), 128, S::kGPlane), b0 = umma_desc(smem_u32(xring), 128, kRowPlane),
+        // A: COUT channels, repeated over the 128 rows (lbo 0); B: CIN channels of consecutive slots
+        const uint64_t a0 = umma_desc_rows<COUT>(smem_u32(gring), 0), b0 = umma_desc_rows<CIN>(smem_u32(xring), S::kXBytes),
                        one = umma_desc(smem_u32(ones), 128, 256);
         constexpr uint32_t id1 = umma_idesc(128, CIN, true, true), id2 = umma_idesc(128, 2 * CIN, true, true),
                            id3 = umma_idesc(128, 3 * CIN, true, true), idOne = umma_idesc(128, 16, true, true);
@@ -577,7 +580,7 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
                     auto column = [&](int c, int dx) {
 #pragma unroll
                         for (int kk = 0; kk < kStripPx / 16; ++kk) {
-                            const uint64_t ak = ad + (uint64_t)(16 * kk), off = (uint64_t)(16 * kk + dx);
+                            const uint64_t ak = ad + (uint64_t)(2 * COUT * kk), off = (uint64_t)((16 * kk + dx) * CIN / 8);
                             const uint32_t d = tmem + (uint32_t)(c * 3 * CIN), go = kk == 0 ? acc : 1u;
                             if (ahead >= 3) {
                                 umma(d, ak, bd + off, id3, go);
@@ -597,7 +600,7 @@ __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CU
                         for (int c = 0; c < S::kCols0; ++c) column(c, c);
 #pragma unroll
                         for (int kk = 0; kk < kStripPx / 16; ++kk)
-                            umma(tmem + (uint32_t)S::kBiasCol, ad + (uint64_t)(16 * kk), one, idOne, kk == 0 ? acc : 1u);
+                            umma(tmem + (uint32_t)S::kBiasCol, ad + (uint64_t)(2 * COUT * kk), one, idOne, kk == 0 ? acc : 1u);
                     }
                     umma_commit(&gEmpty[sg % S::kGRing]);
                     umma_commit(&xEmpty[(sx + j) % S::kXRing]);
@@ -801,18 +804,19 @@ __global__ void k_filter_target(const uint2* __restrict__ rough, size_t P, float
 }
 
 
-// tensor map of an NHWC BF16 activation [B][H][W][C]: boxes of 8 channels x `pixels` pixels x 1 row
-cudaError_t patch_map(CUtensorMap* map, const void* x, int B, int H, int W, int C, int pixels = kRowW) {
+// tensor map of an NHWC BF16 activation [B][H][W][C]: boxes of one row of `pixels` pixels, all channels,
+// swizzled over a pixel's channels
+cudaError_t row_map(CUtensorMap* map, const void* x, int B, int H, int W, int C, int pixels) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return cudaErrorNotSupported;
     if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0) return cudaErrorMisalignedAddress;
     const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
     const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    const cuuint32_t box[4] = {8, (cuuint32_t)pixels, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)C, (cuuint32_t)pixels, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUtensorMapSwizzle swizzle = C == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : C == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
@@ -847,7 +851,7 @@ cudaError_t conv_launch(const FilterConvArgs& a, cudaStream_t s) {
     }
     if (a.B <= 0 || a.H <= 0 || a.W <= 0) return cudaSuccess;
     CUtensorMap map;
-    cudaError_t e = patch_map(&map, a.x, a.B, a.H, a.W, CIN);
+    cudaError_t e = row_map(&map, a.x, a.B, a.H, a.W, CIN, kRowW);
     if (e != cudaSuccess) return e;
     // segments of rows (a multiple of 3): about two items per CTA, at least 9 rows (each item re-reads
     // 2 halo rows)
@@ -871,11 +875,11 @@ cudaError_t dw_launch(const bf16* x, const bf16* g, int B, int H, int W, float* 
         attr.store(true, std::memory_order_release);
     }
     CUtensorMap mx, mg;
-    cudaError_t e = patch_map(&mx, x, B, H, W, CIN);
-    if (e == cudaSuccess) e = patch_map(&mg, g, B, H, W, COUT, kStripPx);
+    cudaError_t e = row_map(&mx, x, B, H, W, CIN, kRowW);
+    if (e == cudaSuccess) e = row_map(&mg, g, B, H, W, COUT, kStripPx);
     if (e != cudaSuccess) return e;
     // one CTA per SM; two groups take half each: both copy every row, which bounds them (two thirds for the
-    // two columns: 106 us for 64 -> 64 on 32 crops against 98)
+    // two columns: 106 us for 64 -> 64 on 32 crops against 96)
     const int all = filter_dw_ctas();
     ctas[0] = S::kGroups == 1 ? all : std::max(1, all / 2);
     ctas[1] = S::kGroups == 1 ? all : std::max(1, all - ctas[0]);
