@@ -327,9 +327,6 @@ cudaError_t launch_resolve_job(const float4* samples, const JobDesc& hostJob, ui
 // 48 when p.countVisits
 cudaError_t launch_trace_queue(const TraceParams& p, const float* rays, uint32_t n, float* tuv, uint32_t* ids, int depth,
                                cudaStream_t s);
-// closest hits of n rays with a traversal stack of `depth` (16, 24, 32 or 48) entries
-cudaError_t launch_trace_rays(const DevScene& sc, const float* rays, uint32_t n, float* tuv, uint32_t* ids,
-                              unsigned long long* counters, int depth, cudaStream_t s);
 
 // ---- learned roughness filter (filter.cu) ----
 // one 3x3 convolution of NHWC BF16 activations (x 16-byte aligned): v = conv(x, w) + bias, then

@@ -2492,29 +2492,6 @@ __global__ void __launch_bounds__(256) k_sort_scatter(const TraceParams P, int q
     }
 }
 
-template <int DEPTH>
-__global__ void __launch_bounds__(kTraceThreads) k_trace_rays(const __grid_constant__ DevScene sc, const float* __restrict__ rays,
-                                                               uint32_t n, float* __restrict__ tuv, uint32_t* __restrict__ ids,
-                                                               unsigned long long* counters) {
-    RG_DECLARE_SMEM_STACK(stk, kTraceThreads, DEPTH);
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const float* r = rays + 8 * (size_t)k;
-    VisitCounts vc = {0, 0, 0};
-    Hit h = closest_hit<false>(sc, r[0], r[1], r[2], r[4], r[5], r[6], r[3], r[7], stk, vc, counters);
-    if (vc.overflow) {  // rays re-traced deep, counted like the frame's
-        atomicAdd(counters + 6, vc.overflow);
-        atomicAdd(counters + 14, vc.overflow);
-    }
-    if (h.hit) {
-        tuv[3 * k] = h.t; tuv[3 * k + 1] = h.u; tuv[3 * k + 2] = h.v;
-        ids[2 * k] = h.inst; ids[2 * k + 1] = h.prim;
-    } else {
-        tuv[3 * k] = tuv[3 * k + 1] = tuv[3 * k + 2] = 0.0f;
-        ids[2 * k] = ids[2 * k + 1] = 0xFFFFFFFFu;
-    }
-}
-
 }  // namespace
 
 cudaError_t launch_trace(const TraceParams& p, cudaStream_t s) {
@@ -2850,21 +2827,6 @@ cudaError_t capture_trace_batch(const TraceParams& p0, const TraceTune& tune, co
 cudaError_t launch_resolve_job(const float4* samples, const JobDesc& j, uint2* base, uint2* normal, uint2* rough, cudaStream_t s) {
     dim3 grid((j.W + 31) / 32, (j.H + 7) / 8);
     k_resolve_job<<<grid, 256, 0, s>>>(samples + 3 * (size_t)j.sampleBase, j.W, j.H, j.S, base, normal, rough);
-    count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_trace_rays(const DevScene& sc, const float* rays, uint32_t n, float* tuv, uint32_t* ids,
-                              unsigned long long* counters, int depth, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    const uint32_t g = (n + kTraceThreads - 1) / kTraceThreads;
-    switch (depth) {
-        case 16: k_trace_rays<16><<<g, kTraceThreads, 0, s>>>(sc, rays, n, tuv, ids, counters); break;
-        case 24: k_trace_rays<24><<<g, kTraceThreads, 0, s>>>(sc, rays, n, tuv, ids, counters); break;
-        case 32: k_trace_rays<32><<<g, kTraceThreads, 0, s>>>(sc, rays, n, tuv, ids, counters); break;
-        case 48: k_trace_rays<48><<<g, kTraceThreads, 0, s>>>(sc, rays, n, tuv, ids, counters); break;
-        default: return cudaErrorInvalidValue;
-    }
     count_launch();
     return cudaGetLastError();
 }

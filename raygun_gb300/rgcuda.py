@@ -423,8 +423,8 @@ class Context:
     def trace_rays(self, rays):
         rays = np.ascontiguousarray(rays, np.float32)
         n = len(rays)
-        tuv = np.zeros((n, 3), np.float32)
-        ids = np.zeros((n, 2), np.uint32)
+        tuv = np.empty((n, 3), np.float32)
+        ids = np.empty((n, 2), np.uint32)
         self._ck(self.L.rg_trace_rays(self.h, _p(rays), n, _p(tuv), _p(ids)))
         return tuv, ids
 

@@ -48,3 +48,31 @@ def test_edge_rays_equal_oracle(rg, orc, kind):
     for t, i in ((th, ih), (d_tuv.cpu().numpy(), d_ids.cpu().numpy().view(np.uint32))):
         assert np.array_equal(i, ids) and np.array_equal(t, tuv)
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 12288, 12289, 172032, 172033])
+def test_host_query_routes(rg, n):
+    """rg_trace_rays at the edges of its routes (page-locked rays; device copies; two launches whose overflow
+    lists lie in each other's buffers), one ray in 50 overflowing a 16-word stack, against the
+    device query."""
+    import torch
+    from test_gpu_parity import camera_rays, stacked_scene
+    sc = stacked_scene(4096)
+    ctx = rg.Context()
+    rg.load_scene(ctx, sc)
+    ctx.set_batch_tune(128, 16, "none")
+    cam = camera_rays(sc)
+    rays = np.ascontiguousarray(cam[(np.arange(n) * 7) % len(cam)], np.float32)
+    rays[np.arange(n) % 50 != 0, 4:7] *= np.float32(-1.0)
+    rays[::50] = cam[len(cam) // 2 + 24]  # the image's middle
+    tuv, ids = ctx.trace_rays(rays)
+    st = ctx.stats()
+    hits = int((ids[:, 0] != 0xFFFFFFFF).sum())
+    assert st["stack_overflows"] == hits == -(-n // 50) and st["deep_overflows"] == 0
+    d_rays = torch.from_numpy(rays).cuda()
+    d_tuv, d_ids = torch.full((n, 3), -1.0, device="cuda"), torch.zeros((n, 2), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ctx.trace_rays_device(d_rays.data_ptr(), n, d_tuv.data_ptr(), d_ids.data_ptr())
+    ctx.synchronize()
+    assert np.array_equal(d_ids.cpu().numpy().view(np.uint32), ids) and np.array_equal(d_tuv.cpu().numpy(), tuv)
+    ctx.close()
