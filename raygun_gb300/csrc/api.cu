@@ -100,7 +100,7 @@ struct rg_ctx {
     SceneState* sc = nullptr;
     uint32_t scId = 0;
     // shared sort scratch
-    DevBuf keysA, keysB, valsA, valsB, sortState, bounds, sahQueue;
+    DevBuf keysA, keysB, valsA, valsB, sortState, sahQueue;
     // images (raytracer.cpp:173-195)
     uint32_t W = 0, H = 0;
     DevBuf base, normal, rough, finalImg, fxaaOut, fb, dbgT, dbgA, dbgB;
@@ -303,7 +303,6 @@ rg_status ensure_sort_scratch(rg_ctx* c, uint32_t n) {
     TRY(ensure(c, c->valsB, 4ull * n));
     TRY(ensure(c, c->sortState, 4ull * sort_state_words(n)));
     TRY(ensure(c, c->sahQueue, sah_queue_bytes(std::min(n, kSahBlasMaxPrims))));
-    TRY(ensure(c, c->bounds, 64));
     return RG_OK;
 }
 
@@ -338,7 +337,6 @@ LbvhBuffers buffers(rg_ctx* c, const BvhSet& s) {
     b.sortState = c->sortState.as<uint32_t>();
     b.parents = s.parents.as<uint32_t>();
     b.flags = s.flags.as<uint32_t>();
-    b.bounds = c->bounds.as<uint32_t>();
     b.sahQueue = c->sahQueue.as<unsigned char>();
     b.status = wait_status(c);
     return b;
@@ -581,7 +579,7 @@ rg_status rg_destroy(rg_ctx* c) {
         if (c->copied[k]) cudaEventDestroy(c->copied[k]);
     }
     if (c->copyStream) cudaStreamDestroy(c->copyStream);
-    DevBuf* bufs[] = {&c->keysA, &c->keysB, &c->valsA, &c->valsB, &c->sortState, &c->bounds, &c->sahQueue, &c->base, &c->normal, &c->rough,
+    DevBuf* bufs[] = {&c->keysA, &c->keysB, &c->valsA, &c->valsB, &c->sortState, &c->sahQueue, &c->base, &c->normal, &c->rough,
                       &c->finalImg, &c->fxaaOut, &c->fb, &c->dbgT, &c->dbgA, &c->dbgB, &c->counters, &c->tmpA, &c->tmpB, &c->tmpC,
                       &c->tmpD, &c->samples, &c->workCounter, &c->wfPayload, &c->wfMeta, &c->wfFrames, &c->wfQO0, &c->wfQO1,
                       &c->wfQD0, &c->wfQD1, &c->wfQP0, &c->wfQP1, &c->wfHitTUV, &c->wfHitInst, &c->wfCounts, &c->wfOverflow, &c->jobTable,

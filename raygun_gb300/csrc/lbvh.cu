@@ -6,9 +6,12 @@
 //   2. centroid bounds (order-preserving uint atomics: exact, order independent)
 //   3. 30-bit Morton codes of the centroids, normalised to the cube of the largest centroid extent
 //   4. stable LSD radix sort of (code, primitive) in four 8-bit passes, one onesweep kernel each
-//   5. Karras 2012 hierarchy (n-1 internal nodes; equal codes split on the index)
-//   6. bottom-up boxes: one thread per leaf climbs; the second arrival at a node writes its box
-// Refit (topology kept, boxes recomputed) reruns step 6 only.
+//   5. Karras 2012 hierarchy (n-1 internal nodes; equal codes split on the index) and its boxes, bottom
+//      up: one thread per leaf climbs; the second arrival at a split goes on with the node
+// Refit keeps the topology and recomputes the boxes in a climb of its own.
+#include <cooperative_groups.h>
+
+#include <atomic>
 #include <cstdlib>
 
 #include "rg_internal.cuh"
@@ -17,10 +20,13 @@ namespace rg {
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortRounds = 8;
 static_assert(kSortWarps * kSortRounds * 32 == kSortTileKeys, "one onesweep tile per block");
+constexpr uint32_t kNoBox = 0xFFFFFFFFu;        // a box word not yet written (no union of boxes is this NaN)
 constexpr uint32_t kMortonMaxBlocks = 608;  // grid-stride: bounds the global histogram atomics
 
 __global__ void k_tri_boxes(const rg_vertex* __restrict__ v, const uint32_t* __restrict__ idx, uint32_t vOff, uint32_t iOff,
@@ -62,11 +68,7 @@ __device__ inline void centroid(const float* b, float* c) {
     for (int a = 0; a < 3; ++a) c[a] = __fmul_rn(__fadd_rn(b[a], b[3 + a]), 0.5f);
 }
 
-__global__ void k_bounds_init(uint32_t* bounds) {
-    if (threadIdx.x < 3) bounds[threadIdx.x] = 0xFFFFFFFFu;
-    else if (threadIdx.x < 6) bounds[threadIdx.x] = 0u;
-}
-
+// the centroid bounds as words that start at zero: ~f2ord of the minima, f2ord of the maxima
 __global__ void __launch_bounds__(256) k_centroid_bounds(const float* __restrict__ boxes, uint32_t n, uint32_t* bounds) {
     __shared__ float red[6][8];
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -99,18 +101,20 @@ __global__ void __launch_bounds__(256) k_centroid_bounds(const float* __restrict
             hi = fmaxf(hi, red[3 + a][k]);
         }
         if (lo <= hi) {  // the block saw a centroid
-            atomicMin(&bounds[a], f2ord(lo));
+            atomicMax(&bounds[a], ~f2ord(lo));
             atomicMax(&bounds[3 + a], f2ord(hi));
         }
     }
 }
 
-// codes, the sort's input (keys, and values = primitive ids in BOTH value buffers, so that every
-// word of either is a valid primitive id whatever a pass writes), and the four digit histograms of
-// the sort (grid-stride; one shared-memory histogram per block, flushed with global atomics)
+// codes, the sort's input (keys, and values = primitive ids in every buffer that a pass writes values
+// to, so that each word is a valid primitive id whatever a pass writes), cleared arrival words of the
+// hierarchy, and the four digit histograms of the sort (grid-stride; one shared-memory histogram per
+// block, flushed with global atomics)
 __global__ void __launch_bounds__(256) k_morton(const float* __restrict__ boxes, uint32_t n, const uint32_t* __restrict__ bounds,
-                                                uint32_t* __restrict__ morton, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                                                uint32_t* __restrict__ valsAlt, uint32_t* __restrict__ hist) {
+                                                uint32_t* morton, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                uint32_t* __restrict__ valsAlt, uint32_t* order, uint32_t* __restrict__ arrivals,
+                                                uint32_t* __restrict__ nodeBoxes, uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[4 * 256];
     for (int i = threadIdx.x; i < 4 * 256; i += 256) h[i] = 0;
     // every axis is scaled by the LARGEST centroid extent (a cube), so a thin axis spends few of its
@@ -118,7 +122,7 @@ __global__ void __launch_bounds__(256) k_morton(const float* __restrict__ boxes,
     float lo[3], inv[3];
     float emax = 0.0f;
     for (int a = 0; a < 3; ++a) {
-        lo[a] = ord2f(bounds[a]);
+        lo[a] = ord2f(~bounds[a]);
         emax = fmaxf(emax, __fsub_rn(ord2f(bounds[3 + a]), lo[a]));
     }
     for (int a = 0; a < 3; ++a) inv[a] = emax > 0.0f ? __fdiv_rn(1.0f, emax) : 0.0f;
@@ -132,6 +136,11 @@ __global__ void __launch_bounds__(256) k_morton(const float* __restrict__ boxes,
         keys[p] = m;
         vals[p] = p;
         valsAlt[p] = p;
+        order[p] = p;
+        if (p + 1 < n) {
+            arrivals[p] = 0u;
+            for (int a = 0; a < 6; ++a) nodeBoxes[6 * (size_t)p + a] = kNoBox;
+        }
 #pragma unroll
         for (int d = 0; d < 4; ++d) atomicAdd(&h[256 * d + ((m >> (8 * d)) & 0xFFu)], 1u);
     }
@@ -163,6 +172,19 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
 
 __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// lanes of the warp with the same 8-bit digit: eight ballots (__match_any_sync takes 250 cycles of
+// the SM's quarter, five times as long)
+__device__ __forceinline__ uint32_t digit_peers(bool ok, uint32_t digit) {
+    uint32_t peers = __ballot_sync(0xFFFFFFFFu, ok);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool one = (digit >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, one);
+        peers &= one ? m : ~m;
+    }
+    return peers;
 }
 
 // exclusive prefix sum over the block's 256 threads (one value each); `warpSums` holds 8 words
@@ -204,9 +226,9 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_onesweep(const uint32_t* 
         bool ok = i < n;
         key[r] = ok ? keysIn[i] : 0u;
         val[r] = ok ? valsIn[i] : 0u;
-        uint32_t digit = ok ? ((key[r] >> shift) & 0xFFu) : (256u + lane);
-        uint32_t peers = __match_any_sync(0xFFFFFFFFu, digit);
-        uint32_t before = ok ? wc[w][digit] : 0u;
+        uint32_t digit = (key[r] >> shift) & 0xFFu;
+        uint32_t peers = digit_peers(ok, digit);
+        uint32_t before = wc[w][digit];
         __syncwarp();
         pos[r] = before + __popc(peers & ltmask);
         if (ok && (peers & ltmask) == 0) wc[w][digit] = before + __popc(peers);
@@ -260,6 +282,261 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_onesweep(const uint32_t* 
     }
 }
 
+// ---- codes and sort of up to 65536 primitives in one launch ----------------------------------------
+// As separate launches (bounds, codes, four onesweep passes) a build of this size is a chain of launches
+// and of waits on words in L2, 8 us a pass for 0.1 us of traffic.  One thread-block cluster holds all of it
+// in shared memory: every thread keeps ROUNDS keys in registers, the blocks exchange their centroid
+// bounds and digit counts through distributed shared memory and scatter the (code, primitive) pairs
+// straight into each other's (sorted by digit first: 1900 clocks a pass
+// against 5500 in key order).  Stable: blocks, warps and rounds in key order, lanes in key order.  Two
+// cluster barriers a pass.  As many blocks of 1024 threads as there are keys for, up to 16 (beyond
+// the portable 8, which hold 32768 keys), so that a thread ranks few keys one after another.
+// 50000 keys: 31 us, against 45 us in eight launches with their gaps.  (Ranking, 5000 clocks a pass, and
+// the scatter, 1900, are what is left; lane masks by shared-memory atomics in place of the ballots:
+// 2 % less for 32 KB more.)
+constexpr int kClusterThreads = 1024;
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kClusterRounds = 4;  // keys a thread at most
+struct ClusterSort {
+    unsigned long long pair[kClusterThreads * kClusterRounds];    // code << 32 | primitive, from all blocks
+    unsigned long long sorted[kClusterThreads * kClusterRounds];  // the block's pairs by digit
+    uint32_t wc[kClusterWarps][256];  // counts by warp and digit, then offsets within a quarter of the warps
+    uint32_t part[4][256];            // counts by quarter, then where a quarter's keys of a digit start in `sorted`
+    uint32_t cnt[256];                // the block's counts: read by the other blocks
+    uint32_t all[4][256], before[4][256];  // keys of a digit in all blocks, in earlier blocks (by quarter of the blocks)
+    uint32_t shift[256];              // from a key's place in `sorted` to its place in the input's order
+    uint32_t warpSums[2][8];
+    float red[kClusterWarps][6];
+    float bounds[6], total[6];        // centroid bounds: the block's (read by the others), the input's
+};
+
+template <int ROUNDS>
+__global__ void __launch_bounds__(kClusterThreads) k_sort_cluster(const float* __restrict__ boxes, uint32_t n, uint32_t* morton,
+                                                                  uint32_t* __restrict__ keysOut, uint32_t* order,
+                                                                  uint32_t* __restrict__ arrivals, uint32_t* __restrict__ nodeBoxes) {
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+    ClusterSort& S = *reinterpret_cast<ClusterSort*>(smemRaw);
+    const cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), size = cluster.num_blocks();
+    constexpr uint32_t kBlockKeys = kClusterThreads * ROUNDS;
+    const uint32_t tid = threadIdx.x, w = tid >> 5, lane = tid & 31, ltmask = (1u << lane) - 1u;
+    const uint32_t base = rank * kBlockKeys + w * (ROUNDS * 32) + lane;  // the thread's keys: base + 32 r
+    uint32_t key[ROUNDS] = {}, val[ROUNDS] = {}, pos[ROUNDS];
+    {
+        float c[ROUNDS][3];
+        float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            const uint32_t p = base + 32 * r;
+            if (p >= n) continue;
+            centroid(boxes + 6 * (size_t)p, c[r]);
+            for (int a = 0; a < 3; ++a) {
+                v[a] = fminf(v[a], c[r][a]);
+                v[3 + a] = fmaxf(v[3 + a], c[r][a]);
+            }
+        }
+        auto reduce = [&]() {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    v[a] = fminf(v[a], __shfl_xor_sync(0xFFFFFFFFu, v[a], off));
+                    v[3 + a] = fmaxf(v[3 + a], __shfl_xor_sync(0xFFFFFFFFu, v[3 + a], off));
+                }
+        };
+        reduce();
+        if (lane == 0)
+            for (int a = 0; a < 6; ++a) S.red[w][a] = v[a];
+        __syncthreads();
+        if (w == 0) {
+            for (int a = 0; a < 6; ++a) v[a] = S.red[lane][a];
+            reduce();
+            if (lane == 0)
+                for (int a = 0; a < 6; ++a) S.bounds[a] = v[a];
+        }
+        // meanwhile: the hierarchy's words
+        for (uint32_t i = rank * kClusterThreads + tid; i + 1 < n; i += size * kClusterThreads) arrivals[i] = 0u;
+        for (uint32_t i = rank * kClusterThreads + tid; i < 6 * (n - 1); i += size * kClusterThreads) nodeBoxes[i] = kNoBox;
+        cluster.sync();
+        if (w == 0) {
+            for (int a = 0; a < 6; ++a) v[a] = lane < size ? cluster.map_shared_rank(S.bounds, lane)[a] : a < 3 ? INFINITY : -INFINITY;
+            reduce();
+            if (lane == 0)
+                for (int a = 0; a < 6; ++a) S.total[a] = v[a];
+        }
+        __syncthreads();
+        // every axis is scaled by the largest centroid extent, as in k_morton; an axis without a
+        // centroid (all NaN) has NaN bounds
+        float lo[3], inv, emax = 0.0f;
+        for (int a = 0; a < 3; ++a) {
+            const bool any = S.total[a] <= S.total[3 + a];
+            lo[a] = any ? S.total[a] : ord2f(0xFFFFFFFFu);
+            emax = fmaxf(emax, __fsub_rn(any ? S.total[3 + a] : ord2f(0u), lo[a]));
+        }
+        inv = emax > 0.0f ? __fdiv_rn(1.0f, emax) : 0.0f;
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            const uint32_t p = base + 32 * r;
+            if (p >= n) continue;
+            const uint32_t x = quant10(c[r][0], lo[0], inv), y = quant10(c[r][1], lo[1], inv), z = quant10(c[r][2], lo[2], inv);
+            key[r] = (expand10(x) << 2) | (expand10(y) << 1) | expand10(z);
+            val[r] = p;
+            morton[p] = key[r];
+        }
+    }
+    const uint32_t held = min(kBlockKeys, n - min(n, rank * kBlockKeys));  // the block's keys
+#pragma unroll 1
+    for (int pass = 0; pass < 4; ++pass) {
+        const int bits = 8 * pass;
+        if (pass) {
+#pragma unroll
+            for (int r = 0; r < ROUNDS; ++r) {
+                const unsigned long long kv = S.pair[w * (ROUNDS * 32) + 32 * r + lane];
+                key[r] = (uint32_t)(kv >> 32);
+                val[r] = (uint32_t)kv;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kClusterWarps * 256 / kClusterThreads; ++i) (&S.wc[0][0])[tid + kClusterThreads * i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            const bool ok = base + 32 * r < n;
+            const uint32_t digit = (key[r] >> bits) & 0xFFu;
+            const uint32_t peers = digit_peers(ok, digit);
+            const uint32_t ahead = S.wc[w][digit];
+            __syncwarp();
+            pos[r] = ahead + __popc(peers & ltmask);
+            if (ok && (peers & ltmask) == 0) S.wc[w][digit] = ahead + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        const uint32_t q = tid >> 8, d = tid & 255u;  // a quarter of the warps, then of the blocks; a digit
+        {
+            uint32_t c[kClusterWarps / 4], run = 0;
+#pragma unroll
+            for (int i = 0; i < kClusterWarps / 4; ++i) c[i] = S.wc[q * (kClusterWarps / 4) + i][d];
+#pragma unroll
+            for (int i = 0; i < kClusterWarps / 4; ++i) {
+                S.wc[q * (kClusterWarps / 4) + i][d] = run;
+                run += c[i];
+            }
+            S.part[q][d] = run;
+        }
+        __syncthreads();
+        // exclusive prefix over the digits, 8 warps of it: within the warp here, the warps before by their sums
+        auto prefix = [&](uint32_t v, uint32_t* sums) {
+            uint32_t x = v;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+                if (lane >= (uint32_t)off) x += y;
+            }
+            if (lane == 31) sums[w] = x;
+            return x - v;
+        };
+        uint32_t mineAt = 0;
+        if (q == 0) {
+            const uint32_t c = S.part[0][d] + S.part[1][d] + S.part[2][d] + S.part[3][d];
+            S.cnt[d] = c;
+            mineAt = prefix(c, S.warpSums[0]);
+        }
+        cluster.barrier_arrive();  // the counts are there
+        __syncthreads();
+        if (q == 0) {
+            for (uint32_t k = 0; k < w; ++k) mineAt += S.warpSums[0][k];
+            uint32_t at = mineAt;
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t c = S.part[i][d];
+                S.part[i][d] = at;
+                at += c;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            if (base + 32 * r >= n) continue;
+            const uint32_t dg = (key[r] >> bits) & 0xFFu;
+            S.sorted[S.part[w / (kClusterWarps / 4)][dg] + S.wc[w][dg] + pos[r]] = (unsigned long long)key[r] << 32 | val[r];
+        }
+        cluster.barrier_wait();
+        {
+            uint32_t all = 0, before = 0;
+#pragma unroll 4
+            for (uint32_t b = q; b < size; b += 4) {
+                const uint32_t c = cluster.map_shared_rank(S.cnt, b)[d];
+                all += c;
+                before += b < rank ? c : 0u;
+            }
+            S.all[q][d] = all;
+            S.before[q][d] = before;
+        }
+        if (pass == 3) cluster.barrier_arrive();  // the last look into the other blocks' memory
+        __syncthreads();
+        uint32_t at = 0;
+        if (q == 0)
+            at = prefix(S.all[0][d] + S.all[1][d] + S.all[2][d] + S.all[3][d], S.warpSums[1]) + S.before[0][d] + S.before[1][d] +
+                 S.before[2][d] + S.before[3][d];
+        __syncthreads();
+        if (q == 0) {
+            for (uint32_t k = 0; k < w; ++k) at += S.warpSums[1][k];
+            S.shift[d] = at - mineAt;
+        }
+        __syncthreads();
+        // neighbours in `sorted` mostly stay neighbours: whole stretches go to a block
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) {
+            const uint32_t i = tid + kClusterThreads * r;
+            if (i >= held) continue;
+            const unsigned long long kv = S.sorted[i];
+            const uint32_t dst = i + S.shift[(uint32_t)(kv >> (32 + bits)) & 0xFFu];
+            if (pass < 3) {
+                cluster.map_shared_rank(S.pair, dst / kBlockKeys)[dst % kBlockKeys] = kv;
+            } else {
+                keysOut[dst] = (uint32_t)(kv >> 32);
+                order[dst] = (uint32_t)kv;
+            }
+        }
+        if (pass < 3) cluster.sync();
+    }
+    cluster.barrier_wait();
+}
+
+// cluster size that this device schedules for k_sort_cluster: 16, 8, or 0 (none)
+uint32_t cluster_limit() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];  // 0: not asked yet
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 0;
+    int v = known[dev].load(std::memory_order_acquire);
+    if (!v) {
+        v = -1;
+        const void* fn[3] = {(const void*)k_sort_cluster<1>, (const void*)k_sort_cluster<2>, (const void*)k_sort_cluster<4>};
+        bool ok = true;
+        for (const void* f : fn)
+            ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterSort)) == cudaSuccess &&
+                 cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        for (int size = 16; ok && v < 0 && size >= 8; size /= 2) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(size);
+            cfg.blockDim = dim3(kClusterThreads);
+            cfg.dynamicSmemBytes = sizeof(ClusterSort);
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim = {(unsigned)size, 1, 1};
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            bool all = true;
+            for (const void* f : fn) all = all && cudaOccupancyMaxActiveClusters(&clusters, f, &cfg) == cudaSuccess && clusters > 0;
+            if (all) v = size;
+        }
+        if (v < 0) cudaGetLastError();  // a refused attribute is no error of the build
+        known[dev].store(v, std::memory_order_release);
+    }
+    return v < 0 ? 0u : (uint32_t)v;
+}
+
 // TLAS leaf k: the instance at sorted position k with its inverse rows and its BLAS's root box
 // and record pointers copied in
 __global__ void k_inst_records(const uint32_t* __restrict__ order, uint32_t n, const DevInstance* __restrict__ inst,
@@ -286,45 +563,161 @@ __global__ void k_inst_records(const uint32_t* __restrict__ order, uint32_t n, c
     out[k] = r;
 }
 
-// ---- Karras 2012 hierarchy ----------------------------------------------------------------------
-__device__ inline int delta(const uint32_t* __restrict__ k, int n, int i, int j) {
-    if (j < 0 || j >= n) return -1;
-    uint32_t a = k[i], b = k[j];
-    if (a == b) return 32 + __clz((uint32_t)i ^ (uint32_t)j);
-    return __clz(a ^ b);
+// ---- hierarchy -----------------------------------------------------------------------------------
+// The binary radix tree of the sorted codes (Karras 2012: its nodes and their numbering), built bottom
+// up with the boxes (Apetrei 2014).  A node covers a range [l, r] of leaves and splits after leaf s; its
+// parent splits where the range borders on the closer neighbour: after r if leaf r + 1 shares more bits
+// with leaf r than leaf l - 1 with leaf l, else after l - 1.  The node is then its parent's left (right)
+// child, and Karras' number for it is r (l); the root's is 0.  One thread per leaf climbs: of a
+// split's two arrivals the first leaves its far end and stops, the second goes on with the union.
+//
+// The climb is a chain of dependent memory accesses, some 25 levels of it for 50000 leaves, so
+//   - a block keeps the nodes whose range lies in its own kHierLeaves leaves in shared memory;
+//   - of the others a level is ONE round trip: the arrival word carries the far end and the common bits
+//     with the leaf beyond it (up to 2^25 leaves; more read them from the codes), no fence orders it
+//     after the box, and the sibling's box is requested together with it.  Box words start as
+//     kNoBox, which no union is, so a box still on its way is seen and asked for again; after
+//     kHierPolls requests the box is taken from the leaves instead, so no wait is unbounded.
+// 50000 leaves: 23 us (37 us with an acquire-release arrival and its box after it), against 12 us for
+// the nodes and 36 us for the boxes as two kernels.
+#ifndef RG_HIER_LEAVES
+#define RG_HIER_LEAVES 512
+#endif
+constexpr int kHierLeaves = RG_HIER_LEAVES;
+constexpr int kHierPolls = 4096;
+
+__device__ __forceinline__ int delta(uint32_t a, uint32_t b, uint32_t i, uint32_t j) {  // common leading bits of (code, position)
+    return a == b ? 32 + __clz(i ^ j) : __clz(a ^ b);
 }
 
-__global__ void k_karras(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* __restrict__ left, uint32_t* __restrict__ right,
-                         uint32_t* __restrict__ parents) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int N = (int)n;
-    if (i >= N - 1) return;
-    int d = (delta(keys, N, i, i + 1) - delta(keys, N, i, i - 1)) >= 0 ? 1 : -1;
-    int dmin = delta(keys, N, i, i - d);
-    int lmax = 2;
-    while (delta(keys, N, i, i + lmax * d) > dmin) lmax *= 2;
-    int l = 0;
-    for (int t = lmax / 2; t >= 1; t /= 2)
-        if (delta(keys, N, i, i + (l + t) * d) > dmin) l += t;
-    int j = i + l * d;
-    int dnode = delta(keys, N, i, j);
-    int s = 0, t = l;
-    do {
-        t = (t + 1) >> 1;
-        if (delta(keys, N, i, i + (s + t) * d) > dnode) s += t;
-    } while (t > 1);
-    int gamma = i + s * d + min(d, 0);
-    int lo = min(i, j), hi = max(i, j);
-    uint32_t L = (lo == gamma) ? (kLeaf | (uint32_t)gamma) : (uint32_t)gamma;
-    uint32_t R = (hi == gamma + 1) ? (kLeaf | (uint32_t)(gamma + 1)) : (uint32_t)(gamma + 1);
-    left[i] = L;
-    right[i] = R;
-    parents[(L & kLeaf) ? (n - 1) + (L & ~kLeaf) : L] = (uint32_t)i;
-    parents[(R & kLeaf) ? (n - 1) + (R & ~kLeaf) : R] = (uint32_t)i;
-    if (i == 0) parents[0] = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t swap_relaxed(uint32_t* p, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.exch.relaxed.gpu.global.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
 }
 
-// ---- bottom-up boxes ----------------------------------------------------------------------------
+__device__ __forceinline__ void load_box_relaxed(const float* p, uint32_t* b) {
+#pragma unroll
+    for (int a = 0; a < 6; ++a) b[a] = ld_relaxed(reinterpret_cast<const uint32_t*>(p) + a);
+}
+__device__ __forceinline__ bool box_there(const uint32_t* b) {
+    bool there = true;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) there = there && b[a] != kNoBox;
+    return there;
+}
+
+__global__ void __launch_bounds__(kHierLeaves) k_hierarchy(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ order,
+                                                           const float* __restrict__ primBoxes, uint32_t n, uint32_t* __restrict__ left,
+                                                           uint32_t* __restrict__ right, uint32_t* __restrict__ parents,
+                                                           uint32_t* arrivals, float* nodeBoxes) {
+    __shared__ uint32_t sKeys[kHierLeaves + 2];      // leaves first - 1 .. first + kHierLeaves
+    __shared__ uint32_t sArrive[kHierLeaves];        // by split
+    __shared__ float sLeaf[kHierLeaves][6], sNode[kHierLeaves][6];  // boxes by leaf and by node number
+    const uint32_t first = blockIdx.x * kHierLeaves, k = first + threadIdx.x;
+    const uint32_t end = min(n, first + kHierLeaves);  // one past the block's last leaf
+    const bool packed = n < (1u << 25);
+    float cur[6];
+    if (k < n) {
+        const float* b = primBoxes + 6 * (size_t)order[k];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) sLeaf[threadIdx.x][a] = cur[a] = b[a];
+        sKeys[threadIdx.x + 1] = keys[k];
+        sArrive[threadIdx.x] = 0u;
+    }
+    if (threadIdx.x == 0) {
+        sKeys[0] = first ? keys[first - 1] : 0u;
+        sKeys[end - first + 1] = end < n ? keys[end] : 0u;
+    }
+    __syncthreads();
+    if (k >= n) return;
+    auto key = [&](uint32_t i) { return i + 1 >= first && i <= end ? sKeys[i + 1 - first] : keys[i]; };
+    auto between = [&](uint32_t i, uint32_t j) { return delta(key(i), key(j), i, j); };
+    uint32_t l = k, r = k, node = kLeaf | k;
+    int dl = l > 0 ? between(l - 1, l) : -1, dr = r + 1 < n ? between(r, r + 1) : -1;
+    // a radix tree has at most 62 levels; the bounds also hold for words that another build is writing
+    for (int level = 0; level < 128; ++level) {
+        if (dl < 0 && dr < 0) return;  // the root is done
+        const bool isLeft = dr > dl;
+        const uint32_t s = isLeft ? r : l - 1;  // the parent's split
+        if (s >= n - 1u) return;                // never in a build that runs alone
+        // the parent's range lies in the block if mine does and the sibling's does not reach past it
+        const int ds = isLeft ? dr : dl;
+        const bool local = l >= first && r < end &&
+                           (isLeft ? r + 1 < end && !(end < n && between(r + 1, end) > ds)
+                                   : l > first && !(first > 0 && between(first - 1, l - 1) > ds));
+        const uint32_t mine = (isLeft ? l : r) + 1u + (packed ? (uint32_t)((isLeft ? dl : dr) + 1) << 25 : 0u);
+        const uint32_t sibNode = isLeft ? s + 1 : s;  // the sibling's number if it is not a leaf
+        uint32_t got, ob[6];
+        if (local) {
+            if (!(node & kLeaf)) {
+#pragma unroll
+                for (int a = 0; a < 6; ++a) sNode[node - first][a] = cur[a];
+                __threadfence_block();
+            }
+            got = atomicExch(&sArrive[s - first], mine);
+            __threadfence_block();
+        } else {
+            got = swap_relaxed(&arrivals[s], mine);
+            load_box_relaxed(nodeBoxes + 6 * (size_t)min(sibNode, n - 2u), ob);
+        }
+        if (got == 0u) return;
+        const uint32_t far = (packed ? got & 0x1FFFFFFu : got) - 1u;  // the other side's far end
+        if (isLeft ? far <= s || far >= n : far > s) return;  // never in a build that runs alone
+        const bool sibLeaf = far == sibNode;
+        const uint32_t L = (isLeft ? l : far) == s ? (kLeaf | s) : s;
+        const uint32_t R = (isLeft ? far : r) == s + 1 ? (kLeaf | (s + 1)) : s + 1;
+        if (isLeft) {
+            r = far;
+            dr = packed ? (int)(got >> 25) - 1 : r + 1 < n ? between(r, r + 1) : -1;
+        } else {
+            l = far;
+            dl = packed ? (int)(got >> 25) - 1 : l > 0 ? between(l - 1, l) : -1;
+        }
+        if (local) {
+            const float* b = sibLeaf ? sLeaf[sibNode - first] : sNode[sibNode - first];
+#pragma unroll
+            for (int a = 0; a < 6; ++a) ob[a] = __float_as_uint(b[a]);
+        } else if (sibLeaf) {
+            const float* b = primBoxes + 6 * (size_t)order[sibNode];
+#pragma unroll
+            for (int a = 0; a < 6; ++a) ob[a] = __float_as_uint(b[a]);
+        } else {
+            for (int i = 0; i < kHierPolls && !box_there(ob); ++i) load_box_relaxed(nodeBoxes + 6 * (size_t)sibNode, ob);
+            if (!box_there(ob)) {
+                float u[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                const uint32_t i0 = isLeft ? s + 1 : far, i1 = isLeft ? far : s;
+                for (uint32_t i = i0; i <= i1; ++i) {
+                    const float* b = primBoxes + 6 * (size_t)order[i];
+                    for (int a = 0; a < 3; ++a) {
+                        u[a] = fminf(u[a], b[a]);
+                        u[3 + a] = fmaxf(u[3 + a], b[3 + a]);
+                    }
+                }
+                for (int a = 0; a < 6; ++a) ob[a] = __float_as_uint(u[a]);
+            }
+        }
+        node = dl < 0 && dr < 0 ? 0u : dr > dl ? r : l;
+        if (node >= n - 1u) return;  // never in a build that runs alone
+        float* o = nodeBoxes + 6 * (size_t)node;
+        // the left child's box is the first operand
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float c0 = __uint_as_float(ob[a]), c1 = __uint_as_float(ob[3 + a]);
+            cur[a] = isLeft ? fminf(cur[a], c0) : fminf(c0, cur[a]);
+            cur[3 + a] = isLeft ? fmaxf(cur[3 + a], c1) : fmaxf(c1, cur[3 + a]);
+        }
+#pragma unroll
+        for (int a = 0; a < 6; ++a) st_relaxed(reinterpret_cast<uint32_t*>(o) + a, __float_as_uint(cur[a]));
+        left[node] = L;
+        right[node] = R;
+        parents[(L & kLeaf) ? (n - 1) + (L & ~kLeaf) : L] = node;
+        parents[(R & kLeaf) ? (n - 1) + (R & ~kLeaf) : R] = node;
+        if (dl < 0 && dr < 0) parents[0] = 0xFFFFFFFFu;
+    }
+}
+
+// ---- refit ---------------------------------------------------------------------------------------
 __device__ inline void load_box_cg(const float* p, float* b) {
     for (int a = 0; a < 6; ++a) b[a] = __ldcg(p + a);
 }
@@ -1595,33 +1988,55 @@ cudaError_t lbvh_build(const LbvhBuffers& b, cudaStream_t s) {
     const uint32_t n = b.n;
     if (n == 0) return cudaSuccess;
     if (n > kStatCount) return cudaErrorInvalidValue;  // the sort's status words count in 30 bits
-    const uint32_t nTiles = (uint32_t)sort_tiles(n);
-    cudaError_t e = cudaMemsetAsync(b.sortState, 0, 4 * sort_state_words(n), s);
-    if (e != cudaSuccess) return e;
-    k_bounds_init<<<1, 32, 0, s>>>(b.bounds);
-    uint32_t gb = min(blocks(n, 256), 1024u);
-    k_centroid_bounds<<<gb, 256, 0, s>>>(b.primBoxes, n, b.bounds);
-    k_morton<<<min(blocks(n, 256), kMortonMaxBlocks), 256, 0, s>>>(b.primBoxes, n, b.bounds, b.morton, b.keysA, b.valsA, b.valsB,
-                                                                   b.sortState);
-    count_launch(3);
-    // polls of an unpublished predecessor tile before a look-back counts that tile itself
-    // (RG_SORT_SPIN_LIMIT overrides; 0 makes every such look-back count, which tests use)
-    uint32_t spinLimit = 1u << 16;
-    if (const char* env = getenv("RG_SORT_SPIN_LIMIT")) spinLimit = (uint32_t)strtoul(env, nullptr, 10);
-    uint32_t *kin = b.keysA, *vin = b.valsA, *kout = b.keysB, *vout = b.valsB;
-    for (int pass = 0; pass < 4; ++pass) {
-        k_sort_onesweep<<<nTiles, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, pass, b.sortState, nTiles, spinLimit);
+    const uint32_t limit = cluster_limit();
+    if (n <= limit * kClusterThreads * kClusterRounds) {  // one cluster holds the keys
+        // as many blocks as there are keys for, so that a thread ranks few keys one after another
+        uint32_t size = 1, rounds = 1;
+        while (size < limit && size * kClusterThreads < n) size *= 2;
+        while (size * kClusterThreads * rounds < n) rounds *= 2;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(size);
+        cfg.blockDim = dim3(kClusterThreads);
+        cfg.dynamicSmemBytes = sizeof(ClusterSort);
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim = {size, 1, 1};
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        const auto kernel = rounds == 1 ? k_sort_cluster<1> : rounds == 2 ? k_sort_cluster<2> : k_sort_cluster<4>;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const float*)b.primBoxes, n, b.morton, b.keysA, b.order, b.flags,
+                                                 reinterpret_cast<uint32_t*>(b.nodeBoxes));
+        if (e != cudaSuccess) return e;
         count_launch();
-        uint32_t* t = kin; kin = kout; kout = t;
-        t = vin; vin = vout; vout = t;
+    } else {
+        const uint32_t nTiles = (uint32_t)sort_tiles(n);
+        cudaError_t e = cudaMemsetAsync(b.sortState, 0, 4 * sort_state_words(n), s);
+        if (e != cudaSuccess) return e;
+        uint32_t* bounds = b.sortState + kSortBounds;
+        uint32_t gb = min(blocks(n, 256), 1024u);
+        k_centroid_bounds<<<gb, 256, 0, s>>>(b.primBoxes, n, bounds);
+        k_morton<<<min(blocks(n, 256), kMortonMaxBlocks), 256, 0, s>>>(b.primBoxes, n, bounds, b.morton, b.keysA, b.valsA, b.valsB, b.order,
+                                                                       b.flags, reinterpret_cast<uint32_t*>(b.nodeBoxes), b.sortState);
+        count_launch(2);
+        // polls of an unpublished predecessor tile before a look-back counts that tile itself
+        // (RG_SORT_SPIN_LIMIT overrides; 0 makes every such look-back count, which tests use)
+        uint32_t spinLimit = 1u << 16;
+        if (const char* env = getenv("RG_SORT_SPIN_LIMIT")) spinLimit = (uint32_t)strtoul(env, nullptr, 10);
+        const uint32_t *kin = b.keysA, *vin = b.valsA;  // keys A -> B -> A -> B -> A, values A -> B -> A -> B -> order
+        uint32_t* kout[4] = {b.keysB, b.keysA, b.keysB, b.keysA};
+        uint32_t* vout[4] = {b.valsB, b.valsA, b.valsB, b.order};
+        for (int pass = 0; pass < 4; ++pass) {
+            k_sort_onesweep<<<nTiles, kSortThreads, 0, s>>>(kin, vin, kout[pass], vout[pass], n, pass, b.sortState, nTiles, spinLimit);
+            count_launch();
+            kin = kout[pass];
+            vin = vout[pass];
+        }
     }
-    // after 4 passes the sorted data is back in keysA / valsA
-    e = cudaMemcpyAsync(b.order, vin, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return e;
     if (n == 1) return cudaGetLastError();
-    k_karras<<<blocks(n - 1, 256), 256, 0, s>>>(kin, n, b.left, b.right, b.parents);
+    k_hierarchy<<<blocks(n, kHierLeaves), kHierLeaves, 0, s>>>(b.keysA, b.order, b.primBoxes, n, b.left, b.right, b.parents, b.flags, b.nodeBoxes);
     count_launch();
-    return lbvh_refit(b, s);
+    return cudaGetLastError();
 }
 
 }  // namespace rg

@@ -32,8 +32,7 @@ constexpr size_t kKeysBytes = align_up(4ull * kMaxPrims);
 constexpr size_t kSortStateBytes = align_up(4ull * sort_state_words(kMaxPrims));
 constexpr size_t kParentsBytes = align_up(8ull * kMaxPrims);
 constexpr size_t kFlagsBytes = align_up(4ull * kMaxPrims);
-constexpr size_t kBoundsBytes = align_up(64);
-constexpr size_t kScratchBytes = 4 * kKeysBytes + kSortStateBytes + kParentsBytes + kFlagsBytes + kBoundsBytes;
+constexpr size_t kScratchBytes = 4 * kKeysBytes + kSortStateBytes + kParentsBytes + kFlagsBytes;
 
 static __device__ __align__(256) unsigned char g_lbvh_scratch[kScratchBytes];
 
@@ -85,8 +84,7 @@ extern "C" rg_status rg_lbvh_build_device_noalloc(const float* d_boxes, uint32_t
     b.valsB = reinterpret_cast<uint32_t*>(p); p += kKeysBytes;
     b.sortState = reinterpret_cast<uint32_t*>(p); p += kSortStateBytes;  // zeroed by the build
     b.parents = reinterpret_cast<uint32_t*>(p); p += kParentsBytes;
-    b.flags = reinterpret_cast<uint32_t*>(p); p += kFlagsBytes;  // zeroed inside lbvh_build (refit step)
-    b.bounds = reinterpret_cast<uint32_t*>(p);                    // reset by the build's first kernel
+    b.flags = reinterpret_cast<uint32_t*>(p);  // zeroed inside lbvh_build
     cudaError_t e = lbvh_build(b, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? RG_OK : RG_ERR_CUDA;
 }

@@ -132,10 +132,9 @@ struct LbvhBuffers {  // scratch + outputs of one LBVH build, sized by the calle
     float* nodeBoxes;      // (n-1) x 6
     // scratch
     uint32_t* keysA; uint32_t* keysB; uint32_t* valsA; uint32_t* valsB;
-    uint32_t* sortState;   // sort_state_words(n): digit histograms, tile counters, look-back words
+    uint32_t* sortState;   // sort_state_words(n): digit histograms, tile counters, centroid bounds, look-back words
     uint32_t* parents;     // 2n (internal n-1 then leaves n)
     uint32_t* flags;       // n-1
-    uint32_t* bounds;      // 6 (ordered uints)
     // binned-SAH builds: the task queue of k_sah_tasks (sah_queue_bytes(n), 16-byte aligned) and a
     // status word set to 2 when one of its waits gave up (nullable)
     unsigned char* sahQueue = nullptr;
@@ -157,6 +156,7 @@ constexpr size_t sah_queue_bytes(size_t n) { return 20 * n + 64; }
 // (tile, digit)
 constexpr uint32_t kSortTileKeys = 2048;
 constexpr uint32_t kSortTileCounters = 4 * 256;
+constexpr uint32_t kSortBounds = kSortTileCounters + 8;  // the centroid bounds (6 words)
 constexpr uint32_t kSortStatusOffset = kSortTileCounters + 32;
 constexpr size_t sort_tiles(size_t n) { return (n + kSortTileKeys - 1) / kSortTileKeys; }
 constexpr size_t sort_state_words(size_t n) { return kSortStatusOffset + 4 * 256 * sort_tiles(n); }
