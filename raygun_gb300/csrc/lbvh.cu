@@ -837,14 +837,24 @@ __global__ void k_wide_records(const float* __restrict__ primBoxes, const uint32
 // sides non-empty, so each level shortens every range.  From level medianLevel on, ranges are halved
 // without binning, so no tree is deeper than medianLevel + ceil(log2 n) levels, whatever the centroid
 // distribution (a surface-area split can peel one primitive off a range per level).
-// Internal nodes are numbered in level order (a level's tasks follow the previous levels' nodes), so
-// a task is just its range.  The result has the LBVH's layout (order, left, right, nodeBoxes), so
+// A level's tasks are numbered after the previous levels' nodes, so a task is just its range; the nodes of
+// the subtrees that single warps finish are numbered from the upper end.  The result has the LBVH's layout (order, left, right, nodeBoxes), so
 // records, refits and traversal are shared.
 constexpr int kSahBins = 16;
 constexpr int kSahWarps = 32;
 constexpr int kSahTaskWarps = 8;               // warps per block of k_sah_tasks
 constexpr uint32_t kSahHandoff = 64;           // tasks of a level from which k_sah_tasks takes over
-constexpr int kSahParallelLevels = 6;          // levels built by k_sah_level, one launch each
+constexpr int kSahParallelLevels = 13;         // levels built by k_sah_level at most, one launch each
+constexpr uint32_t kSahSmall = 4096;           // up to here one CTA holds the primitives of the top levels
+// The level kernels run until a level's tasks hold some kSahTask primitives: a task of some hundreds costs a
+// CTA 10 us and one warp of k_sah_tasks 20 us and more (61442 triangles: levels until 64, 128, 256, 512
+// primitives 2.43, 2.47, 2.53, 2.68 ms for the whole scene load).  A small build's levels cost its CTA 6 us
+// each, a level through k_sah_tasks' queue 9 us, so it hands over when its warps all have a task.
+constexpr uint32_t kSahTask = 64;
+constexpr uint32_t kSahSmallHandoff = 32;
+// A subtree of m primitives on one warp takes m - 1 nodes one after another, 1.5 us each: 32 where the warps
+// have enough of them, 16 in a small build, which has more warps than tasks.
+constexpr uint32_t kSahSubtree = 32, kSahSubtreeSmall = 16;
 constexpr uint32_t kSahWaitLimit = 1u << 22;   // polls of an unpublished task before k_sah_tasks gives up
 
 __device__ __forceinline__ int ord_float(float f) {
@@ -857,43 +867,70 @@ __device__ __forceinline__ float half_area3(const float* lo, const float* hi) {
     return dx * dy + dy * dz + dz * dx;
 }
 
+// minimum and maximum over the warp (redux: one instruction each; as fminf a NaN is passed over)
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // The cheapest of the 3 x 15 surface-area splits of a task's bins (ties to the lowest candidate),
-// reduced over the calling warp (all 32 lanes call it); -1 when no split leaves both sides
-// non-empty.  cnt(a, k), lo(a, k, c), hi(a, k, c) read bin k of axis a (bounds as ordered ints).
+// found by the calling warp (all 32 lanes call it); -1 when no split leaves both sides non-empty.
+// cnt(a, k), lo(a, k, c), hi(a, k, c) read bin k of axis a (bounds as ordered ints).  A half-warp takes
+// an axis, a lane a bin: boxes and counts left and right of each split are prefix and suffix scans (four
+// steps), a third of the instructions of a lane going over the 16 bins for its split.
 template <class Cnt, class Lo, class Hi>
 __device__ __forceinline__ int sah_best_split(const float* scale, int lane, Cnt cnt, Lo lo, Hi hi) {
+    constexpr unsigned full = 0xFFFFFFFFu;
     float bestCost = INFINITY;
     int bestCand = -1;
-    for (int cand = lane; cand < 3 * (kSahBins - 1); cand += 32) {
-        const int a = cand / (kSahBins - 1), sp = cand % (kSahBins - 1) + 1;
-        if (scale[a] <= 0.0f) continue;
-        float L0[3] = {INFINITY, INFINITY, INFINITY}, L1[3] = {-INFINITY, -INFINITY, -INFINITY};
-        float R0[3] = {INFINITY, INFINITY, INFINITY}, R1[3] = {-INFINITY, -INFINITY, -INFINITY};
-        int nl = 0, nr = 0;
-        for (int k = 0; k < kSahBins; ++k) {
-            const int n = cnt(a, k);
-            if (!n) continue;
-            float* X0 = k < sp ? L0 : R0;
-            float* X1 = k < sp ? L1 : R1;
+    const int k = lane & 15;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int a = 2 * half + (lane >> 4);
+        const float sc = a == 0 ? scale[0] : a == 1 ? scale[1] : a == 2 ? scale[2] : 0.0f;
+        float L[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY}, R[6];
+        int nl = sc > 0.0f ? cnt(a, k) : 0;
+        if (nl)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                X0[c] = fminf(X0[c], unord_float(lo(a, k, c)));
-                X1[c] = fmaxf(X1[c], unord_float(hi(a, k, c)));
+                L[c] = fminf(L[c], unord_float(lo(a, k, c)));
+                L[3 + c] = fmaxf(L[3 + c], unord_float(hi(a, k, c)));
             }
-            if (k < sp) nl += n;
-            else nr += n;
+        int nr = nl;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) R[c] = L[c];
+#pragma unroll
+        for (int off = 1; off < 16; off <<= 1) {  // L, nl: bins 0 .. k; R, nr: bins k .. 15
+            const int pn = __shfl_up_sync(full, nl, off, 16), sn = __shfl_down_sync(full, nr, off, 16);
+            if (k >= off) nl += pn;
+            if (k + off < 16) nr += sn;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {  // beyond the half-warp a lane gets its own value
+                L[c] = fminf(L[c], __shfl_up_sync(full, L[c], off, 16));
+                L[3 + c] = fmaxf(L[3 + c], __shfl_up_sync(full, L[3 + c], off, 16));
+                R[c] = fminf(R[c], __shfl_down_sync(full, R[c], off, 16));
+                R[3 + c] = fmaxf(R[3 + c], __shfl_down_sync(full, R[3 + c], off, 16));
+            }
         }
-        if (!nl || !nr) continue;
-        const float cost = half_area3(L0, L1) * (float)nl + half_area3(R0, R1) * (float)nr;
-        if (cost < bestCost) {
+        nr = __shfl_down_sync(full, nr, 1, 16);  // bins k + 1 .. 15
+#pragma unroll
+        for (int c = 0; c < 6; ++c) R[c] = __shfl_down_sync(full, R[c], 1, 16);
+        const float cost = half_area3(L, L + 3) * (float)nl + half_area3(R, R + 3) * (float)nr;
+        if (sc > 0.0f && k < kSahBins - 1 && nl && nr && cost < bestCost) {
             bestCost = cost;
-            bestCand = cand;
+            bestCand = a * (kSahBins - 1) + k;  // split before bin k + 1
         }
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
-        const float oc = __shfl_xor_sync(0xFFFFFFFFu, bestCost, off);
-        const int oi = __shfl_xor_sync(0xFFFFFFFFu, bestCand, off);
+        const float oc = __shfl_xor_sync(full, bestCost, off);
+        const int oi = __shfl_xor_sync(full, bestCand, off);
         if (oi >= 0 && (bestCand < 0 || oc < bestCost || (oc == bestCost && oi < bestCand))) {
             bestCost = oc;
             bestCand = oi;
@@ -902,20 +939,137 @@ __device__ __forceinline__ int sah_best_split(const float* scale, int lane, Cnt 
     return bestCand;
 }
 
-// One level with fewer tasks than warps: G warps share a task (G * count <= 32), each taking a
-// contiguous chunk of the task's range.  The same computation as one warp per task -- bounds and bin
-// contents are order-independent minima, maxima and counts, the split is chosen by the same rule, and
-// the partition stays stable (each warp writes its chunk at the offsets of the chunks before it) --
-// so the tree is the same; the top levels just run on the whole CTA instead of a few warps.
+// One primitive a lane into the bins of one axis (bins in shared memory, this warp's own).  The
+// primitives of a range keep the mesh's order, so a warp's mostly fall into a few bins, and 32 atomics on
+// one word take their turns: lanes of one bin are reduced first while the groups are large.
+__device__ __forceinline__ void sah_bin(bool valid, int bin, const float* bx, int* cnt, int (*lo)[3], int (*hi)[3], int lane) {
+    constexpr int kGroup = 8;
+    unsigned todo = __ballot_sync(0xFFFFFFFFu, valid);
+    while (__popc(todo) >= kGroup) {
+        const int b0 = __shfl_sync(0xFFFFFFFFu, bin, __ffs(todo) - 1);
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, valid && bin == b0) & todo;
+        if (__popc(m) < kGroup) break;
+        if (m >> lane & 1u) {
+            int l[3], h[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                l[c] = __reduce_min_sync(m, ord_float(bx[c]));
+                h[c] = __reduce_max_sync(m, ord_float(bx[3 + c]));
+            }
+            if (lane == __ffs(m) - 1) {
+                cnt[bin] += __popc(m);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    lo[bin][c] = min(lo[bin][c], l[c]);
+                    hi[bin][c] = max(hi[bin][c], h[c]);
+                }
+            }
+        }
+        todo &= ~m;
+        __syncwarp();
+    }
+    if (todo >> lane & 1u) {
+        atomicAdd(&cnt[bin], 1);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            atomicMin(&lo[bin][c], ord_float(bx[c]));
+            atomicMax(&hi[bin][c], ord_float(bx[3 + c]));
+        }
+    }
+    __syncwarp();
+}
+
+// f(valid, primitive, box) for order[b, e), a lane each, the loads of four rounds in flight together
+template <bool COHERENT, int kRounds, class F>
+__device__ __forceinline__ void sah_each(const float* __restrict__ boxes, const uint32_t* order, uint32_t b, uint32_t e, int lane, F&& f) {
+    for (uint32_t i0 = b; i0 < e; i0 += 32 * kRounds) {
+        uint32_t prim[kRounds];
+        float bx[kRounds][6];
+#pragma unroll
+        for (int j = 0; j < kRounds; ++j) {
+            const uint32_t i = i0 + 32 * j + lane;
+            prim[j] = i < e ? (COHERENT ? __ldcg(order + i) : order[i]) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < kRounds; ++j)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) bx[j][c] = i0 + 32 * j + lane < e ? boxes[6 * (size_t)prim[j] + c] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < kRounds; ++j)
+            if (i0 + 32 * j < e) f(i0 + 32 * j + lane < e, prim[j], bx[j]);
+    }
+}
+
+// a range's box (v[0..5]) and centroid box (v[6..11]), lane by lane; sah_bounds_warp: over the warp
+__device__ __forceinline__ void sah_bounds_init(float* v) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        v[a] = v[6 + a] = INFINITY;
+        v[3 + a] = v[9 + a] = -INFINITY;
+    }
+}
+__device__ __forceinline__ void sah_bounds_add(float* v, const float* bx) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        v[a] = fminf(v[a], bx[a]);
+        v[3 + a] = fmaxf(v[3 + a], bx[3 + a]);
+        const float c = 0.5f * (bx[a] + bx[3 + a]);
+        v[6 + a] = fminf(v[6 + a], c);
+        v[9 + a] = fmaxf(v[9 + a], c);
+    }
+}
+__device__ __forceinline__ void sah_bounds_warp(float* v) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        v[a] = warp_min(v[a]);
+        v[3 + a] = warp_max(v[3 + a]);
+        v[6 + a] = warp_min(v[6 + a]);
+        v[9 + a] = warp_max(v[9 + a]);
+    }
+}
+__device__ __forceinline__ float sah_scale(float clo, float chi) {
+    const float ext = chi - clo;
+    return ext > 0.0f ? (float)kSahBins / ext : 0.0f;
+}
+__device__ __forceinline__ int sah_bin_of(float lo, float hi, float origin, float scale) {
+    const float c = 0.5f * (lo + hi);
+    return max(0, min((int)((c - origin) * scale), kSahBins - 1));
+}
+__device__ __forceinline__ float pick3(const float* v, int a) { return a == 0 ? v[0] : a == 1 ? v[1] : v[2]; }
+// a warp's bins cleared
+__device__ __forceinline__ void sah_bins_clear(int (&lo)[3][kSahBins][3], int (&hi)[3][kSahBins][3], int (&cnt)[3][kSahBins], int lane) {
+    for (int k = lane; k < 3 * kSahBins; k += 32) (&cnt[0][0])[k] = 0;
+    for (int k = lane; k < 9 * kSahBins; k += 32) {
+        (&lo[0][0][0])[k] = ord_float(INFINITY);
+        (&hi[0][0][0])[k] = ord_float(-INFINITY);
+    }
+    __syncwarp();
+}
+
+// One level with fewer tasks than warps: G warps share a task (G * count <= 32, and about 64
+// primitives of the largest task a warp at least), each taking a contiguous chunk of the task's range.
+// The same computation as one warp per task -- bounds and bin contents are order-independent minima,
+// maxima and counts, the split is chosen by the same rule, and the partition stays stable (each warp
+// writes its chunk at the offsets of the chunks before it) -- so the tree is the same; the top levels
+// just run on the whole CTA instead of a few warps.  1024 primitives in shared memory: 9 us a level, half
+// of it instruction fetches of code that runs once (14 us and a launch with 32 warps a task and the
+// group's bins and bounds merged by its first warp).
+template <int kRounds>
 __device__ __forceinline__ void sah_level_grouped(const float* __restrict__ boxes, uint32_t* __restrict__ order, uint32_t* __restrict__ tmp,
                                                   uint32_t* __restrict__ left, uint32_t* __restrict__ right, float* __restrict__ nodeBoxes,
                                                   const uint2* cur, uint2* nxt, uint32_t count, bool median, uint32_t baseCur,
                                                   uint32_t baseNext, uint32_t& nNext, int (*bLo)[3][kSahBins][3],
                                                   int (*bHi)[3][kSahBins][3], int (*bCnt)[3][kSahBins], float (*gPart)[12],
-                                                  float (*tClo)[3], float (*tScale)[3], int* tBest, uint32_t* wLeft) {
+                                                  int* tBest, uint32_t* wLeft) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t largest = 0;
+    if ((uint32_t)lane < count) {
+        const uint2 tk = cur[lane];
+        largest = tk.y - tk.x;
+    }
+    largest = __reduce_max_sync(0xFFFFFFFFu, largest);
     uint32_t G = kSahWarps;
-    while (G * count > (uint32_t)kSahWarps) G >>= 1;
+    while (G > 1 && (G * count > (uint32_t)kSahWarps || (G - 1) * 64 >= largest)) G >>= 1;
     const uint32_t t = (uint32_t)warp / G, m = (uint32_t)warp % G;
     const bool has = t < count;  // warp-uniform
     const int lw = (int)(t * G);  // the task's leader warp (owner of its bins)
@@ -930,165 +1084,93 @@ __device__ __forceinline__ void sah_level_grouped(const float* __restrict__ boxe
         ce = min(e, cb + chunk);
     }
     // bounds and centroid bounds of the chunk, then of the task
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    float clo[3] = {INFINITY, INFINITY, INFINITY}, chi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t i = cb + lane; i < ce; i += 32) {
-        const float* bx = boxes + 6 * (size_t)order[i];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], bx[a]);
-            hi[a] = fmaxf(hi[a], bx[3 + a]);
-            const float c = 0.5f * (bx[a] + bx[3 + a]);
-            clo[a] = fminf(clo[a], c);
-            chi[a] = fmaxf(chi[a], c);
-        }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xFFFFFFFFu, lo[a], off));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xFFFFFFFFu, hi[a], off));
-            clo[a] = fminf(clo[a], __shfl_xor_sync(0xFFFFFFFFu, clo[a], off));
-            chi[a] = fmaxf(chi[a], __shfl_xor_sync(0xFFFFFFFFu, chi[a], off));
-        }
+    float v[12];
+    sah_bounds_init(v);
+    sah_each<false, kRounds>(boxes, order, cb, ce, lane, [&](bool valid, uint32_t, const float* bx) {
+        if (valid) sah_bounds_add(v, bx);
+    });
+    sah_bounds_warp(v);
     if (lane == 0)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            gPart[warp][a] = lo[a];
-            gPart[warp][3 + a] = hi[a];
-            gPart[warp][6 + a] = clo[a];
-            gPart[warp][9 + a] = chi[a];
-        }
-    __syncthreads();
-    if (has && m == 0) {
-        if (lane == 0) {
-            for (uint32_t g = 1; g < G; ++g)
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    lo[a] = fminf(lo[a], gPart[lw + g][a]);
-                    hi[a] = fmaxf(hi[a], gPart[lw + g][3 + a]);
-                    clo[a] = fminf(clo[a], gPart[lw + g][6 + a]);
-                    chi[a] = fmaxf(chi[a], gPart[lw + g][9 + a]);
-                }
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                nodeBoxes[6 * (size_t)node + a] = lo[a];
-                nodeBoxes[6 * (size_t)node + 3 + a] = hi[a];
-                const float ext = chi[a] - clo[a];
-                tClo[t][a] = clo[a];
-                tScale[t][a] = ext > 0.0f ? (float)kSahBins / ext : 0.0f;
-            }
-        }
-    }
+        for (int k = 0; k < 12; ++k) gPart[warp][k] = v[k];
+    if (has && !median) sah_bins_clear(bLo[warp], bHi[warp], bCnt[warp], lane);
     __syncthreads();
     float tc[3] = {0.0f, 0.0f, 0.0f}, ts[3] = {0.0f, 0.0f, 0.0f};
-    if (has)
+    if (has) {  // every warp of the group: lane g takes the g-th chunk's
+#pragma unroll
+        for (int k = 0; k < 12; ++k) v[k] = gPart[lw + ((uint32_t)lane < G ? lane : 0)][k];
+        sah_bounds_warp(v);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            tc[a] = tClo[t][a];
-            ts[a] = tScale[t][a];
+            tc[a] = v[6 + a];
+            ts[a] = sah_scale(v[6 + a], v[9 + a]);
         }
-    auto bin_of = [&](const float* bx, int a) {
-        const float c = 0.5f * (bx[a] + bx[3 + a]);
-        return max(0, min((int)((c - tc[a]) * ts[a]), kSahBins - 1));
-    };
-    if (has && !median) {  // every warp bins its chunk into its own bins (no atomics across warps)
-        for (int k = lane; k < 3 * kSahBins; k += 32) {
-            const int a = k / kSahBins, bn = k % kSahBins;
-            bCnt[warp][a][bn] = 0;
+        if (m == 0 && lane == 0)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                bLo[warp][a][bn][c] = ord_float(INFINITY);
-                bHi[warp][a][bn][c] = ord_float(-INFINITY);
-            }
-        }
-        __syncwarp();
-        for (uint32_t i = cb + lane; i < ce; i += 32) {
-            const float* bx = boxes + 6 * (size_t)order[i];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (ts[a] <= 0.0f) continue;
-                const int k = bin_of(bx, a);
-                atomicAdd(&bCnt[warp][a][k], 1);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    atomicMin(&bLo[warp][a][k][c], ord_float(bx[c]));
-                    atomicMax(&bHi[warp][a][k][c], ord_float(bx[3 + c]));
-                }
+            for (int k = 0; k < 6; ++k) nodeBoxes[6 * (size_t)node + k] = v[k];
+        if (!median)  // every warp bins its chunk into its own bins (no atomics across warps)
+            sah_each<false, kRounds>(boxes, order, cb, ce, lane, [&](bool valid, uint32_t, const float* bx) {
+#pragma unroll 1
+                for (int a = 0; a < 3; ++a)
+                    if (pick3(ts, a) > 0.0f)
+                        sah_bin(valid, sah_bin_of(pick3(bx, a), pick3(bx + 3, a), pick3(tc, a), pick3(ts, a)), bx, bCnt[warp][a],
+                                bLo[warp][a], bHi[warp][a], lane);
+            });
+    }
+    __syncthreads();
+    if (has && !median && G > 1) {  // the group's bins into the leader's (counts add, bounds are minima and maxima: exact)
+        constexpr int kWords = 3 * kSahBins;
+#pragma unroll 1
+        for (uint32_t k = m * 32 + lane; k < 7 * kWords; k += 32 * G) {
+            if (k < kWords) {
+                int r = 0;
+                for (uint32_t g = 1; g < G; ++g) r += (&bCnt[lw + g][0][0])[k];
+                (&bCnt[lw][0][0])[k] += r;
+            } else if (k < 4 * kWords) {
+                int r = (&bLo[lw][0][0][0])[k - kWords];
+                for (uint32_t g = 1; g < G; ++g) r = min(r, (&bLo[lw + g][0][0][0])[k - kWords]);
+                (&bLo[lw][0][0][0])[k - kWords] = r;
+            } else {
+                int r = (&bHi[lw][0][0][0])[k - 4 * kWords];
+                for (uint32_t g = 1; g < G; ++g) r = max(r, (&bHi[lw + g][0][0][0])[k - 4 * kWords]);
+                (&bHi[lw][0][0][0])[k - 4 * kWords] = r;
             }
         }
     }
     __syncthreads();
     if (has && m == 0) {  // the leader picks the split: cheapest surface-area cost, ties to the lowest candidate
         int bestCand = -1;
-        if (!median) {
-            // the group's bins into the leader's (counts add, bounds are minima and maxima: exact)
-            for (int k = lane; k < 3 * kSahBins; k += 32) {
-                const int a = k / kSahBins, bn = k % kSahBins;
-                int cnt = bCnt[lw][a][bn];
-                int l[3], h[3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    l[c] = bLo[lw][a][bn][c];
-                    h[c] = bHi[lw][a][bn][c];
-                }
-                for (uint32_t g = 1; g < G; ++g) {
-                    cnt += bCnt[lw + g][a][bn];
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        l[c] = min(l[c], bLo[lw + g][a][bn][c]);
-                        h[c] = max(h[c], bHi[lw + g][a][bn][c]);
-                    }
-                }
-                bCnt[lw][a][bn] = cnt;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    bLo[lw][a][bn][c] = l[c];
-                    bHi[lw][a][bn][c] = h[c];
-                }
-            }
-            __syncwarp();
+        if (!median)
             bestCand = sah_best_split(ts, lane, [&](int a, int k) { return bCnt[lw][a][k]; },
                                       [&](int a, int k, int c) { return bLo[lw][a][k][c]; },
                                       [&](int a, int k, int c) { return bHi[lw][a][k][c]; });
-        }
         if (lane == 0) tBest[t] = bestCand;
     }
     __syncthreads();
     const int best = has ? tBest[t] : -1;
     const int sa = best >= 0 ? best / (kSahBins - 1) : 0, sp = best >= 0 ? best % (kSahBins - 1) + 1 : 0;
-    if (best >= 0) {  // left count of the chunk
-        uint32_t nl = 0;
-        for (uint32_t i0 = cb; i0 < ce; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const bool isL = i < ce && bin_of(boxes + 6 * (size_t)order[i], sa) < sp;
-            nl += __popc(__ballot_sync(0xFFFFFFFFu, isL));
-        }
-        if (lane == 0) wLeft[warp] = nl;
+    if (best >= 0) {  // left count of the chunk: its bins before the split (the leader's hold the task's)
+        const int c = __reduce_add_sync(0xFFFFFFFFu, lane < sp ? bCnt[warp][sa][lane] : 0);
+        if (lane == 0) wLeft[warp] = (uint32_t)c;
     }
     __syncthreads();
     uint32_t nlTotal = 0;
     if (best >= 0) {  // stable partition: this chunk's lefts after the lefts of the chunks before it, rights likewise
-        uint32_t before = 0;
-        for (uint32_t g = 0; g < G; ++g) {
-            const uint32_t c = wLeft[lw + g];
-            if (g < m) before += c;
-            nlTotal += c;
-        }
+        const uint32_t c = (uint32_t)lane < G ? wLeft[lw + lane] : 0u;
+        nlTotal = wLeft[lw];
+        const uint32_t others = __reduce_add_sync(0xFFFFFFFFu, lane > 0 ? c : 0u);  // all chunks but the leader's
+        const uint32_t ahead = __reduce_add_sync(0xFFFFFFFFu, lane > 0 && (uint32_t)lane < m ? c : 0u);
+        const uint32_t before = m ? nlTotal - others + ahead : 0u;
         uint32_t lb = b + before, rb = b + nlTotal + ((cb - b) - before);
-        for (uint32_t i0 = cb; i0 < ce; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const bool valid = i < ce;
-            const uint32_t prim = valid ? order[i] : 0u;
-            const bool isL = valid && bin_of(boxes + 6 * (size_t)prim, sa) < sp;
+        sah_each<false, kRounds>(boxes, order, cb, ce, lane, [&](bool valid, uint32_t prim, const float* bx) {
+            const bool isL = valid && sah_bin_of(pick3(bx, sa), pick3(bx + 3, sa), pick3(tc, sa), pick3(ts, sa)) < sp;
             const unsigned lm = __ballot_sync(0xFFFFFFFFu, isL), rm = __ballot_sync(0xFFFFFFFFu, valid && !isL);
             const unsigned below = (1u << lane) - 1u;
             if (isL) tmp[lb + __popc(lm & below)] = prim;
             else if (valid) tmp[rb + __popc(rm & below)] = prim;
             lb += __popc(lm);
             rb += __popc(rm);
-        }
+        });
     }
     __syncthreads();
     if (best >= 0)
@@ -1117,204 +1199,36 @@ __device__ __forceinline__ void sah_level_grouped(const float* __restrict__ boxe
 // order[b, e) through tmp, then emit(mid) creates the children and writes the node's refs.
 // COHERENT: order[] and tmp[] may have been written by other SMs (the task kernel), so they are read
 // through L2.
-// The same for a task of at most 32 * R primitives, with each lane's primitives (ids and boxes)
-// loaded once into registers: every pass reads them there, and the partition writes order[]
-// directly.  Same bounds, bins, costs and stable partition, so the same split.
-template <int R, bool COHERENT, class Emit>
-__device__ __forceinline__ void sah_task_warp_small(const float* __restrict__ boxes, uint32_t* __restrict__ order,
-                                                    float* __restrict__ nodeBoxes, uint32_t b, uint32_t e, uint32_t node, bool median,
-                                                    int (&wLo)[3][kSahBins][3], int (&wHi)[3][kSahBins][3], int (&wCnt)[3][kSahBins],
-                                                    int lane, Emit&& emit) {
-    uint32_t prim[R];
-    float bx[R][6];
-    bool valid[R];
-#pragma unroll
-    for (int j = 0; j < R; ++j) {
-        const uint32_t i = b + (uint32_t)(32 * j + lane);
-        valid[j] = i < e;
-        prim[j] = valid[j] ? (COHERENT ? __ldcg(order + i) : order[i]) : 0u;
-    }
-#pragma unroll
-    for (int j = 0; j < R; ++j)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) bx[j][c] = valid[j] ? boxes[6 * (size_t)prim[j] + c] : 0.0f;
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    float clo[3] = {INFINITY, INFINITY, INFINITY}, chi[3] = {-INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-    for (int j = 0; j < R; ++j)
-        if (valid[j])
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = fminf(lo[a], bx[j][a]);
-                hi[a] = fmaxf(hi[a], bx[j][3 + a]);
-                const float c = 0.5f * (bx[j][a] + bx[j][3 + a]);
-                clo[a] = fminf(clo[a], c);
-                chi[a] = fmaxf(chi[a], c);
-            }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xFFFFFFFFu, lo[a], off));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xFFFFFFFFu, hi[a], off));
-            clo[a] = fminf(clo[a], __shfl_xor_sync(0xFFFFFFFFu, clo[a], off));
-            chi[a] = fmaxf(chi[a], __shfl_xor_sync(0xFFFFFFFFu, chi[a], off));
-        }
-    if (lane == 0)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            nodeBoxes[6 * (size_t)node + a] = lo[a];
-            nodeBoxes[6 * (size_t)node + 3 + a] = hi[a];
-        }
-    float scale[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const float ext = chi[a] - clo[a];
-        scale[a] = ext > 0.0f ? (float)kSahBins / ext : 0.0f;
-    }
-    // bin of primitive j on axis a (a may be a runtime value: selects, not indexing, keep the boxes
-    // in registers)
-    auto bin_of = [&](int j, int a) {
-        const float l = a == 0 ? bx[j][0] : (a == 1 ? bx[j][1] : bx[j][2]);
-        const float h = a == 0 ? bx[j][3] : (a == 1 ? bx[j][4] : bx[j][5]);
-        const float o = a == 0 ? clo[0] : (a == 1 ? clo[1] : clo[2]);
-        const float s = a == 0 ? scale[0] : (a == 1 ? scale[1] : scale[2]);
-        const float c = 0.5f * (l + h);
-        return max(0, min((int)((c - o) * s), kSahBins - 1));
-    };
-    int bestCand = -1;
-    if (!median) {
-        for (int k = lane; k < 3 * kSahBins; k += 32) {
-            const int a = k / kSahBins, bn = k % kSahBins;
-            wCnt[a][bn] = 0;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                wLo[a][bn][c] = ord_float(INFINITY);
-                wHi[a][bn][c] = ord_float(-INFINITY);
-            }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < R; ++j)
-            if (valid[j])
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    if (scale[a] <= 0.0f) continue;
-                    const int k = bin_of(j, a);
-                    atomicAdd(&wCnt[a][k], 1);
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        atomicMin(&wLo[a][k][c], ord_float(bx[j][c]));
-                        atomicMax(&wHi[a][k][c], ord_float(bx[j][3 + c]));
-                    }
-                }
-        __syncwarp();
-        bestCand = sah_best_split(scale, lane, [&](int a, int k) { return wCnt[a][k]; },
-                                  [&](int a, int k, int c) { return wLo[a][k][c]; },
-                                  [&](int a, int k, int c) { return wHi[a][k][c]; });
-    }
-    uint32_t mid = b + (e - b) / 2;  // no usable split (coincident centroids): halve the range
-    if (bestCand >= 0) {
-        const int a = bestCand / (kSahBins - 1), sp = bestCand % (kSahBins - 1) + 1;
-        bool isL[R];
-        uint32_t nl = 0;
-#pragma unroll
-        for (int j = 0; j < R; ++j) {
-            isL[j] = valid[j] && bin_of(j, a) < sp;
-            nl += __popc(__ballot_sync(0xFFFFFFFFu, isL[j]));
-        }
-        uint32_t lb = 0, rb = 0;
-        const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-        for (int j = 0; j < R; ++j) {  // every lane holds its primitives already: write order[] in place
-            const unsigned lm = __ballot_sync(0xFFFFFFFFu, isL[j]), rm = __ballot_sync(0xFFFFFFFFu, valid[j] && !isL[j]);
-            if (isL[j]) order[b + lb + __popc(lm & below)] = prim[j];
-            else if (valid[j]) order[b + nl + rb + __popc(rm & below)] = prim[j];
-            lb += __popc(lm);
-            rb += __popc(rm);
-        }
-        __syncwarp();
-        mid = b + nl;
-    }
-    emit(mid);
-    __syncwarp();
-}
-
-template <bool COHERENT, class Emit>
+template <bool COHERENT, int kRounds, class Emit>
 __device__ __forceinline__ void sah_task_warp(const float* __restrict__ boxes, uint32_t* __restrict__ order, uint32_t* __restrict__ tmp,
                                               float* __restrict__ nodeBoxes, uint32_t b, uint32_t e, uint32_t node, bool median,
                                               int (&wLo)[3][kSahBins][3], int (&wHi)[3][kSahBins][3], int (&wCnt)[3][kSahBins],
                                               int lane, Emit&& emit) {
-    if (e - b <= 64) {
-        sah_task_warp_small<2, COHERENT>(boxes, order, nodeBoxes, b, e, node, median, wLo, wHi, wCnt, lane, emit);
-        return;
-    }
-    auto ord = [&](uint32_t i) { return COHERENT ? __ldcg(order + i) : order[i]; };
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    float clo[3] = {INFINITY, INFINITY, INFINITY}, chi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t i = b + lane; i < e; i += 32) {
-        const float* bx = boxes + 6 * (size_t)ord(i);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], bx[a]);
-            hi[a] = fmaxf(hi[a], bx[3 + a]);
-            const float c = 0.5f * (bx[a] + bx[3 + a]);
-            clo[a] = fminf(clo[a], c);
-            chi[a] = fmaxf(chi[a], c);
-        }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xFFFFFFFFu, lo[a], off));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xFFFFFFFFu, hi[a], off));
-            clo[a] = fminf(clo[a], __shfl_xor_sync(0xFFFFFFFFu, clo[a], off));
-            chi[a] = fmaxf(chi[a], __shfl_xor_sync(0xFFFFFFFFu, chi[a], off));
-        }
+    float v[12];
+    sah_bounds_init(v);
+    sah_each<COHERENT, kRounds>(boxes, order, b, e, lane, [&](bool valid, uint32_t, const float* bx) {
+        if (valid) sah_bounds_add(v, bx);
+    });
+    sah_bounds_warp(v);
     if (lane == 0)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            nodeBoxes[6 * (size_t)node + a] = lo[a];
-            nodeBoxes[6 * (size_t)node + 3 + a] = hi[a];
-        }
-    float scale[3];
+        for (int k = 0; k < 6; ++k) nodeBoxes[6 * (size_t)node + k] = v[k];
+    float clo[3], scale[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const float ext = chi[a] - clo[a];
-        scale[a] = ext > 0.0f ? (float)kSahBins / ext : 0.0f;
+        clo[a] = v[6 + a];
+        scale[a] = sah_scale(v[6 + a], v[9 + a]);
     }
-    auto bin_of = [&](const float* bx, int a) {
-        const float c = 0.5f * (bx[a] + bx[3 + a]);
-        return max(0, min((int)((c - clo[a]) * scale[a]), kSahBins - 1));
-    };
     int bestCand = -1;
     if (!median) {
-        for (int k = lane; k < 3 * kSahBins; k += 32) {
-            const int a = k / kSahBins, bn = k % kSahBins;
-            wCnt[a][bn] = 0;
+        sah_bins_clear(wLo, wHi, wCnt, lane);
+        sah_each<COHERENT, kRounds>(boxes, order, b, e, lane, [&](bool valid, uint32_t, const float* bx) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                wLo[a][bn][c] = ord_float(INFINITY);
-                wHi[a][bn][c] = ord_float(-INFINITY);
-            }
-        }
-        __syncwarp();
-        for (uint32_t i = b + lane; i < e; i += 32) {
-            const float* bx = boxes + 6 * (size_t)ord(i);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (scale[a] <= 0.0f) continue;
-                const int k = bin_of(bx, a);
-                atomicAdd(&wCnt[a][k], 1);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    atomicMin(&wLo[a][k][c], ord_float(bx[c]));
-                    atomicMax(&wHi[a][k][c], ord_float(bx[3 + c]));
-                }
-            }
-        }
-        __syncwarp();
+            for (int a = 0; a < 3; ++a)
+                if (pick3(scale, a) > 0.0f)
+                    sah_bin(valid, sah_bin_of(pick3(bx, a), pick3(bx + 3, a), pick3(clo, a), pick3(scale, a)), bx, wCnt[a], wLo[a], wHi[a],
+                            lane);
+        });
         bestCand = sah_best_split(scale, lane, [&](int a, int k) { return wCnt[a][k]; },
                                   [&](int a, int k, int c) { return wLo[a][k][c]; },
                                   [&](int a, int k, int c) { return wHi[a][k][c]; });
@@ -1322,25 +1236,17 @@ __device__ __forceinline__ void sah_task_warp(const float* __restrict__ boxes, u
     uint32_t mid = b + (e - b) / 2;  // no usable split (coincident centroids): halve the range
     if (bestCand >= 0) {
         const int a = bestCand / (kSahBins - 1), sp = bestCand % (kSahBins - 1) + 1;
-        uint32_t nl = 0;
-        for (uint32_t i0 = b; i0 < e; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const bool isL = i < e && bin_of(boxes + 6 * (size_t)ord(i), a) < sp;
-            nl += __popc(__ballot_sync(0xFFFFFFFFu, isL));
-        }
+        const uint32_t nl = (uint32_t)__reduce_add_sync(0xFFFFFFFFu, lane < sp ? wCnt[a][lane] : 0);
         uint32_t lb = 0, rb = 0;
-        for (uint32_t i0 = b; i0 < e; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const bool valid = i < e;
-            const uint32_t prim = valid ? ord(i) : 0u;
-            const bool isL = valid && bin_of(boxes + 6 * (size_t)prim, a) < sp;
+        sah_each<COHERENT, kRounds>(boxes, order, b, e, lane, [&](bool valid, uint32_t prim, const float* bx) {
+            const bool isL = valid && sah_bin_of(pick3(bx, a), pick3(bx + 3, a), pick3(clo, a), pick3(scale, a)) < sp;
             const unsigned lm = __ballot_sync(0xFFFFFFFFu, isL), rm = __ballot_sync(0xFFFFFFFFu, valid && !isL);
             const unsigned below = (1u << lane) - 1u;
             if (isL) tmp[b + lb + __popc(lm & below)] = prim;
             else if (valid) tmp[b + nl + rb + __popc(rm & below)] = prim;
             lb += __popc(lm);
             rb += __popc(rm);
-        }
+        });
         __syncwarp();
         for (uint32_t i = b + lane; i < e; i += 32) order[i] = COHERENT ? __ldcg(tmp + i) : tmp[i];
         __syncwarp();
@@ -1348,6 +1254,129 @@ __device__ __forceinline__ void sah_task_warp(const float* __restrict__ boxes, u
     }
     emit(mid);
     __syncwarp();
+}
+
+// The whole subtree of a task of at most 32 primitives on one warp, a primitive a lane: a node costs no
+// access to memory but its own results.  Nodes are taken from a stack (lane i holds entry i); the
+// lanes of a node's range are reordered by its partition.  Bounds, bins, costs, ties and partition as
+// sah_task_warp's; two primitives need no bins: every split between them costs the same, so it is the
+// first on the first axis that tells them apart.  Node ids: the root has its own, the others are
+// first .. first + (e - b - 2) - 1.  Returns the level below the deepest node.
+__device__ __forceinline__ uint32_t sah_subtree_warp(const float* __restrict__ boxes, uint32_t* __restrict__ order, uint32_t* __restrict__ left,
+                                                     uint32_t* __restrict__ right, float* __restrict__ nodeBoxes, uint32_t b, uint32_t e,
+                                                     uint32_t node, uint32_t first, uint32_t level, uint32_t medianLevel,
+                                                     int (&wLo)[3][kSahBins][3], int (&wHi)[3][kSahBins][3], int (&wCnt)[3][kSahBins],
+                                                     int lane) {
+    constexpr unsigned full = 0xFFFFFFFFu;
+    const int m = (int)(e - b);
+    uint32_t prim = lane < m ? __ldcg(order + b + lane) : 0u;
+    float bx[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) bx[c] = lane < m ? boxes[6 * (size_t)prim + c] : 0.0f;
+    uint32_t stRange = (uint32_t)m << 8 | level << 16, stNode = node;  // entry 0: lanes 0 .. m - 1
+    uint32_t deepest = 0;
+    for (int sp = 1; sp > 0;) {
+        --sp;
+        const uint32_t rg = __shfl_sync(full, stRange, sp), nd = __shfl_sync(full, stNode, sp);
+        const int lb = (int)(rg & 0xFFu), le = (int)(rg >> 8 & 0xFFu);
+        const uint32_t lv = rg >> 16;
+        const bool in = lane >= lb && lane < le;
+        deepest = max(deepest, lv + 1);
+        float v[12];
+        sah_bounds_init(v);
+        if (in) sah_bounds_add(v, bx);
+        sah_bounds_warp(v);
+        const float mineOut = lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : lane == 3 ? v[3] : lane == 4 ? v[4] : v[5];
+        if (lane < 6) nodeBoxes[6 * (size_t)nd + lane] = mineOut;
+        float scale[3];
+        int bin[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            scale[a] = sah_scale(v[6 + a], v[9 + a]);
+            bin[a] = sah_bin_of(bx[a], bx[3 + a], v[6 + a], scale[a]);
+        }
+        int axis = -1, before = 0;  // left: bin[axis] < before
+        if (lv < medianLevel) {
+            if (le - lb == 2) {
+                float q[6];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    q[c] = fminf(INFINITY, bx[c]);
+                    q[3 + c] = fmaxf(-INFINITY, bx[3 + c]);
+                }
+                const float area = half_area3(q, q + 3);
+                const float cost = __shfl_sync(full, area, lb) + __shfl_sync(full, area, lb + 1);
+                if (cost < INFINITY)
+#pragma unroll
+                    for (int a = 2; a >= 0; --a) {
+                        const int b0 = __shfl_sync(full, bin[a], lb), b1 = __shfl_sync(full, bin[a], lb + 1);
+                        if (scale[a] > 0.0f && b0 != b1) {
+                            axis = a;
+                            before = min(b0, b1) + 1;
+                        }
+                    }
+            } else {
+                sah_bins_clear(wLo, wHi, wCnt, lane);
+                if (in)
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        if (pick3(scale, a) <= 0.0f) continue;
+                        const int k = a == 0 ? bin[0] : a == 1 ? bin[1] : bin[2];
+                        atomicAdd(&wCnt[a][k], 1);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            atomicMin(&wLo[a][k][c], ord_float(bx[c]));
+                            atomicMax(&wHi[a][k][c], ord_float(bx[3 + c]));
+                        }
+                    }
+                __syncwarp();
+                const int cand = sah_best_split(scale, lane, [&](int a, int k) { return wCnt[a][k]; },
+                                                [&](int a, int k, int c) { return wLo[a][k][c]; },
+                                                [&](int a, int k, int c) { return wHi[a][k][c]; });
+                __syncwarp();
+                if (cand >= 0) {
+                    axis = cand / (kSahBins - 1);
+                    before = cand % (kSahBins - 1) + 1;
+                }
+            }
+        }
+        int mid = lb + (le - lb) / 2;  // no usable split: halve the range
+        if (axis >= 0) {
+            const bool isL = in && (axis == 0 ? bin[0] : axis == 1 ? bin[1] : bin[2]) < before;
+            const unsigned lm = __ballot_sync(full, isL), rm = __ballot_sync(full, in && !isL);
+            mid = lb + __popc(lm);
+            const unsigned below = (1u << lane) - 1u;
+            int* perm = &wCnt[0][0];  // the bins are done with
+            if (in) perm[isL ? lb + __popc(lm & below) : mid + __popc(rm & below)] = lane;
+            __syncwarp();
+            const int src = in ? perm[lane] : lane;
+            __syncwarp();
+            prim = __shfl_sync(full, prim, src);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) bx[c] = __shfl_sync(full, bx[c], src);
+        }
+        uint32_t ref[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int r0 = c ? mid : lb, r1 = c ? le : mid;
+            if (r1 - r0 == 1) {
+                ref[c] = kLeaf | (b + (uint32_t)r0);
+            } else {
+                ref[c] = first++;
+                if (lane == sp) {
+                    stRange = (uint32_t)r0 | (uint32_t)r1 << 8 | (lv + 1) << 16;
+                    stNode = ref[c];
+                }
+                ++sp;
+            }
+        }
+        if (lane == 0) {
+            left[nd] = ref[0];
+            right[nd] = ref[1];
+        }
+    }
+    if (lane < m) order[b + lane] = prim;
+    return deepest;
 }
 
 // The first kSahParallelLevels levels, one launch per level: CTA t of level L splits task t of the
@@ -1365,7 +1394,6 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_level(const float* __
     __shared__ int bLo[kSahWarps][3][kSahBins][3], bHi[kSahWarps][3][kSahBins][3];
     __shared__ int bCnt[kSahWarps][3][kSahBins];
     __shared__ float gPart[kSahWarps][12];
-    __shared__ float tClo[kSahWarps][3], tScale[kSahWarps][3];
     __shared__ int tBest[kSahWarps];
     __shared__ uint32_t wLeft[kSahWarps];
     uint2* cur = (level & 1) ? tasksB : tasksA;
@@ -1380,8 +1408,8 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_level(const float* __
     if (blockIdx.x >= count) return;
     uint32_t base = level == 0 ? 0u : 1u;
     for (int k = 1; k < level; ++k) base += lvCount[k];
-    sah_level_grouped(boxes, order, tmp, left, right, nodeBoxes, cur + blockIdx.x, nxt, 1u, (uint32_t)level >= medianLevel,
-                      base + blockIdx.x, base + count, lvCount[level + 1], bLo, bHi, bCnt, gPart, tClo, tScale, tBest, wLeft);
+    sah_level_grouped<4>(boxes, order, tmp, left, right, nodeBoxes, cur + blockIdx.x, nxt, 1u, (uint32_t)level >= medianLevel,
+                      base + blockIdx.x, base + count, lvCount[level + 1], bLo, bHi, bCnt, gPart, tBest, wLeft);
 }
 
 // ---- one task over many CTAs (the top levels of large builds) -------------------------------------
@@ -1415,25 +1443,19 @@ __device__ __forceinline__ int bin_slot_cnt(int a, int bn) { return a * kSahBins
 __device__ __forceinline__ int bin_slot_lo(int a, int bn, int c) { return 3 * kSahBins + (a * kSahBins + bn) * 3 + c; }
 __device__ __forceinline__ int bin_slot_hi(int a, int bn, int c) { return 3 * kSahBins + 9 * kSahBins + (a * kSahBins + bn) * 3 + c; }
 
-// the task's frame (box, centroid origin and bin scale) from the parts of all its CTAs
-__device__ __forceinline__ void split_frame(const float* part, float* lo, float* hi, float* clo, float* scale) {
-    float chi[3];
+// the task's frame (box, centroid origin and bin scale) from the parts of all its CTAs, a part a lane
+static_assert(kSplitCtas == 32, "a lane takes a part");
+__device__ __forceinline__ void split_frame(const float* part, int lane, float* lo, float* hi, float* clo, float* scale) {
+    float v[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = part[12 * lane + k];
+    sah_bounds_warp(v);
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-        lo[a] = clo[a] = INFINITY;
-        hi[a] = chi[a] = -INFINITY;
-    }
-    for (int m = 0; m < kSplitCtas; ++m) {
-        const float* p = part + 12 * m;
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], p[a]);
-            hi[a] = fmaxf(hi[a], p[3 + a]);
-            clo[a] = fminf(clo[a], p[6 + a]);
-            chi[a] = fmaxf(chi[a], p[9 + a]);
-        }
-    }
-    for (int a = 0; a < 3; ++a) {
-        const float ext = chi[a] - clo[a];
-        scale[a] = ext > 0.0f ? (float)kSahBins / ext : 0.0f;
+        lo[a] = v[a];
+        hi[a] = v[3 + a];
+        clo[a] = v[6 + a];
+        scale[a] = sah_scale(v[6 + a], v[9 + a]);
     }
 }
 
@@ -1505,7 +1527,7 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_split(const float* __
         return;
     }
     float lo[3], hi[3], clo[3], scale[3];
-    split_frame(part, lo, hi, clo, scale);
+    split_frame(part, lane, lo, hi, clo, scale);
     auto bin_of = [&](const float* bx, int a) {
         const float c = 0.5f * (bx[a] + bx[3 + a]);
         return max(0, min((int)((c - clo[a]) * scale[a]), kSahBins - 1));
@@ -1521,21 +1543,20 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_split(const float* __
             }
         }
         __syncwarp();
-        for (uint32_t i = cb + threadIdx.x; i < ce; i += blockDim.x) {
-            const float* bx = boxes + 6 * (size_t)order[i];
-            for (int a = 0; a < 3; ++a) {
-                if (scale[a] <= 0.0f) continue;
-                const int k = bin_of(bx, a);
-                atomicAdd(&sb[warp][bin_slot_cnt(a, k)], 1);
-                for (int c = 0; c < 3; ++c) {
-                    atomicMin(&sb[warp][bin_slot_lo(a, k, c)], ord_float(bx[c]));
-                    atomicMax(&sb[warp][bin_slot_hi(a, k, c)], ord_float(bx[3 + c]));
-                }
-            }
+        for (uint32_t i0 = cb + warp * 32; i0 < ce; i0 += blockDim.x) {
+            const bool valid = i0 + lane < ce;
+            float bx[6];
+            const uint32_t prim = valid ? order[i0 + lane] : 0u;
+            for (int c = 0; c < 6; ++c) bx[c] = valid ? boxes[6 * (size_t)prim + c] : 0.0f;
+            for (int a = 0; a < 3; ++a)
+                if (scale[a] > 0.0f)
+                    sah_bin(valid, bin_of(bx, a), bx, &sb[warp][bin_slot_cnt(a, 0)], reinterpret_cast<int(*)[3]>(&sb[warp][bin_slot_lo(a, 0, 0)]),
+                            reinterpret_cast<int(*)[3]>(&sb[warp][bin_slot_hi(a, 0, 0)]), lane);
         }
         __syncthreads();
         for (int k = threadIdx.x; k < kBinInts; k += blockDim.x) {
             int r = sb[0][k];
+#pragma unroll 8
             for (int w = 1; w < kSahWarps; ++w)
                 r = k < 3 * kSahBins ? r + sb[w][k] : (k < 3 * kSahBins + 9 * kSahBins ? min(r, sb[w][k]) : max(r, sb[w][k]));
             binsT[(size_t)m * kBinInts + k] = r;
@@ -1546,6 +1567,7 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_split(const float* __
         if (!median)
             for (int k = threadIdx.x; k < kBinInts; k += blockDim.x) {
                 int r = binsT[k];
+#pragma unroll 8
                 for (int c = 1; c < kSplitCtas; ++c) {
                     const int o = binsT[(size_t)c * kBinInts + k];
                     r = k < 3 * kSahBins ? r + o : (k < 3 * kSahBins + 9 * kSahBins ? min(r, o) : max(r, o));
@@ -1649,34 +1671,52 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_split(const float* __
 // with fewer tasks than warps spread each task over a group of warps), until a level has `handoff`
 // tasks or more.  That level's tasks go to the queue Q, whose slots are the node ids from baseCur
 // on, and k_sah_tasks finishes the tree.
-__global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_build(const float* __restrict__ boxes, uint32_t n, uint32_t* __restrict__ order,
-                                                                 uint32_t* __restrict__ tmp, uint32_t* __restrict__ left,
+// SMALL: all levels from the root, for builds of up to kSahSmall primitives (a TLAS), whose boxes, order and
+// partition buffer the CTA keeps in shared memory.
+constexpr size_t kSahSmallSmem = kSahSmall * (24 + 4 + 4);
+template <bool SMALL>
+__global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_build(const float* __restrict__ boxesIn, uint32_t n, uint32_t* orderOut,
+                                                                 uint32_t* tmpBuf, uint32_t* __restrict__ left,
                                                                  uint32_t* __restrict__ right, float* __restrict__ nodeBoxes,
                                                                  uint2* __restrict__ tasksA, uint2* __restrict__ tasksB,
-                                                                 uint32_t medianLevel, uint32_t handoff, SahQueue Q,
+                                                                 uint32_t firstLevel, uint32_t medianLevel, uint32_t handoff, SahQueue Q,
                                                                  const uint32_t* __restrict__ lvCount, uint32_t* __restrict__ levelsOut) {
+    constexpr int kRounds = SMALL ? 1 : 4;
+    extern __shared__ float sahSmem[];
+    const float* boxes = SMALL ? sahSmem : boxesIn;
+    uint32_t* order = SMALL ? reinterpret_cast<uint32_t*>(sahSmem) + 6 * kSahSmall : orderOut;
+    uint32_t* tmp = SMALL ? reinterpret_cast<uint32_t*>(sahSmem) + 7 * kSahSmall : tmpBuf;
     __shared__ int bLo[kSahWarps][3][kSahBins][3], bHi[kSahWarps][3][kSahBins][3];
     __shared__ int bCnt[kSahWarps][3][kSahBins];
     __shared__ uint32_t nCur, nNext, baseCur, baseNext, levels;
     // levels with fewer tasks than warps: per-warp partial bounds, per-task centroid frame and split,
     // per-warp left counts
     __shared__ float gPart[kSahWarps][12];
-    __shared__ float tClo[kSahWarps][3], tScale[kSahWarps][3];
     __shared__ int tBest[kSahWarps];
     __shared__ uint32_t wLeft[kSahWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {  // the state after the level kernels (their counts; level 0: the root)
-        uint32_t base = 1, lv = 1;
-        while (lv < (uint32_t)kSahParallelLevels && lvCount[lv]) base += lvCount[lv++];
-        nCur = lv < (uint32_t)kSahParallelLevels ? 0u : lvCount[lv];
+        uint32_t base = 0, lv = 0;
+        nCur = 1;
+        while (lv < firstLevel && nCur) {
+            base += nCur;
+            nCur = lvCount[++lv];
+        }
         nNext = 0;
         baseCur = base;          // node id of the current level's first task
         baseNext = base + nCur;  // node id of the next level's first task
         levels = lv;
     }
     __syncthreads();
-    uint2* cur = (kSahParallelLevels & 1) ? tasksB : tasksA;
-    uint2* nxt = (kSahParallelLevels & 1) ? tasksA : tasksB;
+    uint2* cur = (firstLevel & 1) ? tasksB : tasksA;
+    uint2* nxt = (firstLevel & 1) ? tasksA : tasksB;
+    if (SMALL) {  // no level kernels: the preparations of level 0
+        for (uint32_t i = threadIdx.x; i < 6 * n; i += blockDim.x) sahSmem[i] = boxesIn[i];
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) order[i] = i;
+        for (uint32_t i = threadIdx.x; i + 1 < n; i += blockDim.x) left[i] = right[i] = kLeaf;
+        if (threadIdx.x == 0) cur[0] = make_uint2(0u, n);
+        __syncthreads();
+    }
     for (;;) {
         const uint32_t count = nCur;
         if (count == 0) break;
@@ -1690,18 +1730,20 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_build(const float* __
                 Q.ctr[1] = count;
                 Q.ctr[2] = baseCur;
                 Q.ctr[3] = n - 1 - baseCur;
+                Q.ctr[4] = n - 1;           // ids from here down go to the subtrees
+                Q.ctr[5] = n - 1 - baseCur;  // nodes not yet made
             }
             break;
         }
         const bool median = levels >= medianLevel;  // from here on ranges are halved: the depth stays bounded
         if (count < (uint32_t)kSahWarps) {
-            sah_level_grouped(boxes, order, tmp, left, right, nodeBoxes, cur, nxt, count, median, baseCur, baseNext, nNext, bLo, bHi,
-                              bCnt, gPart, tClo, tScale, tBest, wLeft);
+            sah_level_grouped<kRounds>(boxes, order, tmp, left, right, nodeBoxes, cur, nxt, count, median, baseCur, baseNext, nNext, bLo, bHi,
+                              bCnt, gPart, tBest, wLeft);
         } else
         for (uint32_t t = warp; t < count; t += kSahWarps) {
             const uint2 tk = cur[t];
             const uint32_t b = tk.x, e = tk.y, node = baseCur + t;
-            sah_task_warp<false>(boxes, order, tmp, nodeBoxes, b, e, node, median, bLo[warp], bHi[warp], bCnt[warp], lane,
+            sah_task_warp<false, kRounds>(boxes, order, tmp, nodeBoxes, b, e, node, median, bLo[warp], bHi[warp], bCnt[warp], lane,
                                  [&](uint32_t mid) {  // single primitives become leaf refs, the rest next-level tasks
                                      if (lane != 0) return;
                                      const uint32_t rb0[2] = {b, mid}, re0[2] = {mid, e};
@@ -1732,20 +1774,24 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_build(const float* __
         nxt = sw;
         __syncthreads();
     }
+    if (SMALL)
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) orderOut[i] = order[i];
     if (threadIdx.x == 0 && levelsOut) *levelsOut = levels;
 }
 
 // The rest of the tree on every SM: a warp claims the next queue slot, waits (bounded) until the
 // slot's task is published, splits it as k_sah_build does, and publishes its children's tasks in
-// the next free slots (node id = first node id of the queue + slot).  Every internal node is one
-// task, so the queue holds exactly n - 1 - (first node id) tasks and a warp whose claim lies beyond
-// that is done.  A slot's task is published by the warp that split its parent, which claimed an
-// earlier slot and runs, so every wait ends; a wait that still runs out sets *status to 2 and
-// leaves that subtree as prepared (valid refs, unset boxes).
+// the next free slots (node id = first node id of the queue + slot).  A task of at most 32 primitives is
+// finished by its warp, whose node ids come from the upper end; a warp whose slot will not be
+// used sees that every node is made, and is done.  A slot's task is published by the warp that split
+// its parent, which claimed an earlier slot and runs, so every wait ends; a wait that still runs out
+// sets *status to 2 and leaves that subtree as prepared (valid refs, unset boxes).
+// A task costs its warp some 9 us of waits on L2 (claim, publication, order, boxes, children), which
+// small ones would pay per node: 191 us for 61442 triangles (601 us with every node a task).
 __global__ void __launch_bounds__(kSahTaskWarps * 32, 3) k_sah_tasks(const float* __restrict__ boxes, uint32_t* __restrict__ order,
                                                                   uint32_t* __restrict__ tmp, uint32_t* __restrict__ left,
                                                                   uint32_t* __restrict__ right, float* __restrict__ nodeBoxes,
-                                                                  SahQueue Q, uint32_t medianLevel, uint32_t* __restrict__ levelsOut,
+                                                                  SahQueue Q, uint32_t medianLevel, uint32_t subtree, uint32_t* __restrict__ levelsOut,
                                                                   int* __restrict__ status, uint32_t waitLimit) {
     __shared__ int bLo[kSahTaskWarps][3][kSahBins][3], bHi[kSahTaskWarps][3][kSahBins][3];
     __shared__ int bCnt[kSahTaskWarps][3][kSahBins];
@@ -1758,6 +1804,10 @@ __global__ void __launch_bounds__(kSahTaskWarps * 32, 3) k_sah_tasks(const float
             slot = atomicAdd(Q.ctr, 1u);
             if (slot < total) {
                 for (uint32_t spins = 0; ld_relaxed(Q.ready + slot) == 0; ++spins) {
+                    if (ld_relaxed(Q.ctr + 5) == 0) {  // every node is made: no task is left for the slot
+                        slot = total;
+                        break;
+                    }
                     if (spins >= waitLimit) {
                         ok = 0;
                         if (status) atomicExch(status, 2);
@@ -1773,23 +1823,35 @@ __global__ void __launch_bounds__(kSahTaskWarps * 32, 3) k_sah_tasks(const float
         __threadfence();  // after the publication: the task and its order[] range
         const uint4 tk = __ldcg(Q.tasks + slot);
         const uint32_t b = tk.x, e = tk.y, node = tk.z, level = tk.w;
+        if (e - b <= subtree) {
+            uint32_t first = 0;
+            if (lane == 0 && e - b > 2) first = atomicSub(Q.ctr + 4, e - b - 2) - (e - b - 2);
+            first = __shfl_sync(0xFFFFFFFFu, first, 0);
+            deepest = max(deepest, sah_subtree_warp(boxes, order, left, right, nodeBoxes, b, e, node, first, level, medianLevel, bLo[warp],
+                                                    bHi[warp], bCnt[warp], lane));
+            if (lane == 0) atomicSub(Q.ctr + 5, e - b - 1);
+            continue;
+        }
         deepest = max(deepest, level + 1);
-        sah_task_warp<true>(boxes, order, tmp, nodeBoxes, b, e, node, level >= medianLevel, bLo[warp], bHi[warp], bCnt[warp], lane,
+        sah_task_warp<true, 4>(boxes, order, tmp, nodeBoxes, b, e, node, level >= medianLevel, bLo[warp], bHi[warp], bCnt[warp], lane,
                             [&](uint32_t mid) {
                                 const uint32_t rb0[2] = {b, mid}, re0[2] = {mid, e};
                                 uint32_t ref[2] = {0u, 0u};
                                 if (lane == 0) {
+                                    const uint32_t inner = (mid - b > 1 ? 1u : 0u) + (e - mid > 1 ? 1u : 0u);
+                                    uint32_t q = inner ? atomicAdd(Q.ctr + 1, inner) : 0u;
                                     for (int c = 0; c < 2; ++c) {
                                         if (re0[c] - rb0[c] == 1) {
                                             ref[c] = kLeaf | rb0[c];
                                         } else {
-                                            const uint32_t q = atomicAdd(Q.ctr + 1, 1u);
                                             ref[c] = base + q;
                                             Q.tasks[q] = make_uint4(rb0[c], re0[c], base + q, level + 1);
+                                            ++q;
                                         }
                                     }
                                     left[node] = ref[0];
                                     right[node] = ref[1];
+                                    atomicSub(Q.ctr + 5, 1u);
                                 }
                                 __threadfence();  // every lane's order[] writes and the new tasks, then the publication
                                 __syncwarp();
@@ -1914,6 +1976,9 @@ cudaError_t lbvh_refit(const LbvhBuffers& b, cudaStream_t s) {
 }
 
 static int sah_task_grid() {  // persistent grid of k_sah_tasks (every resident block)
+    // (per device and process; the shared memory of the small build is asked for on every device)
+    if (cudaFuncSetAttribute((const void*)k_sah_build<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSahSmallSmem) != cudaSuccess)
+        return 0;
     static std::atomic<int> grid{0};
     int g = grid.load(std::memory_order_acquire);
     if (g) return g;
@@ -1936,7 +2001,7 @@ cudaError_t sah_build(const LbvhBuffers& b, bool parents, uint32_t* levels, cuda
     Q.ready = reinterpret_cast<uint32_t*>(b.sahQueue + 16 * (size_t)b.n);
     Q.ctr = Q.ready + b.n;
     uint32_t* lvCount = Q.ctr + 8;  // tasks per level of the level kernels
-    cudaError_t e = cudaMemsetAsync(Q.ready, 0, 4 * (size_t)b.n + 64, s);  // ready words and counters
+    cudaError_t e = cudaMemsetAsync(Q.ready, 0, 4 * (size_t)b.n + 96, s);  // ready words and counters
     if (e != cudaSuccess) return e;
     // scratch: the sort buffers (n words each); at most n / 2 tasks per level, 2 words each
     uint2* tasksA = reinterpret_cast<uint2*>(b.valsA);
@@ -1958,18 +2023,25 @@ cudaError_t sah_build(const LbvhBuffers& b, bool parents, uint32_t* levels, cuda
                 count_launch();
             }
     }
-    for (int lv = lv0; lv < kSahParallelLevels; ++lv)
+    const bool small = b.n <= kSahSmall;
+    int levelKernels = 0;  // until a level's tasks hold some kSahTask primitives
+    while (!small && levelKernels < kSahParallelLevels && (b.n >> levelKernels) > kSahTask) ++levelKernels;
+    for (int lv = lv0; lv < levelKernels; ++lv)
         k_sah_level<<<1u << lv, kSahWarps * 32, 0, s>>>(b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA,
                                                          tasksB, lvCount, lv, kSahMedianLevel);
-    k_sah_build<<<1, kSahWarps * 32, 0, s>>>(b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA, tasksB,
-                                              kSahMedianLevel, kSahHandoff, Q, lvCount, levels);
+    if (small)
+        k_sah_build<true><<<1, kSahWarps * 32, kSahSmallSmem, s>>>(b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA,
+                                                                   tasksB, 0u, kSahMedianLevel, kSahSmallHandoff, Q, lvCount, levels);
+    else
+        k_sah_build<false><<<1, kSahWarps * 32, 0, s>>>(b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA, tasksB,
+                                                        (uint32_t)levelKernels, kSahMedianLevel, kSahHandoff, Q, lvCount, levels);
     // polls of an unpublished task before a warp gives up (RG_SAH_WAIT_LIMIT overrides; 0 makes
     // the first unpublished slot end the wait, which tests use to check the reported status)
     uint32_t waitLimit = kSahWaitLimit;
     if (const char* env = getenv("RG_SAH_WAIT_LIMIT")) waitLimit = (uint32_t)strtoul(env, nullptr, 10);
     k_sah_tasks<<<grid, kSahTaskWarps * 32, 0, s>>>(b.primBoxes, b.order, b.keysA, b.left, b.right, b.nodeBoxes, Q, kSahMedianLevel,
-                                                     levels, b.status, waitLimit);
-    count_launch(kSahParallelLevels - lv0 + 2);
+                                                     small ? kSahSubtreeSmall : kSahSubtree, levels, b.status, waitLimit);
+    count_launch(levelKernels - lv0 + 2);
     if (parents) {
         k_parents<<<blocks(b.n - 1, 256), 256, 0, s>>>(b.left, b.right, b.n, b.parents);
         count_launch();

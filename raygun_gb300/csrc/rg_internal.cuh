@@ -142,14 +142,14 @@ struct LbvhBuffers {  // scratch + outputs of one LBVH build, sized by the calle
 };
 
 // task queue of the SAH builder's task kernel: n task records (range, node id, level), n ready
-// words, 8 counters (claims, pushes, first node id, tasks in total), 8 per-level task counts of its
-// level kernels
+// words, 8 counters (claims, pushes, first node id, nodes in total, end of the node ids that are left,
+// nodes not yet made), 16 per-level task counts of its level kernels
 struct SahQueue {
     uint4* tasks;
     uint32_t* ready;
     uint32_t* ctr;
 };
-constexpr size_t sah_queue_bytes(size_t n) { return 20 * n + 64; }
+constexpr size_t sah_queue_bytes(size_t n) { return 20 * n + 96; }
 
 // onesweep radix sort of the Morton codes: keys per tile, and the layout of its state words (zeroed
 // by each build): 4 passes x 256 digit counts, 4 tile counters, then per pass one status word per
