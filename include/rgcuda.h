@@ -127,7 +127,7 @@ typedef struct {
     uint64_t tris;       /* triangle tests (RG_FLAG_COUNT_VISITS) */
     uint64_t stack_overflows; /* rays whose short traversal stack overflowed; each was traced again with a deep
                                  stack, so its hit is complete (a cost, not an error) */
-    uint64_t iterations; /* trace/shade rounds of the wavefront loop (0 for the megakernel) */
+    uint64_t iterations; /* rounds of the ray trees (0 for the megakernel) */
     uint64_t deep_overflows; /* rays that overflowed even the deep stack: 0 for every tree this library builds
                                 (at most 64 BVH2 levels); non-zero means hits may be missing */
 } rg_stats;
@@ -275,13 +275,13 @@ typedef struct rg_batch_tune {
     int32_t sort_key;     /* RG_SORT_*: rays sorted per round by direction octant or origin Morton code */
 } rg_batch_tune;
 
-/* Renders every job: one wavefront loop traces the paths of all jobs together (path slots that
- * finish take the next job's work), then each job's samples are resolved and run through the
+/* Renders every job: the ray trees of all jobs' samples are grown, checked and composed together (chunk
+ * after chunk of the samples, numbered job after job), then each job's samples are resolved and run through the
  * roughness, postprocess and FXAA passes into its own RGBA32F image.  Each image equals what
  * rg_render of that job's scene, resolution and UBO produces.  rg_get_stats then counts the rays
- * of the whole batch.  The batch runs as one CUDA graph launch whose round loop is a device-side
- * while node (re-captured only when the batch's shape changes: job sizes, samples, post options,
- * tune); RG_FLAG_HOST_LOOP, RG_FLAG_KERNEL_TIMING and RG_FLAG_COUNT_VISITS use the host-polled
+ * of the whole batch.  The batch runs as one CUDA graph launch whose loops are device-side
+ * while nodes (re-captured only when the batch's shape changes: job sizes, samples, the largest recursion
+ * limit, post options, tune); RG_FLAG_HOST_LOOP, RG_FLAG_KERNEL_TIMING and RG_FLAG_COUNT_VISITS use the host-polled
  * loop instead.  In graph mode rg_timings.rtOnly covers the whole batch (post included). */
 rg_status rg_render_batch(rg_ctx* ctx, const rg_job* jobs, uint32_t n);
 /* Device pointer of job `job`'s RGBA32F image of the last batch (width*height*4 floats). */
@@ -338,10 +338,9 @@ rg_status rg_set_glossy(rg_ctx* ctx, uint32_t seed);
 /* Device memory the context holds (all scene slots, images, path state, scratch) and its budget
  * (rg_device_opts.hbm_budget_bytes, 0 = none), in bytes. */
 rg_status rg_get_memory(rg_ctx* ctx, uint64_t* allocated_bytes, uint64_t* budget_bytes);
-/* Path slots of the batch loop: at most this many samples are in flight, and a slot whose path ends
- * takes the next sample.  Default 2^25, about 1.6 KB of device memory each (54 GB when a batch has
- * that many samples; a batch of fewer samples takes one slot per sample).  Fewer slots narrow every
- * round: 2^23 slots rendered the 64-scene benchmark batch 4 % slower, 2^20 slots 34 % slower. */
+/* Samples of a batch in flight: its samples go through their ray trees in chunks of at most this many.
+ * Default 2^25, 0.8 to 1.6 KB of device memory each (a batch of fewer samples takes one slot per
+ * sample).  Fewer slots mean more chunks of narrower rounds. */
 rg_status rg_set_batch_slots(rg_ctx* ctx, uint32_t slots);
 /* Autotuner of the batch loop: renders the batch once (warm-up, capture) and then `reps` times
  * with every launch shape of the grid threads {64,128,256} x stack depth {16,24,32,48} x sort key

@@ -108,19 +108,19 @@ struct rg_ctx {
     // misc
     DevBuf counters, tmpA, tmpB, tmpC, tmpD;  // counters: 8 per-frame + 8 cumulative
     DevBuf samples, workCounter;               // per-sample payload sums, persistent-kernel work counter
-    // wavefront path state
-    DevBuf wfPayload, wfMeta, wfFrames, wfQO0, wfQO1, wfQD0, wfQD1, wfQP0, wfQP1, wfHitTUV, wfHitInst, wfCounts, wfOverflow;
+    // ray queries: traversal counters, overflow list
+    DevBuf wfCounts, wfOverflow;
     // ray trees of the frames: node pool (its nodes per sample grow when a frame filled it)
     DevBuf trO, trD, trState, trHit, trInst, trSurf, trLink, trOver, trCand, trCtl;
     uint32_t treeNodes = kTreeNodesMin;
     uint32_t* hostCount = nullptr;             // pinned words for polling the queue length and work counter
     int lastIterations = 0;
-    // batch rendering: job table, per-slot job / sample index, ray-sort scratch, per-job images
-    DevBuf jobTable, slotJob, slotSample, sortKeys, sortPerm, sortHist;
+    // batch rendering: job table, ray-sort scratch, per-job images
+    DevBuf jobTable, sortKeys, sortPerm, sortHist;
     DevBuf bBase, bNormal, bRough, bFinal, bFxaa, batchFb;
     std::vector<size_t> batchOffset;           // per job: first pixel in batchFb
     std::vector<uint32_t> batchW, batchH;
-    uint32_t batchSlots = 1u << 25;            // path slots of the batch loop (path state ~1.6 KB each: 54 GB at most)
+    uint32_t batchSlots = 1u << 25;            // samples of a batch's chunk (7 to 13 nodes of 112 bytes each: 49 GB at most)
     TraceTune tune;
     // graph form of the batch: second stream (loop body capture), instantiated graph and what it
     // was captured for, loop words (device), launch accounting
@@ -130,8 +130,7 @@ struct rg_ctx {
     std::vector<uint8_t> graphKey;
     DevBuf loopWords;
     uint64_t graphFixedKernels = 0;
-    int graphBodyKernels = 0;
-    uint32_t bodyRunsSeen = 0;
+    uint32_t kernelsSeen = 0;
     bool graphPending = false;
     // learned roughness filter used by the frames (nullable), glossy reference shading seed (0 = off),
     // samples of the last frame
@@ -272,14 +271,14 @@ rg_status ensure(rg_ctx* c, DevBuf& b, size_t bytes) {
 }
 
 // bookkeeping of finished batch-graph launches (call after the stream was synchronized): launch
-// accounting of the loop body runs, iteration count, the loop's iteration-limit flag
+// accounting of the graph's loops, round count, the loops' limit flag, a larger pool after a full one
 rg_status settle_graph(rg_ctx* c) {
     if (!c->graphPending) return RG_OK;
     c->graphPending = false;
-    const uint32_t runs = c->hostCount[6];
-    count_launch((uint64_t)(runs - c->bodyRunsSeen) * (uint64_t)c->graphBodyKernels);
-    c->bodyRunsSeen = runs;
-    c->lastIterations = 2 * (int)c->hostCount[4];
+    count_launch(c->hostCount[6] - c->kernelsSeen);
+    c->kernelsSeen = c->hostCount[6];
+    c->lastIterations = (int)c->hostCount[7];
+    if (c->hostCount[8] && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
     if (c->hostCount[5]) {
         CK(cudaMemsetAsync(c->loopWords.as<uint32_t>() + 1, 0, sizeof(uint32_t), c->stream));
         return fail(c, RG_ERR_CUDA, "batch round loop stopped at its iteration limit");
@@ -455,48 +454,8 @@ uint64_t scene_bytes(const SceneState& st) {
     return b;
 }
 
-// path state of the wavefront loop for `paths` path slots
-// path state for `paths` paths; queues and hit records for max(paths, hitSlots) entries
-rg_status ensure_wavefront(rg_ctx* c, size_t paths, WavefrontBuffers& w) {
-    const size_t P = paths ? paths : 1, Q = P;
-    TRY(ensure(c, c->wfPayload, 64 * P));
-    TRY(ensure(c, c->wfMeta, 8 * P));
-    TRY(ensure(c, c->wfFrames, 144ull * kMaxFrames * P));
-    TRY(ensure(c, c->wfQO0, 16 * Q));
-    TRY(ensure(c, c->wfQO1, 16 * Q));
-    TRY(ensure(c, c->wfQD0, 16 * Q));
-    TRY(ensure(c, c->wfQD1, 16 * Q));
-    TRY(ensure(c, c->wfQP0, 4 * Q));
-    TRY(ensure(c, c->wfQP1, 4 * Q));
-    TRY(ensure(c, c->wfHitTUV, 16 * Q));
-    TRY(ensure(c, c->wfHitInst, 4 * Q));
-    TRY(ensure(c, c->wfOverflow, 4 * Q));
-    if (!c->wfCounts.p) {  // the overflow list length and the finished-block count start at zero
-        TRY(ensure(c, c->wfCounts, 32));
-        CK(cudaMemsetAsync(c->wfCounts.p, 0, 32, c->stream));
-    }
-    w.payload = c->wfPayload.as<float4>();
-    w.meta = c->wfMeta.as<int2>();
-    w.frames = c->wfFrames.p;
-    w.qO[0] = c->wfQO0.as<float4>();
-    w.qO[1] = c->wfQO1.as<float4>();
-    w.qD[0] = c->wfQD0.as<float4>();
-    w.qD[1] = c->wfQD1.as<float4>();
-    w.qPath[0] = c->wfQP0.as<uint32_t>();
-    w.qPath[1] = c->wfQP1.as<uint32_t>();
-    w.hitTUV = c->wfHitTUV.as<float4>();
-    w.hitInst = c->wfHitInst.as<uint32_t>();
-    w.counts = c->wfCounts.as<uint32_t>();
-    w.overflow = c->wfOverflow.as<uint32_t>();
-    return RG_OK;
-}
-
-// ray-tree buffers for a frame of `work` samples; frames of more than 2^25 samples go in chunks
-rg_status ensure_tree(rg_ctx* c, size_t work, RayTree& t) {
-    const size_t roots = std::min<size_t>(work, 1u << 25);
-    size_t cap = std::max<size_t>(roots * c->treeNodes, 1u << 16);
-    // (RG_TREE_POOL overrides the pool's nodes; tests use a small pool to make chunks fill it)
-    if (const char* env = getenv("RG_TREE_POOL")) cap = std::max<size_t>(strtoull(env, nullptr, 10), 4608);
+// buffers of a pool of `cap` ray-tree nodes
+rg_status ensure_tree_nodes(rg_ctx* c, size_t cap, RayTree& t) {
     TRY(ensure(c, c->trO, 16 * cap));
     TRY(ensure(c, c->trD, 16 * cap));
     TRY(ensure(c, c->trState, 16 * cap));
@@ -520,6 +479,18 @@ rg_status ensure_tree(rg_ctx* c, size_t work, RayTree& t) {
     t.ctl = c->trCtl.as<uint32_t>();
     t.capacity = (uint32_t)cap;
     return RG_OK;
+}
+
+// Frames of more than 2^25 samples go in chunks.  A pool that grew after a chunk had filled it is given
+// up again where memory does not allow it.
+rg_status ensure_tree(rg_ctx* c, size_t roots, size_t least, RayTree& t) {
+    // (RG_TREE_POOL overrides the pool's nodes; tests use a small pool to make chunks fill it)
+    if (const char* env = getenv("RG_TREE_POOL")) return ensure_tree_nodes(c, std::max<size_t>(strtoull(env, nullptr, 10), 4608), t);
+    const rg_status st = ensure_tree_nodes(c, std::max(roots * c->treeNodes, least), t);
+    if ((st != RG_ERR_BUDGET && st != RG_ERR_OUT_OF_MEMORY) || c->treeNodes == kTreeNodesMin) return st;
+    if (st == RG_ERR_OUT_OF_MEMORY) cudaGetLastError();
+    c->treeNodes = kTreeNodesMin;
+    return ensure_tree_nodes(c, std::max(roots * kTreeNodesMin, least), t);
 }
 
 }  // namespace
@@ -553,7 +524,7 @@ rg_status rg_create(rg_ctx** out, const rg_device_opts* opts) {
         return RG_ERR_OUT_OF_MEMORY;
     }
     cudaMemsetAsync(c->counters.p, 0, 18 * sizeof(unsigned long long), c->stream);
-    if (cudaHostAlloc(&c->hostCount, 8 * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess ||
+    if (cudaHostAlloc(&c->hostCount, 12 * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->copyStream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->staged[0], cudaEventDisableTiming) != cudaSuccess ||
@@ -581,9 +552,7 @@ rg_status rg_destroy(rg_ctx* c) {
     if (c->copyStream) cudaStreamDestroy(c->copyStream);
     DevBuf* bufs[] = {&c->keysA, &c->keysB, &c->valsA, &c->valsB, &c->sortState, &c->sahQueue, &c->base, &c->normal, &c->rough,
                       &c->finalImg, &c->fxaaOut, &c->fb, &c->dbgT, &c->dbgA, &c->dbgB, &c->counters, &c->tmpA, &c->tmpB, &c->tmpC,
-                      &c->tmpD, &c->samples, &c->workCounter, &c->wfPayload, &c->wfMeta, &c->wfFrames, &c->wfQO0, &c->wfQO1,
-                      &c->wfQD0, &c->wfQD1, &c->wfQP0, &c->wfQP1, &c->wfHitTUV, &c->wfHitInst, &c->wfCounts, &c->wfOverflow, &c->jobTable,
-                      &c->slotJob, &c->slotSample, &c->sortKeys, &c->sortPerm, &c->sortHist, &c->bBase, &c->bNormal, &c->bRough,
+                      &c->tmpD, &c->samples, &c->workCounter, &c->wfCounts, &c->wfOverflow, &c->jobTable, &c->sortKeys, &c->sortPerm, &c->sortHist, &c->bBase, &c->bNormal, &c->bRough,
                       &c->bFinal, &c->bFxaa, &c->batchFb, &c->trO, &c->trD, &c->trState, &c->trHit, &c->trInst, &c->trSurf, &c->trLink,
                       &c->trOver, &c->trCand, &c->trCtl};
     for (DevBuf* b : bufs) release(c, *b);
@@ -874,7 +843,7 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     tp.glossySeed = c->glossySeed;
     c->lastSamples = (uint32_t)ubo->numSamples;
     const bool mega = (c->flags & RG_FLAG_MEGAKERNEL) != 0;
-    if (!mega) TRY(ensure_tree(c, frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), tp.tree));
+    if (!mega) TRY(ensure_tree(c, std::min<size_t>(frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), 1u << 25), 1u << 16, tp.tree));
     CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
     FrameEvents* fe;
     TRY(cur_events(c, &fe));
@@ -1333,11 +1302,6 @@ std::vector<uint8_t> batch_graph_key(rg_ctx* c, const TraceParams& tp, const Sor
 
 rg_status launch_batch_graph(rg_ctx* c, const TraceParams& tp, const SortScratch& sort, const JobDesc* jd, const rg_job* jobs,
                              uint32_t n) {
-    if (!c->loopWords.p) {
-        TRY(ensure(c, c->loopWords, 16));
-        CK(cudaMemsetAsync(c->loopWords.p, 0, 16, c->stream));
-        c->bodyRunsSeen = 0;
-    }
     std::vector<uint8_t> key = batch_graph_key(c, tp, sort, jd, jobs, n);
     if (!c->graphExec || key != c->graphKey) {
         if (c->graphExec) cudaGraphExecDestroy(c->graphExec);
@@ -1352,7 +1316,9 @@ rg_status launch_batch_graph(rg_ctx* c, const TraceParams& tp, const SortScratch
         if (e == cudaSuccess) e = enqueue_batch_posts(c, jd, jobs, n);
         const uint64_t posts = g_launches.load() - postsBefore;
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(c->hostCount + 4, c->loopWords.p, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
+            e = cudaMemcpyAsync(c->hostCount + 4, c->loopWords.p, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(c->hostCount + 8, tp.tree.ctl + kTreeWasFull, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
         cudaGraph_t g = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
         g_launches.store(before);  // captured launches are counted when the graph runs
@@ -1369,7 +1335,7 @@ rg_status launch_batch_graph(rg_ctx* c, const TraceParams& tp, const SortScratch
         }
         c->graph = g;
         c->graphKey = std::move(key);
-        c->graphFixedKernels = (uint64_t)batch_graph_kernels(c->tune, &c->graphBodyKernels) + posts;
+        c->graphFixedKernels = posts;  // the loops count theirs
     }
     CK(cudaGraphLaunch(c->graphExec, c->stream));
     count_launch(c->graphFixedKernels);
@@ -1462,6 +1428,7 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
             return fail(c, RG_ERR_INVALID_ARG, "job " + std::to_string(j) + ": learned filter asked for, none set (rg_set_filter)");
     std::vector<JobDesc> jd(n);
     uint64_t work = 0, samples = 0, pixels = 0, maxPixels = 0;
+    int maxRecursions = 0;
     for (uint32_t j = 0; j < n; ++j) {
         const rg_job& in = jobs[j];
         if (in.scene >= c->scenes.size() || !c->scenes[in.scene])
@@ -1479,6 +1446,7 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
         std::memset(&d, 0, sizeof(d));
         d.scene = scene_of(st);
         d.ubo = in.ubo;
+        maxRecursions = std::max(maxRecursions, (int)in.ubo.maxRecursions);
         d.W = in.width;
         d.H = in.height;
         d.S = S;
@@ -1497,20 +1465,22 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
     const uint32_t slots = (uint32_t)std::min<uint64_t>(work, c->batchSlots);
     TraceParams tp;
     std::memset(&tp, 0, sizeof(tp));
-    TRY(ensure_wavefront(c, slots, tp.wf));
+    TRY(ensure_tree(c, slots, 4608, tp.tree));
     TRY(ensure(c, c->samples, 48ull * samples));
-    TRY(ensure(c, c->workCounter, 16));
-    TRY(ensure(c, c->slotJob, 4ull * slots));
-    TRY(ensure(c, c->slotSample, 4ull * slots));
     TRY(ensure(c, c->jobTable, sizeof(JobDesc) * n));
     SortScratch sort{};
     if (c->tune.sortKey != RG_SORT_NONE) {
-        TRY(ensure(c, c->sortKeys, 4ull * slots));
-        TRY(ensure(c, c->sortPerm, 4ull * slots));
+        TRY(ensure(c, c->sortKeys, 4ull * tp.tree.capacity));
+        TRY(ensure(c, c->sortPerm, 4ull * tp.tree.capacity));
         TRY(ensure(c, c->sortHist, 8192 * 4));
         sort.keysA = c->sortKeys.as<uint32_t>();
         sort.valsA = c->sortPerm.as<uint32_t>();
         sort.hist = c->sortHist.as<uint32_t>();
+    }
+    if (!c->loopWords.p) {
+        TRY(ensure(c, c->loopWords, 16));
+        CK(cudaMemsetAsync(c->loopWords.p, 0, 16, c->stream));
+        c->kernelsSeen = 0;
     }
     TRY(ensure(c, c->bBase, 8 * maxPixels));
     TRY(ensure(c, c->bNormal, 8 * maxPixels));
@@ -1522,13 +1492,11 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
     tp.counters = c->counters.as<unsigned long long>();
     tp.countVisits = (c->flags & RG_FLAG_COUNT_VISITS) ? 1 : 0;
     tp.samples = c->samples.as<float4>();
-    tp.workCounter = c->workCounter.as<uint32_t>();
     tp.jobs = c->jobTable.as<JobDesc>();
     tp.njobs = n;
     tp.totalWork = (uint32_t)work;
     tp.slots = slots;
-    tp.slotJob = c->slotJob.as<uint32_t>();
-    tp.slotSample = c->slotSample.as<uint32_t>();
+    tp.batchRounds = maxRecursions + 1;
     CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
     c->batchOffset.assign(n, 0);
     c->batchW.assign(n, 0);
@@ -1547,10 +1515,11 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
     for (uint32_t j = 0; j < n; ++j) filtered |= (jobs[j].options & RG_JOB_FILTER) != 0;
     const bool hostLoop = filtered || (c->flags & (RG_FLAG_HOST_LOOP | RG_FLAG_KERNEL_TIMING | RG_FLAG_COUNT_VISITS)) != 0;
     if (hostLoop) {
-        if (c->flags & RG_FLAG_KERNEL_TIMING)
-            CK(launch_trace_batch(tp, c->tune, sort, c->stream, c->hostCount, &c->lastIterations, next_kernel_events, fe));
-        else
-            CK(launch_trace_batch(tp, c->tune, sort, c->stream, c->hostCount, &c->lastIterations));
+        const bool timed = (c->flags & RG_FLAG_KERNEL_TIMING) != 0;
+        bool full = false;
+        CK(launch_trace_batch(tp, c->tune, sort, c->loopWords.as<uint32_t>(), c->stream, c->hostCount, &c->lastIterations, &full,
+                              timed ? next_kernel_events : nullptr, timed ? fe : nullptr));
+        if (full && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
         CK(cudaEventRecord(fe->ev[EV_POST0], c->stream));
         CK(enqueue_batch_posts(c, jd.data(), jobs, n));
     } else {

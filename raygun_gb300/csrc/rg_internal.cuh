@@ -186,19 +186,11 @@ cudaError_t setup_instances(const rg_instance* in, uint32_t n, const DevBlas* bl
 cudaError_t inst_records(const uint32_t* order, uint32_t n, const DevInstance* inst, const DevBlas* blas, InstRec* out,
                          cudaStream_t s);
 
-// device buffers of the wavefront path (one path per pixel sample; P = paths)
+// counters and overflow list of the traversal kernel
 struct WavefrontBuffers {
-    float4* payload;   // P x 4 float4: the reference payload (payload.h:29-39)
-    int2* meta;        // P: frame-stack depth, miss index of the pending ray
-    void* frames;      // P x kMaxFrames paused closest-hit frames (144 B each)
-    float4* qO[2];     // ray queues: origin + tmin
-    float4* qD[2];     //             direction + tmax
-    uint32_t* qPath[2];
-    float4* hitTUV;    // per queue slot: t, u, v, primitive bits
-    uint32_t* hitInst; // per queue slot: instance or 0xFFFFFFFF (miss)
-    uint32_t* counts;  // [0], [1] queue lengths, [2] trace work counter, [3] overflow list length,
-                       // [4] trace blocks finished (both zero between launches)
-    uint32_t* overflow; // per queue slot: slots of rays whose short traversal stack overflowed
+    uint32_t* counts;  // [2] trace work counter, [3] overflow list length, [4] trace blocks finished
+                       // (the last two zero between launches)
+    uint32_t* overflow; // rays whose short traversal stack overflowed
 };
 
 // Ray trees (trace.cu): one node per traced ray.  The roots, one per sample of the chunk, are nodes
@@ -219,16 +211,31 @@ struct RayTree {
 // words of RayTree::ctl: nodes appended after the roots; rays that the last check changed, 16 minus the
 // least recursion depth of the rays replaced since the last round, nodes traced when the last check ran;
 // the traversal kernel's work counter, overflow list length and finished blocks; lengths of the candidate
-// lists; then the first node of every round
+// lists; then the first node of every round, and a batch's words
 enum : int { kTreeAlloc = 0, kTreeChanges = 1, kTreeLevels = 2, kTreeTraced = 3, kTreeFetch = 4, kTreeCand = 7, kTreeBounds = 9 };
 constexpr uint32_t kTreeMaxNodes = 1u << 29;
 // a sample's GENERIC hits (at most 2^9 - 1 at 8 recursions) bound the checks that can change a ray
 constexpr int kTreeMaxRounds = 512 * 9;
-constexpr int kTreeCtlWords = kTreeBounds + kTreeMaxRounds + 1;
+// of a batch: more rounds are needed, the chunk filled the pool, rounds run, a chunk is set up (polled together);
+// the chunk's roots and first work item, the candidate list in use, the round to trace next and the one
+// traced last, samples a chunk, and whether any chunk filled the pool
+enum : int {
+    kTreeMore = kTreeBounds + kTreeMaxRounds + 1, kTreeFull, kTreeTop, kTreeLive, kTreeRoots, kTreeBase, kTreeCandList, kTreeRound,
+    kTreeTracedRound, kTreeChunk, kTreeWasFull, kTreeCtlWords
+};
+constexpr int kTreeComposeRun = 4;  // rounds composed per run of that loop
+// loops of a batch's graph: their conditions; words: runs of the loops in this launch (at most maxRuns), sticky limit
+// flag, kernels launched in total, rounds in this launch; kernels of a chunk, a run of rounds, a run of compositions
+struct TreeLoop {
+    bool graph;
+    cudaGraphConditionalHandle chunks, rounds, composes;
+    uint32_t* words;
+    uint32_t maxRuns, chunkKernels, roundKernels, composeKernels;
+};
 // Pool size: nodes per sample.  The benchmark scenes trace 2.5 to 4 rays a sample; a chunk of samples
 // that fills the pool goes again in smaller chunks, and the next frame's pool is twice as large, up to
-// kTreeNodesMax a sample (less than the 1.6 KB that a path of the batch loop takes).
-constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 14;
+// kTreeNodesMax a sample.
+constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 13;
 
 // one render job of a batch: a scene, its UBO and its image size.  Work items of the batch are
 // numbered job after job; job j owns [workBase, workBase + workCount) and writes its per-sample
@@ -255,17 +262,14 @@ struct TraceParams {
     uint32_t* workCounter;         // work-item counter of the persistent kernel
     int countVisits;
     WavefrontBuffers wf;
-    // batch form of the wavefront loop (launch_trace_batch): the job table in device memory, the
-    // batch's work-item count, and per path slot the job and the output sample index.  A slot whose
-    // path finished takes the next work item (path regeneration), so `slots` bounds the path state.
+    // batch (launch_trace_batch): the job table in device memory, the batch's work items, samples a chunk at
+    // most, and the rounds every chunk runs (1 + the largest recursion limit)
     const JobDesc* jobs;
     uint32_t njobs;
     uint32_t totalWork;
     uint32_t slots;
-    uint32_t pad2;
-    uint32_t* slotJob;
-    uint32_t* slotSample;
-    const uint32_t* perm;  // nullable: order in which the trace kernel takes the queue's rays
+    int batchRounds;
+    const uint32_t* perm;  // nullable: order in which the trace kernel takes the round's rays
     uint32_t glossySeed;   // 0: the reference's mirror shading; else glossy reference shading (seed)
     // ray trees: the first round computes the camera rays of the roots itself
     int firstRound;
@@ -306,18 +310,14 @@ bool tune_supported(const TraceTune& t);
 struct SortScratch {
     uint32_t *keysA, *keysB, *valsA, *valsB, *hist;
 };
-// the wavefront loop over every job of p.jobs (raygen with regeneration, trace/shade rounds, tail);
-// hostWords: two pinned words (queue length, work counter) polled every few rounds
-cudaError_t launch_trace_batch(const TraceParams& p, const TraceTune& tune, const SortScratch& sort, cudaStream_t s,
-                               uint32_t* hostWords, int* iterations, EventPairFn kernelEvents = nullptr, void* user = nullptr);
-// graph form of launch_trace_batch, enqueued on stream s while it captures: prologue, a while node
-// (body captured on the idle stream s2: two trace/shade rounds and the device-side loop condition)
-// and the tail launch.  loopWords: 3 device words (body runs of the launch, sticky iteration-limit
-// flag, body runs in total), the last two zeroed by the caller once.
+// every job of p.jobs through ray trees, the loops on the host; hostWords: four pinned words polled after each check
+// and chunk; loopWords as below
+cudaError_t launch_trace_batch(const TraceParams& p, const TraceTune& tune, const SortScratch& sort, uint32_t* loopWords, cudaStream_t s,
+                               uint32_t* hostWords, int* iterations, bool* poolFull, EventPairFn kernelEvents = nullptr, void* user = nullptr);
+// graph form, enqueued on stream s while it captures; the loops run on the device (bodies captured on the idle stream s2).
+// loopWords: TreeLoop::words, the sticky flag and the kernel count zeroed by the caller once.
 cudaError_t capture_trace_batch(const TraceParams& p, const TraceTune& tune, const SortScratch& sort, cudaStream_t s,
                                 cudaStream_t s2, uint32_t* loopWords);
-// kernels of that graph outside the loop body; *perBody = kernels of one body run
-int batch_graph_kernels(const TraceTune& tune, int* perBody);
 // raygen.rgen:36-38 for one job of a batch: average its samples into RGBA16F G-buffers
 cudaError_t launch_resolve_job(const float4* samples, const JobDesc& hostJob, uint2* base, uint2* normal, uint2* rough,
                                cudaStream_t s);

@@ -22,8 +22,8 @@ import numpy as np
 
 from . import scenes
 
-# device bytes per path slot of the batch loop (payload, meta, 10 frames, two queue entries, hit)
-PATH_SLOT_BYTES = 64 + 8 + 144 * 10 + 2 * 36 + 20
+# device bytes per path slot of a batch: up to 13 ray-tree nodes of 112 bytes, 8 more each with sorted rays
+PATH_SLOT_BYTES = 13 * (112 + 8)
 # per sample (payload sums), per output pixel (batch framebuffer), per pixel of the largest job
 # (G-buffers, post scratch)
 SAMPLE_BYTES, PIXEL_BYTES, SCRATCH_PIXEL_BYTES = 48, 16, 40

@@ -92,3 +92,24 @@ def test_query_sizes(rg, n):
     ctx.synchronize()
     assert np.array_equal(d_ids.cpu().numpy().view(np.uint32), ids) and np.array_equal(d_tuv.cpu().numpy(), tuv)
     ctx.close()
+
+
+@pytest.mark.parametrize("pool", [None, 4608, 30000])
+@pytest.mark.parametrize("host_loop,sort", [(False, "none"), (False, "morton"), (True, "octant")])
+def test_batch_trees(rg, monkeypatch, pool, host_loop, sort):
+    """A batch of scenes of different recursion limits (0 to 8) and sizes through ray trees, its loops on the
+    device or on the host, in chunks that fill the node pool, equals the scenes' own frames."""
+    scs = [glass_scene(97, 55, 2, 5, seed=3), glass_scene(40, 30, 1, 0, seed=4), glass_scene(64, 64, 1, 8, seed=5, spheres=24),
+           glass_scene(1, 1, 3, 2, seed=6)]
+    ref = [render(rg, sc) for sc in scs]
+    if pool:
+        monkeypatch.setenv("RG_TREE_POOL", str(pool))
+    br = rg.BatchRenderer(scs, flags=rg.RG_FLAG_HOST_LOOP if host_loop else 0)
+    br.ctx.set_batch_tune(128, 48, sort)
+    for _ in range(2):
+        for img, (r, _) in zip(br.render(), ref):
+            assert np.array_equal(img, r[0])
+        st = br.ctx.stats()
+        assert {k: st[k] for k in ("primary", "shadow", "secondary", "masked")} == \
+            {k: sum(s[k] for _, s in ref) for k in ("primary", "shadow", "secondary", "masked")}
+    br.ctx.close()
