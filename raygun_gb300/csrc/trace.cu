@@ -1129,6 +1129,10 @@ __global__ void k_resolve_job(const float4* __restrict__ samples, uint32_t W, ui
 // ---------------------------------------------------------------------------------------------
 // Frames and batches: rays traced by launches of one traversal kernel, between them what the hits need.
 
+// Start of a kernel of a frame's chain of launches (launch_next): from here on everything before it is finished
+// and visible.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
     const unsigned mask = __ballot_sync(0xFFFFFFFFu, want);
     if (!mask) return 0;
@@ -1420,6 +1424,7 @@ __device__ __forceinline__ uint32_t trace_workers(uint32_t count, uint32_t threa
 
 template <bool COUNT, TraceForm FORM, int THREADS, int DEPTH>
 __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k_wf_trace(const __grid_constant__ TraceParams P, int q) {
+    chain_wait();
     RG_DECLARE_SMEM_STACK(stk, THREADS, DEPTH);
     const WavefrontBuffers& wf = P.wf;
     constexpr bool BATCH = FORM == kFormBatch, QUERY = FORM == kFormQuery, TREE = !QUERY;
@@ -1744,6 +1749,7 @@ __device__ __forceinline__ void refraction_left(const TraceParams& P, uint32_t y
 // then its refraction rays, with one atomic: 32 hits of a few surfaces give runs of similar rays.
 template <bool BATCH, bool GLOSSY>
 __global__ void __launch_bounds__(128) k_tree_expand(const __grid_constant__ TraceParams P, int round) {
+    chain_wait();
     const RayTree& t = P.tree;
     const bool first = P.firstRound != 0, counted = BATCH && round < 0;
     if (counted) round = (int)t.ctl[kTreeTracedRound];
@@ -1926,6 +1932,7 @@ __device__ float exact_ref_depth(const TraceParams& P, uint32_t x, uint32_t fres
 // next rounds; candidates whose subtree could still change stay in the other list.
 template <bool BATCH, bool GLOSSY>
 __global__ void __launch_bounds__(128) k_tree_check(const __grid_constant__ TraceParams P, int round) {
+    chain_wait();
     const RayTree& t = P.tree;
     if (BATCH) round = (int)t.ctl[kTreeRound];
     const uint32_t n = min(t.ctl[kTreeCand + tree_cand<BATCH>(P)], t.capacity), fresh = t.ctl[kTreeBounds + round];
@@ -2114,6 +2121,7 @@ __device__ V3 shadow_chain(const TraceParams& P, const DevScene& sc, const V3 L,
 // longer needed once its own colour is known); roots write their sample's payload sums.
 template <bool BATCH>
 __global__ void __launch_bounds__(128) k_tree_compose(const __grid_constant__ TraceParams P, int round) {
+    chain_wait();
     const RayTree& t = P.tree;
     if (BATCH) {  // round < 0: counted from the last round down, rounds before P.batchRounds have launches of their own
         if (t.ctl[kTreeFull]) return;
@@ -2512,6 +2520,24 @@ cudaError_t launch_trace_queue(const TraceParams& p, const float* rays, uint32_t
     return cudaGetLastError();
 }
 
+// A launch that is set up while the one before it still runs (its blocks are placed as soon as that one's have
+// ended, and chain_wait for its memory): 1.5 us less between two launches, of which a frame has 20 to 50.
+// 160x90 frame 401 -> 363 us, 640x360 spheres 997 -> 927 us, 1080p game frame 16.24 -> 16.08 ms.  Letting the blocks
+// in earlier (launch_dependents) costs more than it gives: they hold places of blocks still working (16.41 ms).
+static cudaError_t launch_next(void (*kernel)(const TraceParams, int), int grid, int threads, cudaStream_t s, const TraceParams& p, int round) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    count_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, p, round);
+}
+
 cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, uint32_t* hostWords, int* iterations, bool* poolFull,
                               EventPairFn kernelEvents, void* user) {
     TraceParams p = p0;
@@ -2550,15 +2576,12 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, uint32_t* h
                 cudaEvent_t e0 = nullptr, e1 = nullptr;
                 if (kernelEvents && !kernelEvents(user, &e0, &e1)) e0 = e1 = nullptr;
                 if (e0) cudaEventRecord(e0, s);
-                trace<<<gTrace, kTraceThreads, 0, s>>>(p, k);
+                if ((e = launch_next(trace, gTrace, kTraceThreads, s, p, k)) != cudaSuccess) return e;
                 if (e1) cudaEventRecord(e1, s);
-                expand<<<gExpand, 128, 0, s>>>(p, k);
-                count_launch(2);
+                if ((e = launch_next(expand, gExpand, 128, s, p, k)) != cudaSuccess) return e;
             }
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
             if (maxRec == 0) break;  // no hit issues a ray
-            check<<<gCheck, 128, 0, s>>>(p, k);
-            count_launch();
+            if ((e = launch_next(check, gCheck, 128, s, p, k)) != cudaSuccess) return e;
             if ((e = cudaMemcpyAsync(hostWords, p.tree.ctl, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
             if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
             full = p.treeRoots + hostWords[kTreeAlloc] > cap;
@@ -2575,10 +2598,8 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, uint32_t* h
             split(p.treeBase, p.treeRoots, (p.treeRoots + 7) / 8);
             continue;
         }
-        while (k--) {
-            k_tree_compose<false><<<gCompose, 128, 0, s>>>(p, k);
-            count_launch();
-        }
+        while (k--)
+            if ((e = launch_next(k_tree_compose<false>, gCompose, 128, s, p, k)) != cudaSuccess) return e;
     }
     if (iterations) *iterations = it;
     dim3 grid((p.W + 31) / 32, (p.H + 7) / 8);
