@@ -203,6 +203,7 @@ __device__ __forceinline__ uint32_t pack_pair(float x, float y) {
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kConvThreads, 1) k_filter_conv(const __grid_constant__ CUtensorMap tmapX, const FilterConvArgs a,
                                                                  int segRows) {
+    chain_wait();
     using S = ConvShape<CIN, COUT>;
     using bf16 = __nv_bfloat16;
     constexpr int CC = S::CC, NW = S::kWindows, KK = CIN / 16;
@@ -478,6 +479,7 @@ template <int CIN, int COUT>
 __global__ void __launch_bounds__(128, 1) k_filter_dw(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapG, int B,
                                                       int H, int W, int ctas0, float* __restrict__ partial, float* __restrict__ biasPartial,
                                                       int* status) {
+    chain_wait();
     using S = DwShape<CIN, COUT>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -682,6 +684,7 @@ __global__ void k_filter_pack(const float* __restrict__ W, int coutReal, int cin
 // sum a quarter of the CTAs each (in a fixed order: a step is deterministic).  lr = 0: gradients only.
 // The five reductions of 152 partials took 244 us one thread a parameter; all of this takes 17 us.
 __global__ void __launch_bounds__(256) k_filter_finish(const FilterFinish f) {
+    chain_wait();
     __shared__ float part[4][64];
     const int j = threadIdx.x & 63, q = threadIdx.x >> 6;
     int l = 0;
@@ -722,6 +725,7 @@ __global__ void __launch_bounds__(256) k_filter_finish(const FilterFinish f) {
 // mean-squared error over the 3 predicted channels; g = d(loss)/d(out) into channels 0..2 of [P][16]
 __global__ void __launch_bounds__(256) k_filter_loss(const float4* __restrict__ out, const float4* __restrict__ target, size_t P,
                                                      float scale, bf16* __restrict__ g, float* __restrict__ partial) {
+    chain_wait();
     __shared__ float red[256];
     float s = 0.0f;
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (size_t)gridDim.x * blockDim.x) {
@@ -757,6 +761,7 @@ __device__ __forceinline__ float4 unpack_half4(uint2 u) {
 //   7 roughness term (rough.a), 8-10 base colour, 11 reflect contribution
 __global__ void k_filter_gbuffer(const uint2* __restrict__ base, const uint2* __restrict__ normal, const uint2* __restrict__ rough, size_t P,
                                  float samples, bf16* __restrict__ out) {
+    chain_wait();
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (size_t)gridDim.x * blockDim.x) {
         const float4 b = unpack_half4(base[p]), n = unpack_half4(normal[p]), r = unpack_half4(rough[p]);
         // normal.w = log(sum of sample depths) * 0.25 / S  ->  mean depth
@@ -777,6 +782,7 @@ __global__ void k_filter_gbuffer(const uint2* __restrict__ base, const uint2* __
 // postprocess.comp:28-50 with the filter's prediction in place of roughColorsA
 __global__ void k_filter_composite(const uint2* __restrict__ base, const float4* __restrict__ pred, size_t P, float4 fade, int showAlpha,
                                    uint2* __restrict__ finalImg) {
+    chain_wait();
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (size_t)gridDim.x * blockDim.x) {
         const float4 b = unpack_half4(base[p]), r = pred[p];
         float cr = fminf(fmaxf(b.x * (1.0f - b.w) + r.x * b.w, 0.0f), 1.0f);
@@ -859,7 +865,7 @@ cudaError_t conv_launch(const FilterConvArgs& a, cudaStream_t s) {
     int segRows = (int)std::min<long long>(a.H, std::max<long long>(9, (rowsTotal + 2LL * grid - 1) / (2LL * grid)));
     segRows = (segRows + kGroupRows - 1) / kGroupRows * kGroupRows;
     const long long items = (long long)a.B * strips * ((a.H + segRows - 1) / segRows);
-    k_filter_conv<CIN, COUT><<<(int)std::min<long long>(items, grid), kConvThreads, S::kSmem, s>>>(map, a, segRows);
+    launch_chain(k_filter_conv<CIN, COUT>, (int)std::min<long long>(items, grid), kConvThreads, S::kSmem, s, map, a, segRows);
     count_launch();
     return cudaGetLastError();
 }
@@ -884,7 +890,7 @@ cudaError_t dw_launch(const bf16* x, const bf16* g, int B, int H, int W, float* 
     ctas[0] = S::kGroups == 1 ? all : std::max(1, all / 2);
     ctas[1] = S::kGroups == 1 ? all : std::max(1, all - ctas[0]);
     const int grid = S::kGroups == 1 ? all : ctas[0] + ctas[1];
-    k_filter_dw<CIN, COUT><<<grid, 128, S::kSmem, s>>>(mx, mg, B, H, W, ctas[0], partial, biasPartial, status);
+    launch_chain(k_filter_dw<CIN, COUT>, grid, 128, S::kSmem, s, mx, mg, B, H, W, ctas[0], partial, biasPartial, status);
     count_launch();
     return cudaGetLastError();
 }
@@ -931,19 +937,19 @@ cudaError_t filter_finish(FilterFinish& f, cudaStream_t s) {
         l.block0 = blocks;
         blocks += (l.coutReal * (9 * l.cinReal + 1) + 63) / 64;
     }
-    k_filter_finish<<<blocks, 256, 0, s>>>(f);
+    launch_chain(k_filter_finish, blocks, 256, 0, s, f);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t filter_loss(const float4* out, const float4* target, size_t P, float scale, void* g, float* partial, int blocks, cudaStream_t s) {
-    k_filter_loss<<<blocks, 256, 0, s>>>(out, target, P, scale, static_cast<bf16*>(g), partial);
+    launch_chain(k_filter_loss, blocks, 256, 0, s, out, target, P, scale, static_cast<bf16*>(g), partial);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t filter_gbuffer(const uint2* base, const uint2* normal, const uint2* rough, size_t P, float samples, void* out, cudaStream_t s) {
-    k_filter_gbuffer<<<(unsigned)((P + 255) / 256 < 4096 ? (P + 255) / 256 : 4096), 256, 0, s>>>(base, normal, rough, P, samples,
+    launch_chain(k_filter_gbuffer, (unsigned)((P + 255) / 256 < 4096 ? (P + 255) / 256 : 4096), 256, 0, s, base, normal, rough, P, samples,
                                                                                                  static_cast<bf16*>(out));
     count_launch();
     return cudaGetLastError();
@@ -951,7 +957,7 @@ cudaError_t filter_gbuffer(const uint2* base, const uint2* normal, const uint2* 
 
 cudaError_t filter_composite(const uint2* base, const float4* pred, size_t P, const float fade[4], int showAlpha, uint2* finalImg,
                              cudaStream_t s) {
-    k_filter_composite<<<(unsigned)((P + 255) / 256 < 4096 ? (P + 255) / 256 : 4096), 256, 0, s>>>(
+    launch_chain(k_filter_composite, (unsigned)((P + 255) / 256 < 4096 ? (P + 255) / 256 : 4096), 256, 0, s, 
         base, pred, P, make_float4(fade[0], fade[1], fade[2], fade[3]), showAlpha, finalImg);
     count_launch();
     return cudaGetLastError();

@@ -31,6 +31,7 @@ constexpr uint32_t kMortonMaxBlocks = 608;  // grid-stride: bounds the global hi
 
 __global__ void k_tri_boxes(const rg_vertex* __restrict__ v, const uint32_t* __restrict__ idx, uint32_t vOff, uint32_t iOff,
                             uint32_t n, float* __restrict__ boxes) {
+    chain_wait();
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     float lo[3], hi[3];
@@ -49,6 +50,7 @@ __global__ void k_tri_boxes(const rg_vertex* __restrict__ v, const uint32_t* __r
 // triangle records in leaf order: v0 (w = primitive id), v1, v2
 __global__ void k_tri_records(const rg_vertex* __restrict__ v, const uint32_t* __restrict__ idx, uint32_t vOff, uint32_t iOff,
                               const uint32_t* __restrict__ order, uint32_t n, float4* __restrict__ tris) {
+    chain_wait();
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     uint32_t p = order[k];
@@ -70,6 +72,7 @@ __device__ inline void centroid(const float* b, float* c) {
 
 // the centroid bounds as words that start at zero: ~f2ord of the minima, f2ord of the maxima
 __global__ void __launch_bounds__(256) k_centroid_bounds(const float* __restrict__ boxes, uint32_t n, uint32_t* bounds) {
+    chain_wait();
     __shared__ float red[6][8];
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
@@ -115,6 +118,7 @@ __global__ void __launch_bounds__(256) k_morton(const float* __restrict__ boxes,
                                                 uint32_t* morton, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                                 uint32_t* __restrict__ valsAlt, uint32_t* order, uint32_t* __restrict__ arrivals,
                                                 uint32_t* __restrict__ nodeBoxes, uint32_t* __restrict__ hist) {
+    chain_wait();
     __shared__ uint32_t h[4 * 256];
     for (int i = threadIdx.x; i < 4 * 256; i += 256) h[i] = 0;
     // every axis is scaled by the LARGEST centroid extent (a cube), so a thin axis spends few of its
@@ -207,6 +211,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_onesweep(const uint32_t* 
                                                                  uint32_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut,
                                                                  uint32_t n, int pass, uint32_t* __restrict__ state, uint32_t nTiles,
                                                                  uint32_t spinLimit) {
+    chain_wait();
     __shared__ uint32_t wc[kSortWarps][256];
     __shared__ uint32_t digitBase[256];
     __shared__ uint32_t warpSums[kSortWarps];
@@ -314,6 +319,7 @@ template <int ROUNDS>
 __global__ void __launch_bounds__(kClusterThreads) k_sort_cluster(const float* __restrict__ boxes, uint32_t n, uint32_t* morton,
                                                                   uint32_t* __restrict__ keysOut, uint32_t* order,
                                                                   uint32_t* __restrict__ arrivals, uint32_t* __restrict__ nodeBoxes) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smemRaw[];
     ClusterSort& S = *reinterpret_cast<ClusterSort*>(smemRaw);
     const cg::cluster_group cluster = cg::this_cluster();
@@ -541,6 +547,7 @@ uint32_t cluster_limit() {
 // and record pointers copied in
 __global__ void k_inst_records(const uint32_t* __restrict__ order, uint32_t n, const DevInstance* __restrict__ inst,
                                const DevBlas* __restrict__ blas, InstRec* __restrict__ out) {
+    chain_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t ii = order[k];
@@ -611,6 +618,7 @@ __global__ void __launch_bounds__(kHierLeaves) k_hierarchy(const uint32_t* __res
                                                            const float* __restrict__ primBoxes, uint32_t n, uint32_t* __restrict__ left,
                                                            uint32_t* __restrict__ right, uint32_t* __restrict__ parents,
                                                            uint32_t* arrivals, float* nodeBoxes) {
+    chain_wait();
     __shared__ uint32_t sKeys[kHierLeaves + 2];      // leaves first - 1 .. first + kHierLeaves
     __shared__ uint32_t sArrive[kHierLeaves];        // by split
     __shared__ float sLeaf[kHierLeaves][6], sNode[kHierLeaves][6];  // boxes by leaf and by node number
@@ -737,6 +745,7 @@ __device__ __forceinline__ uint32_t arrive(uint32_t* flag) {  // release my box,
 __global__ void k_bottom_up(const float* __restrict__ primBoxes, const uint32_t* __restrict__ order, uint32_t n,
                             const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
                             const uint32_t* __restrict__ parents, uint32_t* flags, float* nodeBoxes) {
+    chain_wait();
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     uint32_t node = parents[(n - 1) + k];
@@ -786,6 +795,7 @@ __device__ inline void child_box(const float* __restrict__ primBoxes, const uint
 __global__ void k_wide_records(const float* __restrict__ primBoxes, const uint32_t* __restrict__ order, uint32_t n,
                                const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
                                const float* __restrict__ nodeBoxes, WideNode* __restrict__ out) {
+    chain_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i + 1 >= n) return;
     uint32_t refs[4];
@@ -1391,6 +1401,7 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_level(const float* __
                                                                  uint32_t* __restrict__ right, float* __restrict__ nodeBoxes,
                                                                  uint2* __restrict__ tasksA, uint2* __restrict__ tasksB,
                                                                  uint32_t* __restrict__ lvCount, int level, uint32_t medianLevel) {
+    chain_wait();
     __shared__ int bLo[kSahWarps][3][kSahBins][3], bHi[kSahWarps][3][kSahBins][3];
     __shared__ int bCnt[kSahWarps][3][kSahBins];
     __shared__ float gPart[kSahWarps][12];
@@ -1461,6 +1472,7 @@ __device__ __forceinline__ void split_frame(const float* part, int lane, float* 
 
 __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_init(uint32_t n, uint32_t* __restrict__ order, uint32_t* __restrict__ left,
                                                                 uint32_t* __restrict__ right, uint2* __restrict__ tasksA) {
+    chain_wait();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         order[i] = i;
         if (i + 1 < n) left[i] = right[i] = kLeaf;  // every node starts as (leaf 0, leaf 0)
@@ -1474,6 +1486,7 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_split(const float* __
                                                                  uint2* __restrict__ tasksA, uint2* __restrict__ tasksB,
                                                                  uint32_t* __restrict__ lvCount, SplitScratch X, int level, int phase,
                                                                  uint32_t medianLevel) {
+    chain_wait();
     __shared__ int sb[kSahWarps][kBinInts];  // per-warp bins; merged bins in sb[0]
     __shared__ float red[kSahWarps][12];
     __shared__ uint32_t wl[kSahWarps];
@@ -1681,6 +1694,7 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_build(const float* __
                                                                  uint2* __restrict__ tasksA, uint2* __restrict__ tasksB,
                                                                  uint32_t firstLevel, uint32_t medianLevel, uint32_t handoff, SahQueue Q,
                                                                  const uint32_t* __restrict__ lvCount, uint32_t* __restrict__ levelsOut) {
+    chain_wait();
     constexpr int kRounds = SMALL ? 1 : 4;
     extern __shared__ float sahSmem[];
     const float* boxes = SMALL ? sahSmem : boxesIn;
@@ -1793,6 +1807,7 @@ __global__ void __launch_bounds__(kSahTaskWarps * 32, 3) k_sah_tasks(const float
                                                                   uint32_t* __restrict__ right, float* __restrict__ nodeBoxes,
                                                                   SahQueue Q, uint32_t medianLevel, uint32_t subtree, uint32_t* __restrict__ levelsOut,
                                                                   int* __restrict__ status, uint32_t waitLimit) {
+    chain_wait();
     __shared__ int bLo[kSahTaskWarps][3][kSahBins][3], bHi[kSahTaskWarps][3][kSahBins][3];
     __shared__ int bCnt[kSahTaskWarps][3][kSahBins];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1867,6 +1882,7 @@ __global__ void __launch_bounds__(kSahTaskWarps * 32, 3) k_sah_tasks(const float
 // at parents[n - 1 + k], the root's 0xFFFFFFFF), which the bottom-up refit walks
 __global__ void k_parents(const uint32_t* __restrict__ left, const uint32_t* __restrict__ right, uint32_t n,
                           uint32_t* __restrict__ parents) {
+    chain_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i + 1 >= n) return;
     const uint32_t L = left[i], R = right[i];
@@ -1880,6 +1896,7 @@ __global__ void k_parents(const uint32_t* __restrict__ left, const uint32_t* __r
 // ---- instances ----------------------------------------------------------------------------------
 __global__ void k_instances(const rg_instance* __restrict__ in, uint32_t n, const DevBlas* __restrict__ blas, uint32_t nblas,
                             DevInstance* __restrict__ out, float* __restrict__ boxes, bool checkOffsets, uint32_t nm) {
+    chain_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     rg_instance I = in[i];
@@ -1937,7 +1954,7 @@ inline uint32_t blocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
 
 cudaError_t tri_boxes(const rg_vertex* v, const uint32_t* idx, uint32_t vOff, uint32_t iOff, uint32_t n, float* boxes, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_tri_boxes<<<blocks(n, 256), 256, 0, s>>>(v, idx, vOff, iOff, n, boxes);
+    launch_chain(k_tri_boxes, blocks(n, 256), 256, 0, s, v, idx, vOff, iOff, n, boxes);
     count_launch();
     return cudaGetLastError();
 }
@@ -1945,7 +1962,7 @@ cudaError_t tri_boxes(const rg_vertex* v, const uint32_t* idx, uint32_t vOff, ui
 cudaError_t tri_records(const rg_vertex* v, const uint32_t* idx, uint32_t vOff, uint32_t iOff, const uint32_t* order, uint32_t n,
                         float4* tris, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_tri_records<<<blocks(n, 256), 256, 0, s>>>(v, idx, vOff, iOff, order, n, tris);
+    launch_chain(k_tri_records, blocks(n, 256), 256, 0, s, v, idx, vOff, iOff, order, n, tris);
     count_launch();
     return cudaGetLastError();
 }
@@ -1953,7 +1970,7 @@ cudaError_t tri_records(const rg_vertex* v, const uint32_t* idx, uint32_t vOff, 
 cudaError_t inst_records(const uint32_t* order, uint32_t n, const DevInstance* inst, const DevBlas* blas, InstRec* out,
                          cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_inst_records<<<blocks(n, 128), 128, 0, s>>>(order, n, inst, blas, out);
+    launch_chain(k_inst_records, blocks(n, 128), 128, 0, s, order, n, inst, blas, out);
     count_launch();
     return cudaGetLastError();
 }
@@ -1961,7 +1978,7 @@ cudaError_t inst_records(const uint32_t* order, uint32_t n, const DevInstance* i
 cudaError_t setup_instances(const rg_instance* in, uint32_t n, const DevBlas* blas, uint32_t nblas, DevInstance* out, float* boxes,
                             bool checkOffsets, uint32_t nm, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_instances<<<blocks(n, 128), 128, 0, s>>>(in, n, blas, nblas, out, boxes, checkOffsets, nm);
+    launch_chain(k_instances, blocks(n, 128), 128, 0, s, in, n, blas, nblas, out, boxes, checkOffsets, nm);
     count_launch();
     return cudaGetLastError();
 }
@@ -1970,7 +1987,7 @@ cudaError_t lbvh_refit(const LbvhBuffers& b, cudaStream_t s) {
     if (b.n <= 1) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(b.flags, 0, sizeof(uint32_t) * (b.n - 1), s);
     if (e != cudaSuccess) return e;
-    k_bottom_up<<<blocks(b.n, 256), 256, 0, s>>>(b.primBoxes, b.order, b.n, b.left, b.right, b.parents, b.flags, b.nodeBoxes);
+    launch_chain(k_bottom_up, blocks(b.n, 256), 256, 0, s, b.primBoxes, b.order, b.n, b.left, b.right, b.parents, b.flags, b.nodeBoxes);
     count_launch();
     return cudaGetLastError();
 }
@@ -2013,11 +2030,11 @@ cudaError_t sah_build(const LbvhBuffers& b, bool parents, uint32_t* levels, cuda
         X.bins = reinterpret_cast<int*>(X.part + 4 * kSplitCtas * 12);
         X.left = reinterpret_cast<uint32_t*>(X.bins + 4 * kSplitCtas * kBinInts);
         X.best = reinterpret_cast<int*>(X.left + 4 * kSplitCtas);
-        k_sah_init<<<2 * kSplitCtas, kSahWarps * 32, 0, s>>>(b.n, b.order, b.left, b.right, tasksA);
+        launch_chain(k_sah_init, 2 * kSplitCtas, kSahWarps * 32, 0, s, b.n, b.order, b.left, b.right, tasksA);
         count_launch();
         for (; lv0 < kSahSplitLevels; ++lv0)
             for (int ph = 0; ph < 5; ++ph) {
-                k_sah_split<<<(1u << lv0) * kSplitCtas, kSahWarps * 32, 0, s>>>(b.primBoxes, b.order, b.keysA, b.left, b.right,
+                launch_chain(k_sah_split, (1u << lv0) * kSplitCtas, kSahWarps * 32, 0, s, b.primBoxes, b.order, b.keysA, b.left, b.right,
                                                                                  b.nodeBoxes, tasksA, tasksB, lvCount, X, lv0, ph,
                                                                                  kSahMedianLevel);
                 count_launch();
@@ -2027,23 +2044,23 @@ cudaError_t sah_build(const LbvhBuffers& b, bool parents, uint32_t* levels, cuda
     int levelKernels = 0;  // until a level's tasks hold some kSahTask primitives
     while (!small && levelKernels < kSahParallelLevels && (b.n >> levelKernels) > kSahTask) ++levelKernels;
     for (int lv = lv0; lv < levelKernels; ++lv)
-        k_sah_level<<<1u << lv, kSahWarps * 32, 0, s>>>(b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA,
+        launch_chain(k_sah_level, 1u << lv, kSahWarps * 32, 0, s, b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA,
                                                          tasksB, lvCount, lv, kSahMedianLevel);
     if (small)
-        k_sah_build<true><<<1, kSahWarps * 32, kSahSmallSmem, s>>>(b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA,
+        launch_chain(k_sah_build<true>, 1, kSahWarps * 32, kSahSmallSmem, s, b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA,
                                                                    tasksB, 0u, kSahMedianLevel, kSahSmallHandoff, Q, lvCount, levels);
     else
-        k_sah_build<false><<<1, kSahWarps * 32, 0, s>>>(b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA, tasksB,
+        launch_chain(k_sah_build<false>, 1, kSahWarps * 32, 0, s, b.primBoxes, b.n, b.order, b.keysA, b.left, b.right, b.nodeBoxes, tasksA, tasksB,
                                                         (uint32_t)levelKernels, kSahMedianLevel, kSahHandoff, Q, lvCount, levels);
     // polls of an unpublished task before a warp gives up (RG_SAH_WAIT_LIMIT overrides; 0 makes
     // the first unpublished slot end the wait, which tests use to check the reported status)
     uint32_t waitLimit = kSahWaitLimit;
     if (const char* env = getenv("RG_SAH_WAIT_LIMIT")) waitLimit = (uint32_t)strtoul(env, nullptr, 10);
-    k_sah_tasks<<<grid, kSahTaskWarps * 32, 0, s>>>(b.primBoxes, b.order, b.keysA, b.left, b.right, b.nodeBoxes, Q, kSahMedianLevel,
+    launch_chain(k_sah_tasks, grid, kSahTaskWarps * 32, 0, s, b.primBoxes, b.order, b.keysA, b.left, b.right, b.nodeBoxes, Q, kSahMedianLevel,
                                                      small ? kSahSubtreeSmall : kSahSubtree, levels, b.status, waitLimit);
     count_launch(levelKernels - lv0 + 2);
     if (parents) {
-        k_parents<<<blocks(b.n - 1, 256), 256, 0, s>>>(b.left, b.right, b.n, b.parents);
+        launch_chain(k_parents, blocks(b.n - 1, 256), 256, 0, s, b.left, b.right, b.n, b.parents);
         count_launch();
     }
     return cudaGetLastError();
@@ -2051,7 +2068,7 @@ cudaError_t sah_build(const LbvhBuffers& b, bool parents, uint32_t* levels, cuda
 
 cudaError_t wide_records(const LbvhBuffers& b, WideNode* out, cudaStream_t s) {
     if (b.n <= 1) return cudaSuccess;
-    k_wide_records<<<blocks(b.n - 1, 256), 256, 0, s>>>(b.primBoxes, b.order, b.n, b.left, b.right, b.nodeBoxes, out);
+    launch_chain(k_wide_records, blocks(b.n - 1, 256), 256, 0, s, b.primBoxes, b.order, b.n, b.left, b.right, b.nodeBoxes, out);
     count_launch();
     return cudaGetLastError();
 }
@@ -2071,11 +2088,13 @@ cudaError_t lbvh_build(const LbvhBuffers& b, cudaStream_t s) {
         cfg.blockDim = dim3(kClusterThreads);
         cfg.dynamicSmemBytes = sizeof(ClusterSort);
         cfg.stream = s;
-        cudaLaunchAttribute at[1];
+        cudaLaunchAttribute at[2];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim = {size, 1, 1};
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_chain
+        at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         const auto kernel = rounds == 1 ? k_sort_cluster<1> : rounds == 2 ? k_sort_cluster<2> : k_sort_cluster<4>;
         const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const float*)b.primBoxes, n, b.morton, b.keysA, b.order, b.flags,
                                                  reinterpret_cast<uint32_t*>(b.nodeBoxes));
@@ -2087,8 +2106,8 @@ cudaError_t lbvh_build(const LbvhBuffers& b, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         uint32_t* bounds = b.sortState + kSortBounds;
         uint32_t gb = min(blocks(n, 256), 1024u);
-        k_centroid_bounds<<<gb, 256, 0, s>>>(b.primBoxes, n, bounds);
-        k_morton<<<min(blocks(n, 256), kMortonMaxBlocks), 256, 0, s>>>(b.primBoxes, n, bounds, b.morton, b.keysA, b.valsA, b.valsB, b.order,
+        launch_chain(k_centroid_bounds, gb, 256, 0, s, b.primBoxes, n, bounds);
+        launch_chain(k_morton, min(blocks(n, 256), kMortonMaxBlocks), 256, 0, s, b.primBoxes, n, bounds, b.morton, b.keysA, b.valsA, b.valsB, b.order,
                                                                        b.flags, reinterpret_cast<uint32_t*>(b.nodeBoxes), b.sortState);
         count_launch(2);
         // polls of an unpublished predecessor tile before a look-back counts that tile itself
@@ -2099,14 +2118,14 @@ cudaError_t lbvh_build(const LbvhBuffers& b, cudaStream_t s) {
         uint32_t* kout[4] = {b.keysB, b.keysA, b.keysB, b.keysA};
         uint32_t* vout[4] = {b.valsB, b.valsA, b.valsB, b.order};
         for (int pass = 0; pass < 4; ++pass) {
-            k_sort_onesweep<<<nTiles, kSortThreads, 0, s>>>(kin, vin, kout[pass], vout[pass], n, pass, b.sortState, nTiles, spinLimit);
+            launch_chain(k_sort_onesweep, nTiles, kSortThreads, 0, s, kin, vin, kout[pass], vout[pass], n, pass, b.sortState, nTiles, spinLimit);
             count_launch();
             kin = kout[pass];
             vin = vout[pass];
         }
     }
     if (n == 1) return cudaGetLastError();
-    k_hierarchy<<<blocks(n, kHierLeaves), kHierLeaves, 0, s>>>(b.keysA, b.order, b.primBoxes, n, b.left, b.right, b.parents, b.flags, b.nodeBoxes);
+    launch_chain(k_hierarchy, blocks(n, kHierLeaves), kHierLeaves, 0, s, b.keysA, b.order, b.primBoxes, n, b.left, b.right, b.parents, b.flags, b.nodeBoxes);
     count_launch();
     return cudaGetLastError();
 }

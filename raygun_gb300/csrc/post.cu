@@ -460,6 +460,7 @@ __device__ float4 fxaa_pixel(const Tex& T, int x, int y) {
 }
 
 __global__ void __launch_bounds__(256) k_fxaa(const PostParams P) {
+    chain_wait();
     const int x = blockIdx.x * 16 + (threadIdx.x & 15), y = blockIdx.y * 16 + (threadIdx.x >> 4);
     if (x >= (int)P.W || y >= (int)P.H) return;
     size_t pix = (size_t)y * P.W + x;
@@ -557,7 +558,7 @@ cudaError_t launch_rough_post(const PostParams& p, cudaStream_t s) {
 
 cudaError_t launch_fxaa(const PostParams& p, cudaStream_t s) {
     dim3 grid((p.W + 15) / 16, (p.H + 15) / 16);
-    k_fxaa<<<grid, 256, 0, s>>>(p);
+    launch_chain(k_fxaa, grid, 256, 0, s, p);
     count_launch();
     return cudaGetLastError();
 }

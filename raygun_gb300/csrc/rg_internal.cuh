@@ -6,6 +6,7 @@
 // out as fmaf() where they are wanted.
 #pragma once
 
+#include <utility>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -119,6 +120,28 @@ namespace rg {
 // kernels launched by this library in this process (rg_launch_count)
 extern std::atomic<uint64_t> g_launches;
 inline void count_launch(uint64_t n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+
+// A chain of short launches: each is set up while the one before it still runs (its blocks are placed as soon as
+// that one's have ended) and waits for that one's memory itself, first thing, with chain_wait.  1.5 us
+// less between two launches, of which a frame has 20 to 50 and a scene load 60: 160x90 frame 401 -> 363 us,
+// 640x360 spheres 997 -> 927 us, 1080p game frame 16.24 -> 16.08 ms.  Letting the next blocks in earlier
+// (launch_dependents) costs more than it gives: they hold places of blocks still working (16.41 ms).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// kernel: one that starts with chain_wait
+template <class... P, class... A>
+cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 struct LbvhBuffers {  // scratch + outputs of one LBVH build, sized by the caller (n primitives)
     uint32_t n;

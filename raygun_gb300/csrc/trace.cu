@@ -1110,6 +1110,7 @@ __device__ __forceinline__ void resolve_pixel(const float4* s, uint32_t S, size_
 }
 
 __global__ void k_resolve(const TraceParams P) {
+    chain_wait();
     const uint32_t x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
     if (x >= P.W || y >= P.H) return;
     const uint32_t S = (uint32_t)P.ubo.numSamples;
@@ -1128,10 +1129,6 @@ __global__ void k_resolve_job(const float4* __restrict__ samples, uint32_t W, ui
 
 // ---------------------------------------------------------------------------------------------
 // Frames and batches: rays traced by launches of one traversal kernel, between them what the hits need.
-
-// Start of a kernel of a frame's chain of launches (launch_next): from here on everything before it is finished
-// and visible.
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
     const unsigned mask = __ballot_sync(0xFFFFFFFFu, want);
@@ -2433,7 +2430,7 @@ cudaError_t launch_trace(const TraceParams& p, cudaStream_t s) {
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     dim3 grid((p.W + 31) / 32, (p.H + 7) / 8);
-    k_resolve<<<grid, 256, 0, s>>>(p);
+    launch_chain(k_resolve, grid, 256, 0, s, p);
     count_launch();
     return cudaGetLastError();
 }
@@ -2520,24 +2517,6 @@ cudaError_t launch_trace_queue(const TraceParams& p, const float* rays, uint32_t
     return cudaGetLastError();
 }
 
-// A launch that is set up while the one before it still runs (its blocks are placed as soon as that one's have
-// ended, and chain_wait for its memory): 1.5 us less between two launches, of which a frame has 20 to 50.
-// 160x90 frame 401 -> 363 us, 640x360 spheres 997 -> 927 us, 1080p game frame 16.24 -> 16.08 ms.  Letting the blocks
-// in earlier (launch_dependents) costs more than it gives: they hold places of blocks still working (16.41 ms).
-static cudaError_t launch_next(void (*kernel)(const TraceParams, int), int grid, int threads, cudaStream_t s, const TraceParams& p, int round) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    count_launch();
-    return cudaLaunchKernelEx(&cfg, kernel, p, round);
-}
-
 cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, uint32_t* hostWords, int* iterations, bool* poolFull,
                               EventPairFn kernelEvents, void* user) {
     TraceParams p = p0;
@@ -2576,12 +2555,14 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, uint32_t* h
                 cudaEvent_t e0 = nullptr, e1 = nullptr;
                 if (kernelEvents && !kernelEvents(user, &e0, &e1)) e0 = e1 = nullptr;
                 if (e0) cudaEventRecord(e0, s);
-                if ((e = launch_next(trace, gTrace, kTraceThreads, s, p, k)) != cudaSuccess) return e;
+                if ((e = launch_chain(trace, gTrace, kTraceThreads, 0, s, p, k)) != cudaSuccess) return e;
                 if (e1) cudaEventRecord(e1, s);
-                if ((e = launch_next(expand, gExpand, 128, s, p, k)) != cudaSuccess) return e;
+                count_launch(2);
+                if ((e = launch_chain(expand, gExpand, 128, 0, s, p, k)) != cudaSuccess) return e;
             }
             if (maxRec == 0) break;  // no hit issues a ray
-            if ((e = launch_next(check, gCheck, 128, s, p, k)) != cudaSuccess) return e;
+            count_launch();
+            if ((e = launch_chain(check, gCheck, 128, 0, s, p, k)) != cudaSuccess) return e;
             if ((e = cudaMemcpyAsync(hostWords, p.tree.ctl, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
             if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
             full = p.treeRoots + hostWords[kTreeAlloc] > cap;
@@ -2598,12 +2579,13 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, uint32_t* h
             split(p.treeBase, p.treeRoots, (p.treeRoots + 7) / 8);
             continue;
         }
+        count_launch(k);
         while (k--)
-            if ((e = launch_next(k_tree_compose<false>, gCompose, 128, s, p, k)) != cudaSuccess) return e;
+            if ((e = launch_chain(k_tree_compose<false>, gCompose, 128, 0, s, p, k)) != cudaSuccess) return e;
     }
     if (iterations) *iterations = it;
     dim3 grid((p.W + 31) / 32, (p.H + 7) / 8);
-    k_resolve<<<grid, 256, 0, s>>>(p);
+    launch_chain(k_resolve, grid, 256, 0, s, p);
     count_launch();
     return cudaGetLastError();
 }
