@@ -884,10 +884,10 @@ rg_status rg_download(rg_ctx* c, float* host) {
     if (!c->haveFrame) return fail(c, RG_ERR_NOT_READY, "no frame rendered");
     TRY(set_device(c));
     CK(cudaMemcpyAsync(host, c->fb.p, 16ull * c->W * c->H, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(&c->hostCount[7], wait_status(c), 4, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(&c->hostCount[9], wait_status(c), 4, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     TRY(settle_graph(c));
-    if (c->hostCount[7]) return fail(c, RG_ERR_CUDA, wait_failure(c->hostCount[7]));
+    if (c->hostCount[9]) return fail(c, RG_ERR_CUDA, wait_failure(c->hostCount[9]));
     return RG_OK;
 }
 
@@ -955,11 +955,11 @@ rg_status rg_download_image(rg_ctx* c, int32_t which, float* host) {
 rg_status rg_synchronize(rg_ctx* c) {
     if (!c) return RG_ERR_INVALID_ARG;
     TRY(set_device(c));
-    CK(cudaMemcpyAsync(&c->hostCount[7], wait_status(c), 4, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(&c->hostCount[9], wait_status(c), 4, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     CK(cudaStreamSynchronize(c->copyStream));
     TRY(settle_graph(c));
-    if (c->hostCount[7]) return fail(c, RG_ERR_CUDA, wait_failure(c->hostCount[7]));
+    if (c->hostCount[9]) return fail(c, RG_ERR_CUDA, wait_failure(c->hostCount[9]));
     return RG_OK;
 }
 

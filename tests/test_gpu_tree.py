@@ -112,4 +112,5 @@ def test_batch_trees(rg, monkeypatch, pool, host_loop, sort):
         st = br.ctx.stats()
         assert {k: st[k] for k in ("primary", "shadow", "secondary", "masked")} == \
             {k: sum(s[k] for _, s in ref) for k in ("primary", "shadow", "secondary", "masked")}
+        assert st["iterations"] >= 9  # the largest recursion limit + 1
     br.ctx.close()
