@@ -125,6 +125,7 @@ struct rg_ctx {
     // graph form of the batch: second stream (loop body capture), instantiated graph and what it
     // was captured for, loop words (device), launch accounting
     cudaStream_t stream2 = nullptr;
+    cudaEvent_t laneEvent[2] = {nullptr, nullptr};  // tie it to `stream` while it runs a frame's second lane
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graphExec = nullptr;
     std::vector<uint8_t> graphKey;
@@ -465,7 +466,7 @@ rg_status ensure_tree_nodes(rg_ctx* c, size_t cap, RayTree& t) {
     TRY(ensure(c, c->trLink, 16 * cap));
     TRY(ensure(c, c->trOver, 4 * cap));
     TRY(ensure(c, c->trCand, 8 * cap));
-    TRY(ensure(c, c->trCtl, kTreeCtlWords * sizeof(uint32_t)));
+    TRY(ensure(c, c->trCtl, 2 * kTreeCtlWords * sizeof(uint32_t)));  // a frame's two lanes
     t.rayO = c->trO.as<float4>();
     t.rayD = c->trD.as<float4>();
     t.state = c->trState.as<uint4>();
@@ -524,9 +525,11 @@ rg_status rg_create(rg_ctx** out, const rg_device_opts* opts) {
         return RG_ERR_OUT_OF_MEMORY;
     }
     cudaMemsetAsync(c->counters.p, 0, 18 * sizeof(unsigned long long), c->stream);
-    if (cudaHostAlloc(&c->hostCount, 12 * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess ||
+    if (cudaHostAlloc(&c->hostCount, 16 * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->copyStream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->laneEvent[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->laneEvent[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->staged[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->staged[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->copied[0], cudaEventDisableTiming) != cudaSuccess ||
@@ -573,6 +576,8 @@ rg_status rg_destroy(rg_ctx* c) {
     if (c->graphExec) cudaGraphExecDestroy(c->graphExec);
     if (c->graph) cudaGraphDestroy(c->graph);
     release(c, c->loopWords);
+    for (cudaEvent_t e : c->laneEvent)
+        if (e) cudaEventDestroy(e);
     if (c->stream2) cudaStreamDestroy(c->stream2);
     if (c->hostCount) cudaFreeHost(c->hostCount);
     if (c->queryStage) cudaFreeHost(c->queryStage);
@@ -854,7 +859,9 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     } else {
         bool full = false;
         const bool timed = (c->flags & RG_FLAG_KERNEL_TIMING) != 0;
-        CK(launch_trace_tree(tp, c->stream, c->hostCount, &c->lastIterations, &full, timed ? next_kernel_events : nullptr, timed ? fe : nullptr));
+        const TreeLane second = {c->stream2, c->laneEvent[0], c->laneEvent[1], tp.tree.ctl + kTreeCtlWords, c->hostCount + 12};
+        CK(launch_trace_tree(tp, c->stream, second, c->hostCount, &c->lastIterations, &full, timed ? next_kernel_events : nullptr,
+                             timed ? fe : nullptr));
         if (full && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
     }
     return run_post(c, ubo, fxaa);

@@ -319,9 +319,16 @@ inline size_t frame_work_items(uint32_t W, uint32_t H, uint32_t S) {
 // kernelEvents (nullable): callback that returns a (start, end) event pair to record around each
 // traversal launch
 typedef bool (*EventPairFn)(void* user, cudaEvent_t* start, cudaEvent_t* end);
-// a frame through ray trees, and its resolve.  hostWords: three pinned words polled after each check;
+// what a frame's second lane of chunks runs with: an idle stream, events that tie it to the frame's stream, control
+// words and pinned words of its own
+struct TreeLane {
+    cudaStream_t stream;
+    cudaEvent_t fork, join;
+    uint32_t *ctl, *hostWords;
+};
+// a frame through ray trees, and its resolve.  hostWords: four pinned words polled after each check;
 // iterations: rounds run; *poolFull: a chunk of samples filled the node pool
-cudaError_t launch_trace_tree(const TraceParams& p, cudaStream_t s, uint32_t* hostWords, int* iterations, bool* poolFull,
+cudaError_t launch_trace_tree(const TraceParams& p, cudaStream_t s, const TreeLane& second, uint32_t* hostWords, int* iterations, bool* poolFull,
                               EventPairFn kernelEvents = nullptr, void* user = nullptr);
 // traversal launch shape of the batch loop: block size {64,128,256}, stack entries {16,24,32,48},
 // ray-sort key applied to each queue before it is traced

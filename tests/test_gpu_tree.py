@@ -62,6 +62,20 @@ def test_full_node_pool(rg, monkeypatch, pool):
         assert np.array_equal(x, y)
 
 
+@pytest.mark.parametrize("pool", [None, 2000000])
+def test_two_lanes(rg, monkeypatch, pool):
+    """A frame large enough for two lanes of chunks, with a pool that holds all trees or a fraction of them."""
+    sc = glass_scene(1283, 409, 2, 3)
+    ref, sr = render(rg, sc, flags=rg.RG_FLAG_MEGAKERNEL)
+    if pool:
+        monkeypatch.setenv("RG_TREE_POOL", str(pool))
+    for _ in range(2):
+        got, sg = render(rg, sc)
+        assert sg == sr
+        for x, y in zip(got, ref):
+            assert np.array_equal(x, y)
+
+
 def test_trees_equal_oracle(rg, orc):
     sc = glass_scene(128, 72, 1, 6)
     (img, _, _), st = render(rg, sc)
