@@ -486,7 +486,7 @@ rg_status ensure_tree_nodes(rg_ctx* c, size_t cap, RayTree& t) {
 // up again where memory does not allow it.
 rg_status ensure_tree(rg_ctx* c, size_t roots, size_t least, RayTree& t) {
     // (RG_TREE_POOL overrides the pool's nodes; tests use a small pool to make chunks fill it)
-    if (const char* env = getenv("RG_TREE_POOL")) return ensure_tree_nodes(c, std::max<size_t>(strtoull(env, nullptr, 10), 4608), t);
+    if (const char* env = getenv("RG_TREE_POOL")) return ensure_tree_nodes(c, std::max<size_t>(strtoull(env, nullptr, 10), kTreePoolMin), t);
     const rg_status st = ensure_tree_nodes(c, std::max(roots * c->treeNodes, least), t);
     if ((st != RG_ERR_BUDGET && st != RG_ERR_OUT_OF_MEMORY) || c->treeNodes == kTreeNodesMin) return st;
     if (st == RG_ERR_OUT_OF_MEMORY) cudaGetLastError();
@@ -848,7 +848,7 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     tp.glossySeed = c->glossySeed;
     c->lastSamples = (uint32_t)ubo->numSamples;
     const bool mega = (c->flags & RG_FLAG_MEGAKERNEL) != 0;
-    if (!mega) TRY(ensure_tree(c, std::min<size_t>(frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), 1u << 25), 1u << 16, tp.tree));
+    if (!mega) TRY(ensure_tree(c, std::min<size_t>(frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), 1u << 25), kTreePoolMin, tp.tree));
     CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
     FrameEvents* fe;
     TRY(cur_events(c, &fe));
@@ -1472,7 +1472,7 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
     const uint32_t slots = (uint32_t)std::min<uint64_t>(work, c->batchSlots);
     TraceParams tp;
     std::memset(&tp, 0, sizeof(tp));
-    TRY(ensure_tree(c, slots, 4608, tp.tree));
+    TRY(ensure_tree(c, slots, kTreePoolMin, tp.tree));
     TRY(ensure(c, c->samples, 48ull * samples));
     TRY(ensure(c, c->jobTable, sizeof(JobDesc) * n));
     SortScratch sort{};

@@ -259,6 +259,7 @@ struct TreeLoop {
 // that fills the pool goes again in smaller chunks, and the next frame's pool is twice as large, up to
 // kTreeNodesMax a sample.
 constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 13;
+constexpr size_t kTreePoolMin = 4608;  // nodes: a sample's tree at 8 recursions, replaced rays included
 
 // one render job of a batch: a scene, its UBO and its image size.  Work items of the batch are
 // numbered job after job; job j owns [workBase, workBase + workCount) and writes its per-sample
