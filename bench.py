@@ -338,7 +338,7 @@ def run_ours(args):
     ctx.set_flags(0)
     crays = cst["primary"] + cst["shadow"] + cst["secondary"]
     bytes_per_ray = (crays * BYTES_RAY + cst["nodes"] * BYTES_NODE + cst["tris"] * BYTES_TRI) / max(crays, 1)
-    # k_wf_trace runs once per wavefront round; one frame's launches are taken together as the unit
+    # k_wf_trace runs once per round; one frame's launches are taken together as the unit
     trace_ms = tm["traceKernelSum"] / max(tm["frames"], 1)
     bytes_launch = bytes_per_ray * rays / K
     achieved = bytes_launch / (trace_ms * 1e-3) / 1e9
@@ -532,7 +532,7 @@ def run_batch(args):
                    "instanced_tris": int(sum(sc.instanced_tri_count for sc in scenes)),
                    "unique_tris": int(sum(sc.tri_count for sc in scenes)), "pixels": int(sum(pixels)),
                    "samples": int(sum(p * int(sc.ubo["numSamples"][0]) for p, sc in zip(pixels, scenes))),
-                   "l2": "inputs larger than L2 (path state and scene BVHs of the batch are several GB)",
+                   "l2": "inputs larger than L2 (ray-tree nodes and scene BVHs of the batch are several GB)",
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
         "batches_per_s": K / (ms * 1e-3), "rays_per_batch": rays / K,
         "autotune": None if tune is None else {

@@ -41,7 +41,7 @@ typedef struct {
 } rg_device_opts;
 #define RG_FLAG_DEBUG_IMAGES 1u /* keep roughTransitions / roughColorsA/B for rg_download_image */
 #define RG_FLAG_COUNT_VISITS 2u /* count BVH node / triangle visits (roofline accounting) */
-#define RG_FLAG_MEGAKERNEL 4u   /* trace + shade in one persistent kernel instead of the wavefront loop */
+#define RG_FLAG_MEGAKERNEL 4u   /* trace + shade in one persistent kernel instead of ray trees */
 #define RG_FLAG_KERNEL_TIMING 8u /* CUDA events around every traversal launch (rg_timings.traceKernel) */
 #define RG_FLAG_HOST_LOOP 16u    /* rg_render_batch: host-polled round loop instead of the CUDA graph */
 #define RG_FLAG_TLAS_LBVH 32u    /* build the TLAS as an LBVH (Morton order) instead of by binned SAH; TLASes of more
@@ -335,7 +335,7 @@ rg_status rg_set_filter(rg_ctx* ctx, rg_filter* f);
  * of the material roughness (alpha = roughness^2), seeded per pixel sample from `seed` */
 rg_status rg_set_glossy(rg_ctx* ctx, uint32_t seed);
 
-/* Device memory the context holds (all scene slots, images, path state, scratch) and its budget
+/* Device memory the context holds (all scene slots, images, ray-tree nodes, scratch) and its budget
  * (rg_device_opts.hbm_budget_bytes, 0 = none), in bytes. */
 rg_status rg_get_memory(rg_ctx* ctx, uint64_t* allocated_bytes, uint64_t* budget_bytes);
 /* Samples of a batch in flight: its samples go through their ray trees in chunks of at most this many.

@@ -75,7 +75,7 @@ def scene_bytes_estimate(sc: scenes.Scene) -> int:
 
 
 def working_bytes(reqs, path_slots: int) -> int:
-    """Device memory of one batch beyond its scenes: path state, sample sums, images, post scratch."""
+    """Device memory of one batch beyond its scenes: ray-tree nodes, sample sums, images, post scratch."""
     if not reqs:
         return 0
     samples = sum(r.samples for r in reqs)
