@@ -830,6 +830,10 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     if (!c->W) return fail(c, RG_ERR_NOT_READY, "rg_set_resolution was not called");
     if (!c->sc->tlasReady) return fail(c, RG_ERR_NOT_READY, "no TLAS (call rg_build_tlas after the last rg_build_blas)");
     TRY(set_device(c));
+    const bool mega = (c->flags & RG_FLAG_MEGAKERNEL) != 0;
+    // chunks are numbered in 32 bits (a path per sample at once did not fit in memory from far fewer samples on)
+    if (!mega && frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples) >= (1ull << 31))
+        return fail(c, RG_ERR_TOO_LARGE, "frame too large: at most 2^31 samples per frame");
     TRY(ensure(c, c->samples, 48ull * c->W * c->H * (uint32_t)ubo->numSamples));
     TRY(ensure(c, c->workCounter, 16));
     TraceParams tp;
@@ -847,7 +851,6 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     tp.workCounter = c->workCounter.as<uint32_t>();
     tp.glossySeed = c->glossySeed;
     c->lastSamples = (uint32_t)ubo->numSamples;
-    const bool mega = (c->flags & RG_FLAG_MEGAKERNEL) != 0;
     if (!mega) TRY(ensure_tree(c, std::min<size_t>(frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), 1u << 25), kTreePoolMin, tp.tree));
     CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
     FrameEvents* fe;

@@ -587,10 +587,7 @@ __global__ void k_inst_records(const uint32_t* __restrict__ order, uint32_t n, c
 //     kHierPolls requests the box is taken from the leaves instead, so no wait is unbounded.
 // 50000 leaves: 23 us (37 us with an acquire-release arrival and its box after it), against 12 us for
 // the nodes and 36 us for the boxes as two kernels.
-#ifndef RG_HIER_LEAVES
-#define RG_HIER_LEAVES 512
-#endif
-constexpr int kHierLeaves = RG_HIER_LEAVES;
+constexpr int kHierLeaves = 512;
 constexpr int kHierPolls = 4096;
 
 __device__ __forceinline__ int delta(uint32_t a, uint32_t b, uint32_t i, uint32_t j) {  // common leading bits of (code, position)
