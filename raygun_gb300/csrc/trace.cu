@@ -11,8 +11,9 @@
 // the smaller (instance, primitive).  Box tests only ever accept more than the exact test would (see
 // the ray set-up below), so the hit found does not depend on the tree: it is the brute-force answer.
 //
-// The reference's recursion (nested traceRayEXT calls sharing ONE payload, payload.h:29-43) runs
-// here as an explicit state machine per thread: a paused closest-hit invocation is a Frame on a
+// Frames and batches run the reference's recursion (nested traceRayEXT calls sharing ONE payload,
+// payload.h:29-43) as ray trees, described at k_tree_expand.  The megakernel runs it as written, by an
+// explicit state machine per thread: a paused closest-hit invocation is a Frame on a
 // small per-thread stack with a resume code, and every trace (of any depth) happens in the same
 // outer loop so the threads of a warp traverse together.  Payload fields that the reference leaves
 // stale (depth, rayType, curIOR, refDepth) leak exactly as in the reference.
