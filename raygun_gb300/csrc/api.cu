@@ -268,6 +268,9 @@ rg_status ensure(rg_ctx* c, DevBuf& b, size_t bytes) {
     }
     b.cap = grow;
     c->allocated += grow;
+    // what new device memory holds is undefined, and mostly zeros (RG_FILL_ALLOC fills it with a byte; tests use it
+    // to show that nothing relies on zeros)
+    if (const char* env = getenv("RG_FILL_ALLOC")) CK(cudaMemsetAsync(b.p, (int)strtoul(env, nullptr, 0), grow, c->stream));
     return RG_OK;
 }
 

@@ -2696,6 +2696,10 @@ struct BatchLaunch {
         gSort = grid_of((const void*)k_sort_scatter<RG_SORT_MORTON>, 256);
         return gTrace && gExpand && gCheck && gCompose && gSort;
     }
+    // the bucket counts start at zero; each round's k_sort_offsets leaves them at zero again
+    cudaError_t begin(cudaStream_t s) const {
+        return sortKey == RG_SORT_NONE ? cudaSuccess : cudaMemsetAsync(sort.hist, 0, SortBuckets<RG_SORT_MORTON>::n * sizeof(uint32_t), s);
+    }
     int perRound() const { return 2 + (sortKey != RG_SORT_NONE ? 3 : 0); }
     // round k (negative: the current one)
     cudaError_t round(TraceParams p, int k, cudaStream_t s, cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr) const {
@@ -2749,6 +2753,7 @@ cudaError_t launch_trace_batch(const TraceParams& p0, const TraceTune& tune, con
     cudaError_t e;
     *iterations = 0;
     *poolFull = false;
+    if ((e = B.begin(s)) != cudaSuccess) return e;
     k_tree_next<<<1, 1, 0, s>>>(p, loop, true);
     count_launch();
     for (;;) {
@@ -2814,6 +2819,7 @@ cudaError_t capture_trace_batch(const TraceParams& p0, const TraceTune& tune, co
         cudaError_t e;
         cudaGraphNode_t node;
         cudaGraph_t chunk = nullptr, body = nullptr, done = nullptr;
+        if ((e = B.begin(s)) != cudaSuccess) return e;
         k_tree_next<<<1, 1, 0, s>>>(p, loop, true);
         if ((e = add_while(s, &loop.chunks, true, &node, &chunk)) != cudaSuccess) return e;
         if ((e = cudaStreamBeginCaptureToGraph(s2, chunk, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed)) != cudaSuccess) return e;

@@ -1,0 +1,28 @@
+"""Batches at the edges of their loops: what new device memory holds, loops that give up, many chunks, samples
+whose trees exceed the node pool."""
+import numpy as np
+import pytest
+
+from test_gpu_tree import glass_scene, render
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def glass(rg):
+    scs = [glass_scene(97, 55, 2, 5, seed=3), glass_scene(40, 30, 1, 0, seed=4), glass_scene(64, 64, 1, 8, seed=5, spheres=24)]
+    return scs, [render(rg, sc)[0][0] for sc in scs]
+
+
+@pytest.mark.parametrize("host_loop", [False, True])
+@pytest.mark.parametrize("sort", ["none", "octant", "morton"])
+def test_first_batch_in_filled_memory(rg, glass, monkeypatch, sort, host_loop):
+    """The first batch of a context whose buffers do not start as zeros (the ray sort's bucket counts are added to)."""
+    scs, ref = glass
+    br = rg.BatchRenderer(scs, flags=rg.RG_FLAG_HOST_LOOP if host_loop else 0)
+    br.ctx.set_batch_tune(128, 48, sort)
+    monkeypatch.setenv("RG_FILL_ALLOC", "0x3c")
+    for _ in range(2):
+        for img, r in zip(br.render(), ref):
+            assert np.array_equal(img, r)
+    br.ctx.close()
