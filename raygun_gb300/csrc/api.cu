@@ -274,6 +274,8 @@ rg_status ensure(rg_ctx* c, DevBuf& b, size_t bytes) {
     return RG_OK;
 }
 
+constexpr const char* kLoopLimitError = "batch round loop stopped at its iteration limit";
+
 // bookkeeping of finished batch-graph launches (call after the stream was synchronized): launch
 // accounting of the graph's loops, round count, the loops' limit flag, a larger pool after a full one
 rg_status settle_graph(rg_ctx* c) {
@@ -285,7 +287,7 @@ rg_status settle_graph(rg_ctx* c) {
     if (c->hostCount[8] && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
     if (c->hostCount[5]) {
         CK(cudaMemsetAsync(c->loopWords.as<uint32_t>() + 1, 0, sizeof(uint32_t), c->stream));
-        return fail(c, RG_ERR_CUDA, "batch round loop stopped at its iteration limit");
+        return fail(c, RG_ERR_CUDA, kLoopLimitError);
     }
     return RG_OK;
 }
@@ -1530,8 +1532,10 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
     if (hostLoop) {
         const bool timed = (c->flags & RG_FLAG_KERNEL_TIMING) != 0;
         bool full = false;
-        CK(launch_trace_batch(tp, c->tune, sort, c->loopWords.as<uint32_t>(), c->stream, c->hostCount, &c->lastIterations, &full,
-                              timed ? next_kernel_events : nullptr, timed ? fe : nullptr));
+        const cudaError_t e = launch_trace_batch(tp, c->tune, sort, c->loopWords.as<uint32_t>(), c->stream, c->hostCount, &c->lastIterations,
+                                                 &full, timed ? next_kernel_events : nullptr, timed ? fe : nullptr);
+        if (e == cudaErrorLaunchTimeout) return fail(c, RG_ERR_CUDA, kLoopLimitError);
+        CK(e);
         if (full && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
         CK(cudaEventRecord(fe->ev[EV_POST0], c->stream));
         CK(enqueue_batch_posts(c, jd.data(), jobs, n));

@@ -248,7 +248,7 @@ enum : int {
 };
 constexpr int kTreeComposeRun = 4;  // rounds composed per run of that loop
 // loops of a batch's graph: their conditions; words: runs of the loops in this launch (at most maxRuns), sticky limit
-// flag, kernels launched in total, rounds in this launch; kernels of a chunk, a run of rounds, a run of compositions
+// flag (graph form), kernels launched in total, rounds in this launch; kernels of a chunk, a run of rounds, a run of compositions
 struct TreeLoop {
     bool graph;
     cudaGraphConditionalHandle chunks, rounds, composes;
@@ -342,7 +342,7 @@ struct SortScratch {
     uint32_t *keysA, *keysB, *valsA, *valsB, *hist;
 };
 // every job of p.jobs through ray trees, the loops on the host; hostWords: four pinned words polled after each check
-// and chunk; loopWords as below
+// and chunk; loopWords as below; cudaErrorLaunchTimeout when the loops gave up
 cudaError_t launch_trace_batch(const TraceParams& p, const TraceTune& tune, const SortScratch& sort, uint32_t* loopWords, cudaStream_t s,
                                uint32_t* hostWords, int* iterations, bool* poolFull, EventPairFn kernelEvents = nullptr, void* user = nullptr);
 // graph form, enqueued on stream s while it captures; the loops run on the device (bodies captured on the idle stream s2).

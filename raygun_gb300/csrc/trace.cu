@@ -2238,7 +2238,7 @@ __global__ void k_tree_step(const __grid_constant__ TraceParams P, const TreeLoo
     bool more = !full && (nodes > c[kTreeTraced] || c[kTreeChanges]);
     loop.words[0] += 1u;
     if (more && (loop.words[0] >= loop.maxRuns || rounds + (uint32_t)P.batchRounds >= (uint32_t)kTreeMaxRounds)) {
-        loop.words[1] = 1u;
+        if (loop.graph) loop.words[1] = 1u;
         more = false;
         full = true;  // the chunk is not composed,
         c[kTreeRoots] = 0u;  // and no other follows
@@ -2267,7 +2267,7 @@ __global__ void k_tree_composed(const __grid_constant__ TraceParams P, const Tre
 }
 
 // the next chunk (first: of a launch); one that filled the pool goes again in eight parts, and so do the
-// samples after it
+// samples after it.  kTreeLive: a chunk is set up (1), none is left (0), or the loops gave up (2)
 __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoop loop, bool first) {
     uint32_t* c = P.tree.ctl;
     if (first) {
@@ -2279,10 +2279,7 @@ __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoo
     bool stop = false;
     if (c[kTreeFull]) {
         c[kTreeWasFull] = 1u;
-        if (c[kTreeRoots] <= 1u) {  // stopped, or a sample's tree that is larger than the pool (none is)
-            loop.words[1] = 1u;
-            stop = true;
-        }
+        stop = c[kTreeRoots] <= 1u;  // stopped, or a sample's tree that is larger than the pool (none is)
         c[kTreeChunk] = (c[kTreeRoots] + 7u) / 8u;
     } else {
         c[kTreeBase] += c[kTreeRoots];
@@ -2291,15 +2288,16 @@ __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoo
     if (!first) {
         loop.words[0] += 1u;
         if (more && loop.words[0] >= loop.maxRuns) {
-            loop.words[1] = 1u;
+            stop = true;
             more = false;
         }
     }
     c[kTreeRoots] = more ? min(c[kTreeChunk], P.totalWork - c[kTreeBase]) : 0u;
     c[kTreeAlloc] = c[kTreeChanges] = c[kTreeLevels] = c[kTreeTraced] = c[kTreeFetch] = c[kTreeCand] = c[kTreeCand + 1] = 0u;
     c[kTreeCandList] = c[kTreeRound] = c[kTreeFull] = 0u;
-    c[kTreeLive] = more;
+    c[kTreeLive] = more ? 1u : stop ? 2u : 0u;
     if (loop.graph) {
+        if (stop) loop.words[1] = 1u;
         loop.words[2] += (first ? 1u : 0u) + (more ? loop.chunkKernels : 0u);
         if (!first) cudaGraphSetConditional(loop.chunks, more);
     }
@@ -2734,12 +2732,19 @@ static TraceParams batch_params(const TraceParams& p0) {
     return p;
 }
 
+// loop runs before a batch's loops give up (RG_BATCH_LOOP_LIMIT overrides, read when a graph is captured and
+// at every batch of the host loop; tests use a small limit to check the reported error)
+static uint32_t loop_limit(uint32_t runs) {
+    const char* env = getenv("RG_BATCH_LOOP_LIMIT");
+    return env ? (uint32_t)strtoul(env, nullptr, 10) : runs;
+}
+
 cudaError_t launch_trace_batch(const TraceParams& p0, const TraceTune& tune, const SortScratch& sort, uint32_t* loopWords, cudaStream_t s,
                                uint32_t* hostWords, int* iterations, bool* poolFull, EventPairFn kernelEvents, void* user) {
     const TraceParams p = batch_params(p0);
     BatchLaunch B;
     if (!B.init(p, tune, sort)) return cudaErrorInvalidValue;
-    const TreeLoop loop = {false, 0, 0, 0, loopWords, 1u << 30, 0, 0, 0};
+    const TreeLoop loop = {false, 0, 0, 0, loopWords, loop_limit(1u << 30), 0, 0, 0};
     auto poll = [&]() {
         cudaError_t e = cudaMemcpyAsync(hostWords, p.tree.ctl + kTreeMore, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -2775,6 +2780,7 @@ cudaError_t launch_trace_batch(const TraceParams& p0, const TraceTune& tune, con
         k_tree_next<<<1, 1, 0, s>>>(p, loop, false);
         count_launch();
         if ((e = poll()) != cudaSuccess) return e;
+        if (hostWords[3] == 2u) return cudaErrorLaunchTimeout;  // the loops gave up: samples are missing
         if (!hostWords[3]) break;
     }
     return cudaGetLastError();
@@ -2805,10 +2811,7 @@ cudaError_t capture_trace_batch(const TraceParams& p0, const TraceTune& tune, co
     if (p.countVisits) return cudaErrorInvalidValue;  // the visit-counting build runs the host loop
     BatchLaunch B;
     if (!B.init(p, tune, sort)) return cudaErrorInvalidValue;
-    // loop runs before the loops stop with the limit flag set (RG_BATCH_LOOP_LIMIT overrides, read
-    // when the graph is captured; tests use a small limit to check the reported error)
-    uint32_t maxIter = 50000u;
-    if (const char* env = getenv("RG_BATCH_LOOP_LIMIT")) maxIter = (uint32_t)strtoul(env, nullptr, 10);
+    const uint32_t maxIter = loop_limit(50000u);
     const int R = p.batchRounds, more = std::max(1, R - 1);
     TreeLoop loop = {true, 0, 0, 0, loopWords, maxIter, (uint32_t)(R * B.perRound() + 2 + R + 1), (uint32_t)(more * B.perRound() + 2),
                      (uint32_t)kTreeComposeRun + 1u};

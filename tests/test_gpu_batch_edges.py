@@ -26,3 +26,21 @@ def test_first_batch_in_filled_memory(rg, glass, monkeypatch, sort, host_loop):
         for img, r in zip(br.render(), ref):
             assert np.array_equal(img, r)
     br.ctx.close()
+
+
+def test_host_loop_limit_is_reported(rg, glass, monkeypatch):
+    """The host loop that stops at its limit returns the error itself, and leaves nothing behind for the
+    batches after it, in either form."""
+    scs, ref = glass
+    br = rg.BatchRenderer(scs, flags=rg.RG_FLAG_HOST_LOOP)
+    br.ctx.set_batch_slots(1024)
+    monkeypatch.setenv("RG_BATCH_LOOP_LIMIT", "1")
+    with pytest.raises(rg.RgError) as e:
+        br.ctx.render_batch(br.jobs())
+    assert e.value.code == -2 and "iteration limit" in str(e.value), str(e.value)
+    monkeypatch.delenv("RG_BATCH_LOOP_LIMIT")
+    for flags in (0, rg.RG_FLAG_HOST_LOOP):
+        br.ctx.set_flags(flags)
+        for img, r in zip(br.render(), ref):
+            assert np.array_equal(img, r)
+    br.ctx.close()
