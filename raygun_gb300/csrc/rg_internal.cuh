@@ -229,7 +229,7 @@ struct RayTree {
     uint32_t* overflow; // nodes of rays whose short traversal stack overflowed
     uint32_t* cand[2];  // nodes whose assumptions k_tree_check verifies (the list in use: treeCand)
     uint32_t* ctl;      // kTreeCtlWords words
-    uint32_t capacity;  // nodes, below kTreeMaxNodes
+    uint32_t capacity;  // nodes, at most kTreePoolMax
 };
 // words of RayTree::ctl: nodes appended after the roots; rays that the last check changed, 16 minus the
 // least recursion depth of the rays replaced since the last round, nodes traced when the last check ran;
@@ -260,6 +260,12 @@ struct TreeLoop {
 // kTreeNodesMax a sample.
 constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 13;
 constexpr size_t kTreePoolMin = 4608;  // nodes: a sample's tree at 8 recursions, replaced rays included
+constexpr size_t kTreePoolMax = kTreeMaxNodes - 4;  // links keep 29 bits for a node, three of their values for no node
+// nodes of the pool for `roots` samples; a pool at its bound holds fewer samples a chunk
+constexpr size_t tree_pool_nodes(size_t roots, size_t perRoot, size_t least) {
+    const size_t n = roots > kTreePoolMax / perRoot ? kTreePoolMax : roots * perRoot;
+    return n < least ? (least < kTreePoolMax ? least : kTreePoolMax) : n;
+}
 
 // one render job of a batch: a scene, its UBO and its image size.  Work items of the batch are
 // numbered job after job; job j owns [workBase, workBase + workCount) and writes its per-sample

@@ -1623,6 +1623,7 @@ constexpr uint32_t kNodeMask = kTreeMaxNodes - 1u;  // links: node ids below kTr
 constexpr uint32_t kNoNode = kNodeMask;             //   no ray issued
 constexpr uint32_t kZeroFront = kNodeMask - 1u;     //   a front-face refraction of zero direction: misses,
 constexpr uint32_t kZeroBack = kNodeMask - 2u;      //   leaves curIOR = ior; a back-face one: leaves 1
+static_assert(kTreePoolMax <= kZeroBack, "a node of a pool is never one of the links' values for none");
 constexpr uint32_t kFrontBit = 0x80000000u;         // links.x: the ray hit the front face
 constexpr uint32_t kOffBit = 0x40000000u;           // state.z: a sibling may have changed refDepth
 constexpr uint32_t kDeadBit = 0x80000000u;          // state.z: below a ray that was replaced
