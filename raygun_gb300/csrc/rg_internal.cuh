@@ -247,7 +247,7 @@ enum : int {
     kTreeTracedRound, kTreeChunk, kTreeWasFull, kTreeCtlWords
 };
 constexpr int kTreeComposeRun = 4;  // rounds composed per run of that loop
-// loops of a batch's graph: their conditions; words: runs of the loops in this launch (at most maxRuns), sticky limit
+// loops of a batch's graph: their conditions; words: runs of the loops on this chunk (at most maxRuns), sticky limit
 // flag (graph form), kernels launched in total, rounds in this launch; kernels of a chunk, a run of rounds, a run of compositions
 struct TreeLoop {
     bool graph;

@@ -2278,7 +2278,8 @@ __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoo
         c[kTreeFetch + 1] = c[kTreeFetch + 2] = 0u;
     }
     bool stop = false;
-    if (c[kTreeFull]) {
+    const bool full = c[kTreeFull] != 0u;
+    if (full) {
         c[kTreeWasFull] = 1u;
         stop = c[kTreeRoots] <= 1u;  // stopped, or a sample's tree that is larger than the pool (none is)
         c[kTreeChunk] = (c[kTreeRoots] + 7u) / 8u;
@@ -2292,6 +2293,9 @@ __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoo
             stop = true;
             more = false;
         }
+        // every chunk has the limit's runs for itself (a batch of many small chunks is no endless loop); the parts of a
+        // chunk that filled the pool share them until one is done
+        if (!full) loop.words[0] = 0u;
     }
     c[kTreeRoots] = more ? min(c[kTreeChunk], P.totalWork - c[kTreeBase]) : 0u;
     c[kTreeAlloc] = c[kTreeChanges] = c[kTreeLevels] = c[kTreeTraced] = c[kTreeFetch] = c[kTreeCand] = c[kTreeCand + 1] = 0u;
@@ -2733,11 +2737,11 @@ static TraceParams batch_params(const TraceParams& p0) {
     return p;
 }
 
-// loop runs before a batch's loops give up (RG_BATCH_LOOP_LIMIT overrides, read when a graph is captured and
-// at every batch of the host loop; tests use a small limit to check the reported error)
-static uint32_t loop_limit(uint32_t runs) {
+// runs of the loops on a chunk before a batch gives up (RG_BATCH_LOOP_LIMIT overrides, read when a graph is
+// captured and at every batch of the host loop; tests use a small limit to check the reported error)
+static uint32_t loop_limit() {
     const char* env = getenv("RG_BATCH_LOOP_LIMIT");
-    return env ? (uint32_t)strtoul(env, nullptr, 10) : runs;
+    return env ? (uint32_t)strtoul(env, nullptr, 10) : 50000u;
 }
 
 cudaError_t launch_trace_batch(const TraceParams& p0, const TraceTune& tune, const SortScratch& sort, uint32_t* loopWords, cudaStream_t s,
@@ -2745,7 +2749,7 @@ cudaError_t launch_trace_batch(const TraceParams& p0, const TraceTune& tune, con
     const TraceParams p = batch_params(p0);
     BatchLaunch B;
     if (!B.init(p, tune, sort)) return cudaErrorInvalidValue;
-    const TreeLoop loop = {false, 0, 0, 0, loopWords, loop_limit(1u << 30), 0, 0, 0};
+    const TreeLoop loop = {false, 0, 0, 0, loopWords, loop_limit(), 0, 0, 0};
     auto poll = [&]() {
         cudaError_t e = cudaMemcpyAsync(hostWords, p.tree.ctl + kTreeMore, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -2812,9 +2816,8 @@ cudaError_t capture_trace_batch(const TraceParams& p0, const TraceTune& tune, co
     if (p.countVisits) return cudaErrorInvalidValue;  // the visit-counting build runs the host loop
     BatchLaunch B;
     if (!B.init(p, tune, sort)) return cudaErrorInvalidValue;
-    const uint32_t maxIter = loop_limit(50000u);
     const int R = p.batchRounds, more = std::max(1, R - 1);
-    TreeLoop loop = {true, 0, 0, 0, loopWords, maxIter, (uint32_t)(R * B.perRound() + 2 + R + 1), (uint32_t)(more * B.perRound() + 2),
+    TreeLoop loop = {true, 0, 0, 0, loopWords, loop_limit(), (uint32_t)(R * B.perRound() + 2 + R + 1), (uint32_t)(more * B.perRound() + 2),
                      (uint32_t)kTreeComposeRun + 1u};
     cudaStream_t s3 = nullptr;  // captures the inner loops' bodies
     cudaError_t e = cudaStreamCreateWithFlags(&s3, cudaStreamNonBlocking);

@@ -44,3 +44,17 @@ def test_host_loop_limit_is_reported(rg, glass, monkeypatch):
         for img, r in zip(br.render(), ref):
             assert np.array_equal(img, r)
     br.ctx.close()
+
+
+@pytest.mark.parametrize("host_loop", [False, True])
+def test_loop_limit_counts_a_chunk(rg, glass, monkeypatch, host_loop):
+    """The limit of the loops bounds the work on a chunk, not the number of chunks: a batch of hundreds of them passes
+    with a limit of 40 runs."""
+    scs, ref = glass
+    br = rg.BatchRenderer(scs, flags=rg.RG_FLAG_HOST_LOOP if host_loop else 0)
+    br.ctx.set_batch_slots(1024)
+    monkeypatch.setenv("RG_TREE_POOL", "4700")
+    monkeypatch.setenv("RG_BATCH_LOOP_LIMIT", "40")
+    for img, r in zip(br.render(), ref):
+        assert np.array_equal(img, r)
+    br.ctx.close()
