@@ -1187,6 +1187,7 @@ rg_status rg_trace_rays(rg_ctx* c, const float* rays, uint32_t n, float* tuv, ui
         float* r = static_cast<float*>(c->queryStage);
         float* t = r + 8ull * n;
         uint32_t* id = reinterpret_cast<uint32_t*>(t + 3ull * n);
+        CK(cudaStreamSynchronize(c->stream));  // the rays are read in stream order, as the copies read them
         std::memcpy(r, rays, 32ull * n);
         CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));  // rg_get_stats then reports this call's overflows
         TRY(enqueue_query(c, r, n, t, id, id + 2ull * n, false));
