@@ -490,8 +490,8 @@ rg_status ensure_tree_nodes(rg_ctx* c, size_t cap, RayTree& t) {
 // Frames of more than 2^25 samples go in chunks.  A pool that grew after a chunk had filled it is given
 // up again where memory does not allow it.
 rg_status ensure_tree(rg_ctx* c, size_t roots, size_t least, RayTree& t) {
-    // (RG_TREE_POOL overrides the pool's nodes; tests use a small pool to make chunks fill it)
-    if (const char* env = getenv("RG_TREE_POOL")) return ensure_tree_nodes(c, tree_pool_nodes(strtoull(env, nullptr, 10), 1, kTreePoolMin), t);
+    // (RG_TREE_POOL overrides the pool's nodes; tests use a small pool to make chunks and single samples fill it)
+    if (const char* env = getenv("RG_TREE_POOL")) return ensure_tree_nodes(c, tree_pool_nodes(strtoull(env, nullptr, 10), 1, 8), t);
     const rg_status st = ensure_tree_nodes(c, tree_pool_nodes(roots, c->treeNodes, least), t);
     if ((st != RG_ERR_BUDGET && st != RG_ERR_OUT_OF_MEMORY) || c->treeNodes == kTreeNodesMin) return st;
     if (st == RG_ERR_OUT_OF_MEMORY) cudaGetLastError();

@@ -237,7 +237,7 @@ struct RayTree {
 // lists; then the first node of every round, and a batch's words
 enum : int { kTreeAlloc = 0, kTreeChanges = 1, kTreeLevels = 2, kTreeTraced = 3, kTreeFetch = 4, kTreeCand = 7, kTreeBounds = 9 };
 constexpr uint32_t kTreeMaxNodes = 1u << 29;
-// a sample's GENERIC hits (at most 2^9 - 1 at 8 recursions) bound the checks that can change a ray
+// room for the rounds' bounds (a chunk that needs more goes again in parts, as one that filled the pool)
 constexpr int kTreeMaxRounds = 512 * 9;
 // of a batch: more rounds are needed, the chunk filled the pool, rounds run, a chunk is set up (polled together);
 // the chunk's roots and first work item, the candidate list in use, the round to trace next and the one
@@ -259,7 +259,7 @@ struct TreeLoop {
 // that fills the pool goes again in smaller chunks, and the next frame's pool is twice as large, up to
 // kTreeNodesMax a sample.
 constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 13;
-constexpr size_t kTreePoolMin = 4608;  // nodes: a sample's tree at 8 recursions, replaced rays included
+constexpr size_t kTreePoolMin = 4608;  // nodes of any pool: four times a sample's tree at 8 recursions without replaced rays
 constexpr size_t kTreePoolMax = kTreeMaxNodes - 4;  // links keep 29 bits for a node, three of their values for no node
 // nodes of the pool for `roots` samples; a pool at its bound holds fewer samples a chunk
 constexpr size_t tree_pool_nodes(size_t roots, size_t perRoot, size_t least) {

@@ -448,19 +448,21 @@ __device__ __forceinline__ void trav_step(Trav& T, const DevScene& sc, const STA
 // a BLAS path take at most 3 * 32 + 1 + 3 * 32 = 193 entries.  Should a push still find it full, the
 // ray is counted in counters[7] (rg_stats.deep_overflows), never silently.
 constexpr int kDeepStack = 196;  // 195 entries and the overflow flag
-__device__ __noinline__ void retrace_deep(const DevScene* sc, float4 o, float4 d, Hit* out, unsigned long long* counters) {
-    uint32_t mem[kDeepStack];
-    float world[6];
-    const LocalStackT<kDeepStack> st{mem, world};
+__device__ __forceinline__ Hit deep_hit(const DevScene& sc, float4 o, float4 d, const LocalStackT<kDeepStack>& st, unsigned long long* counters) {
     VisitCounts vc = {0, 0, 0};
     Trav T;
-    trav_begin(T, *sc, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, st);
-    while (T.active) trav_step<false>(T, *sc, st, vc);
+    trav_begin(T, sc, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, st);
+    while (T.active) trav_step<false>(T, sc, st, vc);
     if (st.over() && counters) {
         atomicAdd(counters + 7, 1ull);
         atomicAdd(counters + 15, 1ull);
     }
-    *out = T.h;
+    return T.h;
+}
+__device__ __noinline__ void retrace_deep(const DevScene* sc, float4 o, float4 d, Hit* out, unsigned long long* counters) {
+    uint32_t mem[kDeepStack];
+    float world[6];
+    *out = deep_hit(*sc, o, d, LocalStackT<kDeepStack>{mem, world}, counters);
 }
 
 template <bool COUNT, class STACK>
@@ -2221,6 +2223,47 @@ __global__ void __launch_bounds__(128) k_tree_compose(const __grid_constant__ Tr
     flush_counts(P, c, 4);
 }
 
+// The sample of root k depth first on one thread, as the megakernel runs it.  A chunk that fills the pool goes again in
+// parts, down to single samples; a sample whose tree, replaced rays included, exceeds the pool even then is
+// rendered this way, so no bound on the size of a tree has to hold.  (1013 nodes at 8 recursions without replacements; how
+// many nodes replacements can leave behind depends on the scene.)  Frames and stack lie in shared memory: local
+// memory is reserved for every thread that the chip can hold.
+struct DepthFirstMem {
+    Frame frames[kMaxFrames];
+    uint32_t stack[kDeepStack];
+    float world[6];
+};
+template <bool BATCH>
+__device__ __forceinline__ void sample_depth_first(const TraceParams& P, uint32_t k, DepthFirstMem& m) {
+    uint32_t job, sample;
+    Payload p;
+    RayReq ray;
+    if (!tree_root<BATCH>(P, k, job, sample, p, ray)) return;
+    const DevScene& sc = tree_scene<BATCH>(P, job);
+    const rg_ubo& u = tree_ubo<BATCH>(P, job);
+    RayCounts cnt = {1, 0, 0, 0};
+    Frame cur;
+    int fsp = 0;
+    Hit h;
+    do {
+        h.hit = false;  // a mask-0 trace meets nothing
+        if (!ray.masked)
+            h = deep_hit(sc, make_float4(ray.o.x, ray.o.y, ray.o.z, ray.tmin), make_float4(ray.d.x, ray.d.y, ray.d.z, ray.tmax),
+                         LocalStackT<kDeepStack>{m.stack, m.world}, P.counters);
+    } while (shade_step(sc, light_of(u), u.maxRecursions, h, p, ray, m.frames, fsp, cur, cnt));
+    store_sample(P.samples + 3 * (size_t)sample, p);
+    const uint32_t c[4] = {cnt.primary, cnt.shadow, cnt.secondary, cnt.masked};
+    for (int i = 0; i < 4; ++i) {
+        atomicAdd(P.counters + i, (unsigned long long)c[i]);
+        atomicAdd(P.counters + 8 + i, (unsigned long long)c[i]);
+    }
+}
+// the one sample of a frame's chunk
+__global__ void k_sample_depth_first(const __grid_constant__ TraceParams P) {
+    __shared__ DepthFirstMem m;
+    sample_depth_first<false>(P, 0, m);
+}
+
 // ---- chunks and loops of a batch, on the device -----------------------------------------------------
 // A batch goes through the same trees as a frame, its samples numbered job after job, in chunks that share
 // the node pool.  Its launches are captured once in a graph whose loops run on the device: over the chunks,
@@ -2238,11 +2281,15 @@ __global__ void k_tree_step(const __grid_constant__ TraceParams P, const TreeLoo
     bool full = nodes > P.tree.capacity;
     bool more = !full && (nodes > c[kTreeTraced] || c[kTreeChanges]);
     loop.words[0] += 1u;
-    if (more && (loop.words[0] >= loop.maxRuns || rounds + (uint32_t)P.batchRounds >= (uint32_t)kTreeMaxRounds)) {
+    if (more && loop.words[0] >= loop.maxRuns) {
         if (loop.graph) loop.words[1] = 1u;
         more = false;
         full = true;  // the chunk is not composed,
         c[kTreeRoots] = 0u;  // and no other follows
+    }
+    if (more && rounds + (uint32_t)P.batchRounds >= (uint32_t)kTreeMaxRounds) {  // no room for the rounds' bounds: as a full pool
+        more = false;
+        full = true;
     }
     if (more) c[kTreeCandList] ^= 1u;
     else loop.words[3] += rounds;
@@ -2268,22 +2315,28 @@ __global__ void k_tree_composed(const __grid_constant__ TraceParams P, const Tre
 }
 
 // the next chunk (first: of a launch); one that filled the pool goes again in eight parts, and so do the
-// samples after it.  kTreeLive: a chunk is set up (1), none is left (0), or the loops gave up (2)
+// samples after it (a single sample: depth first).  kTreeLive: a chunk is set up (1), none is left (0), or the loops gave up (2)
 __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoop loop, bool first) {
+    __shared__ DepthFirstMem m;
     uint32_t* c = P.tree.ctl;
+    const uint32_t whole = min(min(P.totalWork, P.slots), max(1u, P.tree.capacity / kTreeNodesMin));
     if (first) {
         loop.words[0] = loop.words[3] = 0u;
         c[kTreeBase] = c[kTreeRoots] = c[kTreeFull] = c[kTreeWasFull] = 0u;
-        c[kTreeChunk] = min(min(P.totalWork, P.slots), max(1u, P.tree.capacity / kTreeNodesMin));
+        c[kTreeChunk] = whole;
         c[kTreeFetch + 1] = c[kTreeFetch + 2] = 0u;
     }
     bool stop = false;
     const bool full = c[kTreeFull] != 0u;
-    if (full) {
-        c[kTreeWasFull] = 1u;
-        stop = c[kTreeRoots] <= 1u;  // stopped, or a sample's tree that is larger than the pool (none is)
+    if (full) c[kTreeWasFull] = 1u;
+    if (full && c[kTreeRoots] != 1u) {
+        stop = c[kTreeRoots] == 0u;  // the check gave up
         c[kTreeChunk] = (c[kTreeRoots] + 7u) / 8u;
     } else {
+        if (full) {
+            sample_depth_first<true>(P, 0, m);
+            c[kTreeChunk] = whole;
+        }
         c[kTreeBase] += c[kTreeRoots];
     }
     bool more = !stop && c[kTreeBase] < P.totalWork;
@@ -2295,7 +2348,7 @@ __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoo
         }
         // every chunk has the limit's runs for itself (a batch of many small chunks is no endless loop); the parts of a
         // chunk that filled the pool share them until one is done
-        if (!full) loop.words[0] = 0u;
+        if (!full || c[kTreeRoots] == 1u) loop.words[0] = 0u;
     }
     c[kTreeRoots] = more ? min(c[kTreeChunk], P.totalWork - c[kTreeBase]) : 0u;
     c[kTreeAlloc] = c[kTreeChanges] = c[kTreeLevels] = c[kTreeTraced] = c[kTreeFetch] = c[kTreeCand] = c[kTreeCand + 1] = 0u;
@@ -2572,7 +2625,7 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
         L.p.wf.overflow = L.p.tree.overflow;
     }
     // chunks of samples (first work item, samples) whose trees share the node pool; a chunk that fills it
-    // goes again in eight parts (one sample's tree, replaced rays included, is far smaller than any pool)
+    // goes again in eight parts, a single sample that does depth first
     std::vector<std::pair<uint32_t, uint32_t>> todo;
     auto split = [&](uint32_t base, uint32_t n, uint32_t m) {
         for (uint32_t b = (n - 1) / m * m + m; b; b -= m) todo.emplace_back(base + b - m, std::min(m, n - (b - m)));  // popped in order
@@ -2616,17 +2669,21 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
             if ((e = cudaStreamSynchronize(L.s)) != cudaSuccess) return e;
             const uint32_t* h = L.hostWords;
             const uint32_t nodes = L.p.treeRoots + h[kTreeAlloc];
-            if (nodes > L.p.tree.capacity) {
+            const bool pending = nodes > h[kTreeTraced], more = pending || h[kTreeChanges];
+            // from the shallowest new ray down
+            L.levels = pending && h[kTreeLevels] ? std::max(1, maxRec + 1 - (16 - (int)h[kTreeLevels])) : 1;
+            if (nodes > L.p.tree.capacity || (more && L.k + L.levels >= kTreeMaxRounds)) {
                 *poolFull = true;
-                if (L.p.treeRoots == 1) return cudaErrorUnknown;
-                split(L.p.treeBase, L.p.treeRoots, (L.p.treeRoots + 7) / 8);
+                if (L.p.treeRoots > 1) {
+                    split(L.p.treeBase, L.p.treeRoots, (L.p.treeRoots + 7) / 8);
+                } else {
+                    k_sample_depth_first<<<1, 1, 0, L.s>>>(L.p);
+                    count_launch();
+                    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                }
                 return start(L);
             }
-            const bool pending = nodes > h[kTreeTraced];
-            if (pending || h[kTreeChanges]) {
-                // from the shallowest new ray down
-                L.levels = pending && h[kTreeLevels] ? std::max(1, maxRec + 1 - (16 - (int)h[kTreeLevels])) : 1;
-                if (L.k + L.levels >= kTreeMaxRounds) return cudaErrorUnknown;
+            if (more) {
                 L.p.treeCand ^= 1u;
                 return rounds(L);
             }

@@ -58,3 +58,47 @@ def test_loop_limit_counts_a_chunk(rg, glass, monkeypatch, host_loop):
     for img, r in zip(br.render(), ref):
         assert np.array_equal(img, r)
     br.ctx.close()
+
+
+def dense_scene(width, height, spp, depth, seed):
+    """Large glass spheres through each other: 8 to 9 rays a sample on average, hundreds for some."""
+    sc = glass_scene(width, height, spp, depth, seed=seed, spheres=24)
+    p = sc.vertices["position"]
+    p[4:] = (p[4:] - p[4:].mean(0)) * np.float32(2.7) + p[4:].mean(0)
+    m = sc.materials[1:]
+    m["transparency"], m["reflectivity"], m["rayConsumption"] = 0.98, 0.9, 1
+    return sc
+
+
+@pytest.mark.parametrize("pool", [8, 40])
+def test_samples_larger_than_the_pool(rg, monkeypatch, pool):
+    """Samples whose trees no pool holds are rendered depth first: frames and both loop forms of a batch equal the
+    megakernel's images and ray counts."""
+    scs = [dense_scene(33, 17, 1, 8, 5), dense_scene(24, 16, 2, 6, 6), glass_scene(9, 7, 1, 0)]
+    ref = [render(rg, sc, flags=rg.RG_FLAG_MEGAKERNEL) for sc in scs]
+    count = ref[0][1]
+    assert sum(count.values()) - count["masked"] > 8 * count["primary"]  # so a tree of more than 8 nodes is among them
+    monkeypatch.setenv("RG_TREE_POOL", str(pool))
+    for sc, (want, st) in zip(scs, ref):
+        got, sg = render(rg, sc)
+        assert sg == st
+        for x, y in zip(got, want):
+            assert np.array_equal(x, y)
+    for flags in (0, rg.RG_FLAG_HOST_LOOP):
+        br = rg.BatchRenderer(scs, flags=flags)
+        for img, (want, _) in zip(br.render(), ref):
+            assert np.array_equal(img, want[0])
+        st = br.ctx.stats()
+        assert {k: st[k] for k in count} == {k: sum(s[k] for _, s in ref) for k in count}
+        br.ctx.close()
+
+
+def test_glossy_sample_larger_than_the_pool(rg, monkeypatch):
+    """The same with glossy reference shading, whose directions hang on the sample's seed."""
+    sc = dense_scene(24, 16, 1, 7, 5)
+    want, st = render(rg, sc, flags=rg.RG_FLAG_MEGAKERNEL, glossy=9)
+    monkeypatch.setenv("RG_TREE_POOL", "8")
+    got, sg = render(rg, sc, glossy=9)
+    assert sg == st
+    for x, y in zip(got, want):
+        assert np.array_equal(x, y)
