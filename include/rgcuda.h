@@ -338,10 +338,9 @@ rg_status rg_set_glossy(rg_ctx* ctx, uint32_t seed);
 /* Device memory the context holds (all scene slots, images, ray-tree nodes, scratch) and its budget
  * (rg_device_opts.hbm_budget_bytes, 0 = none), in bytes. */
 rg_status rg_get_memory(rg_ctx* ctx, uint64_t* allocated_bytes, uint64_t* budget_bytes);
-/* Samples of a batch in flight: its samples go through their ray trees in chunks of at most this many.
- * Default 2^25, 0.8 to 1.6 KB of device memory each (a batch of fewer samples takes one slot per
- * sample; at most 2^29 nodes of 112 bytes are held, so beyond 41 M slots a chunk may hold fewer samples).
- * Fewer slots mean more chunks of narrower rounds. */
+/* Slots of a batch: its samples go through their ray trees in chunks that share the slots' memory, 0.8 to 1.6 KB each;
+ * how many samples a chunk holds follows from the rays they need.  Default 2^25 (a batch of fewer samples takes one slot
+ * per sample; at most 2^29 nodes of 112 bytes are held).  Fewer slots mean more chunks of narrower rounds. */
 rg_status rg_set_batch_slots(rg_ctx* ctx, uint32_t slots);
 /* Autotuner of the batch loop: renders the batch once (warm-up, capture) and then `reps` times
  * with every launch shape of the grid threads {64,128,256} x stack depth {16,24,32,48} x sort key

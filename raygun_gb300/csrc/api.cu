@@ -121,7 +121,7 @@ struct rg_ctx {
     DevBuf bBase, bNormal, bRough, bFinal, bFxaa, batchFb;
     std::vector<size_t> batchOffset;           // per job: first pixel in batchFb
     std::vector<uint32_t> batchW, batchH;
-    uint32_t batchSlots = 1u << 25;            // samples of a batch's chunk (7 to 13 nodes of 112 bytes each: 49 GB at most)
+    uint32_t batchSlots = 1u << 25;            // slots of a batch's chunks (7 to 13 nodes of 112 bytes each: 49 GB at most)
     TraceTune tune;
     // graph form of the batch: second stream (loop body capture), instantiated graph and what it
     // was captured for, loop words (device), launch accounting
@@ -490,14 +490,14 @@ rg_status ensure_tree_nodes(rg_ctx* c, size_t cap, RayTree& t) {
 
 // Frames of more than 2^25 samples go in chunks.  A pool that grew after a chunk had filled it is given
 // up again where memory does not allow it.
-rg_status ensure_tree(rg_ctx* c, size_t roots, size_t least, RayTree& t) {
+rg_status ensure_tree(rg_ctx* c, size_t roots, uint32_t perRoot, RayTree& t) {
     // (RG_TREE_POOL overrides the pool's nodes; tests use a small pool to make chunks and single samples fill it)
     if (const char* env = getenv("RG_TREE_POOL")) return ensure_tree_nodes(c, tree_pool_nodes(strtoull(env, nullptr, 10), 1, 8), t);
-    const rg_status st = ensure_tree_nodes(c, tree_pool_nodes(roots, c->treeNodes, least), t);
-    if ((st != RG_ERR_BUDGET && st != RG_ERR_OUT_OF_MEMORY) || c->treeNodes == kTreeNodesMin) return st;
+    const rg_status st = ensure_tree_nodes(c, tree_pool_nodes(roots, perRoot, kTreePoolMin), t);
+    if ((st != RG_ERR_BUDGET && st != RG_ERR_OUT_OF_MEMORY) || perRoot == kTreeNodesMin) return st;
     if (st == RG_ERR_OUT_OF_MEMORY) cudaGetLastError();
     c->treeNodes = kTreeNodesMin;
-    return ensure_tree_nodes(c, tree_pool_nodes(roots, kTreeNodesMin, least), t);
+    return ensure_tree_nodes(c, tree_pool_nodes(roots, kTreeNodesMin, kTreePoolMin), t);
 }
 
 }  // namespace
@@ -857,7 +857,7 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     tp.workCounter = c->workCounter.as<uint32_t>();
     tp.glossySeed = c->glossySeed;
     c->lastSamples = (uint32_t)ubo->numSamples;
-    if (!mega) TRY(ensure_tree(c, std::min<size_t>(frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), 1u << 25), kTreePoolMin, tp.tree));
+    if (!mega) TRY(ensure_tree(c, std::min<size_t>(frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), 1u << 25), c->treeNodes, tp.tree));
     CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
     FrameEvents* fe;
     TRY(cur_events(c, &fe));
@@ -1485,7 +1485,7 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
     const uint32_t slots = (uint32_t)std::min<uint64_t>(work, c->batchSlots);
     TraceParams tp;
     std::memset(&tp, 0, sizeof(tp));
-    TRY(ensure_tree(c, slots, kTreePoolMin, tp.tree));
+    TRY(ensure_tree(c, slots, slots < work && slots <= kTreeFewSlots ? kTreeNodesMax : c->treeNodes, tp.tree));
     TRY(ensure(c, c->samples, 48ull * samples));
     TRY(ensure(c, c->jobTable, sizeof(JobDesc) * n));
     SortScratch sort{};

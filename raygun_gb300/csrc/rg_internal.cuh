@@ -257,8 +257,10 @@ struct TreeLoop {
 };
 // Pool size: nodes per sample.  The benchmark scenes trace 2.5 to 4 rays a sample; a chunk of samples
 // that fills the pool goes again in smaller chunks, and the next frame's pool is twice as large, up to
-// kTreeNodesMax a sample.
+// kTreeNodesMax a sample (no more than the paths of one ray at a time took, 1.6 KB a sample).
 constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 13;
+// a batch of more samples than slots takes kTreeNodesMax a slot at once up to here (1.5 GB): its chunks are fewer
+constexpr uint32_t kTreeFewSlots = 1u << 20;
 constexpr size_t kTreePoolMin = 4608;  // nodes of any pool: four times a sample's tree at 8 recursions without replaced rays
 constexpr size_t kTreePoolMax = kTreeMaxNodes - 4;  // links keep 29 bits for a node, three of their values for no node
 // nodes of the pool for `roots` samples; a pool at its bound holds fewer samples a chunk

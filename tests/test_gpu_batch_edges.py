@@ -102,3 +102,18 @@ def test_glossy_sample_larger_than_the_pool(rg, monkeypatch):
     assert sg == st
     for x, y in zip(got, want):
         assert np.array_equal(x, y)
+
+
+def test_chunks_grow_again(rg):
+    """A batch with few slots: chunks shrink where samples need many rays and grow again behind them (the rounds of all chunks
+    stay below those of chunks of one sample a slot)."""
+    from raygun_gb300 import scenes as S
+    scs = [dense_scene(64, 64, 1, 8, 5), S.spheres_scene(n_spheres=8, width=640, height=360, num_samples=1, max_recursions=2, seed=3)]
+    ref = [render(rg, sc)[0][0] for sc in scs]
+    br = rg.BatchRenderer(scs)
+    br.ctx.set_batch_slots(1024)
+    for img, r in zip(br.render(), ref):
+        assert np.array_equal(img, r)
+    # 9 rounds a chunk, and 9 for each of up to 8 repetitions in the dense job's
+    assert br.ctx.stats()["iterations"] <= 9 * (640 * 360 // 1024) + 9 * 9 * (64 * 64 // 64)
+    br.ctx.close()
