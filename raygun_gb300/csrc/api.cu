@@ -114,6 +114,8 @@ struct rg_ctx {
     // ray trees of the frames: node pool (its nodes per sample grow when a frame filled it)
     DevBuf trO, trD, trState, trHit, trInst, trSurf, trLink, trOver, trCand, trCtl;
     uint32_t treeNodes = kTreeNodesMin;
+    size_t treeRefused = SIZE_MAX, treeRefusedAt = 0;  // nodes that memory did not allow; what the context held then
+    TreeLoad treeLoad;  // of the last frame
     uint32_t* hostCount = nullptr;             // pinned words for polling the queue length and work counter
     int lastIterations = 0;
     // batch rendering: job table, ray-sort scratch, per-job images
@@ -285,7 +287,7 @@ rg_status settle_graph(rg_ctx* c) {
     count_launch(c->hostCount[6] - c->kernelsSeen);
     c->kernelsSeen = c->hostCount[6];
     c->lastIterations = (int)c->hostCount[7];
-    if (c->hostCount[8] && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
+    if (c->hostCount[8]) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMost);
     if (c->hostCount[5]) {
         CK(cudaMemsetAsync(c->loopWords.as<uint32_t>() + 1, 0, sizeof(uint32_t), c->stream));
         return fail(c, RG_ERR_CUDA, kLoopLimitError);
@@ -488,16 +490,28 @@ rg_status ensure_tree_nodes(rg_ctx* c, size_t cap, RayTree& t) {
     return RG_OK;
 }
 
-// Frames of more than 2^25 samples go in chunks.  A pool that grew after a chunk had filled it is given
-// up again where memory does not allow it.
+// nodes a sample that a pool for `roots` samples may have
+uint32_t tree_nodes_most(const rg_ctx* c, size_t roots) {
+    if (c->budget) return kTreeNodesMax;
+    return (uint32_t)std::min<size_t>(kTreeNodesMost, std::max<size_t>(kTreeNodesMax, kTreeGrowNodes / roots));
+}
+
+// Frames of more than 2^25 samples go in chunks.  A pool of more nodes than the least is given up again where memory
+// does not allow it, and not asked for again until the context holds less.
 rg_status ensure_tree(rg_ctx* c, size_t roots, uint32_t perRoot, RayTree& t) {
     // (RG_TREE_POOL overrides the pool's nodes; tests use a small pool to make chunks and single samples fill it)
     if (const char* env = getenv("RG_TREE_POOL")) return ensure_tree_nodes(c, tree_pool_nodes(strtoull(env, nullptr, 10), 1, 8), t);
-    const rg_status st = ensure_tree_nodes(c, tree_pool_nodes(roots, perRoot, kTreePoolMin), t);
-    if ((st != RG_ERR_BUDGET && st != RG_ERR_OUT_OF_MEMORY) || perRoot == kTreeNodesMin) return st;
+    perRoot = std::min(perRoot, tree_nodes_most(c, roots));
+    const size_t want = tree_pool_nodes(roots, perRoot, kTreePoolMin), least = tree_pool_nodes(roots, kTreeNodesMin, kTreePoolMin);
+    if (c->allocated < c->treeRefusedAt) c->treeRefused = SIZE_MAX;
+    if (want == least || want >= c->treeRefused) return ensure_tree_nodes(c, least, t);
+    const rg_status st = ensure_tree_nodes(c, want, t);
+    if (st != RG_ERR_BUDGET && st != RG_ERR_OUT_OF_MEMORY) return st;
     if (st == RG_ERR_OUT_OF_MEMORY) cudaGetLastError();
-    c->treeNodes = kTreeNodesMin;
-    return ensure_tree_nodes(c, tree_pool_nodes(roots, kTreeNodesMin, kTreePoolMin), t);
+    c->treeRefused = want;
+    const rg_status st2 = ensure_tree_nodes(c, least, t);
+    c->treeRefusedAt = c->allocated;
+    return st2;
 }
 
 }  // namespace
@@ -857,7 +871,8 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
     tp.workCounter = c->workCounter.as<uint32_t>();
     tp.glossySeed = c->glossySeed;
     c->lastSamples = (uint32_t)ubo->numSamples;
-    if (!mega) TRY(ensure_tree(c, std::min<size_t>(frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), 1u << 25), c->treeNodes, tp.tree));
+    const size_t roots = std::min<size_t>(frame_work_items(c->W, c->H, (uint32_t)ubo->numSamples), 1u << 25);
+    if (!mega) TRY(ensure_tree(c, roots, c->treeNodes, tp.tree));
     CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
     FrameEvents* fe;
     TRY(cur_events(c, &fe));
@@ -866,12 +881,19 @@ rg_status rg_render(rg_ctx* c, const rg_ubo* ubo, int32_t fxaa) {
         c->lastIterations = 0;
         CK(launch_trace(tp, c->stream));
     } else {
-        bool full = false;
         const bool timed = (c->flags & RG_FLAG_KERNEL_TIMING) != 0;
-        const TreeLane second = {c->stream2, c->laneEvent[0], c->laneEvent[1], tp.tree.ctl + kTreeCtlWords, c->hostCount + 12};
-        CK(launch_trace_tree(tp, c->stream, second, c->hostCount, &c->lastIterations, &full, timed ? next_kernel_events : nullptr,
-                             timed ? fe : nullptr));
-        if (full && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
+        for (bool grown = true;;) {
+            const TreeLane second = {c->stream2, c->laneEvent[0], c->laneEvent[1], tp.tree.ctl + kTreeCtlWords, c->hostCount + 12};
+            const uint32_t most = tree_nodes_most(c, roots);
+            CK(launch_trace_tree(tp, c->stream, second, c->hostCount, &c->lastIterations, &c->treeLoad, grown && c->treeNodes < most,
+                                 timed ? next_kernel_events : nullptr, timed ? fe : nullptr));
+            if (c->treeLoad.full) c->treeNodes = std::min((c->treeLoad.again ? 4 : 2) * c->treeNodes, most);
+            if (!c->treeLoad.again) break;
+            const uint32_t before = tp.tree.capacity;
+            TRY(ensure_tree(c, roots, c->treeNodes, tp.tree));
+            grown = tp.tree.capacity > before;
+            CK(cudaMemsetAsync(c->counters.p, 0, 64, c->stream));
+        }
     }
     return run_post(c, ubo, fxaa);
 }
@@ -1541,7 +1563,7 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
                                                  &full, timed ? next_kernel_events : nullptr, timed ? fe : nullptr);
         if (e == cudaErrorLaunchTimeout) return fail(c, RG_ERR_CUDA, kLoopLimitError);
         CK(e);
-        if (full && c->treeNodes < kTreeNodesMax) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMax);
+        if (full) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMost);
         CK(cudaEventRecord(fe->ev[EV_POST0], c->stream));
         CK(enqueue_batch_posts(c, jd.data(), jobs, n));
     } else {

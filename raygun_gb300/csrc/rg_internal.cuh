@@ -15,6 +15,7 @@
 #include <atomic>
 
 #include "../../include/rgcuda.h"
+#include "tree_plan.h"
 
 namespace rg {
 
@@ -256,9 +257,11 @@ struct TreeLoop {
     uint32_t maxRuns, chunkKernels, roundKernels, composeKernels;
 };
 // Pool size: nodes per sample.  The benchmark scenes trace 2.5 to 4 rays a sample; a chunk of samples
-// that fills the pool goes again in smaller chunks, and the next frame's pool is twice as large, up to
-// kTreeNodesMax a sample (no more than the paths of one ray at a time took, 1.6 KB a sample).
-constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 13;
+// that fills the pool goes again in smaller chunks, and the next pool is larger, up to kTreeNodesMax a sample (no more
+// than the paths of one ray at a time took, 1.6 KB a sample).  Without a memory budget a pool of up to kTreeGrowNodes
+// (1.9 GB) grows to kTreeNodesMost a sample: a chunk more costs a small frame as much as all of its samples.
+constexpr uint32_t kTreeNodesMin = 7, kTreeNodesMax = 13, kTreeNodesMost = 64;
+constexpr size_t kTreeGrowNodes = 1u << 24;
 // a batch of more samples than slots takes kTreeNodesMax a slot at once up to here (1.5 GB): its chunks are fewer
 constexpr uint32_t kTreeFewSlots = 1u << 20;
 constexpr size_t kTreePoolMin = 4608;  // nodes of any pool: four times a sample's tree at 8 recursions without replaced rays
@@ -336,9 +339,10 @@ struct TreeLane {
     uint32_t *ctl, *hostWords;
 };
 // a frame through ray trees, and its resolve.  hostWords: four pinned words polled after each check;
-// iterations: rounds run; *poolFull: a chunk of samples filled the node pool
-cudaError_t launch_trace_tree(const TraceParams& p, cudaStream_t s, const TreeLane& second, uint32_t* hostWords, int* iterations, bool* poolFull,
-                              EventPairFn kernelEvents = nullptr, void* user = nullptr);
+// iterations: rounds run; load: of the last frame, then of this one; mayGrow: a frame of one chunk that fills the
+// pool is left undone (load->again)
+cudaError_t launch_trace_tree(const TraceParams& p, cudaStream_t s, const TreeLane& second, uint32_t* hostWords, int* iterations, TreeLoad* load,
+                              bool mayGrow, EventPairFn kernelEvents = nullptr, void* user = nullptr);
 // traversal launch shape of the batch loop: block size {64,128,256}, stack entries {16,24,32,48},
 // ray-sort key applied to each queue before it is traced
 struct TraceTune {

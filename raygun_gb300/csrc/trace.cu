@@ -2607,8 +2607,8 @@ static RayTree tree_part(const RayTree& t, size_t at, uint32_t n, uint32_t* ctl)
 // lane has the chip.  2.75 M samples (1279x717, 3 a pixel) 3.07 -> 2.89 ms, 8.3 M 18.24 -> 17.93 ms, 0.92 M 1808 ->
 // 1806 us, 0.23 M 968 -> 1000 us (its rounds no longer fill the chip).
 constexpr uint32_t kTwoLanes = 1u << 20;
-cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeLane& second, uint32_t* hostWords, int* iterations, bool* poolFull,
-                              EventPairFn kernelEvents, void* user) {
+cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeLane& second, uint32_t* hostWords, int* iterations, TreeLoad* load,
+                              bool mayGrow, EventPairFn kernelEvents, void* user) {
     const TraceKernel trace = trace_kernel(false, p0.countVisits != 0, kTraceThreads, kTraversalStack);
     // glossy reference shading has kernels of its own; the reference's shading keeps the lean ones
     const auto expand = p0.glossySeed ? k_tree_expand<false, true> : k_tree_expand<false, false>;
@@ -2619,7 +2619,6 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
     const int maxRec = p0.ubo.maxRecursions;
     const uint32_t work = (uint32_t)frame_work_items(p0.W, p0.H, (uint32_t)p0.ubo.numSamples), cap = p0.tree.capacity;
     int it = 0;
-    *poolFull = false;
     const int lanes = work >= kTwoLanes && !kernelEvents ? 2 : 1;
     FrameLane lane[2];
     for (int l = 0; l < lanes; ++l) {
@@ -2631,14 +2630,10 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
         L.p.wf.counts = L.p.tree.ctl + kTreeFetch - 2;  // the traversal kernel's work counter, overflow list length and finished blocks
         L.p.wf.overflow = L.p.tree.overflow;
     }
-    // chunks of samples (first work item, samples) whose trees share the node pool; a chunk that fills it
-    // goes again in eight parts, a single sample that does depth first
-    std::vector<std::pair<uint32_t, uint32_t>> todo;
-    auto split = [&](uint32_t base, uint32_t n, uint32_t m) {
-        for (uint32_t b = (n - 1) / m * m + m; b; b -= m) todo.emplace_back(base + b - m, std::min(m, n - (b - m)));  // popped in order
-    };
-    const uint32_t part = (work / lanes + 31) / 32 * 32;
-    split(0, work, std::max(1u, std::min(part, lane[0].p.tree.capacity / kTreeNodesMin)));
+    const uint32_t pool = lane[0].p.tree.capacity;
+    ChunkPlan plan(work, (uint32_t)lanes, pool, pool / kTreeNodesMin, std::move(*load));
+    *load = TreeLoad();
+    bool again = false;
     // rounds of a lane, its check and the words that decide what comes next
     auto rounds = [&](FrameLane& L) -> cudaError_t {
         cudaError_t e;
@@ -2658,11 +2653,8 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
         return cudaMemcpyAsync(L.hostWords, L.p.tree.ctl, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, L.s);
     };
     auto start = [&](FrameLane& L) -> cudaError_t {  // the next chunk
-        L.busy = !todo.empty();
+        L.busy = plan.next(L.p.treeBase, L.p.treeRoots);
         if (!L.busy) return cudaSuccess;
-        L.p.treeBase = todo.back().first;
-        L.p.treeRoots = todo.back().second;
-        todo.pop_back();
         L.p.treeCand = 0;
         L.k = 0;
         L.levels = maxRec + 1;
@@ -2680,10 +2672,15 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
             // from the shallowest new ray down
             L.levels = pending && h[kTreeLevels] ? std::max(1, maxRec + 1 - (16 - (int)h[kTreeLevels])) : 1;
             if (nodes > L.p.tree.capacity || (more && L.k + L.levels >= kTreeMaxRounds)) {
-                *poolFull = true;
-                if (L.p.treeRoots > 1) {
-                    split(L.p.treeBase, L.p.treeRoots, (L.p.treeRoots + 7) / 8);
+                if (mayGrow && L.p.treeRoots == work) {  // nothing is composed yet
+                    again = true;
+                    L.busy = false;
+                    return cudaSuccess;
+                }
+                if (L.p.treeRoots > 1) {  // in parts
+                    plan.filled(L.p.treeBase, L.p.treeRoots);
                 } else {
+                    plan.done(L.p.treeBase, 1u, nodes);
                     k_sample_depth_first<<<1, 1, 0, L.s>>>(L.p);
                     count_launch();
                     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -2694,6 +2691,7 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
                 L.p.treeCand ^= 1u;
                 return rounds(L);
             }
+            plan.done(L.p.treeBase, L.p.treeRoots, nodes);
         }
         count_launch(L.k);
         while (L.k--)
@@ -2722,7 +2720,12 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
         if (lanes == 2) cudaStreamSynchronize(second.stream);  // nothing of the frame runs on behind its stream's back
         return e;
     }
+    if (again) {
+        load->full = load->again = true;
+        return cudaSuccess;
+    }
     if (iterations) *iterations = it;
+    *load = plan.load();
     dim3 grid((p0.W + 31) / 32, (p0.H + 7) / 8);
     launch_chain(k_resolve, grid, 256, 0, s, p0);
     count_launch();

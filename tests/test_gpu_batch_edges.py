@@ -117,3 +117,21 @@ def test_chunks_grow_again(rg):
     # 9 rounds a chunk, and 9 for each of up to 8 repetitions in the dense job's
     assert br.ctx.stats()["iterations"] <= 9 * (640 * 360 // 1024) + 9 * 9 * (64 * 64 // 64)
     br.ctx.close()
+
+
+@pytest.mark.parametrize("w,h,spp,swell,budget,rounds", [(160, 90, 1, 1.5, 0, 60), (160, 90, 1, 1.5, 1 << 30, 60), (1283, 409, 2, 2.5, 0, 250)])
+def test_frames_of_many_rays_a_sample(rg, w, h, spp, swell, budget, rounds):
+    """Frames with more nodes than the pool holds: images as the megakernel's from the first on, and later frames in few chunks
+    that fit (9 rounds a chunk and those of replaced rays; 131, 131 and 371 rounds with a pool filled in vain first)."""
+    sc = dense_scene(w, h, spp, 8, 5)
+    p = sc.vertices["position"]
+    p[4:] = (p[4:] - p[4:].mean(0)) * np.float32(swell) + p[4:].mean(0)
+    (want, *_), st = render(rg, sc, flags=rg.RG_FLAG_MEGAKERNEL)
+    assert sum(st.values()) - st["masked"] > 7 * st["primary"]  # so the first pool is too small
+    rt = rg.Raytracer(sc, hbm_budget_bytes=budget).prepare()
+    for k in range(4):
+        assert np.array_equal(rt.render(), want)
+        got = rt.ctx.stats()
+        assert {x: got[x] for x in st} == st
+    assert got["iterations"] <= rounds
+    rt.ctx.close()
