@@ -287,7 +287,7 @@ rg_status settle_graph(rg_ctx* c) {
     count_launch(c->hostCount[6] - c->kernelsSeen);
     c->kernelsSeen = c->hostCount[6];
     c->lastIterations = (int)c->hostCount[7];
-    if (c->hostCount[8]) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMost);
+    if (c->hostCount[8]) c->treeNodes = std::min(4 * c->treeNodes, kTreeNodesMost);
     if (c->hostCount[5]) {
         CK(cudaMemsetAsync(c->loopWords.as<uint32_t>() + 1, 0, sizeof(uint32_t), c->stream));
         return fail(c, RG_ERR_CUDA, kLoopLimitError);
@@ -474,7 +474,10 @@ rg_status ensure_tree_nodes(rg_ctx* c, size_t cap, RayTree& t) {
     TRY(ensure(c, c->trLink, 16 * cap));
     TRY(ensure(c, c->trOver, 4 * cap));
     TRY(ensure(c, c->trCand, 8 * cap));
-    TRY(ensure(c, c->trCtl, 2 * kTreeCtlWords * sizeof(uint32_t)));  // a frame's two lanes
+    if (!c->trCtl.p) {  // a frame's two lanes; the words that launches keep start as of no batch
+        TRY(ensure(c, c->trCtl, 2 * kTreeCtlWords * sizeof(uint32_t)));
+        CK(cudaMemsetAsync(c->trCtl.p, 0, 2 * kTreeCtlWords * sizeof(uint32_t), c->stream));
+    }
     t.rayO = c->trO.as<float4>();
     t.rayD = c->trD.as<float4>();
     t.state = c->trState.as<uint4>();
@@ -1563,7 +1566,7 @@ rg_status rg_render_batch(rg_ctx* c, const rg_job* jobs, uint32_t n) {
                                                  &full, timed ? next_kernel_events : nullptr, timed ? fe : nullptr);
         if (e == cudaErrorLaunchTimeout) return fail(c, RG_ERR_CUDA, kLoopLimitError);
         CK(e);
-        if (full) c->treeNodes = std::min(2 * c->treeNodes, kTreeNodesMost);
+        if (full) c->treeNodes = std::min(4 * c->treeNodes, kTreeNodesMost);
         CK(cudaEventRecord(fe->ev[EV_POST0], c->stream));
         CK(enqueue_batch_posts(c, jd.data(), jobs, n));
     } else {

@@ -242,10 +242,13 @@ constexpr uint32_t kTreeMaxNodes = 1u << 29;
 constexpr int kTreeMaxRounds = 512 * 9;
 // of a batch: more rounds are needed, the chunk filled the pool, rounds run, a chunk is set up (polled together);
 // the chunk's roots and first work item, the candidate list in use, the round to trace next and the one
-// traced last, samples a chunk, and whether any chunk filled the pool
+// traced last, samples a chunk, whether any chunk filled the pool, chunks done, their nodes (float); kept from launch to
+// launch: the chunks of the last one (as many as there is room for; their samples), its nodes, and the batch's samples, the
+// pool's nodes and the slots that they hold for
 enum : int {
     kTreeMore = kTreeBounds + kTreeMaxRounds + 1, kTreeFull, kTreeTop, kTreeLive, kTreeRoots, kTreeBase, kTreeCandList, kTreeRound,
-    kTreeTracedRound, kTreeChunk, kTreeWasFull, kTreeCtlWords
+    kTreeTracedRound, kTreeChunk, kTreeWasFull, kTreeDone, kTreeNodes, kTreeFollow, kTreePlanned, kTreePlanNodes, kTreePlanOf,
+    kTreePlan = kTreePlanOf + 3, kTreeCtlWords = kTreePlan + 16
 };
 constexpr int kTreeComposeRun = 4;  // rounds composed per run of that loop
 // loops of a batch's graph: their conditions; words: runs of the loops on this chunk (at most maxRuns), sticky limit

@@ -2318,33 +2318,53 @@ __global__ void k_tree_composed(const __grid_constant__ TraceParams P, const Tre
 // A chunk has a fixed cost (its launches and loop runs, 0.1 to 0.8 ms), so with fewer slots than samples the next one holds
 // as many as the last one's nodes a sample let expect, at most twice as many as it: 4.1 M samples at 1024
 // slots 165 ms against 1873 ms with chunks of `slots` samples that stayed at an eighth after a full one, 10 M mixed ones at
-// 4096 slots 118 against 1158 ms.  kTreeLive: a chunk is set up (1), none is left (0), or the loops gave up (2)
+// 4096 slots 118 against 1158 ms.  A launch of few chunks leaves their sizes to the next one of the same batch size,
+// which then fills no pool in vain.  kTreeLive: a chunk is set up (1), none is left (0), or the loops gave up (2)
 __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoop loop, bool first) {
     __shared__ DepthFirstMem m;
+    constexpr uint32_t kPlan = kTreeCtlWords - kTreePlan;
     uint32_t* c = P.tree.ctl;
     const uint32_t whole = min(min(P.totalWork, P.slots), max(1u, P.tree.capacity / kTreeNodesMin));
     if (first) {
         loop.words[0] = loop.words[3] = 0u;
-        c[kTreeBase] = c[kTreeRoots] = c[kTreeFull] = c[kTreeWasFull] = 0u;
-        c[kTreeChunk] = whole;
+        c[kTreeBase] = c[kTreeRoots] = c[kTreeFull] = c[kTreeWasFull] = c[kTreeDone] = c[kTreeNodes] = 0u;
+        const bool follow = c[kTreePlanned] && c[kTreePlanOf] == P.totalWork && c[kTreePlanOf + 1] == P.tree.capacity && c[kTreePlanOf + 2] == P.slots;
+        c[kTreeFollow] = follow;
+        if (!follow) c[kTreePlanned] = 0u;
+        c[kTreeChunk] = follow ? c[kTreePlan] : whole;
         c[kTreeFetch + 1] = c[kTreeFetch + 2] = 0u;
     }
     bool stop = false;
     const bool full = c[kTreeFull] != 0u;
-    if (full && c[kTreeRoots] <= whole) c[kTreeWasFull] = 1u;  // (more samples than the pool is meant for: no larger pool)
-    if (full && c[kTreeRoots] != 1u) {
-        stop = c[kTreeRoots] == 0u;  // the check gave up
-        c[kTreeChunk] = (c[kTreeRoots] + 1u) / 2u;
-    } else {
-        const uint32_t roots = c[kTreeRoots];
+    const uint32_t roots = c[kTreeRoots];
+    if (full && roots <= whole) c[kTreeWasFull] = 1u;  // (more samples than the pool is meant for: no larger pool)
+    if (full && roots != 1u) {
+        stop = roots == 0u;  // the check gave up
+        c[kTreeChunk] = (roots + 1u) / 2u;
+        c[kTreeFollow] = c[kTreePlanned] = 0u;
+    } else if (roots) {
+        const uint32_t nodes = roots + c[kTreeAlloc], done = c[kTreeDone] + 1u;
+        const float all = __uint_as_float(c[kTreeNodes]) + (float)nodes;
         if (full) {
             sample_depth_first<true>(P, 0, m);
             c[kTreeChunk] = whole;
-        } else if (roots) {  // samples that fill 7/8 of the pool if they are like these
-            const unsigned long long fit = (unsigned long long)(P.tree.capacity - P.tree.capacity / 8u) * roots / (roots + c[kTreeAlloc]);
+        } else {  // samples that fill 7/8 of the pool if they are like these
+            const unsigned long long fit = (unsigned long long)(P.tree.capacity - P.tree.capacity / 8u) * roots / nodes;
             c[kTreeChunk] = (uint32_t)max(1ull, min(fit, 2ull * roots));
         }
+        if (done <= kPlan) c[kTreePlan + done - 1u] = roots;  // (that place of the last plan is done with)
+        if (c[kTreeFollow] && done < c[kTreePlanned]) c[kTreeChunk] = c[kTreePlan + done];
         c[kTreeBase] += roots;
+        c[kTreeDone] = done;
+        c[kTreeNodes] = __float_as_uint(all);
+        if (c[kTreeBase] >= P.totalWork) {  // the plan of the next launch, unless the rays got far fewer under it
+            const bool fewer = c[kTreeFollow] && all < 0.5f * __uint_as_float(c[kTreePlanNodes]);
+            if (!c[kTreeFollow]) c[kTreePlanNodes] = __float_as_uint(all);
+            c[kTreePlanned] = done <= kPlan && !fewer ? done : 0u;
+            c[kTreePlanOf] = P.totalWork;
+            c[kTreePlanOf + 1] = P.tree.capacity;
+            c[kTreePlanOf + 2] = P.slots;
+        }
     }
     bool more = !stop && c[kTreeBase] < P.totalWork;
     if (!first) {
@@ -2355,9 +2375,9 @@ __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoo
         }
         // every chunk has the limit's runs for itself (a batch of many small chunks is no endless loop); the parts of a
         // chunk that filled the pool share them until one is done
-        if (!full || c[kTreeRoots] == 1u) loop.words[0] = 0u;
+        if (!full || roots == 1u) loop.words[0] = 0u;
     }
-    c[kTreeRoots] = more ? min(c[kTreeChunk], P.totalWork - c[kTreeBase]) : 0u;
+    c[kTreeRoots] = more ? min(min(c[kTreeChunk], P.tree.capacity), P.totalWork - c[kTreeBase]) : 0u;
     c[kTreeAlloc] = c[kTreeChanges] = c[kTreeLevels] = c[kTreeTraced] = c[kTreeFetch] = c[kTreeCand] = c[kTreeCand + 1] = 0u;
     c[kTreeCandList] = c[kTreeRound] = c[kTreeFull] = 0u;
     c[kTreeLive] = more ? 1u : stop ? 2u : 0u;

@@ -135,3 +135,24 @@ def test_frames_of_many_rays_a_sample(rg, w, h, spp, swell, budget, rounds):
         assert {x: got[x] for x in st} == st
     assert got["iterations"] <= rounds
     rt.ctx.close()
+
+
+@pytest.mark.parametrize("host_loop", [False, True])
+@pytest.mark.parametrize("budget", [0, 1 << 30])
+def test_batches_of_many_rays_a_sample(rg, budget, host_loop):
+    """The same for a batch, whose later launches take the chunks that fit in the last one; then a batch of as many samples
+    and far fewer rays through the same context."""
+    sc = dense_scene(160, 90, 1, 8, 5)
+    p = sc.vertices["position"]
+    p[4:] = (p[4:] - p[4:].mean(0)) * np.float32(1.5) + p[4:].mean(0)
+    light = glass_scene(160, 90, 1, 8, seed=2, spheres=1)
+    want = [render(rg, s)[0][0] for s in (sc, light)]
+    br = rg.BatchRenderer([sc, light], flags=rg.RG_FLAG_HOST_LOOP if host_loop else 0, hbm_budget_bytes=budget)
+    jobs = br.jobs()
+    for k in (0, 0, 0, 0, 1, 1, 0):
+        assert np.array_equal(br.render(jobs[k:k + 1])[0], want[k])
+        its = br.ctx.stats()["iterations"]
+        if k == 0:
+            last = its
+    assert last <= 60
+    br.ctx.close()
