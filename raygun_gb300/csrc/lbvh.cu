@@ -11,7 +11,6 @@
 // Refit keeps the topology and recomputes the boxes in a climb of its own.
 #include <cooperative_groups.h>
 
-#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 
@@ -612,10 +611,12 @@ __device__ __forceinline__ bool box_there(const uint32_t* b) {
     return there;
 }
 
+// LEAVES: every box of another block's node is taken from the leaves (tests; a limit passed at run time cost 0.4 us)
+template <bool LEAVES>
 __global__ void __launch_bounds__(kHierLeaves) k_hierarchy(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ order,
                                                            const float* __restrict__ primBoxes, uint32_t n, uint32_t* __restrict__ left,
                                                            uint32_t* __restrict__ right, uint32_t* __restrict__ parents,
-                                                           uint32_t* arrivals, float* nodeBoxes, int polls) {
+                                                           uint32_t* arrivals, float* nodeBoxes) {
     chain_wait();
     __shared__ uint32_t sKeys[kHierLeaves + 2];      // leaves first - 1 .. first + kHierLeaves
     __shared__ uint32_t sArrive[kHierLeaves];        // by split
@@ -689,12 +690,12 @@ __global__ void __launch_bounds__(kHierLeaves) k_hierarchy(const uint32_t* __res
 #pragma unroll
             for (int a = 0; a < 6; ++a) ob[a] = __float_as_uint(b[a]);
         } else {
-            for (int i = 0; i < polls && !box_there(ob); ++i) load_box_relaxed(nodeBoxes + 6 * (size_t)sibNode, ob);
-            if (polls == 0 || !box_there(ob)) {
-                const uint32_t i0 = isLeft ? s + 1 : far, i1 = isLeft ? far : s;  // two leaves at least
-                float u[6];
-                for (int a = 0; a < 6; ++a) u[a] = primBoxes[6 * (size_t)order[i0] + a];
-                for (uint32_t i = i0 + 1; i <= i1; ++i) {
+            for (int i = 0; !LEAVES && i < kHierPolls && !box_there(ob); ++i) load_box_relaxed(nodeBoxes + 6 * (size_t)sibNode, ob);
+            if (LEAVES || !box_there(ob)) {
+                const float none = __uint_as_float(0x7FFFFFFFu);  // passed over, and what a union of NaN boxes is
+                float u[6] = {none, none, none, none, none, none};
+                const uint32_t i0 = isLeft ? s + 1 : far, i1 = isLeft ? far : s;
+                for (uint32_t i = i0; i <= i1; ++i) {
                     const float* b = primBoxes + 6 * (size_t)order[i];
                     for (int a = 0; a < 3; ++a) {
                         u[a] = fminf(u[a], b[a]);
@@ -2124,12 +2125,10 @@ cudaError_t lbvh_build(const LbvhBuffers& b, cudaStream_t s) {
         }
     }
     if (n == 1) return cudaGetLastError();
-    // requests of a sibling's box before it is taken from the leaves (RG_HIER_POLL_LIMIT overrides; 0 takes every
-    // such box from the leaves, which tests use)
-    int polls = kHierPolls;
-    if (const char* env = getenv("RG_HIER_POLL_LIMIT")) polls = (int)std::min(strtoul(env, nullptr, 10), (unsigned long)kHierPolls);
-    launch_chain(k_hierarchy, blocks(n, kHierLeaves), kHierLeaves, 0, s, b.keysA, b.order, b.primBoxes, n, b.left, b.right, b.parents, b.flags,
-                 b.nodeBoxes, polls);
+    // (RG_HIER_POLL_LIMIT=0: no sibling's box is waited for, which tests use)
+    const char* env = getenv("RG_HIER_POLL_LIMIT");
+    launch_chain(env && strtoul(env, nullptr, 10) == 0 ? k_hierarchy<true> : k_hierarchy<false>, blocks(n, kHierLeaves), kHierLeaves, 0, s, b.keysA,
+                 b.order, b.primBoxes, n, b.left, b.right, b.parents, b.flags, b.nodeBoxes);
     count_launch();
     return cudaGetLastError();
 }
