@@ -116,7 +116,7 @@ struct rg_ctx {
     uint32_t treeNodes = kTreeNodesMin;
     size_t treeRefused = SIZE_MAX, treeRefusedAt = 0;  // nodes that memory did not allow; what the context held then
     TreeLoad treeLoad;  // of the last frame
-    uint32_t* hostCount = nullptr;             // pinned words for polling the queue length and work counter
+    uint32_t* hostCount = nullptr;             // 16 pinned words: polls of frames and host loops (4), a graph's loop words (5), wait status, second lane
     int lastIterations = 0;
     // batch rendering: job table, ray-sort scratch, per-job images
     DevBuf jobTable, sortKeys, sortPerm, sortHist;
@@ -1186,7 +1186,7 @@ rg_status enqueue_query(rg_ctx* c, const float* rays, uint32_t n, float* tuv, ui
 // A call of a few thousand rays waited for three copies of pageable memory, a memset and a kernel of one ray
 // a thread.  Up to kQueryStage rays the traversal kernel reads and writes page-locked memory itself (the
 // CPU's memory is on the same coherent link), so two copies by the CPU remain.  Sphere scene, from the
-// host: 100 rays 69 -> 43 us, 4097 rays 94 -> 63 us, 12000 rays 103 -> 89 us.  At 16384 rays the CPU's
+// host: 100 rays 69 -> 43 us, 4097 rays 99 -> 67 us, 12000 rays 103 -> 89 us.  At 16384 rays the CPU's
 // copies make it 104 us, the driver's 92 us, so above it the rays go to device memory.
 // The overflow list (4 bytes a ray) takes no device memory of its own: page-locked up to kQueryOver rays;
 // above, the call is two launches, the list of the first three quarters lies where the last

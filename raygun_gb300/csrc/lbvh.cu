@@ -1795,7 +1795,7 @@ __global__ void __launch_bounds__(kSahWarps * 32, 1) k_sah_build(const float* __
 
 // The rest of the tree on every SM: a warp claims the next queue slot, waits (bounded) until the
 // slot's task is published, splits it as k_sah_build does, and publishes its children's tasks in
-// the next free slots (node id = first node id of the queue + slot).  A task of at most 32 primitives is
+// the next free slots (node id = first node id of the queue + slot).  A task of at most `subtree` primitives is
 // finished by its warp, whose node ids come from the upper end; a warp whose slot will not be
 // used sees that every node is made, and is done.  A slot's task is published by the warp that split
 // its parent, which claimed an earlier slot and runs, so every wait ends; a wait that still runs out

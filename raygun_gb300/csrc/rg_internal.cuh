@@ -124,9 +124,9 @@ inline void count_launch(uint64_t n = 1) { g_launches.fetch_add(n, std::memory_o
 
 // A chain of short launches: each is set up while the one before it still runs (its blocks are placed as soon as
 // that one's have ended) and waits for that one's memory itself, first thing, with chain_wait.  1.5 us
-// less between two launches, of which a frame has 20 to 50 and a scene load 60: 160x90 frame 401 -> 363 us,
-// 640x360 spheres 997 -> 927 us, 1080p game frame 16.24 -> 16.08 ms.  Letting the next blocks in earlier
-// (launch_dependents) costs more than it gives: they hold places of blocks still working (16.41 ms).
+// less between two launches, of which a frame has 20 to 50 and a scene load 60: 160x90 frame 10 % shorter,
+// 640x360 spheres 7.6 %, 1080p game frame 1 %.  Letting the next blocks in earlier (launch_dependents) costs more
+// than it gives, 2 % of the game frame: they hold places of blocks still working.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // kernel: one that starts with chain_wait
 template <class... P, class... A>
@@ -324,9 +324,8 @@ struct TraceParams {
     uint32_t queryCount;
 };
 cudaError_t launch_trace(const TraceParams& p, cudaStream_t s);
-// Work items of the frame loop: W x H pixels padded to whole 8 x 4 tiles, times S samples.  The first
-// round indexes its hit records by work item, so the hit buffers hold this many entries (more than
-// W * H * S when W or H is not a multiple of the tile).
+// Work items of a frame: W x H pixels padded to whole 8 x 4 tiles, times S samples (more than W * H * S when W or H is
+// not a multiple of the tile).  Each is the root of a ray tree, those outside the image an idle one.
 constexpr int kTileW = 8, kTileH = 4;
 inline size_t frame_work_items(uint32_t W, uint32_t H, uint32_t S) {
     return (size_t)((W + kTileW - 1) / kTileW) * ((H + kTileH - 1) / kTileH) * (kTileW * kTileH) * S;
@@ -347,14 +346,15 @@ struct TreeLane {
 cudaError_t launch_trace_tree(const TraceParams& p, cudaStream_t s, const TreeLane& second, uint32_t* hostWords, int* iterations, TreeLoad* load,
                               bool mayGrow, EventPairFn kernelEvents = nullptr, void* user = nullptr);
 // traversal launch shape of the batch loop: block size {64,128,256}, stack entries {16,24,32,48},
-// ray-sort key applied to each queue before it is traced
+// ray-sort key applied to each round but the first before it is traced
 struct TraceTune {
     int threads = 128, depth = 48, sortKey = RG_SORT_NONE;
 };
 bool tune_supported(const TraceTune& t);
-// scratch of the ray sort (each of the first three: `slots` words; hist: 8192 words)
+// scratch of the ray sort (keys and permutation: a word a node of the pool; hist: 4096 bucket counts, zero between
+// rounds, and 4096 offsets)
 struct SortScratch {
-    uint32_t *keysA, *keysB, *valsA, *valsB, *hist;
+    uint32_t *keysA, *valsA, *hist;
 };
 // every job of p.jobs through ray trees, the loops on the host; hostWords: four pinned words polled after each check
 // and chunk; loopWords as below; cudaErrorLaunchTimeout when the loops gave up

@@ -273,7 +273,7 @@ using TravStack = LocalStackT<kTraversalStack>;
 #endif
 
 // Resumable traversal of one ray: trav_begin sets it up, each trav_step processes one record or one
-// leaf (a record tests up to eight children and descends into the nearest hit; a TLAS leaf moves
+// leaf (a record tests four children and descends into the nearest hit; a TLAS leaf moves
 // the ray into the instance's object space and descends into its BLAS behind a marker entry; a BLAS
 // leaf runs the triangle test).  The kernel interleaves trav_step with shading so that a lane whose
 // ray finished does not idle.
@@ -317,8 +317,8 @@ __device__ __forceinline__ void trav_begin(Trav& T, const DevScene& sc, float ox
 // One record: an inner node's four boxes, a triangle, an instance, or the way back to the TLAS.  The
 // loop is bound by instruction issue (71 % of the slots) and by the latency of the record behind it, so
 // what counts is instructions a step.  Approximate 1/d, the shear set up at the first triangle, min
-// and max of three, no tests for empty slots and pushes without a branch took the 1920x1080 game frame
-// from 19.4 to 18.5 ms and 512k secondary rays from 538 to 482 us.  Records with each plane pair
+// and max of three, no tests for empty slots and pushes without a branch took 4.5 % of the 1920x1080 game
+// frame and 1M secondary rays from 538 to 482 us.  Records with each plane pair
 // stored both ways round (256-bit loads) gave 1 % more for twice the memory, smaller records with
 // selects lost 2 %, stack entries with their t (culled when popped) lost 0.5 %.
 template <bool COUNT, bool SHARED = false, class STACK>
@@ -2271,7 +2271,7 @@ __global__ void k_sample_depth_first(const __grid_constant__ TraceParams P) {
 // decides (the host loop of launch_trace_batch runs the same kernels and polls the words).
 // Loop runs cost 20 us each, so the rounds that every chunk needs (batchRounds) are launched without a loop,
 // and a run holds the rounds that replaced rays can need at most; rounds without rays end in 3 us.
-// Six scenes, 10 M samples: 3.8 ms against 7.1 ms for a loop of one ray a path and round, whose rounds
+// Six scenes, 10 M samples: half the time of a loop of one ray a path and round (3.8 against 7.1 ms), whose rounds
 // dragged on for the longest path (16 of them, then 1 ms of single threads finishing paths).
 
 // after a check: whether rays are still to be traced or checked, as launch_trace_tree decides
@@ -2624,8 +2624,8 @@ static RayTree tree_part(const RayTree& t, size_t at, uint32_t n, uint32_t* ctl)
 
 // Samples from which a frame runs as two lanes, each with half of the samples and of the pool in a stream of its own:
 // every round ends with its longest rays and walks, and the host polls after every check; meanwhile the other
-// lane has the chip.  2.75 M samples (1279x717, 3 a pixel) 3.07 -> 2.89 ms, 8.3 M 18.24 -> 17.93 ms, 0.92 M 1808 ->
-// 1806 us, 0.23 M 968 -> 1000 us (its rounds no longer fill the chip).
+// lane has the chip.  2.75 M samples (1279x717, 3 a pixel) 6 % shorter, 8.3 M 1.7 %, 0.92 M 0, 0.23 M 3 % longer (its
+// rounds no longer fill the chip).
 constexpr uint32_t kTwoLanes = 1u << 20;
 cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeLane& second, uint32_t* hostWords, int* iterations, TreeLoad* load,
                               bool mayGrow, EventPairFn kernelEvents, void* user) {
