@@ -109,8 +109,8 @@ struct rg_ctx {
     // misc
     DevBuf counters, tmpA, tmpB, tmpC, tmpD;  // counters: 8 per-frame + 8 cumulative
     DevBuf samples, workCounter;               // per-sample payload sums, persistent-kernel work counter
-    // ray queries: traversal counters, overflow list
-    DevBuf wfCounts, wfOverflow;
+    // ray queries: the traversal kernel's work counter, overflow lists
+    DevBuf wfFetch, wfOverflow;
     // ray trees of the frames: node pool (its nodes per sample grow when a frame filled it)
     DevBuf trO, trD, trState, trHit, trInst, trSurf, trLink, trOver, trCand, trCtl;
     uint32_t treeNodes = kTreeNodesMin;
@@ -578,7 +578,7 @@ rg_status rg_destroy(rg_ctx* c) {
     if (c->copyStream) cudaStreamDestroy(c->copyStream);
     DevBuf* bufs[] = {&c->keysA, &c->keysB, &c->valsA, &c->valsB, &c->sortState, &c->sahQueue, &c->base, &c->normal, &c->rough,
                       &c->finalImg, &c->fxaaOut, &c->fb, &c->dbgT, &c->dbgA, &c->dbgB, &c->counters, &c->tmpA, &c->tmpB, &c->tmpC,
-                      &c->tmpD, &c->samples, &c->workCounter, &c->wfCounts, &c->wfOverflow, &c->jobTable, &c->sortKeys, &c->sortPerm, &c->sortHist, &c->bBase, &c->bNormal, &c->bRough,
+                      &c->tmpD, &c->samples, &c->workCounter, &c->wfFetch, &c->wfOverflow, &c->jobTable, &c->sortKeys, &c->sortPerm, &c->sortHist, &c->bBase, &c->bNormal, &c->bRough,
                       &c->bFinal, &c->bFxaa, &c->batchFb, &c->trO, &c->trD, &c->trState, &c->trHit, &c->trInst, &c->trSurf, &c->trLink,
                       &c->trOver, &c->trCand, &c->trCtl};
     for (DevBuf* b : bufs) release(c, *b);
@@ -1167,17 +1167,13 @@ rg_status rg_instance_inverse(rg_ctx* c, float* out) {
 namespace {
 // one query launch: rays, hits and the overflow list anywhere the device can read and write
 rg_status enqueue_query(rg_ctx* c, const float* rays, uint32_t n, float* tuv, uint32_t* ids, uint32_t* overflow, bool countVisits) {
-    if (!c->wfCounts.p) {
-        TRY(ensure(c, c->wfCounts, 32));
-        CK(cudaMemsetAsync(c->wfCounts.p, 0, 32, c->stream));
-    }
+    TRY(ensure(c, c->wfFetch, 16));
     TraceParams tp;
     std::memset(&tp, 0, sizeof(tp));
     tp.scene = scene_of(*c->sc);
     tp.counters = c->counters.as<unsigned long long>();
     tp.countVisits = countVisits ? 1 : 0;
-    tp.wf.counts = c->wfCounts.as<uint32_t>();
-    tp.wf.overflow = overflow;
+    tp.wf = {c->wfFetch.as<uint32_t>(), overflow};
     CK(launch_trace_queue(tp, rays, n, tuv, ids, c->tune.depth, c->stream));
     return RG_OK;
 }

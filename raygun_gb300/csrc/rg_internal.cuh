@@ -210,11 +210,10 @@ cudaError_t setup_instances(const rg_instance* in, uint32_t n, const DevBlas* bl
 cudaError_t inst_records(const uint32_t* order, uint32_t n, const DevInstance* inst, const DevBlas* blas, InstRec* out,
                          cudaStream_t s);
 
-// counters and overflow list of the traversal kernel
-struct WavefrontBuffers {
-    uint32_t* counts;  // [2] trace work counter, [3] overflow list length, [4] trace blocks finished
-                       // (the last two zero between launches)
-    uint32_t* overflow; // rays whose short traversal stack overflowed
+// words of the traversal kernel: its work counter, and one a ray for the lists of rays whose short stack overflowed
+struct TraceWork {
+    uint32_t* fetch;
+    uint32_t* overflow;
 };
 
 // Ray trees (trace.cu): one node per traced ray.  The roots, one per sample of the chunk, are nodes
@@ -227,16 +226,16 @@ struct RayTree {
     uint32_t* hitInst;  // instance or 0xFFFFFFFF (miss)
     float4* surf;       // of a hit: world normal, material index bits
     uint4* link;        // of a hit: its shadow, reflection and refraction node
-    uint32_t* overflow; // nodes of rays whose short traversal stack overflowed
+    uint32_t* overflow; // links of the lists of rays whose short traversal stack overflowed
     uint32_t* cand[2];  // nodes whose assumptions k_tree_check verifies (the list in use: treeCand)
     uint32_t* ctl;      // kTreeCtlWords words
     uint32_t capacity;  // nodes, at most kTreePoolMax
 };
 // words of RayTree::ctl: nodes appended after the roots; rays that the last check changed, 16 minus the
 // least recursion depth of the rays replaced since the last round, nodes traced when the last check ran;
-// the traversal kernel's work counter, overflow list length and finished blocks; lengths of the candidate
-// lists; then the first node of every round, and a batch's words
-enum : int { kTreeAlloc = 0, kTreeChanges = 1, kTreeLevels = 2, kTreeTraced = 3, kTreeFetch = 4, kTreeCand = 7, kTreeBounds = 9 };
+// the traversal kernel's work counter; lengths of the candidate lists; then the first node of every round, and a
+// batch's words
+enum : int { kTreeAlloc = 0, kTreeChanges = 1, kTreeLevels = 2, kTreeTraced = 3, kTreeFetch = 4, kTreeCand = 5, kTreeBounds = 7 };
 constexpr uint32_t kTreeMaxNodes = 1u << 29;
 // room for the rounds' bounds (a chunk that needs more goes again in parts, as one that filled the pool)
 constexpr int kTreeMaxRounds = 512 * 9;
@@ -299,7 +298,7 @@ struct TraceParams {
     float4* samples;               // W*H*S*3 per-sample payload sums (k_trace -> k_resolve)
     uint32_t* workCounter;         // work-item counter of the persistent kernel
     int countVisits;
-    WavefrontBuffers wf;
+    TraceWork wf;
     // batch (launch_trace_batch): the job table in device memory, the batch's work items, samples a chunk at
     // most, and the rounds every chunk runs (1 + the largest recursion limit)
     const JobDesc* jobs;

@@ -229,8 +229,10 @@ constexpr int kTraceThreads = 128;
 // Beside it, six floats per thread keep the world-space ray's origin and clamped inverse direction
 // while the ray is inside a BLAS (the world direction itself stays in registers), so leaving the BLAS
 // restores them instead of dividing again.
-// The last of the DEPTH words flags an overflow (a push that found the other DEPTH - 1 entries
-// full), so the flag costs the traversal loop neither a register nor shared memory beyond the stack.
+// The last of the DEPTH words flags an overflow in bit 0 (a push that found the other DEPTH - 1 entries
+// full), so the flag costs the traversal loop neither a register nor shared memory beyond the stack.  Its other
+// bits are the kernel's (k_wf_trace: the lane's overflowed rays).  Who starts a ray finds the flag clear: a kernel
+// starts the word at zero and clears the flag when it is done with a ray that set it.
 template <int THREADS, int DEPTH>
 struct SmemStackT {
     static constexpr int kDepth = DEPTH - 1;
@@ -295,7 +297,6 @@ struct Trav {
 template <class STACK>
 __device__ __forceinline__ void trav_begin(Trav& T, const DevScene& sc, float ox, float oy, float oz, float dx, float dy, float dz,
                                            float tmin, float tmax, const STACK& stack) {
-    stack.over() = 0u;
     T.h.hit = false;
     T.h.t = tmax;
     T.h.u = T.h.v = 0.0f;
@@ -365,7 +366,7 @@ __device__ __forceinline__ void trav_step(Trav& T, const DevScene& sc, const STA
                     const uint32_t rj = j == 3 ? r[3] : j == 2 ? r[2] : r[1];
                     if (tj == INFINITY) continue;
                     if (T.sp < STACK::kDepth) stack[T.sp++] = rj;
-                    else stack.over() = 1u;
+                    else stack.over() |= 1u;
                 }
             }
             T.ref = r[0];
@@ -411,7 +412,7 @@ __device__ __forceinline__ void trav_step(Trav& T, const DevScene& sc, const STA
                         T.ref = bn == 1 ? kLeaf : 0u;
                         return;
                     }
-                    stack.over() = 1u;
+                    stack.over() |= 1u;
                 }
             }
         }
@@ -451,6 +452,7 @@ constexpr int kDeepStack = 196;  // 195 entries and the overflow flag
 __device__ __forceinline__ Hit deep_hit(const DevScene& sc, float4 o, float4 d, const LocalStackT<kDeepStack>& st, unsigned long long* counters) {
     VisitCounts vc = {0, 0, 0};
     Trav T;
+    st.over() = 0u;
     trav_begin(T, sc, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, st);
     while (T.active) trav_step<false>(T, sc, st, vc);
     if (st.over() && counters) {
@@ -463,19 +465,6 @@ __device__ __noinline__ void retrace_deep(const DevScene* sc, float4 o, float4 d
     uint32_t mem[kDeepStack];
     float world[6];
     *out = deep_hit(*sc, o, d, LocalStackT<kDeepStack>{mem, world}, counters);
-}
-
-template <bool COUNT, class STACK>
-__device__ Hit closest_hit(const DevScene& sc, float ox, float oy, float oz, float dx, float dy, float dz, float tmin, float tmax,
-                           const STACK& stack, VisitCounts& vc, unsigned long long* counters) {
-    Trav T;
-    trav_begin(T, sc, ox, oy, oz, dx, dy, dz, tmin, tmax, stack);
-    while (T.active) trav_step<COUNT>(T, sc, stack, vc);
-    if (stack.over()) {
-        vc.overflow++;
-        retrace_deep(&sc, make_float4(ox, oy, oz, tmin), make_float4(dx, dy, dz, tmax), &T.h, counters);
-    }
-    return T.h;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -970,10 +959,10 @@ enum : int { kIdle = 0, kTraverse = 1, kResult = 2 };
 // starts the traversal of the pending trace; mask-0 traces and zero directions need none
 template <class STACK>
 __device__ __forceinline__ int begin_ray(Trav& T, const DevScene& sc, const RayReq& ray, const STACK& stack) {
+    stack.over() = 0u;
     if (ray.masked) {
         T.h.hit = false;
         T.active = false;
-        stack.over() = 0u;
         return kResult;
     }
     trav_begin(T, sc, ray.o.x, ray.o.y, ray.o.z, ray.d.x, ray.d.y, ray.d.z, ray.tmin, ray.tmax, stack);
@@ -1324,7 +1313,6 @@ __device__ __forceinline__ void drain(Trav& T, uint32_t& slot, const DevScene*& 
                     N.tris = nullptr;
                 }
                 T = N;
-                stk.over() = 0u;
             }
             __syncwarp();
         }
@@ -1362,10 +1350,12 @@ __device__ __forceinline__ void drain(Trav& T, uint32_t& slot, const DevScene*& 
             h.inst = __shfl_sync(full, T.h.inst, f);
             h.prim = __shfl_sync(full, T.h.prim, f);
             h.hit = __shfl_sync(full, (int)T.h.hit, f) != 0;
-            const uint32_t over = __shfl_sync(full, stk.over(), f);
+            const uint32_t over = __shfl_sync(full, stk.over() & 1u, f);
             if ((int)lane == __ffs(peers) - 1) {
                 if (h.hit && accept(h.t, h.t, h.inst, h.prim, T.h)) T.h = h;
-                if (over) stk.over() = 1u;
+                stk.over() |= over;
+            } else if ((int)lane == f) {
+                stk.over() &= ~1u;
             }
         }
     }
@@ -1426,7 +1416,8 @@ template <bool COUNT, TraceForm FORM, int THREADS, int DEPTH>
 __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k_wf_trace(const __grid_constant__ TraceParams P, int q) {
     chain_wait();
     RG_DECLARE_SMEM_STACK(stk, THREADS, DEPTH);
-    const WavefrontBuffers& wf = P.wf;
+    stk.over() = 0u;
+    const TraceWork& wf = P.wf;
     constexpr bool BATCH = FORM == kFormBatch, QUERY = FORM == kFormQuery, TREE = !QUERY;
     const bool first = TREE && P.firstRound;
     uint32_t node0 = 0, count;  // TREE: the round's first node
@@ -1452,13 +1443,13 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
     uint32_t slot = 0;
     const DevScene* scp = nullptr;  // BATCH: scene of the lane's ray
 #define RG_SC (BATCH ? *scp : P.scene)
-    // a finished ray's hit record; a ray whose short stack overflowed also joins the overflow list,
-    // whose rays the kernel's last block traces again with the deep stack (below)
+    // a finished ray's hit record; a ray whose short stack overflowed also joins the lane's list (its first ray, plus 1,
+    // beside the flag; the next one's in the overflow words by ray), which the lane traces again at the end
 #define RG_WF_HIT_OUT()                                                                      \
     do {                                                                                     \
-        if (stk.over()) {                                                                    \
-            vc.overflow++;                                                                   \
-            wf.overflow[atomicAdd(wf.counts + 3, 1u)] = slot;                                \
+        if (stk.over() & 1u) {                                                               \
+            wf.overflow[slot] = stk.over() >> 1;                                             \
+            stk.over() = (slot + 1u) << 1;                                                   \
         }                                                                                    \
         put_hit<FORM>(P, slot, T.h, T.h.hit);                                                \
     } while (0)
@@ -1526,7 +1517,7 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
                 if (needMask) {
                     const int leader = __ffs(needMask) - 1;
                     uint32_t base = 0;
-                    if ((int)lane == leader) base = atomicAdd(wf.counts + 2, (uint32_t)__popc(needMask));
+                    if ((int)lane == leader) base = atomicAdd(wf.fetch, (uint32_t)__popc(needMask));
                     base = __shfl_sync(0xFFFFFFFFu, base, leader);
                     if (need) {
                         const uint32_t k = base + (uint32_t)__popc(needMask & ltmask);
@@ -1541,32 +1532,12 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
     }
 #undef RG_WF_HIT_OUT
 #undef RG_SC
-    unsigned long long c[3] = {vc.nodes, vc.tris, vc.overflow};
-    for (int k = 0; k < 3; ++k) {
-        unsigned long long v = c[k];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
-        if (lane == 0 && v) {
-            atomicAdd(P.counters + 4 + k, v);
-            atomicAdd(P.counters + 12 + k, v);
-        }
-    }
-    // Rays whose short stack overflowed: the last block to finish (every other block has appended its
-    // rays to the list and fenced) traces them again from the start with the deep stack and rewrites
-    // their hit records, then clears the list for the next launch.  No block waits for another.
-    // (thread 0's stack word carries the verdict: every stack is idle once the block is here; no
-    // shared memory is added, which would cost the kernel L1 at 7 blocks per SM)
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        stk.over() = atomicAdd(wf.counts + 4, 1u) == trace_workers(count, THREADS) - 1 ? 1u : 0u;
-    }
-    __syncthreads();
-    const uint32_t lastBlock = *reinterpret_cast<volatile uint32_t*>(&stk_mem[DEPTH - 1][0]);
-    if (!lastBlock) return;
-    __threadfence();
-    const uint32_t nOver = __ldcg(wf.counts + 3);
-    for (uint32_t i = threadIdx.x; i < nOver; i += blockDim.x) {
-        const uint32_t s = __ldcg(wf.overflow + i);
+    // The lane's rays whose short stack overflowed, from the start with the deep stack.  (The last block to finish
+    // did this for the whole launch: 4097 rays that all overflow a 16-word stack took 104 ms.)
+    for (uint32_t next = stk.over() >> 1; next;) {
+        const uint32_t s = next - 1u;
+        next = wf.overflow[s];
+        vc.overflow++;
         float4 o, d;
         const DevScene* sc = &P.scene;
         if (first) {  // root s's camera ray, as the first round computed it
@@ -1589,9 +1560,14 @@ __global__ void __launch_bounds__(THREADS, (RG_WF_MIN_BLOCKS * 128) / THREADS) k
         retrace_deep(sc, o, d, &h, P.counters);
         put_hit<FORM>(P, s, h, h.hit);
     }
-    if (threadIdx.x == 0) {
-        wf.counts[3] = 0;
-        wf.counts[4] = 0;
+    unsigned long long c[3] = {vc.nodes, vc.tris, vc.overflow};
+    for (int k = 0; k < 3; ++k) {
+        unsigned long long v = c[k];
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+        if (lane == 0 && v) {
+            atomicAdd(P.counters + 4 + k, v);
+            atomicAdd(P.counters + 12 + k, v);
+        }
     }
 }
 
@@ -2332,7 +2308,6 @@ __global__ void k_tree_next(const __grid_constant__ TraceParams P, const TreeLoo
         c[kTreeFollow] = follow;
         if (!follow) c[kTreePlanned] = 0u;
         c[kTreeChunk] = follow ? c[kTreePlan] : whole;
-        c[kTreeFetch + 1] = c[kTreeFetch + 2] = 0u;
     }
     bool stop = false;
     const bool full = c[kTreeFull] != 0u;
@@ -2590,16 +2565,17 @@ cudaError_t launch_trace_queue(const TraceParams& p, const float* rays, uint32_t
     TraceParams q = p;
     q.firstRound = 0;
     q.perm = nullptr;
-    q.queryRays = reinterpret_cast<const float4*>(rays);
-    q.queryTuv = tuv;
-    q.queryIds = ids;
-    q.queryCount = n;
-    // the fetch counter, the overflow-list length and the finished-block count (the kernel's last
-    // block clears the latter two again)
-    cudaError_t e = cudaMemsetAsync(q.wf.counts + 2, 0, 3 * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    trace<<<g, kTraceThreads, 0, s>>>(q, 0);
-    count_launch();
+    constexpr uint32_t kPart = 1u << 30;  // rays of a launch: the lists of overflowed rays keep 31 bits for one
+    for (uint32_t at = 0; at < n; at += std::min(n - at, kPart)) {
+        q.queryRays = reinterpret_cast<const float4*>(rays) + 2 * (size_t)at;
+        q.queryTuv = tuv + 3 * (size_t)at;
+        q.queryIds = ids + 2 * (size_t)at;
+        q.queryCount = std::min(n - at, kPart);
+        const cudaError_t e = cudaMemsetAsync(q.wf.fetch, 0, sizeof(uint32_t), s);
+        if (e != cudaSuccess) return e;
+        trace<<<g, kTraceThreads, 0, s>>>(q, 0);
+        count_launch();
+    }
     return cudaGetLastError();
 }
 
@@ -2647,8 +2623,7 @@ cudaError_t launch_trace_tree(const TraceParams& p0, cudaStream_t s, const TreeL
         L.s = l ? second.stream : s;
         L.hostWords = l ? second.hostWords : hostWords;
         if (lanes == 2) L.p.tree = tree_part(p0.tree, (size_t)l * (cap / 2), cap / 2, l ? second.ctl : p0.tree.ctl);
-        L.p.wf.counts = L.p.tree.ctl + kTreeFetch - 2;  // the traversal kernel's work counter, overflow list length and finished blocks
-        L.p.wf.overflow = L.p.tree.overflow;
+        L.p.wf = {L.p.tree.ctl + kTreeFetch, L.p.tree.overflow};
     }
     const uint32_t pool = lane[0].p.tree.capacity;
     ChunkPlan plan(work, (uint32_t)lanes, pool, pool / kTreeNodesMin, std::move(*load));
@@ -2819,8 +2794,7 @@ struct BatchLaunch {
 
 static TraceParams batch_params(const TraceParams& p0) {
     TraceParams p = p0;
-    p.wf.counts = p.tree.ctl + kTreeFetch - 2;  // the traversal kernel's work counter, overflow list length and finished blocks
-    p.wf.overflow = p.tree.overflow;
+    p.wf = {p.tree.ctl + kTreeFetch, p.tree.overflow};
     return p;
 }
 
