@@ -338,7 +338,8 @@ rg_status rg_set_glossy(rg_ctx* ctx, uint32_t seed);
 /* Device memory the context holds (all scene slots, images, ray-tree nodes, scratch) and its budget
  * (rg_device_opts.hbm_budget_bytes, 0 = none), in bytes. */
 rg_status rg_get_memory(rg_ctx* ctx, uint64_t* allocated_bytes, uint64_t* budget_bytes);
-/* Slots of a batch: its samples go through their ray trees in chunks that share the slots' memory, 0.8 to 1.6 KB each;
+/* Slots of a batch: its samples go through their ray trees in chunks that share the slots' memory, 0.8 to 1.6 KB each
+ * (without a memory budget up to 7 KB, 1.9 GB in all, for a batch of one slot per sample whose samples need many rays);
  * how many samples a chunk holds follows from the rays they need.  Default 2^25 (a batch of fewer samples takes one slot
  * per sample; at most 2^29 nodes of 112 bytes are held).  Fewer slots mean more chunks of narrower rounds. */
 rg_status rg_set_batch_slots(rg_ctx* ctx, uint32_t slots);

@@ -512,6 +512,8 @@ rg_status ensure_tree(rg_ctx* c, size_t roots, uint32_t perRoot, RayTree& t) {
     if (st != RG_ERR_BUDGET && st != RG_ERR_OUT_OF_MEMORY) return st;
     if (st == RG_ERR_OUT_OF_MEMORY) cudaGetLastError();
     c->treeRefused = want;
+    // what the larger pool already has of its buffers is not there for the smaller one's others
+    for (DevBuf* b : {&c->trO, &c->trD, &c->trState, &c->trHit, &c->trInst, &c->trSurf, &c->trLink, &c->trOver, &c->trCand}) release(c, *b);
     const rg_status st2 = ensure_tree_nodes(c, least, t);
     c->treeRefusedAt = c->allocated;
     return st2;

@@ -156,3 +156,24 @@ def test_batches_of_many_rays_a_sample(rg, budget, host_loop):
             last = its
     assert last <= 60
     br.ctx.close()
+
+
+def test_pool_falls_back_within_the_budget(rg):
+    """A budget that holds 7 nodes a slot but not the 13 that a batch of few slots asks for first."""
+    sc = glass_scene(640, 360, 1, 3)
+    want = render(rg, sc)[0][0]
+    slots = 1 << 16
+
+    def batch(budget):
+        br = rg.BatchRenderer([sc], hbm_budget_bytes=budget)
+        br.ctx.set_batch_slots(slots)
+        for _ in range(2):
+            assert np.array_equal(br.render()[0], want)
+        held = br.ctx.memory()[0]
+        br.ctx.close()
+        return held
+
+    held = batch(0)
+    assert held > 13 * 112 * slots
+    budget = held - 5 * 112 * slots
+    assert batch(budget) <= budget
